@@ -1,8 +1,8 @@
 """Performance cases of the clustering library.
 
 Each case is one call (or one short sequence of calls) that a program makes
-through the public surface: the Python Context and Server, or the C entry
-points behind them.  Point sets are drawn on the GPU from a seed, with the
+through the public surface: the Python Context, or the C entry points behind
+it.  Point sets are drawn on the GPU from a seed, with the
 shapes the library is used on: Gaussian blobs over uniform noise, Zipf-sized
 blobs, rotated anisotropic 3D blobs with pairs planted at the eps boundary,
 mixtures with eps from the 4th-nearest-neighbour distance, and vehicle tracks
@@ -25,6 +25,9 @@ def listed():
         # a control loop that clusters one sensor sweep out of reserved memory
         {"name": "noalloc_2d_1k", "op": "noalloc", "layout": "blobs", "dim": 2, "n": 1_200,
          "minpts": 5, "precision": FP32_BAND},
+        # the largest sets that entry point takes, 3D, every test in float64
+        {"name": "noalloc_3d_30k", "op": "noalloc", "layout": "blobs", "dim": 3, "n": 30_011,
+         "minpts": 8, "precision": FP64},
         # the smallest ordinary call: an interactive selection
         {"name": "blobs_2d_1k", "op": "dbscan", "layout": "blobs", "dim": 2, "n": 1_000,
          "minpts": 5, "precision": FP64, "core": False},
@@ -55,9 +58,6 @@ def listed():
         # thousands of independent instances in one run, device memory
         {"name": "batch_4096", "op": "batch", "count": 4096, "lo": 256, "hi": 200_000,
          "precision": FP32_BAND},
-        # a burst of requests to the server
-        {"name": "serve_48", "op": "serve", "count": 48, "lo": 1_000, "hi": 400_000,
-         "precision": FP32_BAND},
     ]
 
 
@@ -67,15 +67,13 @@ def _log_int(rng, lo, hi):
 
 def draw(rng):
     op = rng.choice(["noalloc", "dbscan", "dbscan", "dbscan", "sweep", "host", "batch_host",
-                     "batch", "serve"])
+                     "batch"])
     case = {"op": op, "precision": rng.choice([FP64, FP32_BAND])}
-    if op in ("batch", "batch_host", "serve"):
+    if op in ("batch", "batch_host"):
         if op == "batch":
             case.update(count=_log_int(rng, 128, 3000), lo=256, hi=_log_int(rng, 20_000, 200_000))
-        elif op == "batch_host":
-            case.update(count=_log_int(rng, 4, 64), lo=256, hi=_log_int(rng, 2_000, 50_000))
         else:
-            case.update(count=_log_int(rng, 8, 64), lo=1_000, hi=_log_int(rng, 20_000, 400_000))
+            case.update(count=_log_int(rng, 4, 64), lo=256, hi=_log_int(rng, 2_000, 50_000))
         return case
     dim = rng.choice([2, 3])
     top = {"noalloc": 32_768, "dbscan": 20_000_000, "sweep": 3_000_000, "host": 5_000_000}[op]
@@ -237,7 +235,7 @@ def prepare(case, seed):
     gd = importlib.import_module(PKG)
     st = {"case": case, "gd": gd}
     op = case["op"]
-    if op in ("batch", "batch_host", "serve"):
+    if op in ("batch", "batch_host"):
         flat, inst = _mixtures(case, seed)
         if op == "batch":
             api = importlib.import_module(PKG + ".api")
@@ -254,10 +252,7 @@ def prepare(case, seed):
                       clusters=np.zeros(len(inst), dtype=np.int64))
         else:
             st["inst"] = [(p.cpu().numpy(), eps, mp) for p, eps, mp in _split(flat, inst)]
-            if op == "serve":
-                st["server"] = gd.Server(0, workers=2, precision=case["precision"])
-            else:
-                st["ctx"] = gd.Context(0, precision=case["precision"])
+            st["ctx"] = gd.Context(0, precision=case["precision"])
     else:
         st["points"], st["eps"] = _points(case, seed)
         if op == "noalloc":
@@ -314,11 +309,7 @@ def run(st):
         if status != 0:
             raise RuntimeError(st["lib"].gd_last_error().decode())
         return [st["labels"], st["clusters"]]
-    if op == "batch_host":
-        return st["ctx"].batch_dbscan(st["inst"])
-    server = st["server"]
-    ids = [server.submit(*inst) for inst in st["inst"]]
-    return [server.wait(i)[0] for i in ids]
+    return st["ctx"].batch_dbscan(st["inst"])
 
 
 def exact(case, seed):
@@ -328,7 +319,7 @@ def exact(case, seed):
 
 def work(case):
     """Coordinates read once, labels (and core flags) written once; one distance per point."""
-    if case["op"] in ("batch", "batch_host", "serve"):
+    if case["op"] in ("batch", "batch_host"):
         # expected size of a log-uniform instance, half of them 2D and half 3D
         lo, hi = case["lo"], case["hi"]
         n = case["count"] * (hi - lo) / math.log(hi / lo)
