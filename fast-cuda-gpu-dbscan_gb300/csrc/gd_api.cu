@@ -137,8 +137,8 @@ struct gd_ctx {
     return GD_OK;
   }
 
-  // ensure() for temp memory that must be zero when first used (the scan and
-  // sort state): cleared on the stream whenever it is (re)allocated
+  // ensure() for temp memory that must be zero when first used (the scan
+  // state): cleared on the stream whenever it is (re)allocated
   gd_status ensure_zeroed(DevBuf& b, size_t bytes, const char* what) {
     void* before = b.p;
     const size_t had = b.bytes;
@@ -293,8 +293,9 @@ gd_status build_run(gd_ctx* ctx, uint64_t dense_floor, uint64_t dense_per_point)
   GD_TRY(ctx->ensure(ctx->reps, (n + 1) * 4, "cell reps"));
   GD_TRY(ctx->ensure(ctx->cellz, n * 4, "cell coordinates"));
   GD_TRY(ctx->ensure(ctx->bits, gdl::bit_layout(n).words * 4, "bit masks"));
-  GD_TRY(ctx->ensure_zeroed(ctx->sorttemp, gdprim::sort_temp_bytes(n), "sort temp"));
+  GD_TRY(ctx->ensure(ctx->sorttemp, gdprim::sort_temp_bytes(n), "sort temp"));
   size_t sc = std::max({gdprim::scan_temp_bytes(n + 1),
+                        gdprim::scan_temp_bytes(gdprim::sort_scan_elems(n)),
                         gdprim::scan_temp_bytes((int64_t)bi.start_total),
                         gdprim::scan_temp_bytes((int64_t)W)});
   GD_TRY(ctx->ensure_zeroed(ctx->scantemp, sc, "scan temp"));
@@ -306,13 +307,13 @@ gd_status build_run(gd_ctx* ctx, uint64_t dense_floor, uint64_t dense_per_point)
   if (ctx->key64) {
     using U64 = unsigned long long;
     U64* kb[2] = {static_cast<U64*>(ctx->keys0.p), static_cast<U64*>(ctx->keys1.p)};
-    r = gdprim::radix_sort_pairs<U64>(kb, vb, n, key_bits, true, ctx->sorttemp.p, s,
-                                        ctx->dCtr() + gd::kCtrWaitTimeouts);
+    r = gdprim::radix_sort_pairs<U64>(kb, vb, n, key_bits, true, ctx->sorttemp.p,
+                                      ctx->scantemp.p, s, ctx->dCtr() + gd::kCtrWaitTimeouts);
     ctx->skeys = kb[r];
   } else {
     uint32_t* kb[2] = {static_cast<uint32_t*>(ctx->keys0.p), static_cast<uint32_t*>(ctx->keys1.p)};
-    r = gdprim::radix_sort_pairs<uint32_t>(kb, vb, n, key_bits, true, ctx->sorttemp.p, s,
-                                        ctx->dCtr() + gd::kCtrWaitTimeouts);
+    r = gdprim::radix_sort_pairs<uint32_t>(kb, vb, n, key_bits, true, ctx->sorttemp.p,
+                                           ctx->scantemp.p, s, ctx->dCtr() + gd::kCtrWaitTimeouts);
     ctx->skeys = kb[r];
   }
   L += gdprim::sort_launches(n, key_bits);
@@ -474,8 +475,7 @@ gd_status finish_run(gd_ctx* ctx, int32_t* labels, uint8_t* is_core, int32_t on_
   S.precision_used = ctx->f32 ? GD_PREC_FP32_BAND : GD_PREC_FP64;
   S.launches = ctx->launches + ctx->expand_launches + fin;
   if (ctr[gd::kCtrWaitTimeouts]) {
-    // start the scan and sort state afresh for the next run
-    if (ctx->sorttemp.p) cudaMemsetAsync(ctx->sorttemp.p, 0, ctx->sorttemp.bytes, s);
+    // start the scan state afresh for the next run
     if (ctx->scantemp.p) cudaMemsetAsync(ctx->scantemp.p, 0, ctx->scantemp.bytes, s);
     cudaStreamSynchronize(s);
     ctx->stage = 1;

@@ -312,9 +312,10 @@ void exclusive_scan_popc(const uint32_t* words, uint32_t* pre, int64_t nw, void*
 // out[pre[w] + r] = 32 w + (position of the r-th set bit of word w)
 void compact_bits(const uint32_t* words, const uint32_t* pre, int64_t nw, uint32_t* out, int sms,
                   cudaStream_t s);
-// temp bytes needed by radix_sort_pairs for n elements (either key width);
-// zero when first used, as for the scan
+// temp bytes needed by radix_sort_pairs for n elements (either key width), and
+// the elements its scan temp must allow for (scan_temp_bytes of that many)
 size_t sort_temp_bytes(int64_t n);
+int64_t sort_scan_elems(int64_t n);
 // Stable LSD radix sort of (key, value) pairs on the low `bits` key bits,
 // K = uint32_t or unsigned long long.  keys/vals: ping-pong buffers [0] and
 // [1]; input in [0].  If vals_in_is_iota, vals[0] is not read and the values
@@ -322,7 +323,8 @@ size_t sort_temp_bytes(int64_t n);
 // result.  timeouts as for the scan.
 template <class K>
 int radix_sort_pairs(K* keys[2], uint32_t* vals[2], int64_t n, int bits, bool vals_in_is_iota,
-                     void* temp, cudaStream_t s, unsigned long long* timeouts = nullptr);
+                     void* temp, void* scan_temp, cudaStream_t s,
+                     unsigned long long* timeouts = nullptr);
 // kernels one radix_sort_pairs call launches
 int sort_launches(int64_t n, int bits);
 // digit width radix_sort_pairs uses for a `bits`-bit key (8 or 9)

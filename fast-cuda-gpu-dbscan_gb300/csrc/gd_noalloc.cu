@@ -190,6 +190,7 @@ extern "C" gd_status gd_dbscan_noalloc(const double* coords_dev, int64_t n, int3
   if (n == 0) return GD_OK;
   if (gdprim::sort_temp_bytes(kMaxPoints) > kSortTempBytes ||
       gdprim::scan_temp_bytes((int64_t)kTableCells + 1) > kScanTempBytes ||
+      gdprim::scan_temp_bytes(gdprim::sort_scan_elems(kMaxPoints)) > kScanTempBytes ||
       gdprim::scan_temp_bytes(kMaxPoints + 1) > kScanTempBytes)
     return fail(GD_EINVAL, "gd_dbscan_noalloc: scratch layout inconsistent (build error)");
 
@@ -252,14 +253,14 @@ extern "C" gd_status gd_dbscan_noalloc(const double* coords_dev, int64_t n, int3
   if (key64) {
     using U64 = unsigned long long;
     U64* kb[2] = {reinterpret_cast<U64*>(base + kOffKeys0), reinterpret_cast<U64*>(base + kOffKeys1)};
-    r = gdprim::radix_sort_pairs<U64>(kb, vb, n, key_bits, true, base + kOffSortTemp, s,
-                                      dCtr + gd::kCtrWaitTimeouts);
+    r = gdprim::radix_sort_pairs<U64>(kb, vb, n, key_bits, true, base + kOffSortTemp,
+                                      base + kOffScanTemp, s, dCtr + gd::kCtrWaitTimeouts);
     skeys = kb[r];
   } else {
     uint32_t* kb[2] = {reinterpret_cast<uint32_t*>(base + kOffKeys0),
                        reinterpret_cast<uint32_t*>(base + kOffKeys1)};
-    r = gdprim::radix_sort_pairs<uint32_t>(kb, vb, n, key_bits, true, base + kOffSortTemp, s,
-                                           dCtr + gd::kCtrWaitTimeouts);
+    r = gdprim::radix_sort_pairs<uint32_t>(kb, vb, n, key_bits, true, base + kOffSortTemp,
+                                           base + kOffScanTemp, s, dCtr + gd::kCtrWaitTimeouts);
     skeys = kb[r];
   }
   B.keys = skeys;
@@ -318,8 +319,8 @@ extern "C" gd_status gd_dbscan_noalloc(const double* coords_dev, int64_t n, int3
   NA_CUDA(cudaMemcpyAsync(&K, dK, 4, cudaMemcpyDeviceToHost, s), "read cluster count");
   NA_CUDA(cudaStreamSynchronize(s), "DBSCAN pipeline");
   if (ctr[gd::kCtrWaitTimeouts]) {
-    // start the scan and sort state afresh for the next call
-    cudaMemsetAsync(base + kOffSortTemp, 0, kSortTempBytes + kScanTempBytes, s);
+    // start the scan state afresh for the next call
+    cudaMemsetAsync(base + kOffScanTemp, 0, kScanTempBytes, s);
     cudaStreamSynchronize(s);
     return fail(GD_ECUDA, "gd_dbscan_noalloc: a scan or sort look-back wait gave up");
   }

@@ -421,7 +421,7 @@ inline size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
 
 }  // namespace
 
-// temp layout of both primitives: control block (64 B), then their arrays
+// scan temp: control block (64 B), then the status words
 size_t scan_temp_bytes(int64_t n) {
   const int64_t T = (n + kScanTile - 1) / kScanTile;
   return align_up(sizeof(LookbackCtl) + (size_t)(T > 0 ? T : 1) * 8);
@@ -462,23 +462,26 @@ void compact_bits(const uint32_t* words, const uint32_t* pre, int64_t nw, uint32
   k_compact_bits<<<(unsigned)g, 256, 0, s>>>(words, pre, nw, out);
 }
 
-// sort temp: the histogram scan's state (its control block at offset 0 for
-// every sort on this temp), then the [digit][tile] histogram
+// sort temp: the [digit][tile] histogram.  Its scan keeps its state in the
+// caller's scan temp, which holds nothing but scan state: were the two in one
+// buffer, a larger sort's status words would lie where a smaller sort left its
+// histogram, and a count that looks like a tagged word would pass for a prefix.
+int64_t sort_scan_elems(int64_t n) {
+  return (n + kRsMinTile - 1) / kRsMinTile * kRsMaxBins;
+}
+
 size_t sort_temp_bytes(int64_t n) {
-  const int64_t T = (n + kRsMinTile - 1) / kRsMinTile;
-  const int64_t h = T * kRsMaxBins;
-  return scan_temp_bytes(h) + align_up((size_t)h * sizeof(uint32_t));
+  return align_up((size_t)sort_scan_elems(n) * sizeof(uint32_t));
 }
 
 template <class K, int RB>
 int sort_passes(K* keys[2], uint32_t* vals[2], int64_t n, int passes, bool vals_in_is_iota,
-                void* temp, cudaStream_t s, unsigned long long* timeouts) {
+                void* temp, void* scan_temp, cudaStream_t s, unsigned long long* timeouts) {
   constexpr int ITEMS = rs_items<K>();
   constexpr int TILE = kRsThreads * ITEMS;
   const int64_t T = (n + TILE - 1) / TILE;
   const int64_t h = T << RB;
-  void* scan_temp = temp;
-  uint32_t* hist = reinterpret_cast<uint32_t*>(static_cast<char*>(temp) + scan_temp_bytes(h));
+  uint32_t* hist = static_cast<uint32_t*>(temp);
   int cur = 0;
   for (int p = 0; p < passes; ++p) {
     int shift = RB * p;
@@ -505,7 +508,7 @@ int sort_launches(int64_t n, int bits) {
 // else of 8 bits.
 template <class K>
 int radix_sort_pairs(K* keys[2], uint32_t* vals[2], int64_t n, int bits, bool vals_in_is_iota,
-                     void* temp, cudaStream_t s, unsigned long long* timeouts) {
+                     void* temp, void* scan_temp, cudaStream_t s, unsigned long long* timeouts) {
   if (n <= 0) return 0;
   const int rb = sort_digit_bits(bits);
   const int passes = (bits + rb - 1) / rb;
@@ -513,14 +516,16 @@ int radix_sort_pairs(K* keys[2], uint32_t* vals[2], int64_t n, int bits, bool va
     if (vals_in_is_iota) k_iota<<<1024, 256, 0, s>>>(vals[0], n);
     return 0;
   }
-  return rb == 9 ? sort_passes<K, 9>(keys, vals, n, passes, vals_in_is_iota, temp, s, timeouts)
-                 : sort_passes<K, 8>(keys, vals, n, passes, vals_in_is_iota, temp, s, timeouts);
+  return rb == 9 ? sort_passes<K, 9>(keys, vals, n, passes, vals_in_is_iota, temp, scan_temp, s,
+                                     timeouts)
+                 : sort_passes<K, 8>(keys, vals, n, passes, vals_in_is_iota, temp, scan_temp, s,
+                                     timeouts);
 }
 
 template int radix_sort_pairs<uint32_t>(uint32_t* [2], uint32_t* [2], int64_t, int, bool, void*,
-                                        cudaStream_t, unsigned long long*);
+                                        void*, cudaStream_t, unsigned long long*);
 template int radix_sort_pairs<unsigned long long>(unsigned long long* [2], uint32_t* [2], int64_t,
-                                                  int, bool, void*, cudaStream_t,
+                                                  int, bool, void*, void*, cudaStream_t,
                                                   unsigned long long*);
 
 }  // namespace gdprim
