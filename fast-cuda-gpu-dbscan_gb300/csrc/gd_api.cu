@@ -4,12 +4,12 @@
 // A run clusters K >= 1 instances (gd_index_build/gd_dbscan: K = 1;
 // gd_batch_dbscan: K = count).  Stage order on the context's stream; the only
 // host round-trip inside a run is one read of the 64-byte run layout, which
-// sizes the key width, the cell tables and the hash:
+// sizes the key width, the block tables and the hash:
 //   build:  [H2D] per-instance bbox -> grids -> layout -> (read layout) -> keys
-//           -> radix sort -> gather (sorted SoA f64 [+ centred f32]) -> cell runs
-//           -> dense cell tables (counts + exclusive scan) / hash of occupied cells
-//   expand: core flags -> union-find (near pass, far pass, compress, merge
-//           replay) -> root marks -> scan (cluster numbers) -> labels -> borders
+//           -> radix sort -> gather (sorted points, f64 and/or centred f32) -> cells
+//           -> block entries, row tables / hash of occupied block rows
+//   expand: core flags -> union-find (inside blocks, then passes over the stencil,
+//           merge replay) -> root marks -> scan (cluster numbers) -> labels -> borders
 //   finish: scatter labels/core flags to caller order -> [D2H]
 #include <algorithm>
 #include <cmath>
@@ -60,10 +60,13 @@ constexpr double kDefaultCellMult = 0.5 * (1.0 + 1.0 / 65536.0);
 // pair tests one thread spends before handing its work to a warp
 constexpr int kDefaultCoreTests = 256, kDefaultLinkTests = 48, kDefaultBorderTests = 160;
 constexpr int kMaxTests = 65536;
-// A grid takes a cell table (one occupancy bit, one core bit and one prefix bit
-// per cell) when it has at most this many cells per point (or 2^26 cells for a
-// single instance, 4096 per instance in a batch).
-constexpr uint64_t kCellsPerPoint = 64;
+// A grid takes a direct block table (32 bytes per 64-cell block) when it has at
+// most one block per point (or 2^20 blocks for a single instance, 64 per
+// instance in a batch), and a table of its block rows (8 bytes each) when these
+// are few (kRowsPerPoint, or 2^22 for a single instance, 64 in a batch).
+constexpr uint64_t kBlocksPerPoint = 1;
+constexpr uint64_t kBlockFloor = (uint64_t)1 << 20, kRowFloor = (uint64_t)1 << 22;
+constexpr uint64_t kBatchBlockFloor = 64, kBatchRowFloor = 64;
 // largest multipliers allowed: cell diagonal below eps (1 - 2^-20)
 constexpr double kMaxCellMult2 = 0.70710678118654752 * (1.0 - 1.0 / 1048576.0);
 constexpr double kMaxCellMult3 = 0.57735026918962576 * (1.0 - 1.0 / 1048576.0);
@@ -90,8 +93,8 @@ struct gd_ctx {
   double mult2 = kDefaultCellMult2, mult3 = kDefaultCellMult3;
   int tn_core = kDefaultCoreTests, tn_link = kDefaultLinkTests, tn_border = kDefaultBorderTests;
 
-  DevBuf coords, inst, chunks, Pv, Bi, bbox, keys0, keys1, vals0, vals1, X, Xf, table, occ, cellz,
-      hkeys, hvals, reps, bits, core, cellcore, cellmin, parent, cellcid, lab, asym,
+  DevBuf coords, inst, chunks, Pv, Bi, bbox, keys0, keys1, vals0, vals1, X, Xf, ent, links, cellent, blklist,
+      rowtab, hkeys, hvals, reps, bits, core, cellcore, cellmin, cellrep, parent, cellcid, lab, asym,
       hvcell, hvmask, out, coreout, sorttemp, scantemp, small, kcount;
 
   // the current run
@@ -100,6 +103,7 @@ struct gd_ctx {
   int64_t n = 0;
   int dims = 0;   // bit 0: 2D instances present, bit 1: 3D
   bool f32 = false, key64 = false, xf = false;
+  bool x64 = true;  // the run keeps sorted float64 points
   gd::BatchInfo bi{};
   std::vector<gd::InstDesc> hdesc;
   std::vector<gd::Chunk> hchunk;
@@ -113,6 +117,7 @@ struct gd_ctx {
   bool graphs = true;
   cudaGraphExec_t xgraph = nullptr;
   int expands_on_index = 0;
+  bool fresh_index = false;  // no expand has run on this index build yet
   void drop_graph() {
     if (xgraph) cudaGraphExecDestroy(xgraph);
     xgraph = nullptr;
@@ -149,8 +154,8 @@ struct gd_ctx {
 
   void free_all(bool keep_small) {
     DevBuf* a[] = {&coords, &inst,   &chunks,   &Pv,      &Bi,     &bbox,     &keys0,
-                   &keys1,  &vals0,  &vals1,    &X,       &Xf,     &table,    &occ, &cellz, &hkeys,
-                   &hvals,  &reps,   &bits,     &core,    &cellcore, &cellmin,
+                   &keys1,  &vals0,  &vals1,    &X,       &Xf,     &ent,      &links, &cellent, &blklist, &rowtab, &hkeys,
+                   &hvals,  &reps,   &bits,     &core,    &cellcore, &cellmin, &cellrep,
                    &parent, &cellcid,  &lab,     &asym,   &hvcell,   &hvmask,
                    &out,    &coreout, &sorttemp, &scantemp, &small, &kcount};
     for (DevBuf* b : a) {
@@ -183,28 +188,28 @@ struct gd_ctx {
     B.reps = static_cast<int*>(reps.p);
     if (bits.p) gdl::set_bits(B, static_cast<uint32_t*>(bits.p), n);
     B.K = dK();
-    B.start = static_cast<uint32_t*>(table.p);
-    B.occ = static_cast<uint32_t*>(occ.p);
-    B.cellz = static_cast<uint32_t*>(cellz.p);
-    if (bi.occ_total) {
-      // one buffer: occupancy | core occupancy | word prefix counts
-      B.occ_words = bi.occ_total / 32 + 1;
-      B.cocc = B.occ + B.occ_words;
-      B.wpre = B.occ + gdl::occ_wpre_offset(B.occ_words);
-    }
+    B.ckeys = skeys == keys0.p ? keys1.p : keys0.p;
+    B.ent = static_cast<gd::BlockEnt*>(ent.p);
+    B.links = static_cast<gd::BlockLinks*>(links.p);
+    B.ent_base = (uint32_t)bi.ent_total;
+    B.cellent = static_cast<uint32_t*>(cellent.p);
+    B.blklist = static_cast<uint32_t*>(blklist.p);
+    B.rowtab = static_cast<uint2*>(rowtab.p);
     B.hkeys = static_cast<unsigned long long*>(hkeys.p);
-    B.hvals = static_cast<uint32_t*>(hvals.p);
+    B.hvals = static_cast<uint2*>(hvals.p);
     B.hmask = hmask;
-    B.X = static_cast<double*>(X.p);
+    B.X = x64 ? static_cast<double*>(X.p) : nullptr;
     B.Xf = static_cast<float*>(Xf.p);
     B.core = static_cast<uint8_t*>(core.p);
     B.cellcore = static_cast<int*>(cellcore.p);
     B.cellmin = static_cast<int*>(cellmin.p);
+    B.cellrep = static_cast<int*>(cellrep.p);
     B.parent = static_cast<int*>(parent.p);
     B.cellcid = static_cast<int*>(cellcid.p);
     B.lab = static_cast<int*>(lab.p);
     B.asym = static_cast<int*>(asym.p);
     B.hv_cell = static_cast<int*>(hvcell.p);
+    B.compmin = B.lab;
     B.hv_mask = static_cast<unsigned long long*>(hvmask.p);
     B.ctr = dCtr();
     B.tn_core = tn_core;
@@ -232,7 +237,7 @@ void make_chunks(const std::vector<gd::InstDesc>& desc, std::vector<gd::Chunk>& 
 
 // Build stage of a run: ctx->hdesc (internal order, 2D instances first) and
 // ctx->coords_ptr (device) are set by the caller.
-gd_status build_run(gd_ctx* ctx, uint64_t dense_floor, uint64_t dense_per_point) {
+gd_status build_run(gd_ctx* ctx, uint64_t dense_floor, uint64_t rows_floor) {
   ctx->drop_graph();
   cudaStream_t s = ctx->stream;
   const int K = (int)ctx->hdesc.size();
@@ -256,7 +261,7 @@ gd_status build_run(gd_ctx* ctx, uint64_t dense_floor, uint64_t dense_per_point)
   GD_CUDA(cudaMemsetAsync(ctx->Bi.p, 0, sizeof(gd::BatchInfo), s), "clear layout");
   gdl::Bufs B = ctx->bufs();
   const int grid_launches =
-      gdl::grids(B, K, nch, ctx->mult2, ctx->mult3, dense_floor, dense_per_point, s);
+      gdl::grids(B, K, nch, ctx->mult2, ctx->mult3, dense_floor, kBlocksPerPoint, rows_floor, s);
   GD_CUDA(cudaMemcpyAsync(&ctx->bi, ctx->Bi.p, sizeof(gd::BatchInfo), cudaMemcpyDeviceToHost, s),
           "read run layout");
   GD_CUDA(cudaStreamSynchronize(s), "grid parameters");
@@ -278,11 +283,19 @@ gd_status build_run(gd_ctx* ctx, uint64_t dense_floor, uint64_t dense_per_point)
   GD_TRY(ctx->ensure(ctx->keys1, n * kw, "keys"));
   GD_TRY(ctx->ensure(ctx->vals0, n * 4, "ids"));
   GD_TRY(ctx->ensure(ctx->vals1, n * 4, "ids"));
-  GD_TRY(ctx->ensure(ctx->X, (size_t)n * maxd * 8, "sorted coordinates"));
-  if (ctx->xf) GD_TRY(ctx->ensure(ctx->Xf, (size_t)n * maxd * 4, "f32 coordinates"));
-  const uint64_t W = bi.occ_total ? bi.occ_total / 32 + 1 : 0;
-  GD_TRY(ctx->ensure(ctx->table, std::max<uint64_t>(bi.start_total, 1) * 4, "row tables"));
-  if (W) GD_TRY(ctx->ensure(ctx->occ, gdl::occ_buffer_words(W) * 4, "cell occupancy"));
+  ctx->x64 = !ctx->f32 || bi.band_off;
+  if (ctx->x64) GD_TRY(ctx->ensure(ctx->X, (size_t)n * maxd * 8, "sorted coordinates"));
+  if (ctx->xf) GD_TRY(ctx->ensure(ctx->Xf, (size_t)n * (maxd == 3 ? 16 : 8), "f32 coordinates"));
+  // block entries: direct tables, then one slot per cell if some instance has none
+  const bool direct_only = bi.row_total == 0 && !bi.any_sparse;
+  GD_TRY(ctx->ensure(ctx->ent, (bi.ent_total + (direct_only ? 0 : (uint64_t)n)) * sizeof(gd::BlockEnt),
+                     "block entries"));
+  GD_TRY(ctx->ensure(ctx->links,
+                     (bi.ent_total + (direct_only ? 0 : (uint64_t)n)) * sizeof(gd::BlockLinks),
+                     "block links"));
+  GD_TRY(ctx->ensure(ctx->cellent, n * 4, "cell entries"));
+  GD_TRY(ctx->ensure(ctx->blklist, n * 4, "block list"));
+  GD_TRY(ctx->ensure(ctx->rowtab, bi.row_total * 8, "row tables"));
   uint64_t hcap = 1024;
   if (bi.any_sparse) {
     while (hcap < 2 * (uint64_t)n) hcap <<= 1;
@@ -291,13 +304,10 @@ gd_status build_run(gd_ctx* ctx, uint64_t dense_floor, uint64_t dense_per_point)
   }
   ctx->hmask = (uint32_t)(hcap - 1);
   GD_TRY(ctx->ensure(ctx->reps, (n + 1) * 4, "cell reps"));
-  GD_TRY(ctx->ensure(ctx->cellz, n * 4, "cell coordinates"));
   GD_TRY(ctx->ensure(ctx->bits, gdl::bit_layout(n).words * 4, "bit masks"));
   GD_TRY(ctx->ensure(ctx->sorttemp, gdprim::sort_temp_bytes(n), "sort temp"));
-  size_t sc = std::max({gdprim::scan_temp_bytes(n + 1),
-                        gdprim::scan_temp_bytes(gdprim::sort_scan_elems(n)),
-                        gdprim::scan_temp_bytes((int64_t)bi.start_total),
-                        gdprim::scan_temp_bytes((int64_t)W)});
+  const size_t sc = std::max(gdprim::scan_temp_bytes(n + 1),
+                             gdprim::scan_temp_bytes(gdprim::sort_scan_elems(n)));
   GD_TRY(ctx->ensure_zeroed(ctx->scantemp, sc, "scan temp"));
   const int key_bits = bi.LB + bi.IB;
   int r;
@@ -320,24 +330,20 @@ gd_status build_run(gd_ctx* ctx, uint64_t dense_floor, uint64_t dense_per_point)
   ctx->sids = vb[r];
   B = ctx->bufs();
   L += gdl::gather(B, ctx->key64, n, ctx->xf, K == 1, ctx->sms, s);
-  L += gdl::runs(B, ctx->key64, n, ctx->dims == 3, ctx->sms, ctx->scantemp.p, s);
-  // occupancy bits, row-table starts, occupancy ranks
-  GD_CUDA(cudaMemsetAsync(ctx->table.p, 0, bi.start_total * 4, s), "clear row tables");
-  if (W) GD_CUDA(cudaMemsetAsync(ctx->occ.p, 0, W * 4, s), "clear occupancy");
-  L += gdl::cell_counts(B, ctx->key64, n, ctx->sms, s);
-  L += gdl::start_fill(B, ctx->K, s);
-  gdprim::exclusive_scan_u32(B.start, B.start, (int64_t)bi.start_total, ctx->scantemp.p, nullptr,
-                             s, ctx->dCtr() + gd::kCtrWaitTimeouts);
-  L += gdprim::scan_launches((int64_t)bi.start_total);
-  L += gdl::occ_rank(B, ctx->K, ctx->scantemp.p, s);
-  if (bi.any_sparse) {
+  L += gdl::runs(B, ctx->key64, n, ctx->scantemp.p, s);
+  // block entries and row lookups
+  if (bi.ent_total)
+    GD_CUDA(cudaMemsetAsync(ctx->ent.p, 0, bi.ent_total * sizeof(gd::BlockEnt), s), "clear blocks");
+  if (bi.row_total)
+    GD_CUDA(cudaMemsetAsync(ctx->rowtab.p, 0, bi.row_total * 8, s), "clear row tables");
+  if (bi.any_sparse)
     GD_CUDA(cudaMemsetAsync(ctx->hkeys.p, 0xff, hcap * 8, s), "clear row hash");
-    L += gdl::hash_insert(B, ctx->key64, n, ctx->sms, s);
-  }
+  L += gdl::cells(B, ctx->key64, n, ctx->sms, s);
   GD_CUDA(cudaGetLastError(), "index build launch");
   ctx->launches = L;
-  ctx->st.grid_cells = (int64_t)bi.occ_total;
+  ctx->st.grid_cells = (int64_t)bi.grid_cells;
   ctx->st.key_bits = key_bits;
+  ctx->fresh_index = true;
   ctx->stage = 1;
   return GD_OK;
 }
@@ -355,8 +361,8 @@ cudaError_t launch_expand(gd_ctx* ctx, bool capturing) {
                        (gd::kCtrHeavyBorder - gd::kCtrTests64 + 1) * 8, s));
   gdl::Bufs B = ctx->bufs();
   keep(cudaEventRecordWithFlags(ctx->ev[3], s, evf));
-  int L = gdl::core(B, n, ctx->dims, ctx->f32, ctx->key64, ctx->K == 1, ctx->sms,
-                    ctx->scantemp.p, s);
+  int L = gdl::core(B, n, ctx->dims, ctx->f32, ctx->key64, ctx->K == 1,
+                    ctx->fresh_index, ctx->sms, ctx->scantemp.p, s);
   keep(cudaEventRecordWithFlags(ctx->ev[4], s, evf));
   L += gdl::unite(B, n, ctx->dims, ctx->f32, ctx->key64, ctx->sms, ctx->scantemp.p, s);
   keep(cudaEventRecordWithFlags(ctx->ev[5], s, evf));
@@ -365,6 +371,7 @@ cudaError_t launch_expand(gd_ctx* ctx, bool capturing) {
   L += gdl::border(B, n, ctx->dims, ctx->f32, ctx->key64, ctx->sms, s);
   keep(cudaGetLastError());
   ctx->expand_launches = L;
+  ctx->fresh_index = false;
   return e;
 }
 
@@ -374,6 +381,7 @@ gd_status expand_run(gd_ctx* ctx) {
   GD_TRY(ctx->ensure(ctx->core, n, "core flags"));
   GD_TRY(ctx->ensure(ctx->cellcore, n * 4, "cell core counts"));
   GD_TRY(ctx->ensure(ctx->cellmin, n * 4, "cell min index"));
+  GD_TRY(ctx->ensure(ctx->cellrep, n * 4, "cell representatives"));
   GD_TRY(ctx->ensure(ctx->parent, n * 4, "union-find parents"));
   GD_TRY(ctx->ensure(ctx->cellcid, n * 4, "cell cluster ids"));
   GD_TRY(ctx->ensure(ctx->lab, n * 4, "labels"));
@@ -744,7 +752,7 @@ gd_status gd_index_build(gd_ctx* ctx, const gd_points* pts, double eps) {
     ctx->stage = 1;
     return GD_OK;
   }
-  GD_TRY(build_run(ctx, (uint64_t)1 << 26, kCellsPerPoint));
+  GD_TRY(build_run(ctx, kBlockFloor, kRowFloor));
   cudaEventRecord(ctx->ev[2], ctx->stream);
   return GD_OK;
 }
@@ -841,7 +849,7 @@ gd_status gd_batch_dbscan(gd_ctx* ctx, int32_t count, const gd_instance* inst,
     if (stats) *stats = ctx->st;
     return GD_OK;
   }
-  GD_TRY(build_run(ctx, 4096, kCellsPerPoint));
+  GD_TRY(build_run(ctx, kBatchBlockFloor, kBatchRowFloor));
   cudaEventRecord(ctx->ev[2], ctx->stream);
   GD_TRY(expand_run(ctx));
   std::vector<int64_t> kc(cluster_counts ? count : 0);

@@ -5,13 +5,14 @@
 //   keys[n]   u32   fine-cell key of each point, sorted ascending (u64 for
 //                   sparse grids)
 //   ids[n]    u32   original point index of each sorted position
-//   X[k][n]   f64   coordinate k of each sorted position (structure of arrays)
-//   start[C+1] i32  dense cell table: points of cell c are start[c]..start[c+1]
-//                   (grids up to max(2^26, 8n) cells), or, for larger (sparse)
-//                   grids, a hash of the occupied cells' 64-bit keys -> m
+//   X[n][d]   f64   coordinates of each sorted position
+//   ent[]     32 B  block entries: 64 cells each (8x8 in 2D, 4x4x4 in 3D), found
+//                   directly by block key, through a table of block rows, or
+//                   through a hash of the occupied block rows (k_cells)
+//   ckeys[M]        key of every non-empty cell
 //   reps[M+1] i32   sorted position of the first point of every non-empty cell
 // Per non-empty cell, indexed by its cell index m (0..M-1, key order; the
-// walks reach it from occupancy ranks without loading reps):
+// walks reach it from a block entry's occupancy word without loading reps):
 //   cellcore[m]  number of core points in the cell
 //   cellmin[m]   smallest original index among the cell's core points
 //   parent[m]    union-find parent (a cell index)
@@ -52,10 +53,10 @@ struct BatchInfo {
   int32_t LB;          // local key bits (widest instance grid)
   int32_t IB;          // instance-id bits
   int32_t key64;       // 1: keys are 64-bit
-  uint64_t occ_total;  // occupancy bits of all instances (cells of cell tables,
-                       // rows of row tables)
-  uint64_t start_total;// entries of all start tables (rows+1 per row table, 1 otherwise)
-  int32_t any_sparse;  // some instance uses the hash of occupied cells
+  uint64_t ent_total;  // block entries of all directly addressed instances
+  uint64_t row_total;  // row-table entries of all instances that use one
+  uint64_t grid_cells; // cells of direct tables + rows of row tables
+  int32_t any_sparse;  // some instance uses the hash of occupied block rows
   int32_t flags;       // OR of the instances' kFlag* bits
   int32_t any_xf;      // some instance wants the centred float32 copy
   int32_t max_dim;
@@ -78,14 +79,16 @@ struct DevParams {
   float eps2_lo32;     // float32 d2 below this: certainly a neighbour
   float eps2_hi32;     // float32 d2 above this: certainly not a neighbour
   int64_t G[3];        // cells per dimension
-  uint64_t C;          // total cells (G0*G1[*G2])
-  uint64_t rows;       // rows: C / G[dim-1]
+  int32_t Bk[3];       // blocks per dimension (8 cells a side in 2D, 4 in 3D)
+  uint64_t NB;         // total blocks
+  uint64_t rows;       // block rows: NB / Bk[dim-1]
   int32_t dim;
   int32_t minpts;
-  int32_t key_bits;
+  int32_t key_bits;    // bits of a local key (block key, then 6 bits in the block)
+  int32_t cell_bits;   // bits of the plain cell count (the refusal limit is on these)
   int32_t flags;       // kFlag*
-  int32_t sparse;      // grid lookup: 0 dense cell table; 2 dense row table (cells
-                       // inside a row by binary search); 1 hash of occupied rows
+  int32_t sparse;      // block lookup: 0 directly by block key; 2 table of block rows
+                       // (blocks inside a row by binary search); 1 hash of occupied rows
   int32_t prune;       // 1: cell-level inside/outside classification enabled
   float inv_f32;       // fl32(1 / f)
   float uerr;          // bound on the error of a point's in-cell position (cell units)
@@ -94,19 +97,17 @@ struct DevParams {
   int64_t pt_off;      // first point (global index)
   int64_t n;           // points
   int64_t co_off;      // first coordinate in the concatenated buffer
-  uint64_t occ_off;    // first occupancy bit of this instance (cell table: C+1 bits,
-                       // row table: rows+1)
-  uint64_t start_off;  // first start-table entry (row table: rows+1 entries, else 1)
-  int64_t m0;          // first non-empty cell of the instance (index into reps)
-  int64_t m1;          // last non-empty cell of the instance
-  int64_t rank_off;    // cell table: a cell's index into reps = occupancy rank + rank_off
+  uint32_t ent_off;    // direct table: the instance's first block entry
+  uint64_t row_off;    // row table: the instance's first row
   uint64_t kmask;      // mask of the local key bits
   int32_t LB;          // local key bits of the run (copied from BatchInfo)
   int32_t inst;        // instance index
-  // exact division of local keys by G[1] and G[2] (multiply-high method, see
+  // exact division of block keys by Bk[1] and Bk[2] (multiply-high method, see
   // udiv_magic): multiplier and shift per divisor
   uint64_t dm[2];
   int32_t ds[2];
+  uint32_t dm32[2];    // the same on 32 bits, for fewer than 2^32 blocks (small)
+  int32_t small;
   // float32 cell origins without float64 arithmetic (cell_origin32): the cell
   // side and lo - centre per axis as float pairs (hi + lo), valid when fast_origin
   float f_hi, f_lo;
@@ -124,24 +125,36 @@ struct DevParams {
 // Montgomery, "Division by invariant integers using multiplication", 1994,
 // Fig. 4.1, N = 64): with l = ceil(log2 d) and m = floor(2^64 (2^l - d) / d) + 1,
 // q = (t + ((k - t) >> 1)) >> (l - 1), t = mulhi(m, k), for every 64-bit k
-// (l = 0, i.e. d = 1: q = k).  The multiplier is found by long division.
+// (l = 0, i.e. d = 1: q = k).  d < 2^32.
 __host__ __device__ inline void udiv_magic(uint64_t d, uint64_t& m, int32_t& l) {
   l = 0;
   while (l < 64 && (1ull << l) < d) ++l;
   if (l == 0) { m = 0; return; }
-  // floor((2^l - d) * 2^64 / d); exact for d < 2^63 (the remainder never overflows)
-  uint64_t r = (l == 64 ? 0ull : (1ull << l)) - d, q = 0;
-  for (int i = 0; i < 64; ++i) {
-    r <<= 1;
-    q <<= 1;
-    if (r >= d) { r -= d; q |= 1; }
-  }
+  // floor((2^l - d) * 2^64 / d) in two 32-bit digits (d < 2^32: both partial
+  // remainders shifted by 32 fit 64 bits; 2^l - d < d)
+  const uint64_t r0 = ((1ull << l) - d) << 32;
+  const uint64_t q1 = r0 / d, r1 = (r0 - q1 * d) << 32;
+  const uint64_t q = (q1 << 32) | (r1 / d);
   m = q + 1;
 }
 
 __device__ __forceinline__ uint64_t udiv_by(uint64_t k, uint64_t m, int32_t l) {
   if (l == 0) return k;
   const uint64_t t = __umul64hi(m, k);
+  return (t + ((k - t) >> 1)) >> (l - 1);
+}
+
+// The 32-bit form (N = 32): same shift, m = floor(2^32 (2^l - d) / d) + 1.
+__host__ __device__ inline uint32_t udiv_magic32(uint32_t d) {
+  int l = 0;
+  while (l < 32 && (1ull << l) < d) ++l;
+  if (l == 0) return 0;
+  return (uint32_t)((((1ull << l) - d) << 32) / d) + 1u;
+}
+
+__device__ __forceinline__ uint32_t udiv_by32(uint32_t k, uint32_t m, int32_t l) {
+  if (l == 0) return k;
+  const uint32_t t = __umulhi(m, k);
   return (t + ((k - t) >> 1)) >> (l - 1);
 }
 
@@ -168,12 +181,42 @@ __device__ __forceinline__ PredParams pred_params(const DevParams& P) {
   return q;
 }
 
-// A grid too large for a cell table takes a table of its rows when it has at
-// most this many rows per point (or the table floor).
-constexpr uint64_t kRowsPerPoint = 64;
+// Blocks of 64 cells: the low 6 bits of a key are the cell's place in its
+// block, x-major, the bits above the block's key, x-major over the blocks.  A
+// block's occupied cells are one 64-bit word, its cells are consecutive in key
+// order, and the +-2 stencil of a cell meets at most two blocks per axis: 4
+// lookups in 2D and 8 in 3D answer for all 25 or 125 cells.
+constexpr int kBlockBits = 6;
+template <int D>
+__host__ __device__ constexpr int block_shift() { return D == 2 ? 3 : 2; }
+
+// One block.  Direct tables: indexed by block key; otherwise by the block's
+// first cell.
+struct alignas(32) BlockEnt {
+  unsigned long long occ;   // occupied cells
+  uint32_t base;            // index of the block's first cell
+  uint32_t lo;              // the root its core cells share before union pass 1 (kNoEnt:
+                            // unset, kMixedRoot: several); border search: their smallest
+                            // cluster id
+  unsigned long long core;  // cells holding a core point
+  uint32_t hi;              // the root its core cells share before union pass 2
+  uint32_t uni;             // the root its core cells share before union pass 0
+};
+static_assert(sizeof(BlockEnt) == 32, "one sector per block entry");
+constexpr uint32_t kNoEnt = 0xffffffffu, kMixedRoot = 0xfffffffeu;
+
+// Links between core cells of one block that share a face: per axis the cells
+// linked to the next one along it.
+struct alignas(8) BlockLinks {
+  uint32_t w[3][2];
+};
+
+// A grid with too many blocks for a direct table takes a table of its block
+// rows when it has at most this many rows per point (or the table floor).
+constexpr uint64_t kRowsPerPoint = 8;
 
 constexpr int kFlagNonFinite = 1;     // NaN or Inf coordinate
-constexpr int kFlagGridTooLarge = 2;  // keys would not fit 62 bits
+constexpr int kFlagGridTooLarge = 2;  // cell counts and instance ids beyond 62 bits
 constexpr int kFlagNoShortcut = 4;    // |x| too large relative to eps for the
                                       // box-test shortcut / float32 filter
 
@@ -196,13 +239,14 @@ enum Counter {
   kCtrWalkCursor2,      // walk-list entries handed out (2D, 3D); cleared before each walk launch
   kCtrWalkCursor3,
   kCtrWaitTimeouts,     // scan / sort launches whose look-back wait gave up (never expected)
-  kCtrCount = 17
+  kCtrBlocks,           // occupied blocks of the index
+  kCtrCount = 18
 };
 
 // Capacity of the list of one-directional core-core pairs (see k_asym_resolve).
 constexpr int kAsymCap = 2048;
 
-// Hash of occupied cells (sparse grids): open addressing, linear probing.
+// Hash of occupied block rows (sparse grids): open addressing, linear probing.
 constexpr unsigned long long kHashEmpty = ~0ull;
 __host__ __device__ __forceinline__ uint32_t hash_key(unsigned long long k) {
   return (uint32_t)((k * 0x9E3779B97F4A7C15ull) >> 32);
@@ -256,7 +300,7 @@ __device__ __forceinline__ bool pred_from_d2(double d2, const double* p, const d
   return box_f64<D>(p, q, P.eps);
 }
 
-// ---- union-find over cell reps (lock-free, hooks by (cellmin, position)) ---
+// ---- union-find over cells (lock-free; the larger index hooks under the smaller)
 __device__ __forceinline__ int uf_find(int* parent, int x) {
   volatile int* par = parent;
   int p = par[x];
@@ -269,18 +313,13 @@ __device__ __forceinline__ int uf_find(int* parent, int x) {
   return x;
 }
 
-__device__ __forceinline__ bool uf_less(const int* cellmin, int a, int b) {
-  int wa = cellmin[a], wb = cellmin[b];
-  return wa < wb || (wa == wb && a < b);
-}
-
-__device__ __forceinline__ void uf_union(int* parent, const int* cellmin, int a, int b) {
+__device__ __forceinline__ void uf_union(int* parent, int a, int b) {
   while (true) {
     a = uf_find(parent, a);
     b = uf_find(parent, b);
     if (a == b) return;
-    if (uf_less(cellmin, b, a)) { int t = a; a = b; b = t; }
-    // hook b (the heavier root) under a
+    if (b < a) { int t = a; a = b; b = t; }
+    // hook b under a
     int old = atomicCAS(parent + b, b, a);
     if (old == b) return;
     b = old;
@@ -308,10 +347,11 @@ void exclusive_scan_u32(const uint32_t* in, uint32_t* out, int64_t n, void* temp
 void exclusive_scan_popc(const uint32_t* words, uint32_t* pre, int64_t nw, void* temp,
                          uint32_t* total_dev, cudaStream_t s,
                          unsigned long long* timeouts = nullptr);
-// the positions of the set bits of words[0, nw) in ascending order:
-// out[pre[w] + r] = 32 w + (position of the r-th set bit of word w)
-void compact_bits(const uint32_t* words, const uint32_t* pre, int64_t nw, uint32_t* out, int sms,
-                  cudaStream_t s);
+// the set bits of words[0, nw): pre as above, and their positions in ascending
+// order, out[pre[w] + r] = 32 w + (position of the r-th set bit of word w); temp and
+// timeouts as for the scan
+void list_bits(const uint32_t* words, uint32_t* pre, int64_t nw, uint32_t* out, void* temp,
+               uint32_t* total_dev, cudaStream_t s, unsigned long long* timeouts = nullptr);
 // temp bytes needed by radix_sort_pairs for n elements (either key width), and
 // the elements its scan temp must allow for (scan_temp_bytes of that many)
 size_t sort_temp_bytes(int64_t n);

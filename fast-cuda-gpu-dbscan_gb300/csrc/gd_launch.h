@@ -40,22 +40,25 @@ struct Bufs {
   uint32_t* fpre = nullptr;     // core index of each cluster (cluster number = rank)
   int64_t nw = 0;               // words of runbits / lbits
   int64_t nwf = 0;              // words of fbits
-  uint32_t* start = nullptr;    // row tables: first cell (index into reps) per row, after
-                                // the scan; other instances: one entry holding their cells
-  uint32_t* cellz = nullptr;    // per non-empty cell: its last-axis coordinate
-  uint32_t* occ = nullptr;      // occupancy bit per cell (cell tables) or row (row tables)
-  uint32_t* cocc = nullptr;     // the same for cells / rows holding a core point (after
-                                // the core phase; border search)
-  uint32_t* wpre = nullptr;     // per occ word: set bits in the words before it
-  uint64_t occ_words = 0;       // words of occ (and of cocc, wpre); 0 without tables
-  unsigned long long* hkeys = nullptr;  // sparse grids: row hash slots (key of the row's first cell)
-  uint32_t* hvals = nullptr;            // sparse grids: row hash slots (begin, end) pairs
-  uint32_t hmask = 0;                   // sparse grids: slots - 1
-  double* X = nullptr;          // sorted float64 coordinates, max_dim x n
-  float* Xf = nullptr;          // sorted centred float32 coordinates, max_dim x n
+  const void* ckeys = nullptr;  // per non-empty cell: its key (same width as keys)
+  uint32_t* blklist = nullptr;  // first cell of every occupied block
+  uint32_t* cellent = nullptr;  // per non-empty cell: its block's entry
+  gd::BlockEnt* ent = nullptr;  // block entries: direct tables first, then (from ent_base)
+  gd::BlockLinks* links = nullptr;  // per entry, as ent
+  uint32_t ent_base = 0;        // one slot per cell, used at each block's first cell
+  uint2* rowtab = nullptr;      // row tables: cells [x, y) of every block row
+  unsigned long long* hkeys = nullptr;  // row hash slots: key of the block row's start
+  uint2* hvals = nullptr;               // row hash slots: cells [x, y) of the row
+  uint32_t hmask = 0;                   // row hash: slots - 1
+  double* X = nullptr;          // sorted float64 points (2 or 3 doubles each); null in a
+                                // float32-band run whose instances all have a band
+  float* Xf = nullptr;          // sorted centred float32 points (2 or 4 floats each)
   uint8_t* core = nullptr;      // core flag per sorted position
   int* cellcore = nullptr;      // per cell m: number of core points
   int* cellmin = nullptr;       // per cell m: smallest global index of a core point
+  int* compmin = nullptr;       // per root: smallest core index of its component (in lab's
+                                // memory, which holds no labels before the border search)
+  int* cellrep = nullptr;       // per core cell m: its first core point (sorted position)
   int* parent = nullptr;        // per cell m: union-find parent (a cell index)
   int* cellcid = nullptr;       // per cell m: cluster id of its core points (INT_MAX: none)
   int* lab = nullptr;           // label per sorted position
@@ -71,11 +74,6 @@ struct Bufs {
   // (core count per point, link search per cell pair, border search per point)
   int tn_core = 256, tn_link = 48, tn_border = 160;
 };
-
-// Words of the occupancy buffer (occ | cocc | wpre) for W occupancy words, and
-// the offset of wpre: 256-byte aligned, as the scan reads it in 16-byte vectors.
-inline uint64_t occ_wpre_offset(uint64_t W) { return (2 * W + 63) & ~uint64_t(63); }
-inline uint64_t occ_buffer_words(uint64_t W) { return occ_wpre_offset(W) + W; }
 
 // The bit masks of a run of n points (runbits, runpre, lbits, lpre, fbits,
 // fpre) in one buffer: each array nw + 1 (fbits, fpre: nwf + 1) words, at
@@ -114,32 +112,28 @@ inline void set_bits(Bufs& B, uint32_t* words, int64_t n) {
 
 // Host launchers.  Each returns the number of kernels it launched.
 // per-instance bounding boxes, grids and the run layout
+// dense_floor, dense_per_point: blocks a direct table may have; rows_floor: rows a
+// row table may have whatever the point count
 int grids(const Bufs& B, int K, int nchunks, double mult2, double mult3, uint64_t dense_floor,
-          uint64_t dense_per_point, cudaStream_t s);
+          uint64_t dense_per_point, uint64_t rows_floor, cudaStream_t s);
 // cell keys in global point order (width from the run layout)
 int keys(const Bufs& B, bool key64, int nchunks, void* keys_out, cudaStream_t s);
 // sorted float64 (and centred float32) coordinates; one: a single instance
 int gather(const Bufs& B, bool key64, int64_t n, bool xf, bool one, int sms, cudaStream_t s);
-// cell starts: run bits and their ranks, reps, the cell count M, and the split
-// between 2D and 3D cells (mixed: a run holding both)
-int runs(const Bufs& B, bool key64, int64_t n, bool mixed, int sms, void* scan_temp,
-         cudaStream_t s);
-// occupancy bits, row-table cell counts, cellz, each instance's first and last cells
-int cell_counts(const Bufs& B, bool key64, int64_t n, int sms, cudaStream_t s);
-// one-entry start slices (cell counts of instances without a row table); then scan
-int start_fill(const Bufs& B, int K, cudaStream_t s);
-// occupancy ranks: word prefix counts (scan temp: scan_temp_bytes(occ_words)) and each
-// cell table's rank offset
-int occ_rank(const Bufs& B, int K, void* scan_temp, cudaStream_t s);
-// sparse instances: hash of occupied rows (clear the slots first)
-int hash_insert(const Bufs& B, bool key64, int64_t n, int sms, cudaStream_t s);
+// cell starts: run bits and their ranks, reps, ckeys, the cell count M, and the
+// split between 2D and 3D cells
+int runs(const Bufs& B, bool key64, int64_t n, void* scan_temp, cudaStream_t s);
+// block entries, row tables and row hash (direct entries and row tables cleared to
+// 0, hash keys to ~0 first)
+int cells(const Bufs& B, bool key64, int64_t n, int sms, cudaStream_t s);
 // cell phases; dims: bit 0 = 2D instances present, bit 1 = 3D; one: a single instance
-int core(const Bufs& B, int64_t n, int dims, bool f32, bool key64, bool one, int sms,
+// fresh: the first expand of an index build
+int core(const Bufs& B, int64_t n, int dims, bool f32, bool key64, bool one, bool fresh, int sms,
          void* scan_temp, cudaStream_t s);
 int unite(const Bufs& B, int64_t n, int dims, bool f32, bool key64, int sms, void* scan_temp,
           cudaStream_t s);
-// root marks, cluster numbers (total into *B.K), per-cell cluster ids and core
-// occupancy bits
+// root marks, cluster numbers (total into *B.K), per-cell cluster ids and each
+// block's smallest one
 int roots(const Bufs& B, bool key64, int64_t n, int sms, void* scan_temp, cudaStream_t s);
 // the border-search list (non-core points)
 int label(const Bufs& B, int64_t n, int sms, void* scan_temp, cudaStream_t s);

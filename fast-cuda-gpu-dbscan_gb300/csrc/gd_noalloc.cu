@@ -13,8 +13,8 @@
 //
 // Limits and rules:
 //   * n <= GD_NOALLOC_MAX_POINTS (32768); larger inputs are rejected with
-//     GD_ERANGE.  Grids of more than 8*32768 cells use the hash of occupied
-//     cells instead of the dense table, so any extent fits.
+//     GD_ERANGE.  Grids of more than 32768/8 blocks use a table of their block
+//     rows (up to 65536) or the hash of occupied rows, so any extent fits.
 //   * The first call in a CUDA context of a device looks the array's device
 //     address up (cudaGetSymbolAddress, with that device current) and caches it
 //     with the context's id; a new context on that device (after
@@ -45,7 +45,8 @@ void set_error(const std::string& m);
 namespace {
 
 constexpr int64_t kMaxPoints = GD_NOALLOC_MAX_POINTS;
-constexpr uint64_t kTableCells = 8ull * kMaxPoints;      // dense table limit
+constexpr uint64_t kTableBlocks = kMaxPoints / 8;        // direct table limit
+constexpr uint64_t kTableRows = 2ull * kMaxPoints;       // row table limit
 constexpr uint64_t kHashSlots = 2ull * kMaxPoints;       // power of two
 
 constexpr size_t up(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -64,18 +65,20 @@ constexpr size_t kOffVals0 = kOffKeys1 + up(kMaxPoints * 8);
 constexpr size_t kOffVals1 = kOffVals0 + up(kMaxPoints * 4);
 constexpr size_t kOffX = kOffVals1 + up(kMaxPoints * 4);
 constexpr size_t kOffXf = kOffX + up(kMaxPoints * 3 * 8);
-constexpr size_t kOffTable = kOffXf + up(kMaxPoints * 3 * 4);
-constexpr size_t kOffOcc = kOffTable + up((kTableCells + 1) * 4);
-// occupancy, core occupancy, word prefix counts
-constexpr size_t kOffHkeys = kOffOcc + up((3 * (kTableCells / 32 + 1) + 64) * 4);
+constexpr size_t kOffTable = kOffXf + up(kMaxPoints * 4 * 4);
+constexpr size_t kOffEnt = kOffTable + up(kTableRows * 8);
+constexpr size_t kOffLinks = kOffEnt + up((kTableBlocks + kMaxPoints) * sizeof(gd::BlockEnt));
+constexpr size_t kOffHkeys = kOffLinks + up((kTableBlocks + kMaxPoints) * sizeof(gd::BlockLinks));
 constexpr size_t kOffHvals = kOffHkeys + up(kHashSlots * 8);
 constexpr size_t kOffReps = kOffHvals + up(kHashSlots * 8);
-constexpr size_t kOffCellz = kOffReps + up((kMaxPoints + 1) * 4);
-constexpr size_t kOffBits = kOffCellz + up(kMaxPoints * 4);    // cell starts, lists, marks
+constexpr size_t kOffCellent = kOffReps + up((kMaxPoints + 1) * 4);
+constexpr size_t kOffBlklist = kOffCellent + up(kMaxPoints * 4);
+constexpr size_t kOffBits = kOffBlklist + up(kMaxPoints * 4);  // cell starts, lists, marks
 constexpr size_t kOffCore = kOffBits + up(gdl::bit_layout(kMaxPoints).words * 4);
 constexpr size_t kOffCellcore = kOffCore + up(kMaxPoints);
 constexpr size_t kOffCellmin = kOffCellcore + up(kMaxPoints * 4);
-constexpr size_t kOffParent = kOffCellmin + up(kMaxPoints * 4);
+constexpr size_t kOffCellrep = kOffCellmin + up(kMaxPoints * 4);
+constexpr size_t kOffParent = kOffCellrep + up(kMaxPoints * 4);
 constexpr size_t kOffCellcid = kOffParent + up(kMaxPoints * 4);
 constexpr size_t kOffLab = kOffCellcid + up(kMaxPoints * 4);
 constexpr size_t kOffAsym = kOffLab + up(kMaxPoints * 4);
@@ -84,7 +87,7 @@ constexpr size_t kOffHvMask = kOffHvCell + up(kMaxPoints * 4);
 constexpr size_t kOffSortTemp = kOffHvMask + up(kMaxPoints * 8);
 constexpr size_t kSortTempBytes = 64 * 1024;   // >= sort_temp_bytes(kMaxPoints), checked below
 constexpr size_t kOffScanTemp = kOffSortTemp + kSortTempBytes;
-constexpr size_t kScanTempBytes = 4096;        // >= scan_temp_bytes(kTableCells + 1), checked below
+constexpr size_t kScanTempBytes = 4096;        // >= scan_temp_bytes(kMaxPoints + 1), checked below
 constexpr size_t kScratchBytes = kOffScanTemp + kScanTempBytes;
 
 // The scratch.  In host code this name is only a stand-in for the symbol, not
@@ -189,7 +192,6 @@ extern "C" gd_status gd_dbscan_noalloc(const double* coords_dev, int64_t n, int3
   if (n_clusters) *n_clusters = 0;
   if (n == 0) return GD_OK;
   if (gdprim::sort_temp_bytes(kMaxPoints) > kSortTempBytes ||
-      gdprim::scan_temp_bytes((int64_t)kTableCells + 1) > kScanTempBytes ||
       gdprim::scan_temp_bytes(gdprim::sort_scan_elems(kMaxPoints)) > kScanTempBytes ||
       gdprim::scan_temp_bytes(kMaxPoints + 1) > kScanTempBytes)
     return fail(GD_EINVAL, "gd_dbscan_noalloc: scratch layout inconsistent (build error)");
@@ -230,8 +232,8 @@ extern "C" gd_status gd_dbscan_noalloc(const double* coords_dev, int64_t n, int3
   B.M = dM;
   B.ctr = dCtr;
   // index build (the same stages as gd_index_build)
-  gdl::grids(B, 1, nch, 0.5 * (1.0 + 1.0 / 65536.0), 0.5 * (1.0 + 1.0 / 65536.0), kTableCells,
-             0, s);
+  gdl::grids(B, 1, nch, 0.5 * (1.0 + 1.0 / 65536.0), 0.5 * (1.0 + 1.0 / 65536.0),
+             kTableBlocks, 0, kTableRows, s);
   gd::BatchInfo bi;
   NA_CUDA(cudaMemcpyAsync(&bi, base + kOffBi, sizeof bi, cudaMemcpyDeviceToHost, s),
           "read run layout");
@@ -268,45 +270,41 @@ extern "C" gd_status gd_dbscan_noalloc(const double* coords_dev, int64_t n, int3
   B.blist = vb[1 - r];  // the sort's other id and key buffers are free after the sort
   gdl::set_bits(B, reinterpret_cast<uint32_t*>(base + kOffBits), n);
   B.K = dK;
-  B.X = reinterpret_cast<double*>(base + kOffX);
+  B.X = f32 ? nullptr : reinterpret_cast<double*>(base + kOffX);
   B.Xf = reinterpret_cast<float*>(base + kOffXf);
   B.reps = reinterpret_cast<int*>(base + kOffReps);
-  B.cellz = reinterpret_cast<uint32_t*>(base + kOffCellz);
-  B.start = reinterpret_cast<uint32_t*>(base + kOffTable);
-  B.occ = reinterpret_cast<uint32_t*>(base + kOffOcc);
-  if (bi.occ_total) {
-    B.occ_words = bi.occ_total / 32 + 1;
-    B.cocc = B.occ + B.occ_words;
-    B.wpre = B.occ + gdl::occ_wpre_offset(B.occ_words);
-  }
+  B.cellent = reinterpret_cast<uint32_t*>(base + kOffCellent);
+  B.blklist = reinterpret_cast<uint32_t*>(base + kOffBlklist);
+  B.ckeys = skeys == base + kOffKeys0 ? base + kOffKeys1 : base + kOffKeys0;
+  B.ent = reinterpret_cast<gd::BlockEnt*>(base + kOffEnt);
+  B.links = reinterpret_cast<gd::BlockLinks*>(base + kOffLinks);
+  B.ent_base = (uint32_t)bi.ent_total;
+  B.rowtab = reinterpret_cast<uint2*>(base + kOffTable);
   B.hkeys = reinterpret_cast<unsigned long long*>(base + kOffHkeys);
-  B.hvals = reinterpret_cast<uint32_t*>(base + kOffHvals);
+  B.hvals = reinterpret_cast<uint2*>(base + kOffHvals);
   B.hmask = (uint32_t)(kHashSlots - 1);
   gdl::gather(B, key64, n, xf, true, sms, s);
-  gdl::runs(B, key64, n, false, sms, base + kOffScanTemp, s);
-  NA_CUDA(cudaMemsetAsync(B.start, 0, bi.start_total * 4, s), "clear row table");
-  if (B.occ_words) NA_CUDA(cudaMemsetAsync(B.occ, 0, B.occ_words * 4, s), "clear occupancy");
-  gdl::cell_counts(B, key64, n, sms, s);
-  gdl::start_fill(B, 1, s);
-  gdprim::exclusive_scan_u32(B.start, B.start, (int64_t)bi.start_total, base + kOffScanTemp,
-                             nullptr, s, dCtr + gd::kCtrWaitTimeouts);
-  gdl::occ_rank(B, 1, base + kOffScanTemp, s);
-  if (bi.any_sparse) {
+  gdl::runs(B, key64, n, base + kOffScanTemp, s);
+  if (bi.ent_total)
+    NA_CUDA(cudaMemsetAsync(B.ent, 0, bi.ent_total * sizeof(gd::BlockEnt), s), "clear blocks");
+  if (bi.row_total) NA_CUDA(cudaMemsetAsync(B.rowtab, 0, bi.row_total * 8, s), "clear row table");
+  if (bi.any_sparse)
     NA_CUDA(cudaMemsetAsync(B.hkeys, 0xff, kHashSlots * 8, s), "clear row hash");
-    gdl::hash_insert(B, key64, n, sms, s);
-  }
+  gdl::cells(B, key64, n, sms, s);
 
   // expansion (the same stages as gd_expand)
   B.core = base + kOffCore;
   B.cellcore = reinterpret_cast<int*>(base + kOffCellcore);
   B.cellmin = reinterpret_cast<int*>(base + kOffCellmin);
+  B.cellrep = reinterpret_cast<int*>(base + kOffCellrep);
   B.parent = reinterpret_cast<int*>(base + kOffParent);
   B.cellcid = reinterpret_cast<int*>(base + kOffCellcid);
   B.lab = reinterpret_cast<int*>(base + kOffLab);
   B.asym = reinterpret_cast<int*>(base + kOffAsym);
   B.hv_cell = reinterpret_cast<int*>(base + kOffHvCell);
+  B.compmin = B.lab;
   B.hv_mask = reinterpret_cast<unsigned long long*>(base + kOffHvMask);
-  gdl::core(B, n, dims, f32, key64, true, sms, base + kOffScanTemp, s);
+  gdl::core(B, n, dims, f32, key64, true, true, sms, base + kOffScanTemp, s);
   gdl::unite(B, n, dims, f32, key64, sms, base + kOffScanTemp, s);
   gdl::roots(B, key64, n, sms, base + kOffScanTemp, s);
   gdl::label(B, n, sms, base + kOffScanTemp, s);

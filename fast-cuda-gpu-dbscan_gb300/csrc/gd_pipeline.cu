@@ -4,11 +4,12 @@
 //   host bbox + bin widths        main.cu:166-207           -> k_bbox_chunk, k_params_inst
 //   INDEXING_STRUCTURE/insertData indexing.cu:54-118        -> k_keys (cell keys)
 //   thrust::sort_by_key           main.cu:332               -> gdprim::radix_sort_pairs
-//   INDEXING_ADJUSTMENT           indexing.cu:23-51         -> k_run_flags/k_run_scatter/
-//                                                              k_cell_counts + scan / k_row_hash
-//   DBSCAN kernel + searchPoints  dbscan.cu:254-474         -> k_core_point, k_core_heavy
-//   MarkAsCandidate + host merge  dbscan.cu:189-222, 25-187 -> k_union_scan, k_union_heavy,
-//                                                              k_asym_resolve (device union-find)
+//   INDEXING_ADJUSTMENT           indexing.cu:23-51         -> k_runs, k_cells
+//   DBSCAN kernel + searchPoints  dbscan.cu:254-474         -> k_core_cell (float32 band),
+//                                                              k_core_point (float64), k_core_heavy
+//   MarkAsCandidate + host merge  dbscan.cu:189-222, 25-187 -> k_links, k_flood, k_union_scan,
+//                                                              k_union_heavy, k_asym_resolve
+//                                                              (device union-find)
 //   GetDbscanResult               dbscan.cu:225-251         -> k_roots, k_label, k_border_*,
 //                                                              k_scatter_labels
 //
@@ -16,9 +17,9 @@
 // the instance id above the instance's local cell key, so one radix sort, one
 // cell list and one launch per phase (per dimension present) serve them all.
 //
-// Grid: fine cells of side f = eps * m, m = 0.5 * (1 + 2^-16) by default, keyed
-// x-major.  Two points of one cell are always neighbours (cell diagonal
-// <= 0.87 eps), and every neighbour of a point lies within +-2 cells per axis.
+// Grid: fine cells of side f = eps * m (m > 0.5, below 1/sqrt(dim)), in blocks of
+// 64 (8x8 or 4x4x4), keyed by block and place in the block.  Two points of one cell
+// are always neighbours (cell diagonal below eps), and every neighbour of a point lies within +-2 cells per axis.
 // A cell holding >= minpts points is therefore all core ("dense") without a
 // single distance evaluation, and all core points of a cell are in one cluster.
 //
@@ -32,9 +33,11 @@
 #include <algorithm>
 #include <cfloat>
 #include <climits>
+#include <type_traits>
 
 #include "gd_internal.cuh"
 #include "gd_launch.h"
+#include "gd_lookback.cuh"
 
 namespace gd {
 
@@ -172,7 +175,8 @@ __global__ void __launch_bounds__(kBboxThreads) k_bbox_chunk(const gdl::Bufs B) 
 
 // One thread per instance: its grid and float32 band from its bounding box.
 __global__ void k_params_inst(const gdl::Bufs B, int K, double mult2, double mult3,
-                              uint64_t dense_floor, uint64_t dense_per_point) {
+                              uint64_t dense_floor, uint64_t dense_per_point,
+                              uint64_t rows_floor) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= K) return;
   const InstDesc I = B.inst[i];
@@ -199,32 +203,48 @@ __global__ void k_params_inst(const gdl::Bufs B, int K, double mult2, double mul
   p.inst = i;
   double cells = 1.0;
   uint64_t C = 1;
+  uint64_t NB = 1;
+  for (int k = 0; k < 3; ++k) p.Bk[k] = 1;
   for (int k = 0; k < D; ++k) {
     double t = floor(__dmul_rn(__dsub_rn(p.hi[k], p.lo[k]), p.inv_f)) + 1.0;
     if (!(t < 2147483648.0)) { fl |= kFlagGridTooLarge; t = 1.0; }
     p.G[k] = (int64_t)t;
     cells *= t;
     C *= (uint64_t)p.G[k];
+    const int sh = D == 2 ? block_shift<2>() : block_shift<3>();
+    p.Bk[k] = (int32_t)((p.G[k] + (1 << sh) - 1) >> sh);
+    NB *= (uint64_t)p.Bk[k];
   }
-  // local keys must fit 62 bits; a grid beyond the dense-table limit uses the hash
-  if (!(cells < 4.0e18)) fl |= kFlagGridTooLarge;
+  // cell counts must fit 62 bits; keys (whole blocks) then fit 64: rounding the
+  // axes up to blocks costs at most a factor of 4 near the limit (3D, one axis
+  // of a single cell), and 4 * 4e18 < 2^64
+  if (!(cells < 4.0e18)) {
+    fl |= kFlagGridTooLarge;
+    NB = 1;
+  }
+  // Block lookup.  Direct (one 32-byte entry per block, cleared per run) up to
+  // one block per point or the floor; else a table of the block rows (8 bytes
+  // each) up to kRowsPerPoint per point or the floor: a row holds few blocks, so
+  // its search is short and the table stays in cache; else the hash of the
+  // occupied rows.
   uint64_t limit = (uint64_t)I.n * dense_per_point;
   if (limit < dense_floor) limit = dense_floor;
-  p.C = C;
-  p.rows = C / (uint64_t)p.G[D - 1];
-  if (!(cells > (double)limit || C > limit)) {
+  p.NB = NB;
+  p.rows = NB / (uint64_t)p.Bk[D - 1];
+  if (NB <= limit) {
     p.sparse = 0;
   } else {
-    // a grid too large for a cell table may still take a table of its rows
     uint64_t rlimit = dense_per_point ? (uint64_t)I.n * kRowsPerPoint : 0;
-    if (rlimit < dense_floor) rlimit = dense_floor;
+    if (rlimit < rows_floor) rlimit = rows_floor;
     p.sparse = (fl & kFlagGridTooLarge) || p.rows > rlimit ? 1 : 2;
   }
-  udiv_magic((uint64_t)p.G[1], p.dm[0], p.ds[0]);
-  udiv_magic((uint64_t)p.G[2], p.dm[1], p.ds[1]);
-  int bits = 0;
-  while (bits < 63 && (C - 1) >> bits) ++bits;
-  p.key_bits = bits;
+  udiv_magic((uint64_t)p.Bk[1], p.dm[0], p.ds[0]);
+  udiv_magic((uint64_t)p.Bk[2], p.dm[1], p.ds[1]);
+  p.small = NB <= 0xffffffffull ? 1 : 0;
+  p.dm32[0] = udiv_magic32((uint32_t)p.Bk[1]);
+  p.dm32[1] = udiv_magic32((uint32_t)p.Bk[2]);
+  p.key_bits = 64 - __clzll((long long)((NB << kBlockBits) - 1));
+  p.cell_bits = C > 1 ? 64 - __clzll((long long)(C - 1)) : 0;
   // box-test shortcut and float32 filter need every |x| <= eps * 2^30
   double maxabs = 0, R = 0;
   for (int k = 0; k < D; ++k) {
@@ -324,11 +344,8 @@ __global__ void k_params_inst(const gdl::Bufs B, int K, double mult2, double mul
     p.key_fast = kf ? 1 : 0;
   }
   p.flags = fl;
-  p.occ_off = 0;
-  p.start_off = 0;
-  p.m0 = 0;
-  p.m1 = -1;
-  p.rank_off = 0;
+  p.ent_off = 0;
+  p.row_off = 0;
   p.kmask = 0;
   p.LB = 0;
   B.Pv[i] = p;
@@ -338,13 +355,14 @@ __global__ void k_params_inst(const gdl::Bufs B, int K, double mult2, double mul
 // over every instance's table length), flags.
 __global__ void __launch_bounds__(1024) k_layout(const gdl::Bufs B, int K) {
   __shared__ unsigned long long s_part[32], s_part2[32];
-  __shared__ int s_red[4][32];
-  __shared__ unsigned long long s_carry, s_carry2;
+  __shared__ int s_red[5][32];
+  __shared__ unsigned long long s_carry, s_carry2, s_cells;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  int lb = 0, fl = 0, sp = 0, xf = 0, md = 2, k2 = 0;
+  int lb = 0, cb = 0, fl = 0, sp = 0, xf = 0, md = 2, k2 = 0;
   for (int i = threadIdx.x; i < K; i += blockDim.x) {
     const DevParams& p = B.Pv[i];
     if (p.n > 0) lb = max(lb, p.key_bits);
+    if (p.n > 0) cb = max(cb, p.cell_bits);
     fl |= p.flags;
     sp |= p.sparse == 1;
     xf |= p.prune;
@@ -355,6 +373,7 @@ __global__ void __launch_bounds__(1024) k_layout(const gdl::Bufs B, int K) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     lb = max(lb, __shfl_xor_sync(kFull, lb, o));
+    cb = max(cb, __shfl_xor_sync(kFull, cb, o));
     fl |= __shfl_xor_sync(kFull, fl, o);
     sp |= __shfl_xor_sync(kFull, sp, o);
     xf |= __shfl_xor_sync(kFull, xf, o);
@@ -366,15 +385,17 @@ __global__ void __launch_bounds__(1024) k_layout(const gdl::Bufs B, int K) {
     s_red[1][w] = fl | (sp << 16) | (xf << 17);
     s_red[2][w] = md;
     s_red[3][w] = k2;
+    s_red[4][w] = cb;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    int LB = 0, F = 0, MD = 2, K2 = 0;
+    int LB = 0, F = 0, MD = 2, K2 = 0, CB = 0;
     for (int j = 0; j < 32; ++j) {
       LB = max(LB, s_red[0][j]);
       F |= s_red[1][j];
       MD = max(MD, s_red[2][j]);
       K2 += s_red[3][j];
+      CB = max(CB, s_red[4][j]);
     }
     int IB = 0;
     while (IB < 31 && ((K - 1) >> IB)) ++IB;
@@ -385,30 +406,32 @@ __global__ void __launch_bounds__(1024) k_layout(const gdl::Bufs B, int K) {
     bi.key64 = LB + IB > 32 ? 1 : 0;
     bi.any_sparse = (F >> 16) & 1;
     bi.any_xf = (F >> 17) & 1;
-    bi.flags = (F & 0xffff) | B.Bi->flags | (LB + IB > 62 ? kFlagGridTooLarge : 0);
+    bi.flags = (F & 0xffff) | B.Bi->flags |
+               (CB + IB > 62 || LB + IB > 64 ? kFlagGridTooLarge : 0);
     bi.max_dim = MD;
     bi.K2 = K2;
     bi.band_off = (F >> 18) & 1;
-    bi.occ_total = 0;
-    bi.start_total = 0;
+    bi.ent_total = 0;
+    bi.row_total = 0;
+    bi.grid_cells = 0;
     *B.Bi = bi;
     s_carry = 0;
     s_carry2 = 0;
+    s_cells = 0;
   }
   __syncthreads();
   const int LB = B.Bi->LB;
   const uint64_t kmask = LB >= 64 ? ~0ull : ((1ull << LB) - 1ull);
-  // exclusive scans of the table sizes, 1024 instances at a time: occupancy
-  // bits (C+1 per cell table, rows+1 per row table, none for the hash) and
-  // start entries (rows+1 per row table, else one entry holding the point
-  // count, so the start scan stays in sorted-position units)
+  // exclusive scans of the table sizes, 1024 instances at a time: block entries
+  // of direct tables, rows of row tables (none for the hash)
   for (int base = 0; base < K; base += 1024) {
     const int i = base + threadIdx.x;
     unsigned long long vo = 0, vs = 0;
     if (i < K) {
       const DevParams& p = B.Pv[i];
-      vo = p.sparse == 1 ? 0 : (p.sparse == 2 ? p.rows : p.C) + 1;
-      vs = p.sparse == 2 ? p.rows + 1 : 1;
+      vo = p.sparse == 0 ? p.NB : 0;
+      vs = p.sparse == 2 ? p.rows : 0;
+      if (p.sparse != 1) atomicAdd(&s_cells, (vo << kBlockBits) + vs);
     }
     unsigned long long io = vo, is = vs;
 #pragma unroll
@@ -442,8 +465,8 @@ __global__ void __launch_bounds__(1024) k_layout(const gdl::Bufs B, int K) {
     const unsigned long long eo = s_carry + s_part[w] + io - vo;
     const unsigned long long es = s_carry2 + s_part2[w] + is - vs;
     if (i < K) {
-      B.Pv[i].occ_off = eo;
-      B.Pv[i].start_off = es;
+      B.Pv[i].ent_off = (uint32_t)eo;
+      B.Pv[i].row_off = es;
       B.Pv[i].kmask = kmask;
       B.Pv[i].LB = LB;
     }
@@ -455,12 +478,23 @@ __global__ void __launch_bounds__(1024) k_layout(const gdl::Bufs B, int K) {
     __syncthreads();
   }
   if (threadIdx.x == 0) {
-    B.Bi->occ_total = s_carry;
-    B.Bi->start_total = s_carry2;
+    B.Bi->ent_total = s_carry;
+    B.Bi->row_total = s_carry2;
+    B.Bi->grid_cells = s_cells;
   }
 }
 
 // ------------------------------------------------------------------ keys
+// Instance id above the LB local key bits (LB = 64 only for a single instance).
+__device__ __forceinline__ uint64_t inst_key(int inst, int LB) {
+  return LB >= 64 ? 0 : (uint64_t)inst << LB;
+}
+
+template <class Key>
+__device__ __forceinline__ int inst_of(Key key, int LB) {
+  return LB >= 64 ? 0 : (int)((uint64_t)key >> LB);
+}
+
 // floor(fl64(fl64(x - lo) * inv_f)) as an int: t is finite; out-of-range
 // values saturate, and the caller's clamp takes them to the grid's edge.
 __device__ __forceinline__ int cell_index_f64(double x, double lo, double inv_f) {
@@ -476,7 +510,8 @@ __global__ void __launch_bounds__(256) k_keys(const gdl::Bufs B, Key* __restrict
   double lo[3], inv_f = P.inv_f;
   int64_t G[3];
   for (int k = 0; k < 3; ++k) { lo[k] = P.lo[k]; G[k] = P.G[k]; }
-  const uint64_t hi = (uint64_t)P.inst << P.LB;
+  const uint64_t hi = inst_key(P.inst, P.LB);
+  const int B1 = P.Bk[1], B2 = P.Bk[2];
   const bool kfast = P.key_fast != 0;
   const float band = P.key_band, inv32 = P.key_inv32;
   float lo32[3];
@@ -484,7 +519,7 @@ __global__ void __launch_bounds__(256) k_keys(const gdl::Bufs B, Key* __restrict
   const double* __restrict__ pts = B.coords + P.co_off;
   Key* __restrict__ out = keys + P.pt_off;
   auto key_of = [&](int64_t l, const double* xs) {
-    uint64_t key = 0;
+    int c[3] = {0, 0, 0};
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
       if (k >= D) break;
@@ -523,17 +558,18 @@ __global__ void __launch_bounds__(256) k_keys(const gdl::Bufs B, Key* __restrict
       // the float64 formula for the few coordinates near a cell boundary
       if (!fast) q = cell_index_f64(x, lo[k], inv_f);
       q = q < 0 ? 0 : ((int64_t)q >= G[k] ? (int)(G[k] - 1) : q);
-      key = key * (uint64_t)G[k] + (uint64_t)q;
+      c[k] = q;
     }
-    out[l] = (Key)(hi | key);
+    const uint64_t key =
+        D == 2 ? ((uint64_t)(unsigned)(c[0] >> 3) * (unsigned)B1 + (unsigned)(c[1] >> 3)) << kBlockBits |
+                     (unsigned)((c[0] & 7) << 3 | (c[1] & 7))
+               : (((uint64_t)(unsigned)(c[0] >> 2) * (unsigned)B1 + (unsigned)(c[1] >> 2)) * (unsigned)B2 +
+                  (unsigned)(c[2] >> 2)) << kBlockBits |
+                     (unsigned)((c[0] & 3) << 4 | (c[1] & 3) << 2 | (c[2] & 3));
+    out[l] = (Key)(hi + key);
   };
   if (D == 2) for_points<2>(pts, c.begin - P.pt_off, c.end - P.pt_off, key_of);
   else for_points<3>(pts, c.begin - P.pt_off, c.end - P.pt_off, key_of);
-}
-
-template <class Key>
-__device__ __forceinline__ int inst_of(Key key, int LB) {
-  return (int)((uint64_t)key >> LB);
 }
 
 // Coordinates of one point in 16-byte loads where the address allows (a 2D
@@ -566,7 +602,9 @@ __device__ __forceinline__ void load_coords(const double* __restrict__ src, doub
   }
 }
 
-// Sorted structure-of-arrays copy (+ centred float32 copy).  ONE: a single
+// Sorted copies: float64 points (16 or 24 bytes each; X null: none wanted) and
+// centred float32 ones (8 or 16 bytes).  2D positions come first in a mixed run,
+// so each point lies at its position times its own size.  ONE: a single
 // instance (its parameters are Pv[0], no key is read).  kGatherU points per
 // thread and pass, so that as many random loads are in flight.
 #ifndef GD_GATHER_U
@@ -600,11 +638,23 @@ __global__ void k_gather(const gdl::Bufs B, int64_t n) {
       if (i >= n) continue;
       const DevParams& P = *Pp[u];
       const int D = P.dim;
+      if (B.X) {
+        if (D == 2) {
+          reinterpret_cast<double2*>(B.X)[i] = make_double2(v[u][0], v[u][1]);
+        } else {
 #pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        if (k >= D) break;
-        B.X[k * n + i] = v[u][k];
-        if (XF) B.Xf[k * n + i] = __double2float_rn(__dsub_rn(v[u][k], P.centre[k]));
+          for (int k = 0; k < 3; ++k) B.X[3 * i + k] = v[u][k];
+        }
+      }
+      if (XF) {
+        const float f0 = __double2float_rn(__dsub_rn(v[u][0], P.centre[0]));
+        const float f1 = __double2float_rn(__dsub_rn(v[u][1], P.centre[1]));
+        if (D == 2) {
+          reinterpret_cast<float2*>(B.Xf)[i] = make_float2(f0, f1);
+        } else {
+          const float f2 = __double2float_rn(__dsub_rn(v[u][2], P.centre[2]));
+          reinterpret_cast<float4*>(B.Xf)[i] = make_float4(f0, f1, f2, 0.0f);
+        }
       }
     }
   }
@@ -626,156 +676,217 @@ __device__ __forceinline__ int cell_of(const gdl::Bufs& B, int64_t i) {
          1;
 }
 
-// Cell starts: one bit per sorted position (a key differing from the one
-// before it), written a word per warp.
+// Cells, in one pass over the sorted keys: a bit per position that starts a cell
+// (its key differs from the one before) with per-word prefix counts, and every
+// cell's first position (reps) and key (ckeys).  A tile is 8192 positions (16 warps
+// of 16 words): counts are scanned in the block, the tile's prefix comes by look-back
+// while the keys wait in registers.  The last tile closes reps and counts the cells;
+// in runs of 2D and 3D instances the first cell of a 3D instance marks the border.
+// (Bits, scan, list and closing had been four launches reading the keys twice: C2
+// 22 + 6 + 36 + 4 us.)
+constexpr int kRunThreads = 512, kRunWords = 16, kRunTile = kRunThreads * kRunWords;
 template <class Key>
-__global__ void k_run_bits(const Key* __restrict__ keys, int64_t n, uint32_t* __restrict__ bits) {
-  const int lane = threadIdx.x & 31;
-  // four groups of 32 positions per warp and pass, their loads issued together
-  constexpr int U = 4;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t g0 = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); g0 < n;
-       g0 += U * stride) {
-    Key k[U], p[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int64_t i = g0 + u * stride + lane;
-      k[u] = i < n ? keys[i] : (Key)0;
-      p[u] = lane == 0 && i > 0 && i <= n ? keys[i - 1] : (Key)0;
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int64_t i0 = g0 + u * stride;
-      if (i0 >= n) break;  // warp-uniform
-      const int64_t i = i0 + lane;
-      Key prev = __shfl_up_sync(kFull, k[u], 1);
-      if (lane == 0) prev = p[u];
-      const unsigned b = __ballot_sync(kFull, i < n && (i == 0 || k[u] != prev));
-      if (lane == 0) bits[i0 >> 5] = b;
-    }
+__global__ void __launch_bounds__(kRunThreads)
+k_runs(const gdl::Bufs B, int64_t n, Key* __restrict__ ckeys, unsigned tiles,
+       gdprim::LookbackCtl* ctl, unsigned long long* status) {
+  __shared__ uint32_t s_warp[32];
+  __shared__ unsigned s_tile, s_epoch;
+  __shared__ uint32_t s_agg, s_excl;
+  const Key* __restrict__ keys = static_cast<const Key*>(B.keys);
+  unsigned long long* timeouts = B.ctr + kCtrWaitTimeouts;
+  gdprim::lb_begin(ctl, &s_tile, &s_epoch);
+  const unsigned tile = s_tile, epoch = s_epoch;
+  if (tile >= tiles) {
+    // a counter left inconsistent (never expected): no tile, report it
+    if (threadIdx.x == 0) atomicAdd(timeouts, 1ull);
+    gdprim::lb_end(ctl, tiles, epoch);
+    return;
   }
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t seg = (int64_t)tile * kRunTile + (int64_t)w * 32 * kRunWords;
+  Key k[kRunWords];
+#pragma unroll
+  for (int u = 0; u < kRunWords; ++u) {
+    const int64_t i = seg + u * 32 + lane;
+    k[u] = i < n ? keys[i] : (Key)0;
+  }
+  // the key before the segment, then each word's last key
+  Key last = seg > 0 && seg < n ? keys[seg - 1] : (Key)0;
+  unsigned bits[kRunWords], cnt = 0;
+#pragma unroll
+  for (int u = 0; u < kRunWords; ++u) {
+    const int64_t i = seg + u * 32 + lane;
+    Key prev = __shfl_up_sync(kFull, k[u], 1);
+    if (lane == 0) prev = last;
+    last = __shfl_sync(kFull, k[u], 31);
+    bits[u] = __ballot_sync(kFull, i < n && (i == 0 || k[u] != prev));
+    cnt += (unsigned)__popc(bits[u]);
+  }
+  // warp totals scanned in the block (one thread per warp carries the total)
+  const uint32_t ex = gdprim::block_excl_scan<kRunThreads>(lane == 0 ? cnt : 0u, s_warp, &s_agg);
+  const uint32_t excl =
+      gdprim::lb_tile_prefix(status, tile, gdprim::lb_tag(epoch), &s_agg, &s_excl, timeouts);
+  uint32_t m = excl + __shfl_sync(kFull, ex, 0);
+  const int K2 = B.Bi->K2, LB = B.Bi->LB;
+  const bool mixed = K2 > 0 && K2 < B.Bi->K;
+#pragma unroll
+  for (int u = 0; u < kRunWords; ++u) {
+    const int64_t i0 = seg + u * 32, i = i0 + lane;
+    if (i0 >= n) break;  // warp-uniform
+    if (lane == 0) {
+      B.runbits[i0 >> 5] = bits[u];
+      B.runpre[i0 >> 5] = m;
+    }
+    if ((bits[u] >> lane) & 1u) {
+      const uint32_t c = m + (uint32_t)__popc(bits[u] & ((1u << lane) - 1u));
+      B.reps[c] = (int)i;
+      ckeys[c] = k[u];
+      if (mixed && inst_of(k[u], LB) >= K2 && (i == 0 || inst_of(keys[i - 1], LB) < K2))
+        B.ctr[kCtrCells2D] = c;
+    }
+    m += (uint32_t)__popc(bits[u]);
+  }
+  if (tile == tiles - 1u && threadIdx.x == 0) {
+    const uint32_t M = excl + s_agg;
+    *B.M = M;
+    B.reps[M] = (int)n;
+    B.ctr[kCtrCells] = M;
+    if (K2 == 0) B.ctr[kCtrCells2D] = 0;
+    else if (!mixed || inst_of(keys[n - 1], LB) < K2) B.ctr[kCtrCells2D] = M;
+  }
+  gdprim::lb_end(ctl, tiles, epoch);
 }
 
-// After the cell starts are listed in reps: reps[M] = n, the cell count, and
-// (mixed runs) the number of cells of 2D instances -- 2D instances come first,
-// the first cell of a 3D instance is found by binary search.
+// Block entries and row lookups, a lane per cell.  A block's cells are
+// consecutive in key order, mostly within one warp: the run of lanes of one block
+// forms its occupancy word together; the lane of the block's first cell reads on
+// where the block goes past the warp's end (at most 63 cells), and writes the
+// entry (core word and roots empty) and its empty link words.  Every cell notes
+// where its block's entry is.  The first and last cell of a block row write the
+// row's cell range (row table or hash slot).
+constexpr int kCellsThreads = 256, kCellsU = 4;
 template <class Key>
-__global__ void k_runs_finish(const gdl::Bufs B, int64_t n, int mixed) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const int64_t M = *B.M;
-  B.reps[M] = (int)n;
-  B.ctr[kCtrCells] = (unsigned long long)M;
-  const int K2 = B.Bi->K2;
-  int64_t lo = K2 > 0 ? M : 0;
-  if (mixed) {
-    const Key* keys = static_cast<const Key*>(B.keys);
-    const int LB = B.Bi->LB;
-    int64_t hi = M;  // first cell with instance >= K2
-    lo = 0;
-    while (lo < hi) {
-      const int64_t mid = (lo + hi) / 2;
-      if (inst_of(keys[B.reps[mid]], LB) < K2) lo = mid + 1;
-      else hi = mid;
-    }
-  }
-  B.ctr[kCtrCells2D] = (unsigned long long)lo;
-}
-
-// Cell tables: one occupancy bit per non-empty cell (a cell's points are then
-// found by rank, see GridView::rank).  Row tables: one occupancy bit and a cell
-// count per non-empty row (scanned afterwards into each row's first cell).
-// Every cell's last-axis coordinate goes to cellz, and each instance's first
-// and last cells are recorded (k_start_fill turns them into the one-entry start
-// slices of the other instances, so the scan stays in cell units).
-template <class Key>
-__global__ void k_cell_counts(const gdl::Bufs B) {
-  const Key* keys = static_cast<const Key*>(B.keys);
+__global__ void __launch_bounds__(kCellsThreads) k_cells(const gdl::Bufs B) {
+  const Key* __restrict__ ckeys = static_cast<const Key*>(B.ckeys);
   const int LB = B.Bi->LB;
   const int64_t M = *B.M;
-  for (int64_t m = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; m < M;
-       m += (int64_t)gridDim.x * blockDim.x) {
-    const Key key = keys[B.reps[m]];
-    const int inst = inst_of(key, LB);
-    DevParams& P = B.Pv[inst];
-    if (m == 0 || inst_of(keys[B.reps[m - 1]], LB) != inst) P.m0 = m;
-    if (m == M - 1 || inst_of(keys[B.reps[m + 1]], LB) != inst) P.m1 = m;
-    const uint64_t local = (uint64_t)key & P.kmask;
-    const int a = P.dim - 2;
-    const uint64_t row = udiv_by(local, P.dm[a], P.ds[a]);
-    B.cellz[m] = (uint32_t)(local - row * (uint64_t)P.G[P.dim - 1]);
-    if (P.sparse == 1) continue;
-    if (P.sparse == 2) {
-      atomicAdd(B.start + P.start_off + row, 1u);
-      const uint64_t idx = P.occ_off + row;
-      atomicOr(B.occ + (idx >> 5), 1u << (idx & 31));
-      continue;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  // kCellsU groups of 32 cells per warp and round; the round's block list entries
+  // take one atomic (an atomic per warp had bound the kernel: C3 159 us)
+  __shared__ uint32_t s_cnt[32];
+  __shared__ unsigned long long s_at;
+  const int64_t per = (int64_t)kCellsThreads * kCellsU;
+  for (int64_t r0 = blockIdx.x * per; r0 < M; r0 += gridDim.x * per) {
+    uint64_t kk[kCellsU];
+    unsigned ff[kCellsU];
+#pragma unroll
+    for (int u = 0; u < kCellsU; ++u) {
+      const int64_t m0 = r0 + (w * kCellsU + u) * 32, m = m0 + lane;
+      const uint64_t key = (uint64_t)ckeys[m < M ? m : M - 1];
+      const uint64_t blk = key >> kBlockBits;  // with the instance id
+      uint64_t pb = __shfl_up_sync(kFull, blk, 1);
+      if (lane == 0) pb = m > 0 && m < M ? (uint64_t)ckeys[m - 1] >> kBlockBits : ~0ull;
+      kk[u] = key;
+      ff[u] = __ballot_sync(kFull, m < M && (m == 0 || pb != blk));
+      if (lane == 0) s_cnt[w * kCellsU + u] = (uint32_t)__popc(ff[u]);
     }
-    const uint64_t idx = P.occ_off + local;
-    atomicOr(B.occ + (idx >> 5), 1u << (idx & 31));
-  }
-}
-
-// One-entry start slices (instances without a row table): their cell count.
-__global__ void k_start_fill(const gdl::Bufs B, int K) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < K; i += gridDim.x * blockDim.x) {
-    const DevParams& P = B.Pv[i];
-    if (P.sparse != 2) B.start[P.start_off] = P.n > 0 ? (uint32_t)(P.m1 - P.m0 + 1) : 0u;
-  }
-}
-
-// A cell table's cells appear in reps in table order from the instance's first
-// cell on, so a cell's index into reps is its occupancy rank minus the rank of
-// the table's first bit plus that first cell.
-__global__ void k_rank_off(const gdl::Bufs B, int K) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < K; i += gridDim.x * blockDim.x) {
-    DevParams& P = B.Pv[i];
-    if (P.sparse != 0 || P.n == 0) continue;
-    const uint64_t idx = P.occ_off, w = idx >> 5;
-    const int64_t r = (int64_t)B.wpre[w] + __popc(B.occ[w] & ((1u << (idx & 31)) - 1u));
-    P.rank_off = P.m0 - r;
-  }
-}
-
-// sparse instances: hash of the occupied rows, global key of the row's first
-// cell -> [begin, end) of the row's points.  The thread of a row's first cell
-// walks the row's cells to its end.
-template <class Key>
-__global__ void k_row_hash(const gdl::Bufs B) {
-  const Key* keys = static_cast<const Key*>(B.keys);
-  const int LB = B.Bi->LB;
-  const int64_t M = *B.M;
-  const uint32_t mask = B.hmask;
-  for (int64_t m = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; m < M;
-       m += (int64_t)gridDim.x * blockDim.x) {
-    const uint64_t key = (uint64_t)keys[B.reps[m]];
-    const int inst = (int)(key >> LB);
-    const DevParams& P = B.Pv[inst];
-    if (P.sparse != 1) continue;
-    const uint64_t Gl = (uint64_t)P.G[P.dim - 1];
-    const uint64_t hi = key & ~P.kmask;
-    const uint64_t local = key & P.kmask;
-    const uint64_t rowkey = local - local % Gl;
-    if (m > 0) {
-      const uint64_t pk = (uint64_t)keys[B.reps[m - 1]];
-      if ((pk & ~P.kmask) == hi && (pk & P.kmask) >= rowkey) continue;  // not the row's first cell
-    }
-    int64_t m2 = m + 1;
-    while (m2 < M) {
-      const uint64_t k2 = (uint64_t)keys[B.reps[m2]];
-      if ((k2 & ~P.kmask) != hi || (k2 & P.kmask) >= rowkey + Gl) break;
-      ++m2;
-    }
-    const unsigned long long k = hi | rowkey;
-    uint32_t h = hash_key(k) & mask;
-    for (uint32_t probe = 0; probe <= mask; ++probe) {
-      unsigned long long prev = atomicCAS(B.hkeys + h, kHashEmpty, k);
-      if (prev == kHashEmpty || prev == k) {
-        B.hvals[2 * h] = (uint32_t)B.reps[m];
-        B.hvals[2 * h + 1] = (uint32_t)B.reps[m2];
-        break;
+    __syncthreads();
+    if (w == 0) {
+      const uint32_t c = s_cnt[lane];
+      uint32_t inc = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(kFull, inc, o);
+        if (lane >= o) inc += v;
       }
-      h = (h + 1) & mask;
+      s_cnt[lane] = inc - c;
+      if (lane == 31) s_at = atomicAdd(B.ctr + kCtrBlocks, (unsigned long long)inc);
     }
+    __syncthreads();
+    const unsigned long long at0 = s_at;
+#pragma unroll
+    for (int u = 0; u < kCellsU; ++u) {
+    const int64_t m0 = r0 + (w * kCellsU + u) * 32, m = m0 + lane;
+    if (m >= M) continue;
+    const uint64_t key = kk[u], blk = key >> kBlockBits;
+    const unsigned firsts = ff[u];
+    const bool first = (firsts >> lane) & 1u;
+    // the block list, in no particular order
+    if (first)
+      B.blklist[at0 + s_cnt[w * kCellsU + u] + __popc(firsts & ((1u << lane) - 1u))] = (uint32_t)m;
+    const DevParams& P = B.Pv[inst_of(key, LB)];
+    const uint64_t lblk = (key & P.kmask) >> kBlockBits;
+    const int mode = P.sparse;
+    // this lane's run: lanes [rs, re) hold cells of its block
+    const unsigned heads = firsts | 1u;
+    const unsigned upto = (unsigned)((2ull << lane) - 1ull);
+    const int rs = 31 - __clz(heads & upto);
+    const unsigned after = heads & ~upto;
+    const int nv = M - m0 < 32 ? (int)(M - m0) : 32;
+    const int re = after ? __ffs(after) - 1 : nv;
+    const unsigned run = (unsigned)((1ull << re) - (1ull << rs));
+    const uint32_t b = 1u << (key & 31);
+    uint32_t lo = __reduce_or_sync(run, (key & 32) ? 0u : b);
+    uint32_t hi = __reduce_or_sync(run, (key & 32) ? b : 0u);
+    uint32_t e = P.ent_off + (uint32_t)lblk;
+    if (mode != 0) {
+      // the block's first cell: the run's first lane, or cells before the warp
+      int64_t f = m0 + rs;
+      if (rs == 0 && !(firsts & 1u))
+        while (f > 0 && (uint64_t)ckeys[f - 1] >> kBlockBits == blk) --f;
+      e = B.ent_base + (uint32_t)f;
+    }
+    B.cellent[m] = e;
+    if (first) {
+      if (re == 32)
+        for (int64_t c = m0 + 32; c < M; ++c) {
+          const uint64_t k = (uint64_t)ckeys[c];
+          if (k >> kBlockBits != blk) break;
+          if (k & 32) hi |= 1u << (k & 31);
+          else lo |= 1u << (k & 31);
+        }
+      BlockEnt E;
+      E.occ = (unsigned long long)hi << 32 | lo;
+      E.base = (uint32_t)m;
+      E.lo = kNoEnt;
+      E.core = 0;
+      E.hi = kNoEnt;
+      E.uni = kNoEnt;
+      B.ent[e] = E;
+      B.links[e] = BlockLinks{};
+    }
+    if (mode == 0) continue;
+    // the row's first key and the first key past it (no key of the run lies
+    // between a row's last one and the latter)
+    const int a = P.dim - 2;
+    const uint64_t Bz = (uint64_t)P.Bk[P.dim - 1];
+    const uint64_t row = udiv_by(lblk, P.dm[a], P.ds[a]);
+    const uint64_t k0 = inst_key(P.inst, LB) + ((row * Bz) << kBlockBits);
+    const uint64_t k1 = k0 + (Bz << kBlockBits) - 1;  // the row's last possible key
+    const bool rfirst = m == 0 || (uint64_t)ckeys[m - 1] < k0;
+    const bool rlast = m == M - 1 || (uint64_t)ckeys[m + 1] > k1;
+    if (!rfirst && !rlast) continue;
+    uint2* slot = nullptr;
+    if (mode == 2) {
+      slot = B.rowtab + P.row_off + row;
+    } else {
+      const uint32_t mask = B.hmask;
+      uint32_t h = hash_key(k0) & mask;
+      for (uint32_t probe = 0; probe <= mask; ++probe) {
+        const unsigned long long prev = atomicCAS(B.hkeys + h, kHashEmpty, (unsigned long long)k0);
+        if (prev == kHashEmpty || prev == k0) {
+          slot = B.hvals + h;
+          break;
+        }
+        h = (h + 1) & mask;
+      }
+    }
+    if (slot) {
+      if (rfirst) slot->x = (uint32_t)m;
+      if (rlast) slot->y = (uint32_t)(m + 1);
+    }
+    }
+    __syncthreads();
   }
 }
 
@@ -787,38 +898,79 @@ struct CellXYZ {
 
 template <int D>
 __device__ __forceinline__ CellXYZ<D> decompose(uint64_t key, const DevParams& P) {
+  constexpr int S = block_shift<D>(), SM = (1 << S) - 1;
   CellXYZ<D> r;
-  uint64_t k = key;
+  const unsigned in = (unsigned)key & 63u;
+  uint64_t k = key >> kBlockBits;
+  if (P.small) {
+    // fewer than 2^32 blocks: the same division on 32 bits
+    unsigned q = (unsigned)k;
+    if (D == 3) {
+      const unsigned k2 = udiv_by32(q, P.dm32[1], P.ds[1]);
+      r.c[2] = (int)((q - k2 * (unsigned)P.Bk[2]) << S | (in & SM));
+      q = k2;
+    } else {
+      r.c[2] = 0;
+    }
+    const unsigned k1 = udiv_by32(q, P.dm32[0], P.ds[0]);
+    r.c[1] = (int)((q - k1 * (unsigned)P.Bk[1]) << S | (D == 3 ? (in >> S) & SM : in & SM));
+    r.c[0] = (int)(k1 << S | in >> (D == 3 ? 2 * S : S));
+    return r;
+  }
   if (D == 3) {
     const uint64_t k2 = udiv_by(k, P.dm[1], P.ds[1]);
-    r.c[2] = (int)(k - k2 * (uint64_t)P.G[2]);
+    r.c[2] = (int)((unsigned)(k - k2 * (uint64_t)(unsigned)P.Bk[2]) << S | (in & SM));
     k = k2;
   } else {
     r.c[2] = 0;
   }
   const uint64_t k1 = udiv_by(k, P.dm[0], P.ds[0]);
-  r.c[1] = (int)(k - k1 * (uint64_t)P.G[1]);
-  r.c[0] = (int)k1;
+  r.c[1] = (int)((unsigned)(k - k1 * (uint64_t)(unsigned)P.Bk[1]) << S |
+                 (D == 3 ? (in >> S) & SM : in & SM));
+  r.c[0] = (int)((unsigned)k1 << S | in >> (D == 3 ? 2 * S : S));
   return r;
 }
 
-// key of cell (c + o), or -1 when outside the grid
+// Coordinates of sorted position i: float64 copy, centred float32 copy.
 template <int D>
-__device__ __forceinline__ int64_t offset_key(const CellXYZ<D>& c, int ox, int oy, int oz,
-                                              const DevParams& P) {
-  int64_t x = (int64_t)c.c[0] + ox, y = (int64_t)c.c[1] + oy;
-  if (x < 0 || x >= P.G[0] || y < 0 || y >= P.G[1]) return -1;
-  int64_t k = x * P.G[1] + y;
-  if (D == 3) {
-    int64_t z = (int64_t)c.c[2] + oz;
-    if (z < 0 || z >= P.G[2]) return -1;
-    k = k * P.G[2] + z;
+__device__ __forceinline__ void ld_x(const gdl::Bufs& B, int64_t i, double* v) {
+  if (D == 2) {
+    const double2 t = reinterpret_cast<const double2*>(B.X)[i];
+    v[0] = t.x;
+    v[1] = t.y;
+  } else {
+#pragma unroll
+    for (int k = 0; k < D; ++k) v[k] = B.X[3 * i + k];
   }
-  return k;
+}
+template <int D>
+__device__ __forceinline__ void ld_f(const gdl::Bufs& B, int64_t i, float* v) {
+  if (D == 2) {
+    const float2 t = reinterpret_cast<const float2*>(B.Xf)[i];
+    v[0] = t.x;
+    v[1] = t.y;
+  } else {
+    const float4 t = reinterpret_cast<const float4*>(B.Xf)[i];
+    v[0] = t.x;
+    v[1] = t.y;
+    v[D - 1] = t.z;
+  }
+}
+// Float64 coordinates for a band re-test: the sorted copy, or (float32-band runs
+// keep none when every instance has a band) the caller's point.
+template <int D>
+__device__ __forceinline__ void exact_x(const gdl::Bufs& B, const DevParams& P, int64_t i,
+                                        double* v) {
+  if (B.X) {
+    ld_x<D>(B, i, v);
+    return;
+  }
+  const double* src = B.coords + P.co_off + ((int64_t)B.ids[i] - P.pt_off) * D;
+#pragma unroll
+  for (int k = 0; k < D; ++k) v[k] = src[k];
 }
 
-
-// Loads one candidate (sorted position q) in the layout the mode tests with.
+// One candidate (sorted position q) in the layout the mode tests with.
 template <int D, bool F32>
 struct Cand {
   double x[D];
@@ -826,13 +978,9 @@ struct Cand {
 };
 
 template <int D, bool F32>
-__device__ __forceinline__ void load_cand(Cand<D, F32>& c, const double* __restrict__ X,
-                                          const float* __restrict__ Xf, int64_t n, int64_t q) {
-#pragma unroll
-  for (int k = 0; k < D; ++k) {
-    if (F32) c.f[k] = Xf[k * n + q];
-    else c.x[k] = X[k * n + q];
-  }
+__device__ __forceinline__ void load_cand(Cand<D, F32>& c, const gdl::Bufs& B, int64_t q) {
+  if (F32) ld_f<D>(B, q, c.f);
+  else ld_x<D>(B, q, c.x);
 }
 
 // Per-warp staging of up to 32 "A" points (the points of the cell in work).
@@ -867,7 +1015,7 @@ __device__ __forceinline__ float dist2_f32(const float* a, const float* b) {
 // float64 coordinates of both are loaded only for a band re-test.
 template <int D, bool F32, class PP>
 __device__ __forceinline__ bool pair_test(const double* sx, const float* sf, const Cand<D, F32>& c,
-                                          const double* __restrict__ X, int64_t n, int64_t q,
+                                          const gdl::Bufs& B, const DevParams& I, int64_t q,
                                           int64_t si, bool stage_is_centre, const PP& P,
                                           Tally& t) {
   if (F32) {
@@ -877,11 +1025,8 @@ __device__ __forceinline__ bool pair_test(const double* sx, const float* sf, con
     if (s > P.eps2_hi32) return false;
     ++t.band;
     double qx[D], px[D];
-#pragma unroll
-    for (int k = 0; k < D; ++k) {
-      qx[k] = X[k * n + q];
-      px[k] = X[k * n + si];
-    }
+    exact_x<D>(B, I, q, qx);
+    exact_x<D>(B, I, si, px);
     ++t.t64;
     double d2 = dist2_f64<D>(px, qx);
     return stage_is_centre ? pred_from_d2<D>(d2, px, qx, P) : pred_from_d2<D>(d2, qx, px, P);
@@ -896,9 +1041,8 @@ __device__ __forceinline__ bool pair_test(const double* sx, const float* sf, con
 // directions; counts pairs that are neighbours in exactly one direction.
 template <int D, bool F32, class PP>
 __device__ __forceinline__ bool link_test(const double* sx, const float* sf, const Cand<D, F32>& c,
-                                          const double* __restrict__ X, int64_t n, int a, int q,
-                                          const PP& P, Tally& t,
-                                          int* __restrict__ asym_list, unsigned long long* ctr) {
+                                          const gdl::Bufs& B, const DevParams& I, int a, int q,
+                                          const PP& P, Tally& t) {
   double qx[D], ax[D];
   if (F32) {
     ++t.t32;
@@ -907,11 +1051,8 @@ __device__ __forceinline__ bool link_test(const double* sx, const float* sf, con
     if (s > P.eps2_hi32) return false;
     ++t.band;
     // float64 coordinates of both, for the band re-test only
-#pragma unroll
-    for (int k = 0; k < D; ++k) {
-      qx[k] = X[k * n + q];
-      ax[k] = X[k * n + a];
-    }
+    exact_x<D>(B, I, q, qx);
+    exact_x<D>(B, I, a, ax);
   } else {
 #pragma unroll
     for (int k = 0; k < D; ++k) {
@@ -929,10 +1070,10 @@ __device__ __forceinline__ bool link_test(const double* sx, const float* sf, con
     // q is a neighbour of a but not a of q (f), or the reverse: a directed
     // link that the merge replay (k_asym_resolve) needs.
     ++t.asym;
-    unsigned long long slot = atomicAdd(ctr + kCtrAsymEdges, 1ull);
+    unsigned long long slot = atomicAdd(B.ctr + kCtrAsymEdges, 1ull);
     if (slot < (unsigned long long)kAsymCap) {
-      asym_list[2 * slot] = f ? a : q;
-      asym_list[2 * slot + 1] = f ? q : a;
+      B.asym[2 * slot] = f ? a : q;
+      B.asym[2 * slot + 1] = f ? q : a;
     }
   }
   return f && b;
@@ -984,156 +1125,17 @@ __device__ __forceinline__ unsigned run_peers(unsigned act, int v) {
   return (unsigned)(((1ull << e) - 1ull) & ~((1ull << s) - 1ull));
 }
 
-// Cell lookup inside one instance.  Dense grids: the instance's slice of the
-// cell tables gives every cell's point range (an occupancy bit per entry skips
-// empty cells without touching the table).  Sparse grids: a hash of the
-// occupied rows (all cells sharing every coordinate but the last) gives the
-// row's point range, and a binary search on the sorted keys the cells inside
-// it.  The probe loop is bounded by the table size.  The view holds only the
-// instance's scalars; the tables' addresses are read from the kernel's
-// parameter block at each use (B is always the kernel parameter), so they
-// occupy no registers in the walks.
-struct GridView {
-  int sparse;              // DevParams::sparse
-  int key64;
-  uint64_t occ_off;
-  uint64_t start_off;
-  int64_t rank_off;
-  uint64_t hi;             // instance id << LB
-  int64_t Gl;              // cells along the last axis
-  uint64_t glm;            // division by Gl (udiv_by)
-  int32_t gls;
-
-  __device__ __forceinline__ uint64_t gkey(const gdl::Bufs& B, int64_t i) const {
-    return key64 ? static_cast<const unsigned long long*>(B.keys)[i]
-                 : (uint64_t) static_cast<const uint32_t*>(B.keys)[i];
-  }
-  // cell table: index into reps of the first non-empty cell at or after
-  // local key k (its rank among the occupied cells)
-  __device__ __forceinline__ int64_t rank(const gdl::Bufs& B, uint64_t k) const {
-    const uint64_t idx = occ_off + k, w = idx >> 5;
-    return (int64_t)B.wpre[w] + __popc(B.occ[w] & ((1u << (idx & 31)) - 1u)) + rank_off;
-  }
-  __device__ __forceinline__ bool occupied(const gdl::Bufs& B, uint64_t k) const {
-    const uint64_t idx = occ_off + k;
-    return (B.occ[idx >> 5] >> (idx & 31)) & 1u;
-  }
-  // row table: cells [begin, end) (indices into reps) of row ri
-  __device__ __forceinline__ int2 row_cells(const gdl::Bufs& B, uint64_t ri) const {
-    const uint64_t idx = occ_off + ri;
-    if (!((B.occ[idx >> 5] >> (idx & 31)) & 1u)) return make_int2(0, 0);
-    return make_int2((int)B.start[start_off + ri], (int)B.start[start_off + ri + 1]);
-  }
-  // first cell in [b, e) (one row's cells) whose last-axis coordinate is >= z
-  __device__ __forceinline__ int zlower(const gdl::Bufs& B, int b, int e, int64_t z) const {
-    while (b < e) {
-      const int mid = (int)(((unsigned)b + (unsigned)e) >> 1);
-      if ((int64_t)B.cellz[mid] < z) b = mid + 1;
-      else e = mid;
-    }
-    return b;
-  }
-  // row table: whether row ri holds a core point
-  __device__ __forceinline__ bool core_row_at(const gdl::Bufs& B, uint64_t ri) const {
-    const uint64_t idx = occ_off + ri;
-    return (B.cocc[idx >> 5] >> (idx & 31)) & 1u;
-  }
-  // hash: points [begin, end) of the row whose first cell is rowkey
-  __device__ __forceinline__ int2 row(const gdl::Bufs& B, uint64_t rowkey) const {
-    const unsigned long long k = hi | rowkey;
-    const uint32_t hmask = B.hmask;
-    uint32_t h = hash_key(k) & hmask;
-    for (uint32_t probe = 0; probe <= hmask; ++probe) {
-      const unsigned long long kk = B.hkeys[h];
-      if (kk == k) return make_int2((int)B.hvals[2 * h], (int)B.hvals[2 * h + 1]);
-      if (kk == kHashEmpty) break;
-      h = (h + 1) & hmask;
-    }
-    return make_int2(0, 0);
-  }
-  // cell table: occupancy bits of cells z0..z1 (at most 5) of the row whose
-  // first cell is rowkey (bit z - z0), and the reps index of the first
-  // occupied one (the others follow it in reps).  The three words are loaded
-  // at once, whether or not they are needed: word w + 1 past the last
-  // occupancy word is the first core occupancy word, in the same buffer.
-  __device__ __forceinline__ uint32_t occ_cells(const gdl::Bufs& B, uint64_t rowkey, int64_t z0,
-                                                int64_t z1, int64_t& r0) const {
-    const uint64_t i0 = occ_off + rowkey + (uint64_t)z0, w = i0 >> 5;
-    const int len = (int)(z1 - z0) + 1;
-    const int sh = (int)(i0 & 31);
-    const uint32_t lo = B.occ[w], hi = B.occ[w + 1], pre = B.wpre[w];
-    const uint64_t bits = (((uint64_t)hi << 32) | lo) >> sh;
-    const uint32_t mask = (uint32_t)bits & ((1u << len) - 1u);
-    r0 = (int64_t)pre + __popc(lo & ((1u << sh) - 1u)) + rank_off;
-    return mask;
-  }
-  // core occupancy bits of cells z0..z1 of a cell-table row (bit z - z0); word
-  // w + 1 past the last one lies in the padding or the word prefix counts
-  // that follow in the same buffer
-  __device__ __forceinline__ uint32_t core_cells(const gdl::Bufs& B, uint64_t rowkey, int64_t z0,
-                                                 int64_t z1) const {
-    const uint64_t i0 = occ_off + rowkey + (uint64_t)z0;
-    const int len = (int)(z1 - z0) + 1;  // <= 5
-    const uint64_t w = i0 >> 5;
-    const int sh = (int)(i0 & 31);
-    const uint64_t bits = (((uint64_t)B.cocc[w + 1] << 32) | B.cocc[w]) >> sh;
-    return (uint32_t)bits & ((1u << len) - 1u);
-  }
-  // first sorted position in [b, e) whose key is >= g
-  __device__ __forceinline__ int lower(const gdl::Bufs& B, int b, int e, uint64_t g) const {
-    while (b < e) {
-      const int mid = (int)(((unsigned)b + (unsigned)e) >> 1);
-      if (gkey(B, mid) < g) b = mid + 1;
-      else e = mid;
-    }
-    return b;
-  }
-  // points of the cells z0..z1 of the row whose first cell is rowkey: one
-  // contiguous range, because no other key sorts between them
-  __device__ __forceinline__ int2 span_row(const gdl::Bufs& B, uint64_t rowkey, int64_t z0,
-                                           int64_t z1) const {
-    if (!sparse)
-      return make_int2(B.reps[rank(B, rowkey + z0)], B.reps[rank(B, rowkey + z1 + 1)]);
-    if (sparse == 2) {
-      const int2 rc = row_cells(B, udiv_by(rowkey, glm, gls));
-      if (rc.x == rc.y) return make_int2(0, 0);
-      const int ma = zlower(B, rc.x, rc.y, z0), mb = zlower(B, ma, rc.y, z1 + 1);
-      return make_int2(B.reps[ma], B.reps[mb]);
-    }
-    const int2 r = row(B, rowkey);
-    if (r.x == r.y) return r;
-    const int a = lower(B, r.x, r.y, hi | (rowkey + (uint64_t)z0));
-    const int b = lower(B, a, r.y, hi | (rowkey + (uint64_t)z1 + 1));
-    return make_int2(a, b);
-  }
-  // points of the cell with local key k: [x, y)
-  __device__ __forceinline__ int2 cell(const gdl::Bufs& B, uint64_t k) const {
-    if (!sparse) {
-      if (!occupied(B, k)) return make_int2(0, 0);
-      const int64_t r = rank(B, k);
-      return make_int2(B.reps[r], B.reps[r + 1]);
-    }
-    const int64_t z = (int64_t)(k - udiv_by(k, glm, gls) * (uint64_t)Gl);
-    return span_row(B, k - (uint64_t)z, z, z);
-  }
-  // points of the cells k0..k1 (consecutive local keys along one row)
-  __device__ __forceinline__ int2 span(const gdl::Bufs& B, uint64_t k0, uint64_t k1) const {
-    if (!sparse) return make_int2(B.reps[rank(B, k0)], B.reps[rank(B, k1 + 1)]);
-    const int64_t z0 = (int64_t)(k0 - udiv_by(k0, glm, gls) * (uint64_t)Gl);
-    return span_row(B, k0 - (uint64_t)z0, z0, z0 + (int64_t)(k1 - k0));
-  }
-};
-
-__device__ __forceinline__ GridView view_of(const gdl::Bufs& B, const DevParams& P) {
-  const int a = P.dim - 2;
-  return GridView{P.sparse, B.Bi->key64, P.occ_off, P.start_off, P.rank_off,
-                  (uint64_t)P.inst << P.LB, P.G[P.dim - 1], P.dm[a], P.ds[a]};
-}
-
 template <bool KEY64>
 __device__ __forceinline__ uint64_t key_at(const gdl::Bufs& B, int64_t i) {
   if (KEY64) return static_cast<const unsigned long long*>(B.keys)[i];
   return static_cast<const uint32_t*>(B.keys)[i];
+}
+
+// key of cell m (instance id and local key)
+template <bool KEY64>
+__device__ __forceinline__ uint64_t ckey_at(const gdl::Bufs& B, int64_t m) {
+  if (KEY64) return static_cast<const unsigned long long*>(B.ckeys)[m];
+  return static_cast<const uint32_t*>(B.ckeys)[m];
 }
 
 // The cell a kernel thread/warp works on: instance parameters and local key.
@@ -1143,12 +1145,128 @@ struct CellCtx {
 };
 
 template <bool KEY64>
-__device__ __forceinline__ CellCtx cell_ctx(const gdl::Bufs& B, int b, int LB) {
-  const uint64_t key = key_at<KEY64>(B, b);
+__device__ __forceinline__ CellCtx cell_ctx(const gdl::Bufs& B, int64_t m, int LB) {
+  const uint64_t key = ckey_at<KEY64>(B, m);
   CellCtx c;
-  c.P = B.Pv + (int)(key >> LB);
+  c.P = B.Pv + (KEY64 ? inst_of(key, LB) : (int)(key >> LB));
   c.local = key & c.P->kmask;
   return c;
+}
+
+// ------------------------------------------------------------ block lookups
+// Entries of blocks z0 and z0 + 1 (last axis; z0 >= -1) of block row `row`,
+// kNoEnt when unwanted, outside the grid or (row table, hash) not occupied.
+// Direct tables: one address computation, no load.  Row tables and the hash:
+// the row's cell range, then a binary search over its cells' keys for the
+// first cell of the first wanted block; the next block follows its cells.
+template <int D, bool KEY64>
+__device__ __forceinline__ void block_pair(const gdl::Bufs& B, const DevParams& P, uint64_t row,
+                                           int z0, bool want0, bool want1, uint32_t& e0,
+                                           uint32_t& e1) {
+  e0 = kNoEnt;
+  e1 = kNoEnt;
+  const int Bz = P.Bk[D - 1];
+  want0 = want0 && z0 >= 0;
+  want1 = want1 && z0 + 1 < Bz;
+  if (P.sparse == 0) {
+    const uint32_t e = P.ent_off + (uint32_t)row * (uint32_t)Bz + (uint32_t)z0;
+    if (want0) e0 = e;
+    if (want1) e1 = e + 1;
+    return;
+  }
+  if (!want0 && !want1) return;
+  const uint64_t k0 = inst_key(P.inst, P.LB) + ((row * (uint64_t)Bz) << kBlockBits);
+  uint2 rc = make_uint2(0, 0);
+  if (P.sparse == 2) {
+    rc = B.rowtab[P.row_off + row];
+  } else {
+    const uint32_t hmask = B.hmask;
+    uint32_t h = hash_key(k0) & hmask;
+    for (uint32_t probe = 0; probe <= hmask; ++probe) {
+      const unsigned long long kk = B.hkeys[h];
+      if (kk == k0) {
+        rc = B.hvals[h];
+        break;
+      }
+      if (kk == kHashEmpty) break;
+      h = (h + 1) & hmask;
+    }
+  }
+  const uint64_t kf = k0 + ((uint64_t)(want0 ? z0 : z0 + 1) << kBlockBits);
+  uint32_t a = rc.x, b = rc.y;
+  while (a < b) {
+    const uint32_t mid = (a + b) >> 1;
+    if (ckey_at<KEY64>(B, mid) < kf) a = mid + 1;
+    else b = mid;
+  }
+  if (a >= rc.y) return;
+  const uint64_t zb = (ckey_at<KEY64>(B, a) - k0) >> kBlockBits;
+  if (want0 && zb == (uint64_t)z0) {
+    e0 = B.ent_base + a;
+    if (!want1) return;
+    a += (uint32_t)__popcll(B.ent[e0].occ);
+    if (a < rc.y && (ckey_at<KEY64>(B, a) - k0) >> kBlockBits == (uint64_t)(z0 + 1))
+      e1 = B.ent_base + a;
+  } else if (want1 && zb == (uint64_t)(z0 + 1)) {
+    e1 = B.ent_base + a;
+  }
+}
+
+// The first 16 bytes of an entry (occupied cells, first cell, lo); an empty
+// one for kNoEnt.
+struct EntHead {
+  unsigned long long occ;
+  uint32_t base, lo;
+};
+__device__ __forceinline__ EntHead ent_head(const gdl::Bufs& B, uint32_t e) {
+  EntHead h{0, 0, 0};
+  if (e != kNoEnt) {
+    const uint4 v = *reinterpret_cast<const uint4*>(B.ent + e);
+    h.occ = (unsigned long long)v.y << 32 | v.x;
+    h.base = v.z;
+    h.lo = v.w;
+  }
+  return h;
+}
+// its other half: core cells, hi
+struct EntTail {
+  unsigned long long core;
+  uint32_t hi, uni;
+};
+__device__ __forceinline__ EntTail ent_tail(const gdl::Bufs& B, uint32_t e) {
+  EntTail h{0, 0, 0};
+  if (e != kNoEnt) {
+    const uint4 v = *(reinterpret_cast<const uint4*>(B.ent + e) + 1);
+    h.core = (unsigned long long)v.y << 32 | v.x;
+    h.hi = v.z;
+    h.uni = v.w;
+  }
+  return h;
+}
+
+// index of the occupied cell at `bit` of a block
+__device__ __forceinline__ int ent_cell(unsigned long long occ, uint32_t base, int bit) {
+  return (int)(base + (uint32_t)__popcll(occ & ((1ull << bit) - 1ull)));
+}
+
+// Cell (x, y, z): its index, or -1 when outside the grid or empty (the warp
+// kernels' lookup, one cell per lane).
+template <int D, bool KEY64>
+__device__ __forceinline__ int find_cell(const gdl::Bufs& B, const DevParams& P, int64_t x,
+                                         int64_t y, int64_t z) {
+  constexpr int S = block_shift<D>(), SM = (1 << S) - 1;
+  if (x < 0 || x >= P.G[0] || y < 0 || y >= P.G[1]) return -1;
+  if (D == 3 && (z < 0 || z >= P.G[2])) return -1;
+  const int64_t last = D == 3 ? z : y;
+  const uint64_t row = D == 3 ? (uint64_t)(x >> S) * (unsigned)P.Bk[1] + (uint64_t)(y >> S)
+                              : (uint64_t)(x >> S);
+  uint32_t e0, e1;
+  block_pair<D, KEY64>(B, P, row, (int)(last >> S), true, false, e0, e1);
+  const EntHead h = ent_head(B, e0);
+  const int bit = D == 3 ? (int)((x & SM) << (2 * S) | (y & SM) << S | (z & SM))
+                         : (int)((x & SM) << S | (y & SM));
+  if (!((h.occ >> bit) & 1ull)) return -1;
+  return ent_cell(h.occ, h.base, bit);
 }
 
 // cell range of dimension D: 2D instances' cells come first
@@ -1160,43 +1278,20 @@ __device__ __forceinline__ void dim_range(const gdl::Bufs& B, int64_t& mlo, int6
 }
 
 // ------------------------------------------------------------ stencil tables
-// Offsets within +-2 cells, built at compile time.  kRows: the (ox, oy) rows a
-// core count scans, nearest first (by the smallest possible distance to the
-// row, then by how many axes are off), so that points in dense regions reach
-// minPts in fewer rows.  kHalf[d][pass]: the half stencil (o > 0
-// lexicographically) split into the union passes (union_pass).  kFullSt[d]:
-// all offsets (the warp border search).
+// Offsets within +-2 cells, built at compile time.  kHalf[d][pass]: the half
+// stencil (o > 0 lexicographically) split into the union passes (union_pass).
+// kFullSt[d]: all offsets, nearest first (the warp kernels).
 struct OffTab {
   signed char o[128][3];
   int n;
 };
 
-constexpr int row_rank(int x, int y) {
-  const int ax = x < 0 ? -x : x, ay = y < 0 ? -y : y;
-  const int gx = ax > 1 ? ax - 1 : 0, gy = ay > 1 ? ay - 1 : 0;  // empty cells between
-  return (gx * gx + gy * gy) * 8 + ax + ay;
-}
-
-constexpr OffTab make_rows(int D) {
-  OffTab t{};
-  const int order[5] = {0, -1, 1, -2, 2};
-  for (int a = 0; a < 5; ++a)
-    for (int b = 0; b < (D == 3 ? 5 : 1); ++b) {
-      t.o[t.n][0] = (signed char)order[a];
-      t.o[t.n][1] = (signed char)(D == 3 ? order[b] : 0);
-      t.o[t.n][2] = 0;
-      ++t.n;
-    }
-  // stable insertion sort by row_rank
-  for (int i = 1; i < t.n; ++i)
-    for (int j = i; j > 0 && row_rank(t.o[j][0], t.o[j][1]) < row_rank(t.o[j - 1][0], t.o[j - 1][1]);
-         --j)
-      for (int k = 0; k < 2; ++k) {
-        const signed char v = t.o[j][k];
-        t.o[j][k] = t.o[j - 1][k];
-        t.o[j - 1][k] = v;
-      }
-  return t;
+// by the smallest possible distance between the cells, then by how many axes
+// are off
+constexpr int off_rank(int x, int y, int z) {
+  const int ax = x < 0 ? -x : x, ay = y < 0 ? -y : y, az = z < 0 ? -z : z;
+  const int gx = ax > 1 ? ax - 1 : 0, gy = ay > 1 ? ay - 1 : 0, gz = az > 1 ? az - 1 : 0;
+  return (gx * gx + gy * gy + gz * gz) * 8 + ax + ay + az;
 }
 
 // Union passes over the half stencil, run in order with a compression between
@@ -1208,7 +1303,7 @@ constexpr OffTab make_rows(int D) {
 // separate face pass there cost more than it saved).
 constexpr int kUnionPasses = 3;
 
-constexpr int union_passes(int D) { return D == 3 ? 3 : 2; }
+__host__ __device__ constexpr int union_passes(int D) { return D == 3 ? 3 : 2; }
 
 constexpr int union_pass(int D, int x, int y, int z) {
   const int ax = x < 0 ? -x : x, ay = y < 0 ? -y : y, az = z < 0 ? -z : z;
@@ -1238,99 +1333,110 @@ constexpr OffTab make_half(int D, int pass) {
 constexpr OffTab make_full(int D) {
   OffTab t{};
   const int zr = D == 3 ? 2 : 0;
-  for (int x = -2; x <= 2; ++x)
-    for (int y = -2; y <= 2; ++y)
-      for (int z = -zr; z <= zr; ++z) {
-        t.o[t.n][0] = (signed char)x;
-        t.o[t.n][1] = (signed char)y;
-        t.o[t.n][2] = (signed char)z;
-        ++t.n;
-      }
-  return t;
-}
-
-__constant__ OffTab kRows[2] = {make_rows(2), make_rows(3)};
-// rows per dimension, and the 3D rows within one cell of the own row (the
-// first nine of make_rows(3))
-constexpr int kRowsPerDim[2] = {5, 25};
-constexpr int kNearRows3 = 9;
-static_assert(make_rows(2).n == kRowsPerDim[0] && make_rows(3).n == kRowsPerDim[1], "rows");
-static_assert(row_rank(make_rows(3).o[kNearRows3 - 1][0], make_rows(3).o[kNearRows3 - 1][1]) < 8 &&
-                  row_rank(make_rows(3).o[kNearRows3][0], make_rows(3).o[kNearRows3][1]) >= 8,
-              "the near rows come first");
-__constant__ OffTab kHalf[2][kUnionPasses] = {{make_half(2, 0), make_half(2, 1), make_half(2, 2)},
-                                              {make_half(3, 0), make_half(3, 1), make_half(3, 2)}};
-
-// Per union pass and stencil row (ox, oy; oy = 0 in 2D, whose rows run along
-// the second axis): bit dz + 2 set when the cell at last-axis offset dz is in
-// the half stencil and in that pass.
-struct PassZ {
-  unsigned char m[2][kUnionPasses][5][5];
-};
-
-constexpr PassZ make_pass_z() {
-  PassZ t{};
-  for (int p = 0; p < kUnionPasses; ++p)
+  for (int rank = 0; rank < 40; ++rank)
     for (int x = -2; x <= 2; ++x)
       for (int y = -2; y <= 2; ++y)
-        for (int dz = -2; dz <= 2; ++dz) {
-          if (y == 0 && half_pos(x, dz, 0) && union_pass(2, x, dz, 0) == p)
-            t.m[0][p][x + 2][2] |= (unsigned char)(1u << (dz + 2));
-          if (half_pos(x, y, dz) && union_pass(3, x, y, dz) == p)
-            t.m[1][p][x + 2][y + 2] |= (unsigned char)(1u << (dz + 2));
+        for (int z = -zr; z <= zr; ++z) {
+          if (off_rank(x, y, z) != rank) continue;
+          t.o[t.n][0] = (signed char)x;
+          t.o[t.n][1] = (signed char)y;
+          t.o[t.n][2] = (signed char)z;
+          ++t.n;
         }
   return t;
 }
+static_assert(make_full(2).n == 25 && make_full(3).n == 125, "whole stencils");
 
-__constant__ PassZ kPassZ = make_pass_z();
-__constant__ OffTab kFullSt[2] = {make_full(2), make_full(3)};
+__constant__ OffTab kHalf[2][kUnionPasses] = {{make_half(2, 0), make_half(2, 1), make_half(2, 2)},
+                                              {make_half(3, 0), make_half(3, 1), make_half(3, 2)}};
 
-// Per-warp list of candidate rows: row r holds the points lo[r] .. lo[r]+len,
-// and pre[r] is the exclusive prefix of the lengths (rows concatenated in
-// table order).  Lane r looks its row up, so all lookups are in flight at once.
-struct RowList {
-  int lo[32];
-  int pre[32];
+// Union pass masks by a cell's place in its block and the stencil block (row
+// r = first-axis half [x 2 + second-axis half], last-axis half k: 2 r + k;
+// half 0 is the block of c - 2): the block's cells that are in the pass's half
+// stencil of that cell.
+struct PassMasks {
+  unsigned long long m[kUnionPasses][64][8];
 };
 
-template <int D>
-__device__ __forceinline__ int build_rows(const gdl::Bufs& B, RowList& RL, const GridView& gv,
-                                          const CellXYZ<D>& cc,
-                                          const DevParams& P, int lane) {
-  const OffTab& T = kRows[D - 2];
-  const int64_t Gl = P.G[D - 1];
-  const int64_t cl = cc.c[D - 1];
-  const int64_t l0 = cl - 2 < 0 ? 0 : cl - 2;
-  const int64_t l1 = cl + 2 >= Gl ? Gl - 1 : cl + 2;
-  int lo = 0, len = 0;
-  if (lane < T.n) {
-    int64_t rowkey = offset_key<D>(cc, T.o[lane][0], T.o[lane][1], 0, P);
-    if (rowkey >= 0) {
-      rowkey -= cl;
-      const int2 rg = gv.span(B, (uint64_t)(rowkey + l0), (uint64_t)(rowkey + l1));
-      lo = rg.x;
-      len = rg.y - rg.x;
+constexpr PassMasks make_pass_masks(int D) {
+  PassMasks t{};
+  const int S = D == 2 ? 3 : 2, SIDE = 1 << S, zr = D == 3 ? 2 : 0;
+  for (int lb = 0; lb < 64; ++lb) {
+    const int cx = D == 3 ? lb >> 4 : lb >> 3, cy = D == 3 ? (lb >> 2) & 3 : lb & 7;
+    const int cz = D == 3 ? lb & 3 : 0;
+    for (int x = -2; x <= 2; ++x)
+      for (int y = -2; y <= 2; ++y)
+        for (int z = -zr; z <= zr; ++z) {
+          if (!half_pos(x, y, z)) continue;
+          // cell and stencil block start per axis, shifted by one block to stay >= 0
+          const int X = cx + x + SIDE, Y = cy + y + SIDE, Z = cz + z + SIDE;
+          const int hx = (X >> S) - ((cx - 2 + SIDE) >> S), hy = (Y >> S) - ((cy - 2 + SIDE) >> S);
+          const int hz = D == 3 ? (Z >> S) - ((cz - 2 + SIDE) >> S) : 0;
+          const int in = D == 3 ? (X & 3) << 4 | (Y & 3) << 2 | (Z & 3) : (X & 7) << 3 | (Y & 7);
+          const int blk = D == 3 ? hx * 4 + hy * 2 + hz : hx * 2 + hy;
+          t.m[union_pass(D, x, y, z)][lb][blk] |= 1ull << in;
+        }
+  }
+  return t;
+}
+
+// (global memory: the lanes of a warp read different entries)
+__device__ const PassMasks kPassMasks[2] = {make_pass_masks(2), make_pass_masks(3)};
+__constant__ OffTab kFullSt[2] = {make_full(2), make_full(3)};
+
+// Per-warp list of the stencil's non-empty cells, nearest first: cell r holds
+// the points lo[r] .. lo[r] + len, and pre[r] is the exclusive prefix of the
+// lengths (the cells concatenated).
+struct CellList {
+  int lo[128];
+  int pre[128];
+};
+
+// fills the list (each lane looks up every 32nd stencil cell); returns the
+// points, and the cells in ncells
+template <int D, bool KEY64>
+__device__ __forceinline__ int build_cells(const gdl::Bufs& B, CellList& CL, const CellXYZ<D>& cc,
+                                           const DevParams& P, int lane, int& ncells) {
+  const OffTab& T = kFullSt[D - 2];
+  int total = 0, cells = 0;
+  for (int t0 = 0; t0 < T.n; t0 += 32) {
+    const int t = t0 + lane;
+    int lo = 0, len = 0;
+    if (t < T.n) {
+      const int c = find_cell<D, KEY64>(B, P, (int64_t)cc.c[0] + T.o[t][0],
+                                        (int64_t)cc.c[1] + T.o[t][1], (int64_t)cc.c[2] + T.o[t][2]);
+      if (c >= 0) {
+        lo = B.reps[c];
+        len = B.reps[c + 1] - lo;
+      }
     }
-  }
-  int inc = len;
+    int inc = len;
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    int v = __shfl_up_sync(kFull, inc, o);
-    if (lane >= o) inc += v;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(kFull, inc, o);
+      if (lane >= o) inc += v;
+    }
+    const unsigned has = __ballot_sync(kFull, len > 0);
+    if (len > 0) {
+      const int at = cells + __popc(has & ((1u << lane) - 1u));
+      CL.lo[at] = lo;
+      CL.pre[at] = total + inc - len;
+    }
+    cells += __popc(has);
+    total += __shfl_sync(kFull, inc, 31);
   }
-  RL.lo[lane] = lo;
-  RL.pre[lane] = inc - len;
   __syncwarp();
-  return __shfl_sync(kFull, inc, 31);
+  ncells = cells;
+  return total;
 }
 
 // sorted position of concatenated candidate c (0 <= c < total)
-__device__ __forceinline__ int row_pos(const RowList& RL, int nrows, int c) {
+__device__ __forceinline__ int cell_list_pos(const CellList& CL, int ncells, int c) {
   int r = 0;
 #pragma unroll
-  for (int step = 16; step; step >>= 1)
-    if (r + step < nrows && RL.pre[r + step] <= c) r += step;
-  return RL.lo[r] + (c - RL.pre[r]);
+  for (int step = 64; step; step >>= 1)
+    if (r + step < ncells && CL.pre[r + step] <= c) r += step;
+  return CL.lo[r] + (c - CL.pre[r]);
 }
 
 constexpr int kWarpsPerBlock = 8;
@@ -1399,57 +1505,67 @@ __device__ __forceinline__ int classify(const float* u, int ox, int oy, int oz, 
 // Most work items need little: isolated noise points whose stencil holds fewer
 // than minpts points, cells whose neighbour links are found by the first test,
 // border points with a handful of candidate cores.  The front-end kernels give
-// one thread to each point (k_core_point, k_border_point) or core cell
-// (k_union_scan) and finish those cases inline (bounded work per thread); a
+// one thread to each point, chunk of points (core count, border search) or core
+// cell (union scan) and finish those cases inline (bounded work per thread); a
 // cell that needs more is appended to the heavy list and handled by the
-// warp-cooperative *_heavy kernel that follows.  The stencil is walked row by
-// row (5 rows in 2D, 25 in 3D, own row first); a row is one contiguous range of
-// sorted points, and its non-empty cells are visited through the run structure,
-// so empty cells cost nothing.
+// warp-cooperative *_heavy kernel that follows.  The stencil's 25 or 125 cells come
+// as the occupancy words of 4 or 8 blocks, so empty cells cost nothing.  (Rows of 5
+// cells, each looked up by itself, had cost 5 or 25 lookups per walk, by binary
+// search outside the densest grids.)
 constexpr int kScanThreadsPerBlock = 256;
 // The walk kernels (core count, union scan, border search) take their list
-// entries from a global cursor in batches of kWalkBatch, 32 per pass of a
-// warp: work is handed out as it is done, so no warp is left with a tail of
+// entries from a global cursor in batches of 32 (a union scan over a long list: 64,
+// as its entries are short: C3 union 1.32 ms at 32, 1.30 at 64; a 1M-point 2D
+// expand, whose lists are a few passes long: 0.24 ms core at 64, 0.21 at 32), 32 per
+// pass of a warp: work is handed out as it is done, so no warp is left with a tail of
 // costly entries after the others finish (a static grid-stride split left
 // whole SMs idle behind a few slow warps).
-constexpr int kWalkBatch = 64;
+constexpr int kUnionSmall = 1 << 20;
 struct WalkCursor {
   unsigned long long* c;  // kCtrWalkCursor2/3, zero at launch
   int span;               // list entries of this dimension (< 2^31)
+  int batch;              // entries handed out at a time
   int next, end;          // the warp's batch, relative to its first entry (warp-uniform)
   // the warp's next 32 entries are [next, min(next + 32, end)); false when the
   // list is used up (all lanes call it)
   __device__ __forceinline__ bool advance(int lane) {
     if (next < end) return true;
     unsigned long long got = 0;
-    if (lane == 0) got = atomicAdd(c, (unsigned long long)kWalkBatch);
+    if (lane == 0) got = atomicAdd(c, (unsigned long long)batch);
     got = __shfl_sync(kFull, got, 0);
     if (got >= (unsigned long long)span) return false;
     next = (int)got;
-    end = span - next > kWalkBatch ? next + kWalkBatch : span;
+    end = span - next > batch ? next + batch : span;
     return true;
   }
 };
 template <int D>
-__device__ __forceinline__ WalkCursor walk_cursor(const gdl::Bufs& B, int64_t jlo, int64_t jhi) {
-  return WalkCursor{B.ctr + (D == 2 ? kCtrWalkCursor2 : kCtrWalkCursor3), (int)(jhi - jlo), 0, 0};
+__device__ __forceinline__ WalkCursor walk_cursor(const gdl::Bufs& B, int64_t jlo, int64_t jhi,
+                                               int batch) {
+  return WalkCursor{B.ctr + (D == 2 ? kCtrWalkCursor2 : kCtrWalkCursor3), (int)(jhi - jlo), batch,
+                    0, 0};
 }
 // Resident 256-thread blocks per SM the front-end kernels are compiled for
 // (register budget 65536 / (256 * blocks) per thread).  These kernels are
 // bound by memory latency, so occupancy beats registers; the counts were
 // measured on GB300 (a few spilled bytes cost less than a lost block).
 #ifndef GD_CORE_MIN_BLOCKS
-#define GD_CORE_MIN_BLOCKS 4
+#define GD_CORE_MIN_BLOCKS 8
+#endif
+#ifndef GD_CORE_CELL_MIN_BLOCKS
+#define GD_CORE_CELL_MIN_BLOCKS 8
 #endif
 #ifndef GD_UNION_MIN_BLOCKS
-#define GD_UNION_MIN_BLOCKS 5
+#define GD_UNION_MIN_BLOCKS 6
 #endif
 #ifndef GD_BORDER_MIN_BLOCKS
-#define GD_BORDER_MIN_BLOCKS 4
+#define GD_BORDER_MIN_BLOCKS 8
 #endif
 constexpr int kCoreMinBlocks = GD_CORE_MIN_BLOCKS;
+constexpr int kCoreCellMinBlocks = GD_CORE_CELL_MIN_BLOCKS;
 constexpr int kUnionMinBlocks = GD_UNION_MIN_BLOCKS;
 constexpr int kBorderMinBlocks = GD_BORDER_MIN_BLOCKS;
+constexpr int kBorderThreads = 128;
 // The pair-test budgets of one thread (core count per point, link search per
 // cell pair, border search per point) come with the buffers (Bufs::tn_*): the
 // context sets them, the autotuner varies them.
@@ -1472,51 +1588,85 @@ __device__ __forceinline__ void heavy_push(const gdl::Bufs& B, int slot, bool pu
 }
 
 template <int D, bool F32>
-__device__ __forceinline__ void load_point(double* x, float* f, const gdl::Bufs& B, int64_t n,
-                                           int64_t i, bool prune) {
+__device__ __forceinline__ void load_point(double* x, float* f, const gdl::Bufs& B, int64_t i,
+                                           bool prune) {
   // float32-band mode tests from the float32 copy; the float64 coordinates
   // are loaded by the band re-test itself
-#pragma unroll
-  for (int k = 0; k < D; ++k) {
-    if (!F32) x[k] = B.X[k * n + i];
-    if (F32 || prune) f[k] = B.Xf[k * n + i];
-  }
+  if (!F32) ld_x<D>(B, i, x);
+  if (F32 || prune) ld_f<D>(B, i, f);
 }
 
-// Stencil rows of a cell: row r of kRows, its first cell's local key, and the
-// last-axis cell range [l0, l1] around the cell.
+// The +-2 stencil of a cell over its blocks: per axis the first block, and the
+// cells of the axis as bits counted from that block's first cell (w5: within
+// two, w3: within one); the axis' cells fall into two blocks at most.
 template <int D>
-struct RowWalk {
-  CellXYZ<D> cc;
-  int cl, l0, l1;  // the cell's last-axis index and the stencil's range on that axis
-  __device__ __forceinline__ void init(const CellXYZ<D>& c, const DevParams& P) {
-    cc = c;
-    const int64_t Gl = P.G[D - 1];
-    cl = c.c[D - 1];
-    l0 = cl - 2 < 0 ? 0 : cl - 2;
-    l1 = (int64_t)cl + 2 >= Gl ? (int)(Gl - 1) : cl + 2;
+struct Stencil {
+  static constexpr int S = block_shift<D>(), SIDE = 1 << S, ROWS = D == 3 ? 4 : 2;
+  int b0[D];
+  uint32_t w5[D];
+  __device__ __forceinline__ void init(const CellXYZ<D>& cc) {
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
+      b0[k] = (cc.c[k] - 2) >> S;
+      w5[k] = 31u << ((cc.c[k] - 2) & (SIDE - 1));
+    }
   }
-  // local key of row r's first cell, or -1 when the row is outside the grid
-  __device__ __forceinline__ int64_t rowkey(const OffTab& T, int r, const DevParams& P) const {
-    const int64_t k = offset_key<D>(cc, T.o[r][0], T.o[r][1], 0, P);
-    return k < 0 ? k : k - cl;
+  // offset of the first cell of axis k's first block from the cell
+  __device__ __forceinline__ int off0(const CellXYZ<D>& cc, int k) const {
+    return (int)((unsigned)b0[k] << S) - cc.c[k];
   }
-  // index of row r among the grid's rows (its first cell's key is index * G[D-1]),
-  // or -1 when the row is outside the grid
-  __device__ __forceinline__ int64_t rowidx(const OffTab& T, int r, const DevParams& P) const {
-    const int64_t x = (int64_t)cc.c[0] + T.o[r][0];
-    if (x < 0 || x >= P.G[0]) return -1;
-    if (D == 2) return x;
-    const int64_t y = (int64_t)cc.c[1] + T.o[r][1];
-    if (y < 0 || y >= P.G[1]) return -1;
-    return x * P.G[1] + y;
+  static __device__ __forceinline__ uint32_t part(uint32_t w, int i) {
+    return i ? w >> SIDE : w & ((1u << SIDE) - 1u);
+  }
+  // block row r: its index among the grid's block rows, or -1 outside the grid
+  __device__ __forceinline__ int64_t row(int r, const DevParams& P) const {
+    const int bx = b0[0] + (D == 3 ? r >> 1 : r);
+    if (bx < 0 || bx >= P.Bk[0]) return -1;
+    if (D == 2) return bx;
+    const int by = b0[1] + (r & 1);
+    if (by < 0 || by >= P.Bk[1]) return -1;
+    return (int64_t)bx * P.Bk[1] + by;
+  }
+  // place along axis k of the cell at `bit` of a block
+  static __device__ __forceinline__ int bit_off(int bit, int k) {
+    return k == 0 ? bit >> (D == 3 ? 2 * S : S) : (D == 3 && k == 1 ? (bit >> S) & (SIDE - 1)
+                                                                    : bit & (SIDE - 1));
   }
 };
 
-// next cell of a row walk: [q, end), its last-axis offset from the cell in work
-template <bool KEY64>
-__device__ __forceinline__ int cell_end(const gdl::Bufs& B, int q) {
-  return B.reps[cell_of(B, q) + 1];
+// Masks of the stencil's blocks from per-axis cell sets (Stencil::w5 or a part of
+// it): an axis' cells as words of a block mask, for each half of the axis.  The
+// middle (3D) and the last axis repeat in both words.
+template <int D>
+struct StencilWords {
+  using St = Stencil<D>;
+  uint32_t xl[2], xh[2], y[2], z[2];
+  static __device__ __forceinline__ uint32_t first(uint32_t m) {  // half of the axis: one word
+    return D == 3 ? (m & 1u) * 0xffffu | ((m >> 1) & 1u) * 0xffff0000u
+                  : ((m | m << 7 | m << 14 | m << 21) & 0x01010101u) * 255u;
+  }
+  __device__ __forceinline__ void init(const uint32_t* w) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const uint32_t px = St::part(w[0], i), pz = St::part(w[D - 1], i);
+      xl[i] = first(px & ((1u << (St::SIDE / 2)) - 1u));
+      xh[i] = first(px >> (St::SIDE / 2));
+      const uint32_t py = D == 3 ? St::part(w[1], i) : 0u;
+      y[i] = D == 3 ? ((py | py << 3 | py << 6 | py << 9) & 0x1111u) * 15u * 0x10001u : ~0u;
+      z[i] = pz * (D == 3 ? 0x11111111u : 0x01010101u);
+    }
+  }
+  // masks of row r's two blocks
+  __device__ __forceinline__ void row(int r, uint2& m0, uint2& m1) const {
+    const int ri = D == 3 ? r >> 1 : r;
+    const uint32_t a = ri ? xl[1] : xl[0], b = ri ? xh[1] : xh[0];
+    const uint32_t c = D == 3 ? ((r & 1) ? y[1] : y[0]) : ~0u;
+    m0 = make_uint2(a & c & z[0], b & c & z[0]);
+    m1 = make_uint2(a & c & z[1], b & c & z[1]);
+  }
+};
+__device__ __forceinline__ unsigned long long u64_of(uint2 v) {
+  return (unsigned long long)v.y << 32 | v.x;
 }
 
 // Squared largest / smallest distance (plus / minus the position error) along
@@ -1531,40 +1681,33 @@ __device__ __forceinline__ void axis_terms(float a, int o, const PP& P, float& m
   mn2 = mn * mn;
 }
 
-// undecided cells a point queues before testing them (float64 mode): float64
-// tests are costly off the warp-cooperative final flush, and the 3D walks meet
-// more undecided cells.  Float32 tests are cheap enough that testing each
-// undecided cell at once, with the early exit it allows, wins: that mode keeps
-// no queue (lengths measured on GB300).
-__host__ __device__ constexpr int core_queue(int d, bool f32) {
-  return f32 ? 1 : (d == 2 ? 16 : 24);
-}
-constexpr int kCoreWarps = kScanThreadsPerBlock / 32;
-
-// Per-warp staging of the final flush (float64 mode): the points whose core
-// decision waits on their queued cells, with their instances (lanes of one
-// warp may belong to different instances; the predicate constants are read
-// from Pv).
-template <int D, bool F32>
-struct CoreFlushStage {
-  double x[32][D];
-  float f[32][D];
-  int inst[32];
-  int cnt[32];    // neighbours counted so far
-  int incl[32];   // inclusive prefix of the queued candidate counts
-  int nq[32];
-};
+// Axes whose slab distance terms a float64 core walk keeps in shared memory (the
+// 3D walk forms the others again).
+__host__ __device__ constexpr int core_axes(int d) { return d == 3 ? 1 : d; }
+constexpr int kCoreThreads = 128;
+constexpr int kCoreWarps = kCoreThreads / 32;
 
 // Core flags of points in dense cells (at least minpts points: all core, no
 // test), with their cells' core counts and smallest core indices.  Every other
 // point gets its bit in the walk list's mask (listed in sorted order
 // afterwards), so that k_core_point's warps hold only neighbouring points that
 // walk.  ONE: a single instance (its parameters are Pv[0]).
+// chunk: points per walk list entry (1, or k_core_cell's chunk).
 template <bool KEY64, bool ONE>
-__global__ void k_core_split(const gdl::Bufs B, int64_t n) {
+__global__ void k_core_split(const gdl::Bufs B, int64_t n, int chunk, int clear) {
   const int LB = B.Bi->LB;
   const int lane = threadIdx.x & 31;
   unsigned long long dense = 0;
+  // a later expand of the index: the blocks' words start empty again (their link
+  // words do already)
+  const int64_t NBk = clear ? (int64_t)B.ctr[kCtrBlocks] : 0;
+  for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < NBk;
+       j += (int64_t)gridDim.x * blockDim.x) {
+    BlockEnt& E = B.ent[B.cellent[B.blklist[j]]];
+    E.lo = kNoEnt;
+    E.core = 0;
+    E.hi = kNoEnt;
+  }
   // two groups of 32 points per warp and pass, their loads issued together
   constexpr int U = 2;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -1595,8 +1738,8 @@ __global__ void k_core_split(const gdl::Bufs B, int64_t n) {
         B.core[i] = 1;
         if (i == b[u]) ++dense;
       }
-      // the walk list: every point outside a dense cell
-      const unsigned wl = __ballot_sync(kFull, i < n && !dn);
+      // the walk list: the chunk starts among the points outside dense cells
+      const unsigned wl = __ballot_sync(kFull, i < n && !dn && ((int)i - b[u]) % chunk == 0);
       if (lane == 0) B.lbits[i0 >> 5] = wl;
       const unsigned cm = __ballot_sync(kFull, dn);
       const unsigned grp = run_peers(cm, m[u]);
@@ -1614,48 +1757,41 @@ __global__ void k_core_split(const gdl::Bufs B, int64_t n) {
   if (lane == 0 && dense) atomicAdd(B.ctr + kCtrDenseCells, dense);
 }
 
-// Core flags of the listed points (those outside dense cells, in sorted
-// order), one thread per point; warps take the list from the walk cursor.
-// Neighbouring lanes hold neighbouring sorted points, mostly of one cell, so
-// they walk the same stencil rows in step: their loads coincide and their
-// branches agree.  The walk goes row by row, own row first: with cell
-// classification, rows and cells wholly inside eps count without tests, those
-// wholly outside are skipped.  The classification's per-axis terms are formed
-// per row for the fixed axes and per point for the last axis (five pairs in
-// per-thread shared memory).  An undecided cell is tested at once in float32
-// mode.  In float64 mode undecided cells are queued (shared memory); a full
-// queue is tested by its own thread, and what is queued when the walk ends is
-// tested by the whole warp together: the lanes whose decision depends on their
-// queue pool its candidates and every lane tests one candidate per round (one
-// owner's point against one queued point), so the float64 tests run on full
-// warps, and owners stop consuming once they reach minpts.  A point whose
-// tests pass the budget (or a warp whose pooled candidates pass 32 budgets)
-// sends its cell to the warp kernel, which recomputes the whole cell.
-// Per-cell core counts and smallest core indices are warp-aggregated atomics
-// (cleared before the launch).
+// Core flags of the points outside dense cells, float32-band mode: a thread per
+// chunk of up to kCoreChunk consecutive points of one cell, taken from the walk
+// list (chunk starts, in sorted order) through the walk cursor.  The chunk shares
+// one stencil walk: the stencil comes as a few 64-cell occupancy words (4 block
+// lookups in 2D, 8 in 3D, two at a time; home row first), masked to the cells
+// within one (pass 0) and then two (pass 1) of the own cell, whose points count at
+// once; slabs and cells out of reach of the chunk's bounding box leave the walk.
+// Every candidate of an occupied cell is loaded once and tested against all the
+// chunk's points in registers -- a float32 test is about nine instructions, less
+// than the steps that reach a candidate, so sharing those pays more than any
+// finer rule on what to test.  Only cells of more than kCoreBigCell points are
+// classified per point first (wholly inside eps: count, wholly outside: skip).
+// A chunk whose tests pass the budget sends its cell to the warp kernel, which
+// recomputes the whole cell.  Per-cell core counts and smallest core indices are
+// warp-aggregated atomics (cleared before the launch).
 //
-// Rows [r0, r1) of the stencil.  A walk split in two (3D) first takes the 3x3
-// near rows for every listed point (r1 < rows): a point still undecided after
-// them keeps its count in lab[] and its bit in fbits, and the second launch
-// (r0 > 0) walks the remaining rows for that compacted list only.  Most points
-// decide within the near rows, so the second launch's warps hold only the
-// points that need the long walk instead of idling beside them (C3: a warp
-// ran 13.4 rows where its lanes needed 6.2 on average).
-template <int D, bool F32, bool KEY64>
-__global__ void __launch_bounds__(kScanThreadsPerBlock, kCoreMinBlocks)
-k_core_point(const gdl::Bufs B, int64_t n, int r0, int r1) {
-  __shared__ int2 sq[core_queue(D, F32)][kScanThreadsPerBlock];
-  // per thread: squared largest / smallest distance terms to the five cell
-  // slabs along the last axis (offsets -2..2), kept out of registers
-  __shared__ float2 slt[5][kScanThreadsPerBlock];
-  __shared__ CoreFlushStage<D, F32> stage[F32 ? 1 : kCoreWarps];
-  const OffTab& T = kRows[D - 2];
+// Passes [p0, p1).  3D runs pass 0 for every listed chunk first: a chunk with an
+// undecided point keeps its points' counts in lab[] (kDecided for decided ones)
+// and its bit in fbits, and a second launch runs pass 1 for that compacted list
+// only, so that its warps hold only chunks that need the long walk.
+#ifndef GD_CORE_CHUNK
+#define GD_CORE_CHUNK 2
+#endif
+constexpr int kCoreChunk = GD_CORE_CHUNK;
+constexpr int kCoreBigCell = 8;
+constexpr int kDecided = 0x3fffffff;
+template <int D, bool KEY64>
+__global__ void __launch_bounds__(kCoreThreads, kCoreCellMinBlocks)
+k_core_cell(const gdl::Bufs B, int64_t n, int p0, int p1) {
+  using St = Stencil<D>;
+  constexpr int C = kCoreChunk;
   const int lane = threadIdx.x & 31;
-  const int wbase = threadIdx.x & ~31;
-  CoreFlushStage<D, F32>& S = stage[F32 ? 0 : threadIdx.x >> 5];
   const int LB = B.Bi->LB;
-  const bool second = r0 > 0;    // the list and counts of a first launch
-  const bool split = r1 < T.n;   // a second launch follows
+  const bool second = p0 > 0;    // the list and counts of a first launch
+  const bool split = p1 < 2;     // a second launch follows
   // this dimension's part of the walk list: 2D instances' points come first
   const int64_t p3 = B.reps[(int64_t)B.ctr[kCtrCells2D]];
   const int64_t L = (int64_t)*B.lcount;
@@ -1663,217 +1799,475 @@ k_core_point(const gdl::Bufs B, int64_t n, int r0, int r1) {
       p3 < n ? (int64_t)(second ? bit_rank(B.fbits, B.fpre, p3) : bit_rank(B.lbits, B.lpre, p3))
              : L;
   const int64_t jlo = D == 2 ? 0 : L2, jhi = D == 2 ? L2 : L;
-  WalkCursor wc = walk_cursor<D>(B, jlo, jhi);
+  WalkCursor wc = walk_cursor<D>(B, jlo, jhi, 32);
   Tally t;
   while (wc.advance(lane)) {
     const int64_t j = jlo + wc.next + lane;
     const bool valid = wc.next + lane < wc.end;
     wc.next += 32;
     const int64_t i = valid ? (int64_t)B.blist[j] : 0;
-    int m = -1, b = 0;
-    bool isc = false, over = false, pend = false;
-    int cnt = 0, nq = 0, minpts = 0;
-    if (valid && second) cnt = B.lab[i];
+    int m = -1, na = 0, minpts = 0;
+    bool over = false;
+    int cnt[C];
+    uint32_t was = 0;  // points decided by the first launch
     if (valid) {
       m = cell_of(B, i);
-      b = B.reps[m];
-      const CellCtx cx = cell_ctx<KEY64>(B, b, LB);
+      const int b = B.reps[m], e = B.reps[m + 1];
+      na = min(C, e - (int)i);
+      const CellCtx cx = cell_ctx<KEY64>(B, m, LB);
       const DevParams& P = *cx.P;
       const PredParams Q = pred_params(P);
       minpts = Q.minpts;
-      {
-        const GridView gv = view_of(B, P);
-        const bool prune = Q.prune != 0;
-        RowWalk<D> rw;
-        rw.init(decompose<D>(cx.local, P), P);
-        double px[D];
-        float pf[D];
-        load_point<D, F32>(px, pf, B, n, i, prune);
-        float u[D];
+      const bool prune = Q.prune != 0;
+      const CellXYZ<D> cc = decompose<D>(cx.local, P);
+      St st;
+      st.init(cc);
+      // the chunk's points; absent ones repeat the first and count as decided
+      float pf[C][D];
+      int present = 0;
+#pragma unroll
+      for (int a = 0; a < C; ++a) {
+        const int64_t ia = a < na ? i + a : i;
+        ld_f<D>(B, ia, pf[a]);
+        cnt[a] = a < na ? (second ? B.lab[ia] : e - b) : kDecided;
+        if (a < na && second && cnt[a] == kDecided) was |= 1u << a;
+        present += cnt[a] < minpts;
+      }
+      float o[D], ulo[D], uhi[D];  // cell origin, the undecided points' bounds in the cell
+      if (prune) {
+        cell_origin32<D>(cc, P, o);
+#pragma unroll
+        for (int k = 0; k < D; ++k) {
+          float lo = INFINITY, hi = -INFINITY;
+#pragma unroll
+          for (int a = 0; a < C; ++a)
+            if (cnt[a] < minpts) {
+              lo = fminf(lo, pf[a][k]);
+              hi = fmaxf(hi, pf[a][k]);
+            }
+          ulo[k] = __fmul_rn(__fsub_rn(lo, o[k]), Q.inv_f32) - Q.uerr;
+          uhi[k] = __fmul_rn(__fsub_rn(hi, o[k]), Q.inv_f32) + Q.uerr;
+          uint32_t near = 14u;
+          const float l2 = ulo[k] + 1.0f, h2 = 2.0f - uhi[k];  // to the slabs at -2 and +2
+          if (!(l2 > 0.0f && l2 * l2 >= Q.thr_out)) near |= 1u;
+          if (!(h2 > 0.0f && h2 * h2 >= Q.thr_out)) near |= 16u;
+          st.w5[k] = near << ((cc.c[k] - 2) & (St::SIDE - 1));
+        }
+      }
+      int budget = B.tn_core * present;
+      bool done = present == 0;
+      // one occupied cell: place `bit` of block (row r, half h) of the stencil
+      auto visit = [&](int c, int bit, int r, int h) {
+        int off[3] = {0, 0, 0};
+#pragma unroll
+        for (int k = 0; k < D; ++k) {
+          const int half = k == D - 1 ? h : (D == 3 ? (k == 0 ? r >> 1 : r & 1) : r);
+          off[k] = st.off0(cc, k) + (half << St::S) + St::bit_off(bit, k);
+        }
         if (prune) {
-          float o[D];
-          cell_origin32<D>(rw.cc, P, o);
-          frac_pos<D>(pf, o, Q, u);
+          float smin = 0.0f;
+#pragma unroll
+          for (int k = 0; k < D; ++k) {
+            const float d = (float)off[k];
+            const float mn = fmaxf(fmaxf(d - uhi[k], ulo[k] - 1.0f - d), 0.0f);
+            smin = fmaf(mn, mn, smin);
+          }
+          if (smin >= Q.thr_out) return;
+        }
+        const int q0 = B.reps[c], qe = B.reps[c + 1];
+        if (prune && qe - q0 > kCoreBigCell) {
+          int cl[C];
+          bool open = false;
+#pragma unroll
+          for (int a = 0; a < C; ++a) {
+            cl[a] = -1;
+            if (cnt[a] < minpts) {
+              float u[D];
+              frac_pos<D>(pf[a], o, Q, u);
+              cl[a] = classify<D>(u, off[0], off[1], off[2], Q);
+              open |= cl[a] == 0;
+            }
+          }
+          if (!open) {
+#pragma unroll
+            for (int a = 0; a < C; ++a)
+              if (cl[a] > 0) cnt[a] += qe - q0;
+            done = true;
+#pragma unroll
+            for (int a = 0; a < C; ++a) done = done && cnt[a] >= minpts;
+            return;
+          }
+        }
+        for (int q = q0; q < qe; ++q) {
+          budget -= present;
+          if (budget < 0) {
+            over = true;
+            done = true;
+            return;
+          }
+          float f[D];
+          ld_f<D>(B, q, f);
+          bool band = false;
+#pragma unroll
+          for (int a = 0; a < C; ++a) {
+            const float s2 = dist2_f32<D>(pf[a], f);
+            const bool in = s2 < Q.eps2_lo32;
+            cnt[a] += in ? 1 : 0;
+            band |= !in && !(s2 > Q.eps2_hi32);
+          }
+          if (band) {
+            // the float64 predicate for the points whose float32 test cannot say
+            double qx[D];
+            exact_x<D>(B, P, q, qx);
+#pragma unroll
+            for (int a = 0; a < C; ++a) {
+              if (a >= na) continue;
+              const float s2 = dist2_f32<D>(pf[a], f);
+              if (s2 < Q.eps2_lo32 || s2 > Q.eps2_hi32) continue;
+              double px[D];
+              exact_x<D>(B, P, i + a, px);
+              ++t.band;
+              ++t.t64;
+              cnt[a] += pred_from_d2<D>(dist2_f64<D>(px, qx), px, qx, Q) ? 1 : 0;
+            }
+          }
+        }
+        t.t32 += present * (qe - q0);
+        done = true;
+#pragma unroll
+        for (int a = 0; a < C; ++a) done = done && cnt[a] >= minpts;
+      };
+      // the own block's row and half first
+      const int hz = (cc.c[D - 1] >> St::S) - st.b0[D - 1];
+      const int home = D == 3 ? ((cc.c[0] >> St::S) - st.b0[0]) * 2 + (cc.c[1] >> St::S) - st.b0[1]
+                              : (cc.c[0] >> St::S) - st.b0[0];
+      for (int ps = p0; ps < p1 && !done; ++ps) {
+        StencilWords<D> W5, W3;
+        {
+          uint32_t w3[D];
+#pragma unroll
+          for (int k = 0; k < D; ++k) w3[k] = st.w5[k] & (14u << ((cc.c[k] - 2) & (St::SIDE - 1)));
+          W3.init(w3);
+          if (ps > 0) W5.init(st.w5);
+        }
+        for (int tt = 0; tt < St::ROWS && !done; ++tt) {
+          const int r = tt ^ home;
+          const int64_t row = st.row(r, P);
+          if (row < 0) continue;
+          uint2 m0, m1;
+          W3.row(r, m0, m1);
+          if (ps > 0) {
+            uint2 f0, f1;
+            W5.row(r, f0, f1);
+            m0 = make_uint2(f0.x & ~m0.x, f0.y & ~m0.y);
+            m1 = make_uint2(f1.x & ~m1.x, f1.y & ~m1.y);
+          }
+          unsigned long long M0 = u64_of(m0), M1 = u64_of(m1);
+          if (ps == 0 && tt == 0) {
+            // the own cell is counted already
+            const unsigned long long own = ~(1ull << (cx.local & 63));
+            if (hz == 0) M0 &= own;
+            else M1 &= own;
+          }
+          uint32_t e0, e1;
+          block_pair<D, KEY64>(B, P, (uint64_t)row, st.b0[D - 1], M0 != 0, M1 != 0, e0, e1);
+          EntHead a = ent_head(B, e0);
+          const EntHead a1 = ent_head(B, e1);
+          unsigned long long w = a.occ & M0, wn = a1.occ & M1;
+          int h = 0;
+          while (!done) {
+            if (!w) {
+              if (!wn) break;
+              w = wn;
+              wn = 0;
+              a = a1;
+              h = 1;
+            }
+            const int bit = __ffsll((long long)w) - 1;
+            w &= w - 1;
+            visit(ent_cell(a.occ, a.base, bit), bit, r, h);
+          }
+        }
+      }
+    }
+    // results: core flags; in a first launch the undecided chunks go on
+    int ncore = 0;
+    unsigned mn = 0xffffffffu;
+    if (valid && !over) {
+      bool go_on = false;
+#pragma unroll
+      for (int a = 0; a < C; ++a) {
+        if (a >= na || ((was >> a) & 1u)) continue;
+        const bool isc = cnt[a] >= minpts;
+        if (split) {
+          B.lab[i + a] = isc ? kDecided : cnt[a];
+          go_on |= !isc;
+        }
+        if (isc || !split) B.core[i + a] = isc ? 1 : 0;
+        if (isc) {
+          ++ncore;
+          mn = min(mn, B.ids[i + a]);
+        }
+      }
+      if (go_on) atomicOr(B.fbits + (i >> 5), 1u << (i & 31));
+    }
+    // per-cell core count and smallest core index, one atomic pair per cell
+    // and warp
+    const unsigned cm = __ballot_sync(kFull, ncore > 0);
+    const unsigned grp = run_peers(cm, m);
+    if (ncore > 0) {
+      const unsigned mm = __reduce_min_sync(grp, mn);
+      const unsigned nn = __reduce_add_sync(grp, (unsigned)ncore);
+      if (lane == __ffs(grp) - 1) {
+        atomicAdd(B.cellcore + m, (int)nn);
+        atomicMin(reinterpret_cast<unsigned*>(B.cellmin) + m, mm);
+      }
+    }
+    // cells with an undecided chunk, once per warp
+    const unsigned om = __ballot_sync(kFull, over);
+    bool lead = false;
+    if (over) lead = lane == __ffs(__match_any_sync(om, m)) - 1;
+    heavy_push(B, kCtrHeavyCore, lead, m, 0);
+  }
+  flush_tally(t, B.ctr);
+}
+
+// Core flags of the points outside dense cells, float64 mode: a thread per listed
+// point, warps taking the list from the walk cursor.  A float64 test occupies
+// this GPU's narrow float64 pipe for a whole warp slot however few lanes take
+// part, so tests are made only on full warps, and only for points they can
+// decide.  First every point classifies its stencil's occupied cells (same block
+// words as k_core_cell, no float64): wholly inside eps they count, wholly outside
+// they are dropped, the rest stay as bits of their block's word.  A point whose
+// undecided cells cannot lift its count to minpts is no core point, untested.
+// Then the warp pools: each lane hands out its open candidates one at a time into
+// the warp's pair buffer until its count reaches minpts, and whenever the buffer
+// holds 32 pairs the warp tests them, a lane per pair.  A warp whose open
+// candidates pass 32 budgets sends its cells to the warp kernel.
+// Passes as in k_core_cell (2D: both in one walk).
+// a lane's open candidates are counted up to this many (32 lanes' sum fits an int)
+constexpr int kPoolCap = 0x03ffffff;
+template <int D>
+struct PairStage {
+  double x[32][D];
+  double e2in[32], e2[32];
+  int inst[32];
+  int cnt[32];     // hits among the tested pairs
+  int q[64];       // pair buffer: candidate, owner lane
+  int own[64];
+};
+template <int D, bool KEY64>
+__global__ void __launch_bounds__(kCoreThreads, kCoreMinBlocks)
+k_core_point(const gdl::Bufs B, int64_t n, int p0, int p1) {
+  using St = Stencil<D>;
+  constexpr int AX = core_axes(D);
+  // per thread and axis (the last AX): squared largest / smallest distance terms
+  // to the five cell slabs at offsets -2..2
+  __shared__ float2 slt[AX][5][kCoreThreads];
+  // the blocks with undecided cells (their bits, the entry)
+  __shared__ unsigned long long siw[2 * St::ROWS][kCoreThreads];
+  __shared__ uint32_t sie[2 * St::ROWS][kCoreThreads];
+  __shared__ PairStage<D> stage[kCoreWarps];
+  const int lane = threadIdx.x & 31;
+  PairStage<D>& S = stage[threadIdx.x >> 5];
+  const int LB = B.Bi->LB;
+  const bool second = p0 > 0;    // the list and counts of a first launch
+  const bool split = p1 < 2;     // a second launch follows
+  // this dimension's part of the walk list: 2D instances' points come first
+  const int64_t p3 = B.reps[(int64_t)B.ctr[kCtrCells2D]];
+  const int64_t L = (int64_t)*B.lcount;
+  const int64_t L2 =
+      p3 < n ? (int64_t)(second ? bit_rank(B.fbits, B.fpre, p3) : bit_rank(B.lbits, B.lpre, p3))
+             : L;
+  const int64_t jlo = D == 2 ? 0 : L2, jhi = D == 2 ? L2 : L;
+  WalkCursor wc = walk_cursor<D>(B, jlo, jhi, 32);
+  Tally t;
+  while (wc.advance(lane)) {
+    const int64_t j = jlo + wc.next + lane;
+    const bool valid = wc.next + lane < wc.end;
+    wc.next += 32;
+    const int64_t i = valid ? (int64_t)B.blist[j] : 0;
+    int m = -1;
+    int cnt = 0, ptot = 0, ni = 0, minpts = 0;
+    if (valid) {
+      m = cell_of(B, i);
+      const CellCtx cx = cell_ctx<KEY64>(B, m, LB);
+      const DevParams& P = *cx.P;
+      const PredParams Q = pred_params(P);
+      minpts = Q.minpts;
+      cnt = second ? B.lab[i] : B.reps[m + 1] - B.reps[m];
+      const bool prune = Q.prune != 0;
+      const CellXYZ<D> cc = decompose<D>(cx.local, P);
+      St st;
+      st.init(cc);
+      double px[D];
+      float pf[D], u[D];
+      load_point<D, false>(px, pf, B, i, prune);
+#pragma unroll
+      for (int k = 0; k < D; ++k) S.x[lane][k] = px[k];
+      S.e2in[lane] = Q.eps2_in;
+      S.e2[lane] = Q.eps2;
+      S.inst[lane] = P.inst;
+      if (prune) {
+        float o[D];
+        cell_origin32<D>(cc, P, o);
+        frac_pos<D>(pf, o, Q, u);
+#pragma unroll
+        for (int k = 0; k < D; ++k) {
+          uint32_t near = 0;
 #pragma unroll
           for (int j = 0; j < 5; ++j) {
             float a2, b2;
-            axis_terms(u[D - 1], j - 2, Q, a2, b2);
-            slt[j][threadIdx.x] = make_float2(a2, b2);
+            axis_terms(u[k], j - 2, Q, a2, b2);
+            if (k >= D - AX) slt[k - (D - AX)][j][threadIdx.x] = make_float2(a2, b2);
+            if (b2 < Q.thr_out) near |= 1u << j;  // the slab is not beyond eps by itself
           }
+          st.w5[k] = near << ((cc.c[k] - 2) & (St::SIDE - 1));
         }
-        int ptot = 0, budget = B.tn_core;
-        // test the points [q, qe) of one cell until the count reaches minpts
-        auto test_cell = [&](int q, int qe) {
-          for (int qq = q; qq < qe && cnt < Q.minpts; ++qq) {
-            if (budget-- == 0) {
-              over = true;
-              break;
-            }
-            Cand<D, F32> cd;
-            load_cand<D, F32>(cd, B.X, B.Xf, n, qq);
-            cnt += pair_test<D, F32>(px, pf, cd, B.X, n, qq, i, true, Q, t) ? 1 : 0;
-          }
-        };
-        auto flush = [&](void) {
-          for (int j = 0; j < nq && cnt < Q.minpts && !over; ++j) {
-            const int2 c = sq[j][threadIdx.x];
-            test_cell(c.x, c.y);
-          }
-          nq = 0;
-          ptot = 0;
-        };
-        for (int r = r0; r < r1 && cnt < Q.minpts && !over; ++r) {
-          float rmx = 0.0f, rmn = 0.0f;
-          if (prune) {
+      }
+      // cells of this launch: within one (split), the others (second), or all
+      StencilWords<D> W5, W3;
+      {
+        uint32_t w3[D];
 #pragma unroll
-            for (int k = 0; k < D - 1; ++k) {
-              float a2, b2;
-              axis_terms(u[k], (int)T.o[r][k], Q, a2, b2);
-              rmx += a2;
-              rmn += b2;
-            }
-            if (rmn >= Q.thr_out) continue;  // the whole row is beyond eps
-          }
-          const int64_t ri = rw.rowidx(T, r, P);
-          if (ri < 0) continue;
-          const int64_t rk = ri * P.G[D - 1];  // key of the row's first cell
-          // one non-empty cell [q, qe) at last-axis offset d from the point's cell
-          auto visit = [&](int q, int qe, int d) {
+        for (int k = 0; k < D; ++k) w3[k] = st.w5[k] & (14u << ((cc.c[k] - 2) & (St::SIDE - 1)));
+        W3.init(w3);
+        W5.init(st.w5);
+      }
+      const unsigned long long own = 1ull << (cx.local & 63);
+      const int home = D == 3 ? ((cc.c[0] >> St::S) - st.b0[0]) * 2 + (cc.c[1] >> St::S) - st.b0[1]
+                              : (cc.c[0] >> St::S) - st.b0[0];
+      const int hz = (cc.c[D - 1] >> St::S) - st.b0[D - 1];
+      for (int tt = 0; tt < St::ROWS && cnt < minpts; ++tt) {
+        const int r = tt ^ home;
+        const int64_t row = st.row(r, P);
+        if (row < 0) continue;
+        uint2 a[2], f[2];
+        W3.row(r, a[0], a[1]);
+        W5.row(r, f[0], f[1]);
+        unsigned long long M[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          M[h] = split ? u64_of(a[h]) : (second ? u64_of(f[h]) & ~u64_of(a[h]) : u64_of(f[h]));
+          if (tt == 0 && h == hz) M[h] &= ~own;  // the own cell is counted already
+        }
+        uint32_t e[2];
+        block_pair<D, KEY64>(B, P, (uint64_t)row, st.b0[D - 1], M[0] != 0, M[1] != 0, e[0], e[1]);
+        EntHead hd[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) hd[h] = ent_head(B, e[h]);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          unsigned long long w = hd[h].occ & M[h], open = 0;
+          while (w) {
+            const int bit = __ffsll((long long)w) - 1;
+            w &= w - 1;
             int cls = 0;
             if (prune) {
-              const float2 lt = slt[d + 2][threadIdx.x];
-              const float smax = rmx + lt.x, smin = rmn + lt.y;
+              float smax = 0.0f, smin = 0.0f;
+#pragma unroll
+              for (int k = 0; k < D; ++k) {
+                const int half = k == D - 1 ? h : (D == 3 ? (k == 0 ? r >> 1 : r & 1) : r);
+                const int j = st.off0(cc, k) + 2 + (half << St::S) + St::bit_off(bit, k);
+                float2 lt;
+                if (k >= D - AX) lt = slt[k - (D - AX)][j][threadIdx.x];
+                else axis_terms(u[k], j - 2, Q, lt.x, lt.y);
+                smax += lt.x;
+                smin += lt.y;
+              }
               cls = smax <= Q.thr_in ? 1 : (smin >= Q.thr_out ? -1 : 0);
             }
+            if (cls < 0) continue;
+            const int c = ent_cell(hd[h].occ, hd[h].base, bit);
+            const int len = B.reps[c + 1] - B.reps[c];
             if (cls > 0) {
-              cnt += qe - q;
-            } else if (cls == 0) {
-              if constexpr (F32) {
-                test_cell(q, qe);
-              } else {
-                if (nq == core_queue(D, F32)) flush();
-                sq[nq][threadIdx.x] = make_int2(q, qe);
-                ++nq;
-                ptot += qe - q;
-              }
+              cnt += len;
+            } else {
+              open |= 1ull << bit;
+              ptot = min(ptot + min(len, kPoolCap), kPoolCap);
             }
-          };
-          if (gv.sparse == 0) {
-            // cell table: the row's occupied cells from its occupancy bits
-            int64_t rr = 0;
-            uint32_t mask = gv.occ_cells(B, (uint64_t)rk, rw.l0, rw.l1, rr);
-            while (mask && cnt < Q.minpts && !over) {
-              const int z = __ffs(mask) - 1;
-              mask &= mask - 1;
-              visit(B.reps[rr], B.reps[rr + 1], (int)(rw.l0 + z - rw.cl));
-              ++rr;
-            }
-            continue;
           }
-          if (gv.sparse == 2) {
-            // row table: the row's cells from the first at or after l0 to l1
-            const int2 rc = gv.row_cells(B, (uint64_t)ri);
-            for (int mq = gv.zlower(B, rc.x, rc.y, rw.l0); mq < rc.y && cnt < Q.minpts && !over;
-                 ++mq) {
-              const int64_t z = B.cellz[mq];
-              if (z > rw.l1) break;
-              visit(B.reps[mq], B.reps[mq + 1], (int)(z - rw.cl));
-            }
-            continue;
-          }
-          // hash: the row's points, from the first cell at or after l0 to the
-          // first beyond l1
-          const int2 rp = gv.row(B, (uint64_t)rk);
-          if (rp.x == rp.y) continue;
-          const int dmax = (int)(rw.l1 - rw.cl);
-          for (int q = gv.lower(B, rp.x, rp.y, gv.hi | ((uint64_t)rk + (uint64_t)rw.l0));
-               q < rp.y && cnt < Q.minpts && !over;) {
-            const int d = (int)((int64_t)((key_at<KEY64>(B, q) & P.kmask) - (uint64_t)rk) - rw.cl);
-            if (d > dmax) break;
-            const int qe = cell_end<KEY64>(B, q);
-            visit(q, qe, d);
-            q = qe;
+          if (open) {
+            siw[ni][threadIdx.x] = open;
+            sie[ni][threadIdx.x] = e[h];
+            ++ni;
           }
         }
-        // what is still queued decides only if it can lift the count to minpts;
-        // before a second launch it is always counted (that launch walks the
-        // other rows only)
-        pend = !over && cnt < Q.minpts && nq > 0 && (split || cnt + ptot >= Q.minpts);
-        if (pend) {
-#pragma unroll
-          for (int k = 0; k < D; ++k) {
-            S.x[lane][k] = px[k];
-            S.f[lane][k] = pf[k];
-          }
-          S.inst[lane] = P.inst;
-        }
-        isc = !over && cnt >= Q.minpts;
       }
+      // before a second launch the tests are always made (it walks other cells)
+      if (cnt >= minpts || (!split && ptot < kPoolCap && cnt + ptot < minpts)) ni = 0;
+      if (ni == 0) ptot = 0;
     }
-    // ---- warp-cooperative final flush (float64 mode)
-    const unsigned pm = F32 ? 0u : __ballot_sync(kFull, pend);
-    if (!F32 && pm) {
-      int tot = 0;
-      if (pend)
-        for (int j = 0; j < nq; ++j) tot += sq[j][threadIdx.x].y - sq[j][threadIdx.x].x;
-      int incl = tot;
+    // ---- pooled tests
+    bool over = false;
+    int pool = ptot;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(kFull, incl, o);
-        if (lane >= o) incl += v;
-      }
-      const int total = __shfl_sync(kFull, incl, 31);
-      S.incl[lane] = incl;
-      S.nq[lane] = pend ? nq : 0;
-      S.cnt[lane] = cnt;
-      __syncwarp();
-      if (total > 32 * B.tn_core) {
-        if (pend) over = true;  // too much for the warp: the warp kernel takes the cell
-      } else {
-        for (int base = 0; base < total; base += 32) {
-          const int c = base + lane;
-          if (c < total) {
-            // owner: the first lane whose inclusive prefix passes c
-            int lo = 0, hi = 31;
-            while (lo < hi) {
-              const int mid = (lo + hi) >> 1;
-              if (S.incl[mid] > c) hi = mid;
-              else lo = mid + 1;
-            }
-            const int ow = lo;
-            const PredParams Qo = pred_params(B.Pv[S.inst[ow]]);
-            if (S.cnt[ow] < Qo.minpts) {
-              int k = c - (ow > 0 ? S.incl[ow - 1] : 0);  // candidate index within the owner's queue
-              int qq = -1;
-              for (int j = 0; j < S.nq[ow]; ++j) {
-                const int2 sg = sq[j][wbase + ow];
-                const int len = sg.y - sg.x;
-                if (k < len) {
-                  qq = sg.x + k;
-                  break;
-                }
-                k -= len;
-              }
-              if (qq >= 0) {
-                Cand<D, F32> cd;
-                load_cand<D, F32>(cd, B.X, B.Xf, n, qq);
-                // (float64 mode only: the owner's coordinates are staged, no index needed)
-                if (pair_test<D, F32>(S.x[ow], S.f[ow], cd, B.X, n, qq, 0, true, Qo, t))
-                  atomicAdd(&S.cnt[ow], 1);
+    for (int o = 16; o > 0; o >>= 1) pool += __shfl_xor_sync(kFull, pool, o);
+    if (pool > 32 * B.tn_core) {  // too much for the warp: the warp kernel takes the cells
+      over = ni > 0;
+      ni = 0;
+      pool = 0;
+    }
+    S.cnt[lane] = 0;
+    __syncwarp();
+    if (pool > 0) {
+      unsigned long long w = 0, occ = 0;
+      uint32_t base = 0;
+      int k = 0, q = 0, qe = 0, nbuf = 0;
+      bool alive = ni > 0;
+      while (true) {
+        if (alive) {
+          if (q == qe) {
+            if (!w) {
+              if (k == ni) {
+                alive = false;
+              } else {
+                w = siw[k][threadIdx.x];
+                const EntHead a = ent_head(B, sie[k][threadIdx.x]);
+                occ = a.occ;
+                base = a.base;
+                ++k;
               }
             }
+            if (alive) {
+              const int c = ent_cell(occ, base, __ffsll((long long)w) - 1);
+              w &= w - 1;
+              q = B.reps[c];
+              qe = B.reps[c + 1];
+            }
+          }
+          alive = alive && cnt + S.cnt[lane] < minpts;
+        }
+        const unsigned bal = __ballot_sync(kFull, alive);
+        if (alive) {
+          const int at = nbuf + __popc(bal & ((1u << lane) - 1u));
+          S.q[at] = q++;
+          S.own[at] = lane;
+        }
+        nbuf += __popc(bal);
+        __syncwarp();
+        if (nbuf >= 32 || (bal == 0 && nbuf > 0)) {
+          const int take = min(nbuf, 32);
+          nbuf -= take;
+          if (lane < take) {
+            const int qq = S.q[nbuf + lane], ow = S.own[nbuf + lane];
+            double qx[D];
+            ld_x<D>(B, qq, qx);
+            ++t.t64;
+            const double d2 = dist2_f64<D>(S.x[ow], qx);
+            bool hit = d2_le(d2, S.e2in[ow]);
+            if (!hit && d2_le(d2, S.e2[ow])) hit = box_f64<D>(S.x[ow], qx, B.Pv[S.inst[ow]].eps);
+            if (hit) atomicAdd(&S.cnt[ow], 1);
           }
           __syncwarp();
-          if (__all_sync(kFull, !pend || S.cnt[lane] >= minpts)) break;
         }
-        if (pend) {
-          cnt = S.cnt[lane];
-          isc = cnt >= minpts;
-        }
+        if (bal == 0 && nbuf == 0) break;
       }
-      __syncwarp();
+      cnt += S.cnt[lane];
     }
-    // undecided after the near rows: on to the second launch
+    __syncwarp();
+    const bool isc = valid && !over && cnt >= minpts;
+    // undecided after pass 0: on to the second launch
     const bool go_on = split && valid && !over && !isc;
     if (go_on) {
       B.lab[i] = cnt;
@@ -1907,14 +2301,14 @@ k_core_point(const gdl::Bufs B, int64_t n, int r0, int r1) {
 template <int D, bool F32>
 __device__ __forceinline__ int inline_link(const gdl::Bufs& B, int64_t n, int bA, int eA, int bB,
                                            int eB, const float* oA, int ox, int oy, int oz,
-                                           const PredParams& Q, Tally& t) {
+                                           const DevParams& P, const PredParams& Q, Tally& t) {
   const bool prune = Q.prune != 0;
   int budget = B.tn_link;
   for (int a = bA; a < eA; ++a) {
     if (!B.core[a]) continue;
     double ax[D];
     float af[D];
-    load_point<D, F32>(ax, af, B, n, a, prune);
+    load_point<D, F32>(ax, af, B, a, prune);
     if (prune) {
       float u[D];
       frac_pos<D>(af, oA, Q, u);
@@ -1926,11 +2320,40 @@ __device__ __forceinline__ int inline_link(const gdl::Bufs& B, int64_t n, int bA
       if (!B.core[q]) continue;
       if (budget-- == 0) return -1;
       Cand<D, F32> cd;
-      load_cand<D, F32>(cd, B.X, B.Xf, n, q);
-      if (link_test<D, F32>(ax, af, cd, B.X, n, a, q, Q, t, B.asym, B.ctr)) return 1;
+      load_cand<D, F32>(cd, B, q);
+      if (link_test<D, F32>(ax, af, cd, B, P, a, q, Q, t)) return 1;
     }
   }
   return 0;
+}
+
+// Link between core cells m and c (at offset (ox, oy, oz) from m), m's
+// representative in ca: the representatives first -- on the workloads nine face
+// neighbours in ten are linked by that one test -- then the search.
+template <int D, bool F32>
+__device__ __forceinline__ int cell_link(const gdl::Bufs& B, int64_t n, const DevParams& P,
+                                         const CellXYZ<D>& cc, int m, int c,
+                                         const Cand<D, F32>& ca, int ox, int oy, int oz, Tally& t) {
+  Cand<D, F32> cd;
+  load_cand<D, F32>(cd, B, B.cellrep[c]);
+  bool apart;
+  if (F32) {
+    ++t.t32;
+    const float s2 = dist2_f32<D>(ca.f, cd.f);
+    if (s2 < P.eps2_lo32) return 1;
+    apart = s2 > P.eps2_hi32;
+  } else {
+    ++t.t64;
+    const double d2 = dist2_f64<D>(ca.x, cd.x);
+    if (d2_le(d2, P.eps2_in)) return 1;
+    apart = !d2_le(d2, P.eps2);
+  }
+  if (apart && B.cellcore[m] == 1 && B.cellcore[c] == 1) return 0;  // the only pair
+  const PredParams Q = pred_params(P);
+  float oA[D];
+  if (Q.prune) cell_origin32<D>(cc, P, oA);
+  return inline_link<D, F32>(B, n, B.reps[m], B.reps[m + 1], B.reps[c], B.reps[c + 1], oA, ox, oy,
+                             oz, P, Q, t);
 }
 
 // bit of offset (ox, oy, oz) in the kHalf[D][pass] table, or -1 if it is not there
@@ -1959,10 +2382,21 @@ __device__ __forceinline__ int half_bit(int pass, int ox, int oy, int oz) {
   return kHalfBits.b[D - 2][pass][ox + 2][oy + 2][oz + 2];
 }
 
+// Union scan of one pass, one thread per listed core cell A: the pass's half
+// stencil as masks over at most 4 (2D) or 8 (3D) block entries, whose core words
+// leave only the cells holding a core point.  The parents of a block's cells are
+// read in groups of four, through the cache: a parent equal to A's current root,
+// or to A's root when the pass began, settles the cell from one load even if it
+// is stale, since sets only merge.  The others are looked at again from fresh
+// loads and searched for a link.  The entries also hold the
+// root of the block's core cells at the pass's start, where they share one: if it
+// is A's, the whole block is settled by its entry.
 template <int D, bool F32, bool KEY64>
 __global__ void __launch_bounds__(kScanThreadsPerBlock, kUnionMinBlocks)
 k_union_scan(const gdl::Bufs B, int64_t n, int pass) {
-  const OffTab& T = kRows[D - 2];
+  using St = Stencil<D>;
+  __shared__ unsigned long long siw[2 * St::ROWS][kScanThreadsPerBlock];
+  __shared__ uint32_t sie[2 * St::ROWS][kScanThreadsPerBlock];
   const int lane = threadIdx.x & 31;
   const int LB = B.Bi->LB;
   // this dimension's part of the core-cell list: 2D instances' cells come first
@@ -1970,7 +2404,7 @@ k_union_scan(const gdl::Bufs B, int64_t n, int pass) {
   const int64_t L = (int64_t)*B.lcount;
   const int64_t L2 = M2 < n ? (int64_t)bit_rank(B.lbits, B.lpre, M2) : L;
   const int64_t jlo = D == 2 ? 0 : L2, jhi = D == 2 ? L2 : L;
-  WalkCursor wc = walk_cursor<D>(B, jlo, jhi);
+  WalkCursor wc = walk_cursor<D>(B, jlo, jhi, jhi - jlo < kUnionSmall ? 32 : 64);
   Tally t;
   while (wc.advance(lane)) {
     const int64_t j = jlo + wc.next + lane;
@@ -1979,117 +2413,109 @@ k_union_scan(const gdl::Bufs B, int64_t n, int pass) {
     const int64_t m = valid ? (int64_t)B.blist[j] : 0;
     unsigned long long open = 0;
     if (valid) {
-      const int b = B.reps[m];
-      {
-        const int e = B.reps[m + 1];
-        const CellCtx cx = cell_ctx<KEY64>(B, b, LB);
-        const DevParams& P = *cx.P;
-        const PredParams Q = pred_params(P);
-        const GridView gv = view_of(B, P);
-        RowWalk<D> rw;
-        rw.init(decompose<D>(cx.local, P), P);
-        float oA[D];
-        if (Q.prune) cell_origin32<D>(rw.cc, P, oA);
-        // A's parent as the compression before this pass left it: A's root at
-        // the start of the pass.  Neighbours' parents were compressed at the
-        // same time, so one equal to it puts the cell in A's set however the
-        // pass's unions have moved the root since (ra, the current root, is
-        // checked too).
-        const int ra0 = reinterpret_cast<volatile int*>(B.parent)[m];
-        int ra = uf_find(B.parent, (int)m);
-        for (int r = 0; r < T.n; ++r) {
-          const int ox = T.o[r][0], oy = T.o[r][1];
-          // the row's last-axis offsets in this pass (bit dz + 2)
-          const uint32_t zm = kPassZ.m[D - 2][pass][ox + 2][oy + 2];
-          if (!zm) continue;
-          const int64_t rk = rw.rowkey(T, r, P);
-          if (rk < 0) continue;
-          int64_t z0 = (int64_t)rw.cl - 2 + (__ffs(zm) - 1);
-          int64_t z1 = (int64_t)rw.cl - 2 + (31 - __clz(zm));
-          z0 = z0 < rw.l0 ? rw.l0 : z0;
-          z1 = z1 > rw.l1 ? rw.l1 : z1;
-          if (z0 > z1) continue;
-          // bit z - z0: cell z of the row is in this pass
-          const uint32_t allow = zm >> (int)(z0 - ((int64_t)rw.cl - 2));
-          // one cell holding a core point (index c, last-axis offset d).  Its
-          // points are looked up only when a link search is needed.
-          auto visit_core = [&](int c, int d) {
-            // ra: a root of A's set, refreshed only when c's root differs.  A
-            // parent equal to ra puts c in A's set from one load (ra stays in
-            // A's set whatever is hooked later; the pass before compressed the
-            // parents to roots).
-            const int pc = reinterpret_cast<volatile int*>(B.parent)[c];
-            if (pc == ra || pc == ra0) return;
-            const int rc = pc == c ? c : uf_find(B.parent, pc);
-            if (rc == ra) return;
-            ra = uf_find(B.parent, ra);
-            if (rc == ra) return;
-            const int q = B.reps[c], qe = B.reps[c + 1];
-            const int res = D == 3 ? inline_link<D, F32>(B, n, b, e, q, qe, oA, ox, oy, d, Q, t)
-                                   : inline_link<D, F32>(B, n, b, e, q, qe, oA, ox, d, 0, Q, t);
-            if (res > 0) {
-              uf_union(B.parent, B.cellmin, (int)m, c);
-              ra = uf_find(B.parent, ra);
-            } else if (res < 0) {
-              // the pass masks keep every visited offset in this pass's half
-              // stencil
-              const int bit = D == 3 ? half_bit<D>(pass, ox, oy, d) : half_bit<D>(pass, ox, d, 0);
-              if (bit >= 0) open |= 1ull << bit;
-            }
-          };
-          // a cell of unknown core state
-          auto visit = [&](int c, int d) {
-            if (B.cellcore[c] > 0) visit_core(c, d);
-          };
-          if (gv.sparse == 0) {
-            // cell table: the cells holding a core point, from the occupancy and
-            // core occupancy bits (a cell's index into reps: the rank of the
-            // first occupied one plus the occupied cells before it).  Their
-            // parents are read together first, through the cache: a parent
-            // equal to ra settles the cell even if it is stale, since sets only
-            // merge; the others are looked at again from fresh loads.
-            int64_t rr = 0;
-            const uint32_t mask = gv.occ_cells(B, (uint64_t)rk, z0, z1, rr);
-            const uint32_t cm = mask & allow & gv.core_cells(B, (uint64_t)rk, z0, z1);
-            uint32_t slow = 0;
+      const CellCtx cx = cell_ctx<KEY64>(B, m, LB);
+      const DevParams& P = *cx.P;
+      const CellXYZ<D> cc = decompose<D>(cx.local, P);
+      St st;
+      st.init(cc);
+      const unsigned long long* __restrict__ masks = kPassMasks[D - 2].m[pass][cx.local & 63];
+      // A's parent as the compression before this pass left it: A's root at
+      // the start of the pass.  Neighbours' parents were compressed at the
+      // same time, so one equal to it puts the cell in A's set however the
+      // pass's unions have moved the root since (ra, the current root, is
+      // checked too).
+      const int ra0 = reinterpret_cast<volatile int*>(B.parent)[m];
+      int ra = uf_find(B.parent, (int)m);
+      // A's representative: its first core point
+      const int qa = B.cellrep[m];
+      Cand<D, F32> ca;
+      load_cand<D, F32>(ca, B, qa);
+      // one cell holding a core point (index c) at offset (ox, oy, oz).  Its
+      // points are looked up only when a link search is needed.
+      auto visit_core = [&](int c, int ox, int oy, int oz) {
+        // ra: a root of A's set, refreshed only when c's root differs.  A
+        // parent equal to ra puts c in A's set from one load (ra stays in
+        // A's set whatever is hooked later; the pass before compressed the
+        // parents to roots).
+        const int pc = reinterpret_cast<volatile int*>(B.parent)[c];
+        if (pc == ra || pc == ra0) return;
+        const int rc = pc == c ? c : uf_find(B.parent, pc);
+        if (rc == ra) return;
+        ra = uf_find(B.parent, ra);
+        if (rc == ra) return;
+        const int res = cell_link<D, F32>(B, n, P, cc, (int)m, c, ca, ox, oy, oz, t);
+        if (res > 0) {
+          uf_union(B.parent, (int)m, c);
+          ra = uf_find(B.parent, ra);
+        } else if (res < 0) {
+          // the pass masks keep every visited offset in this pass's half stencil
+          const int bit = half_bit<D>(pass, ox, oy, oz);
+          if (bit >= 0) open |= 1ull << bit;
+        }
+      };
+      // the blocks with cells to look at; those are visited afterwards, so that
+      // the warp's lanes visit theirs together whatever blocks they lie in
+      int ni = 0;
+      uint32_t codes = 0;
+      for (int r = 0; r < St::ROWS; ++r) {
+        const unsigned long long M0 = masks[2 * r], M1 = masks[2 * r + 1];
+        if (!(M0 | M1)) continue;
+        const int64_t row = st.row(r, P);
+        if (row < 0) continue;
+        uint32_t e[2];
+        block_pair<D, KEY64>(B, P, (uint64_t)row, st.b0[D - 1], M0 != 0, M1 != 0, e[0], e[1]);
+        EntHead hd[2];
+        EntTail tl[2];
 #pragma unroll
-            for (int z = 0; z < 5; ++z) {
-              if ((cm >> z) & 1u) {
-                const int64_t r = rr + __popc(mask & ((1u << z) - 1u));
-                const int pr = B.parent[r];
-                if (pr != ra && pr != ra0) slow |= 1u << z;
-              }
+        for (int h = 0; h < 2; ++h) {
+          hd[h] = ent_head(B, e[h]);
+          tl[h] = ent_tail(B, e[h]);
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          unsigned long long w = tl[h].core & (h ? M1 : M0), slow;
+          if ((int)(pass == 0 ? tl[h].uni : pass == 1 ? hd[h].lo : tl[h].hi) == ra0) w = 0;
+          slow = 0;
+          while (w) {
+            int bit[4], pr[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              bit[q] = w ? __ffsll((long long)w) - 1 : -1;
+              w &= w - 1;
+              pr[q] = bit[q] >= 0 ? B.parent[ent_cell(hd[h].occ, hd[h].base, bit[q])] : ra;
             }
-            while (slow) {
-              const int z = __ffs(slow) - 1;
-              slow &= slow - 1;
-              const int64_t r = rr + __popc(mask & ((1u << z) - 1u));
-              visit_core((int)r, (int)(z0 + z - rw.cl));
-            }
-            continue;
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              if (pr[q] != ra && pr[q] != ra0) slow |= 1ull << bit[q];
           }
-          if (gv.sparse == 2) {
-            // row table: the row's cells with last-axis coordinate in [z0, z1],
-            // rows without a core point skipped
-            const uint64_t ri = udiv_by((uint64_t)rk, gv.glm, gv.gls);
-            if (!gv.core_row_at(B, ri)) continue;
-            const int2 rc = gv.row_cells(B, ri);
-            for (int mq = gv.zlower(B, rc.x, rc.y, z0); mq < rc.y; ++mq) {
-              const int64_t z = B.cellz[mq];
-              if (z > z1) break;
-              if ((allow >> (int)(z - z0)) & 1u) visit(mq, (int)(z - rw.cl));
-            }
-            continue;
-          }
-          const int2 sp = gv.span_row(B, (uint64_t)rk, z0, z1);
-          for (int q = sp.x; q < sp.y;) {
-            const int c = cell_of(B, q);
-            const int qe = B.reps[c + 1];
-            const int64_t z = (int64_t)((key_at<KEY64>(B, q) & P.kmask) - (uint64_t)rk);
-            if ((allow >> (int)(z - z0)) & 1u) visit(c, (int)(z - rw.cl));
-            q = qe;
+          if (slow) {
+            siw[ni][threadIdx.x] = slow;
+            sie[ni][threadIdx.x] = e[h];
+            codes |= (uint32_t)(2 * r + h) << (4 * ni);
+            ++ni;
           }
         }
+      }
+      unsigned long long w = 0, occ = 0;
+      uint32_t base = 0;
+      int d[3] = {0, 0, 0}, k = 0;
+      while (true) {
+        if (!w) {
+          if (k == ni) break;
+          w = siw[k][threadIdx.x];
+          const EntHead a = ent_head(B, sie[k][threadIdx.x]);
+          occ = a.occ;
+          base = a.base;
+          const int code = (int)(codes >> (4 * k)) & 7;
+          d[0] = st.off0(cc, 0) + ((D == 3 ? code >> 2 : code >> 1) << St::S);
+          if (D == 3) d[1] = st.off0(cc, 1) + (((code >> 1) & 1) << St::S);
+          d[D - 1] = st.off0(cc, D - 1) + ((code & 1) << St::S);
+          ++k;
+        }
+        const int bit = __ffsll((long long)w) - 1;
+        w &= w - 1;
+        visit_core(ent_cell(occ, base, bit), d[0] + St::bit_off(bit, 0), d[1] + St::bit_off(bit, 1),
+                   D == 3 ? d[2] + St::bit_off(bit, 2) : 0);
       }
     }
     heavy_push(B, kCtrHeavyUnion, open != 0, m, open);
@@ -2106,11 +2532,13 @@ k_union_scan(const gdl::Bufs B, int64_t n, int pass) {
 // gives its id without tests and one wholly outside is skipped.  A point whose
 // tests pass the budget sends its cell to the warp kernel.
 template <int D, bool F32, bool KEY64>
-__global__ void __launch_bounds__(kScanThreadsPerBlock, kBorderMinBlocks) k_border_point(const gdl::Bufs B, int64_t n) {
-  // per thread: squared largest / smallest distance terms to the five cell
-  // slabs along the last axis (offsets -2..2), kept out of registers
-  __shared__ float2 slt[5][kScanThreadsPerBlock];
-  const OffTab& T = kRows[D - 2];
+__global__ void __launch_bounds__(kBorderThreads, kBorderMinBlocks) k_border_point(const gdl::Bufs B, int64_t n) {
+  using St = Stencil<D>;
+  // per thread and axis: squared largest / smallest distance terms to the five
+  // cell slabs at offsets -2..2
+  __shared__ float2 slt[D][5][kBorderThreads];
+  __shared__ unsigned long long siw[2 * St::ROWS][kBorderThreads];
+  __shared__ uint32_t sie[2 * St::ROWS][kBorderThreads];
   const int lane = threadIdx.x & 31;
   const int LB = B.Bi->LB;
   // this dimension's part of the list: 2D instances' points come first
@@ -2118,7 +2546,7 @@ __global__ void __launch_bounds__(kScanThreadsPerBlock, kBorderMinBlocks) k_bord
   const int64_t L = (int64_t)*B.lcount;
   const int64_t L2 = p3 < n ? (int64_t)bit_rank(B.lbits, B.lpre, p3) : L;
   const int64_t jlo = D == 2 ? 0 : L2, jhi = D == 2 ? L2 : L;
-  WalkCursor wc = walk_cursor<D>(B, jlo, jhi);
+  WalkCursor wc = walk_cursor<D>(B, jlo, jhi, 32);
   Tally t;
   while (wc.advance(lane)) {
     const int64_t j = jlo + wc.next + lane;
@@ -2129,144 +2557,114 @@ __global__ void __launch_bounds__(kScanThreadsPerBlock, kBorderMinBlocks) k_bord
     if (valid) {
       const int64_t i = (int64_t)B.blist[j];
       m = cell_of(B, i);
-      const int b = B.reps[m];
-      const CellCtx cx = cell_ctx<KEY64>(B, b, LB);
+      const CellCtx cx = cell_ctx<KEY64>(B, m, LB);
       const DevParams& P = *cx.P;
       const PredParams Q = pred_params(P);
-      const GridView gv = view_of(B, P);
       const bool prune = Q.prune != 0;
-      RowWalk<D> rw;
-      rw.init(decompose<D>(cx.local, P), P);
+      const CellXYZ<D> cc = decompose<D>(cx.local, P);
+      St st;
+      st.init(cc);
       double px[D];
       float pf[D];
-      load_point<D, F32>(px, pf, B, n, i, prune);
-      float u[D];
+      load_point<D, F32>(px, pf, B, i, prune);
       if (prune) {
-        float o[D];
-        cell_origin32<D>(rw.cc, P, o);
+        float u[D], o[D];
+        cell_origin32<D>(cc, P, o);
         frac_pos<D>(pf, o, Q, u);
 #pragma unroll
-        for (int k = 0; k < 5; ++k) {
-          float a2, b2;
-          axis_terms(u[D - 1], k - 2, Q, a2, b2);
-          slt[k][threadIdx.x] = make_float2(a2, b2);
+        for (int k = 0; k < D; ++k) {
+          uint32_t near = 0;
+#pragma unroll
+          for (int j = 0; j < 5; ++j) {
+            float a2, b2;
+            axis_terms(u[k], j - 2, Q, a2, b2);
+            slt[k][j][threadIdx.x] = make_float2(a2, b2);
+            if (b2 < Q.thr_out) near |= 1u << j;  // the slab is not beyond eps by itself
+          }
+          st.w5[k] = near << ((cc.c[k] - 2) & (St::SIDE - 1));
         }
       }
       int best = INT_MAX, budget = B.tn_border;
-      for (int r = 0; r < T.n && !over; ++r) {
-        float rmx = 0.0f, rmn = 0.0f;
+      // the blocks with core cells in the stencil, then their cells
+      StencilWords<D> W5;
+      W5.init(st.w5);
+      int ni = 0;
+      uint32_t codes = 0;
+      for (int r = 0; r < St::ROWS; ++r) {
+        const int64_t row = st.row(r, P);
+        if (row < 0) continue;
+        uint2 m[2];
+        W5.row(r, m[0], m[1]);
+        uint32_t e[2];
+        block_pair<D, KEY64>(B, P, (uint64_t)row, st.b0[D - 1], (m[0].x | m[0].y) != 0,
+                             (m[1].x | m[1].y) != 0, e[0], e[1]);
+        unsigned long long w[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) w[h] = e[h] != kNoEnt ? B.ent[e[h]].core & u64_of(m[h]) : 0ull;
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          if (w[h]) {
+            siw[ni][threadIdx.x] = w[h];
+            sie[ni][threadIdx.x] = e[h];
+            codes |= (uint32_t)(2 * r + h) << (4 * ni);
+            ++ni;
+          }
+      }
+      unsigned long long w = 0, occ = 0;
+      uint32_t base = 0;
+      int d[D], kk = 0;
+#pragma unroll
+      for (int k = 0; k < D; ++k) d[k] = 0;
+      while (!over) {
+        if (!w) {
+          if (kk == ni) break;
+          const EntHead a = ent_head(B, sie[kk][threadIdx.x]);
+          const int code = (int)(codes >> (4 * kk)) & 7;
+          w = siw[kk][threadIdx.x];
+          ++kk;
+          if ((int)a.lo >= best) {  // none of its clusters can improve on the best so far
+            w = 0;
+            continue;
+          }
+          occ = a.occ;
+          base = a.base;
+          d[0] = st.off0(cc, 0) + 2 + ((D == 3 ? code >> 2 : code >> 1) << St::S);
+          if (D == 3) d[1] = st.off0(cc, 1) + 2 + (((code >> 1) & 1) << St::S);
+          d[D - 1] = st.off0(cc, D - 1) + 2 + ((code & 1) << St::S);
+        }
+        const int bit = __ffsll((long long)w) - 1;
+        w &= w - 1;
+        const int c = ent_cell(occ, base, bit);
+        const int cB = B.cellcid[c];
+        if (cB >= best) continue;
+        int cls = 0;
         if (prune) {
+          float smax = 0.0f, smin = 0.0f;
 #pragma unroll
-          for (int k = 0; k < D - 1; ++k) {
-            float a2, b2;
-            axis_terms(u[k], (int)T.o[r][k], Q, a2, b2);
-            rmx += a2;
-            rmn += b2;
+          for (int k = 0; k < D; ++k) {
+            const float2 lt = slt[k][d[k] + St::bit_off(bit, k)][threadIdx.x];
+            smax += lt.x;
+            smin += lt.y;
           }
-          if (rmn >= Q.thr_out) continue;  // the whole row is beyond eps
+          cls = smax <= Q.thr_in ? 1 : (smin >= Q.thr_out ? -1 : 0);
         }
-        const int64_t ri = rw.rowidx(T, r, P);
-        if (ri < 0) continue;
-        const int64_t rk = ri * P.G[D - 1];  // key of the row's first cell
-        if (gv.sparse == 0) {
-          // cell table: visit only the cells holding a core point.  The
-          // occupancy, core occupancy and prefix words load together; then the
-          // row's cluster ids, together: a row none of whose ids is below best
-          // is done without looking at its cells.
-          int64_t rr = 0;
-          const uint32_t mask = gv.occ_cells(B, (uint64_t)rk, rw.l0, rw.l1, rr);
-          uint32_t cm = mask & gv.core_cells(B, (uint64_t)rk, rw.l0, rw.l1);
-          int rowmin = INT_MAX;
-#pragma unroll
-          for (int z = 0; z < 5; ++z)
-            if ((cm >> z) & 1u) rowmin = min(rowmin, B.cellcid[rr + __popc(mask & ((1u << z) - 1u))]);
-          if (rowmin >= best) continue;
-          while (cm && !over) {
-            const int z = __ffs(cm) - 1;
-            cm &= cm - 1;
-            const int64_t rq = rr + __popc(mask & ((1u << z) - 1u));
-            const int cB = B.cellcid[rq];
-            if (cB >= best) continue;
-            int cls = 0;
-            if (prune) {
-              const int d = (int)(rw.l0 + z - rw.cl);
-              const float2 lt = slt[d + 2][threadIdx.x];
-              const float smax = rmx + lt.x, smin = rmn + lt.y;
-              cls = smax <= Q.thr_in ? 1 : (smin >= Q.thr_out ? -1 : 0);
+        if (cls > 0) {
+          best = cB;  // every point of that cell, a core among them, is in reach
+        } else if (cls == 0) {
+          const int q = B.reps[c], qe = B.reps[c + 1];
+          for (int qq = q; qq < qe; ++qq) {
+            if (!B.core[qq]) continue;
+            if (budget-- == 0) {
+              over = true;
+              break;
             }
-            if (cls > 0) {
+            Cand<D, F32> cd;
+            load_cand<D, F32>(cd, B, qq);
+            if (pair_test<D, F32>(px, pf, cd, B, P, qq, i, false, Q, t)) {
               best = cB;
-            } else if (cls == 0) {
-              const int q = B.reps[rq], qe = B.reps[rq + 1];
-              for (int qq = q; qq < qe; ++qq) {
-                if (!B.core[qq]) continue;
-                if (budget-- == 0) {
-                  over = true;
-                  break;
-                }
-                Cand<D, F32> cd;
-                load_cand<D, F32>(cd, B.X, B.Xf, n, qq);
-                if (pair_test<D, F32>(px, pf, cd, B.X, n, qq, i, false, Q, t)) {
-                  best = cB;
-                  break;
-                }
-              }
+              break;
             }
           }
-          continue;
-        }
-        if (gv.sparse == 2 && !gv.core_row_at(B, (uint64_t)ri)) continue;
-        // one non-empty cell (index c, points [q, qe)) at last-axis offset d;
-        // cells without core points have cluster id INT_MAX
-        auto visitb = [&](int c, int q, int qe, int d) {
-          const int cB = B.cellcid[c];
-          if (cB >= best) return;
-          int cls = 0;
-          if (prune) {
-            const float2 lt = slt[d + 2][threadIdx.x];
-            const float smax = rmx + lt.x, smin = rmn + lt.y;
-            cls = smax <= Q.thr_in ? 1 : (smin >= Q.thr_out ? -1 : 0);
-          }
-          if (cls > 0) {
-            best = cB;  // every point of that cell, a core among them, is in reach
-          } else if (cls == 0) {
-            for (int qq = q; qq < qe; ++qq) {
-              if (!B.core[qq]) continue;
-              if (budget-- == 0) {
-                over = true;
-                break;
-              }
-              Cand<D, F32> cd;
-              load_cand<D, F32>(cd, B.X, B.Xf, n, qq);
-              if (pair_test<D, F32>(px, pf, cd, B.X, n, qq, i, false, Q, t)) {
-                best = cB;
-                break;
-              }
-            }
-          }
-        };
-        if (gv.sparse == 2) {
-          // row table: the row's cells from the first at or after l0 to l1
-          const int2 rc = gv.row_cells(B, (uint64_t)ri);
-          for (int mq = gv.zlower(B, rc.x, rc.y, rw.l0); mq < rc.y && !over; ++mq) {
-            const int64_t z = B.cellz[mq];
-            if (z > rw.l1) break;
-            visitb(mq, B.reps[mq], B.reps[mq + 1], (int)(z - rw.cl));
-          }
-          continue;
-        }
-        // hash: the row's points from the first cell at or after l0
-        const int2 rp = gv.row(B, (uint64_t)rk);
-        if (rp.x == rp.y) continue;
-        const int dmax = (int)(rw.l1 - rw.cl);
-        for (int q = gv.lower(B, rp.x, rp.y, gv.hi | ((uint64_t)rk + (uint64_t)rw.l0));
-             q < rp.y && !over;) {
-          const int d = (int)((int64_t)((key_at<KEY64>(B, q) & P.kmask) - (uint64_t)rk) - rw.cl);
-          if (d > dmax) break;
-          const int c = cell_of(B, q);
-          const int qe = B.reps[c + 1];
-          visitb(c, q, qe, d);
-          q = qe;
         }
       }
       if (!over) B.lab[i] = best == INT_MAX ? kNoise : best;
@@ -2282,21 +2680,18 @@ __global__ void __launch_bounds__(kScanThreadsPerBlock, kBorderMinBlocks) k_bord
 
 // ------------------------------------------------------------- core flags
 // Heavy cells, one warp each: dense cells (>= minpts points) are all core;
-// other queued cells stream their candidate rows (5 cells along the last axis
-// each, 5 rows in 2D, 25 in 3D, looked up one per lane and concatenated) 32 at
+// other queued cells stream the points of their stencil's cells (looked up one
+// per lane and concatenated, nearest first) 32 at
 // a time, one candidate per lane, and every staged point of the cell gets
 // __ballot_sync + __popc of the lanes holding a neighbour.  The warp stops as
-// soon as every staged point has reached minpts (own row first).
+// soon as every staged point has reached minpts.
 template <int D, bool F32, bool KEY64>
 __global__ void __launch_bounds__(kCellThreads) k_core_heavy(const gdl::Bufs B, int64_t n) {
   __shared__ WarpStage<D> stage[kWarpsPerBlock];
-  __shared__ RowList rows[kWarpsPerBlock];
+  __shared__ CellList lists[kWarpsPerBlock];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   WarpStage<D>& S = stage[w];
-  RowList& RL = rows[w];
-  const int nrows = kRows[D - 2].n;
-  const double* __restrict__ X = B.X;
-  const float* __restrict__ Xf = B.Xf;
+  CellList& CL = lists[w];
   const int LB = B.Bi->LB;
   int64_t mlo, mhi;
   dim_range<D>(B, mlo, mhi);
@@ -2308,7 +2703,7 @@ __global__ void __launch_bounds__(kCellThreads) k_core_heavy(const gdl::Bufs B, 
     const int64_t m = B.hv_cell[h];
     if (m < mlo || m >= mhi) continue;
     const int b = B.reps[m], e = B.reps[m + 1], sz = e - b;
-    const CellCtx cx = cell_ctx<KEY64>(B, b, LB);
+    const CellCtx cx = cell_ctx<KEY64>(B, m, LB);
     const DevParams& P = *cx.P;
     const PredParams Q = pred_params(P);
     if (sz >= Q.minpts) {
@@ -2321,18 +2716,15 @@ __global__ void __launch_bounds__(kCellThreads) k_core_heavy(const gdl::Bufs B, 
       if (lane == 0) { B.cellcore[m] = sz; B.cellmin[m] = mn; ++dense; }
       continue;
     }
-    const GridView gv = view_of(B, P);
     const CellXYZ<D> cc = decompose<D>(cx.local, P);
-    const int total = build_rows<D>(B, RL, gv, cc, P, lane);
+    int ncells = 0;
+    const int total = build_cells<D, KEY64>(B, CL, cc, P, lane, ncells);
     int ncore = 0, mn = INT_MAX;
     for (int c0 = 0; c0 < sz; c0 += 32) {
       const int na = min(32, sz - c0);
       if (lane < na) {
-#pragma unroll
-        for (int k = 0; k < D; ++k) {
-          if (!F32) S.x[lane][k] = X[k * n + b + c0 + lane];
-          if (F32) S.f[lane][k] = Xf[k * n + b + c0 + lane];
-        }
+        if (F32) ld_f<D>(B, b + c0 + lane, S.f[lane]);
+        else ld_x<D>(B, b + c0 + lane, S.x[lane]);
       }
       __syncwarp();
       int mycnt = 0;
@@ -2343,11 +2735,11 @@ __global__ void __launch_bounds__(kCellThreads) k_core_heavy(const gdl::Bufs B, 
         int q = 0;
         Cand<D, F32> cd;
         if (valid) {
-          q = row_pos(RL, nrows, c);
-          load_cand<D, F32>(cd, X, Xf, n, q);
+          q = cell_list_pos(CL, ncells, c);
+          load_cand<D, F32>(cd, B, q);
         }
         for (int j = 0; j < na; ++j) {
-          bool hit = valid && pair_test<D, F32>(S.x[j], S.f[j], cd, X, n, q, b + c0 + j, true, Q, t);
+          bool hit = valid && pair_test<D, F32>(S.x[j], S.f[j], cd, B, P, q, b + c0 + j, true, Q, t);
           unsigned bal = __ballot_sync(kFull, hit);
           if (lane == j) mycnt += __popc(bal);
         }
@@ -2367,38 +2759,159 @@ __global__ void __launch_bounds__(kCellThreads) k_core_heavy(const gdl::Bufs B, 
 }
 
 // ------------------------------------------------------------- union-find
-// Union-find roots, the mask of the core-cell list (cells with a core point,
-// listed in order for k_union_scan; a word per warp over [0, n)), and the
-// core occupancy bit of every core cell's cell-table (row-table) entry, so the
-// link and border searches skip cells (rows) without core points without
-// looking them up.
+// Each core cell's representative (its first core point) and its bit in its
+// block's core word, and the mask of the core-cell list (listed in order for the
+// union; a word per warp over [0, n)).
 template <bool KEY64>
-__global__ void k_parent_init(const gdl::Bufs B, int64_t n) {
+__global__ void k_core_cells(const gdl::Bufs B, int64_t n) {
   const int64_t M = *B.M;
   const int lane = threadIdx.x & 31;
-  const int LB = B.Bi->LB;
   // words of the mask beyond the cells are cleared before the launch
   for (int64_t m0 = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); m0 < M;
        m0 += (int64_t)gridDim.x * blockDim.x) {
     const int64_t m = m0 + lane;
-    bool f = false;
-    if (m < M) {
-      B.parent[m] = (int)m;
-      f = B.cellcore[m] > 0;
-      if (f && B.occ_words) {
-        const uint64_t key = key_at<KEY64>(B, B.reps[m]);
-        const DevParams& P = B.Pv[(int)(key >> LB)];
-        if (P.sparse != 1) {
-          const uint64_t local = key & P.kmask;
-          const int a = P.dim - 2;
-          const uint64_t idx =
-              P.occ_off + (P.sparse == 2 ? udiv_by(local, P.dm[a], P.ds[a]) : local);
-          atomicOr(B.cocc + (idx >> 5), 1u << (idx & 31));
-        }
-      }
+    const bool f = m < M && B.cellcore[m] > 0;
+    if (f) {
+      int q = B.reps[m];
+      while (!B.core[q]) ++q;
+      B.cellrep[m] = q;
+      B.compmin[m] = B.cellmin[m];
+      atomicOr(&B.ent[B.cellent[m]].core, 1ull << ((unsigned)ckey_at<KEY64>(B, m) & 63u));
     }
     const unsigned bl = __ballot_sync(kFull, f);
     if (lane == 0) B.lbits[m0 >> 5] = bl;
+  }
+}
+
+// Union inside blocks, in two steps without a chain to follow: which of a block's
+// core cells that share a face are linked through their representatives (in float64
+// mode: or because all of the neighbour is in the representative's reach), as one
+// word per direction (k_links, a thread per listed core cell), then the connected
+// parts of those words by bit floods (k_flood, a thread per block), whose cells get
+// the part's first cell as parent.  The union passes then start from blocks mostly
+// in one part each, and look for the links that the representatives do not show.
+// (A first pass over single cells had spent its time in the finds and hooks of
+// these links: C3 0.95 ms.)
+template <int D>
+struct LinkDirs {
+  static constexpr int N = D;
+  // the neighbour along axis d: its bit distance, and the places that have it in the block
+  static __device__ constexpr int sh(int d) {
+    return D == 3 ? (d == 0 ? 16 : d == 1 ? 4 : 1) : (d == 0 ? 8 : 1);
+  }
+  static __device__ constexpr unsigned long long in(int d) {
+    return D == 3 ? (d == 0 ? 0x0000ffffffffffffull
+                            : d == 1 ? 0x0fff0fff0fff0fffull : 0x7777777777777777ull)
+                  : (d == 0 ? 0x00ffffffffffffffull : 0x7f7f7f7f7f7f7f7full);
+  }
+};
+
+template <int D, bool F32, bool KEY64>
+__global__ void __launch_bounds__(256) k_links(const gdl::Bufs B, int64_t n) {
+  using Dir = LinkDirs<D>;
+  const int LB = B.Bi->LB;
+  const int64_t M2 = (int64_t)B.ctr[kCtrCells2D];
+  const int64_t L = (int64_t)*B.lcount;
+  const int64_t L2 = M2 < n ? (int64_t)bit_rank(B.lbits, B.lpre, M2) : L;
+  const int64_t jlo = D == 2 ? 0 : L2, jhi = D == 2 ? L2 : L;
+  Tally t;
+  for (int64_t j = jlo + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < jhi;
+       j += (int64_t)gridDim.x * blockDim.x) {
+    const int a = (int)B.blist[j];
+    const uint64_t key = ckey_at<KEY64>(B, a);
+    const int bit = (int)key & 63;
+    const uint32_t e = B.cellent[a];
+    const int qa = B.cellrep[a];
+    const EntHead hd = ent_head(B, e);
+    const unsigned long long core = ent_tail(B, e).core;
+    const DevParams& P = B.Pv[inst_of(key, LB)];
+    unsigned has = 0;
+    int rq[Dir::N];
+#pragma unroll
+    for (int d = 0; d < Dir::N; ++d)
+      if ((((core >> Dir::sh(d)) & Dir::in(d)) >> bit) & 1ull) {
+        has |= 1u << d;
+        rq[d] = B.cellrep[ent_cell(hd.occ, hd.base, bit + Dir::sh(d))];
+      }
+    if (!has) continue;
+    unsigned hit = 0;
+    if constexpr (F32) {
+      float f[D];
+      ld_f<D>(B, qa, f);
+#pragma unroll
+      for (int d = 0; d < Dir::N; ++d)
+        if ((has >> d) & 1u) {
+          float g[D];
+          ld_f<D>(B, rq[d], g);
+          ++t.t32;
+          if (dist2_f32<D>(f, g) < P.eps2_lo32) hit |= 1u << d;
+        }
+    } else {
+      if (P.prune) {
+        const PredParams Q = pred_params(P);
+        float o[D], f[D], u[D];
+        cell_origin32<D>(decompose<D>(key & P.kmask, P), P, o);
+        ld_f<D>(B, qa, f);
+        frac_pos<D>(f, o, Q, u);
+#pragma unroll
+        for (int d = 0; d < Dir::N; ++d)
+          if (classify<D>(u, d == 0, d == 1, d == 2, Q) > 0) hit |= 1u << d;
+        hit &= has;
+      }
+      if (hit != has) {
+        double x[D];
+        ld_x<D>(B, qa, x);
+#pragma unroll
+        for (int d = 0; d < Dir::N; ++d)
+          if (((has & ~hit) >> d) & 1u) {
+            double y[D];
+            ld_x<D>(B, rq[d], y);
+            ++t.t64;
+            if (d2_le(dist2_f64<D>(x, y), P.eps2_in)) hit |= 1u << d;
+          }
+      }
+    }
+#pragma unroll
+    for (int d = 0; d < Dir::N; ++d)
+      if ((hit >> d) & 1u) atomicOr(&B.links[e].w[d][bit >> 5], 1u << (bit & 31));
+  }
+  flush_tally(t, B.ctr);
+}
+
+__global__ void k_flood(const gdl::Bufs B) {
+  const int64_t M2 = (int64_t)B.ctr[kCtrCells2D];
+  const int64_t NBk = (int64_t)B.ctr[kCtrBlocks];
+  for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < NBk;
+       j += (int64_t)gridDim.x * blockDim.x) {
+    const int m0 = (int)B.blklist[j];
+    const uint32_t e = B.cellent[m0];
+    unsigned long long left = B.ent[e].core;
+    if (!left) continue;
+    const unsigned long long occ = B.ent[e].occ;
+    const BlockLinks lk = B.links[e];
+    B.links[e] = BlockLinks{};  // for the next expand
+    uint32_t uni = kNoEnt;
+    unsigned long long l[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) l[d] = (unsigned long long)lk.w[d][1] << 32 | lk.w[d][0];
+    const bool two = m0 < M2;
+    const int s0 = two ? LinkDirs<2>::sh(0) : LinkDirs<3>::sh(0);
+    const int s1 = two ? LinkDirs<2>::sh(1) : LinkDirs<3>::sh(1);
+    while (left) {
+      unsigned long long part = left & (0ull - left), before;
+      const int root = ent_cell(occ, (uint32_t)m0, __ffsll((long long)part) - 1);
+      do {
+        before = part;
+        part |= (part & l[0]) << s0 | ((part >> s0) & l[0]);
+        part |= (part & l[1]) << s1 | ((part >> s1) & l[1]);
+        part |= (part & l[2]) << 1 | ((part >> 1) & l[2]);  // (3D; no bits in 2D)
+      } while (part != before);
+      left &= ~part;
+      uni = uni == kNoEnt ? (uint32_t)root : kMixedRoot;
+      for (unsigned long long w = part; w; w &= w - 1)
+        B.parent[ent_cell(occ, (uint32_t)m0, __ffsll((long long)w) - 1)] = root;
+    }
+    B.ent[e].uni = uni;
   }
 }
 
@@ -2410,8 +2923,6 @@ __global__ void k_parent_init(const gdl::Bufs B, int64_t n) {
 template <int D, bool F32, bool KEY64>
 __global__ void __launch_bounds__(kCellThreads) k_union_heavy(const gdl::Bufs B, int64_t n, int pass) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const double* __restrict__ X = B.X;
-  const float* __restrict__ Xf = B.Xf;
   const int LB = B.Bi->LB;
   int64_t mlo, mhi;
   dim_range<D>(B, mlo, mhi);
@@ -2425,25 +2936,23 @@ __global__ void __launch_bounds__(kCellThreads) k_union_heavy(const gdl::Bufs B,
     const unsigned long long open = B.hv_mask[h];
     const int b = B.reps[m];
     const int e = B.reps[m + 1];
-    const CellCtx cx = cell_ctx<KEY64>(B, b, LB);
+    const CellCtx cx = cell_ctx<KEY64>(B, m, LB);
     const DevParams& P = *cx.P;
     const PredParams Q = pred_params(P);
-    const GridView gv = view_of(B, P);
     const CellXYZ<D> cc = decompose<D>(cx.local, P);
     for (int t0 = 0; t0 < T.n; t0 += 32) {
       const int tt = t0 + lane;
       bool cand = false;
       int bB = 0, eB = 0, cB = 0;
       if (tt < T.n && ((open >> tt) & 1ull)) {
-        const int64_t kb = offset_key<D>(cc, T.o[tt][0], T.o[tt][1], T.o[tt][2], P);
-        if (kb >= 0) {
-          const int2 cb = gv.cell(B, (uint64_t)kb);
-          bB = cb.x;
-          eB = cb.y;
-          if (bB < eB) {
-            cB = cell_of(B, bB);
-            cand = B.cellcore[cB] > 0 && uf_find(B.parent, cB) != uf_find(B.parent, (int)m);
-          }
+        const int c = find_cell<D, KEY64>(B, P, (int64_t)cc.c[0] + T.o[tt][0],
+                                          (int64_t)cc.c[1] + T.o[tt][1],
+                                          (int64_t)cc.c[2] + T.o[tt][2]);
+        if (c >= 0) {
+          cB = c;
+          bB = B.reps[c];
+          eB = B.reps[c + 1];
+          cand = B.cellcore[cB] > 0 && uf_find(B.parent, cB) != uf_find(B.parent, (int)m);
         }
       }
       unsigned mask = __ballot_sync(kFull, cand);
@@ -2459,21 +2968,18 @@ __global__ void __launch_bounds__(kCellThreads) k_union_heavy(const gdl::Bufs B,
           const int q = qb + lane;
           const bool valid = q < ceB && B.core[q];
           Cand<D, F32> c;
-          if (valid) load_cand<D, F32>(c, X, Xf, n, q);
+          if (valid) load_cand<D, F32>(c, B, q);
           for (int a = b; a < e && !found; ++a) {
             if (!B.core[a]) continue;
             double ax[D];
             float af[D];
-#pragma unroll
-            for (int k = 0; k < D; ++k) {
-              if (!F32) ax[k] = X[k * n + a];
-              if (F32) af[k] = Xf[k * n + a];
-            }
-            bool hit = valid && link_test<D, F32>(ax, af, c, X, n, a, q, Q, t, B.asym, B.ctr);
+            if (F32) ld_f<D>(B, a, af);
+            else ld_x<D>(B, a, ax);
+            bool hit = valid && link_test<D, F32>(ax, af, c, B, P, a, q, Q, t);
             found = __any_sync(kFull, hit);
           }
         }
-        if (found && lane == 0) uf_union(B.parent, B.cellmin, (int)m, ccB);
+        if (found && lane == 0) uf_union(B.parent, (int)m, ccB);
         __syncwarp();
       }
     }
@@ -2494,7 +3000,7 @@ __global__ void __launch_bounds__(kCellThreads) k_union_heavy(const gdl::Bufs B,
 // links.  Absorbed roots are re-parented under the opening root.  One thread;
 // the list holds at most kAsymCap links (more is reported as an error).
 __global__ void k_asym_resolve(const gdl::Bufs B) {
-  const int* __restrict__ cellmin = B.cellmin;
+  const int* __restrict__ cellmin = B.compmin;  // per root: the component's smallest core index
   int* parent = B.parent;
   const int* __restrict__ asym_list = B.asym;
   unsigned long long* ctr = B.ctr;
@@ -2556,13 +3062,60 @@ __global__ void k_asym_resolve(const gdl::Bufs B) {
     if (assigned[v] != node[v]) parent[node[v]] = assigned[v];
 }
 
-// parent[m] <- root (full path compression)
-__global__ void k_compress(const gdl::Bufs B) {
+// parent[m] <- root (full path compression).  slot[D] (for the cells of that
+// dimension, -1: none): the word of each block's entry (0: lo, 1: hi) that gets
+// the block's root when all its core cells have the same one, kMixedRoot when not,
+// for the next union pass (one atomic per run of lanes of one block).
+__global__ void k_compress(const gdl::Bufs B, int slot2, int slot3) {
+  const int64_t M = *B.M, M2 = (int64_t)B.ctr[kCtrCells2D];
+  const int lane = threadIdx.x & 31;
+  for (int64_t m0 = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); m0 < M;
+       m0 += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t m = m0 + lane;
+    const bool on = m < M && B.cellcore[m] > 0;
+    int r = 0;
+    uint32_t e = 0;
+    if (on) {
+      r = uf_find(B.parent, (int)m);
+      B.parent[m] = r;
+      e = B.cellent[m];
+    }
+    const int slot = m < M2 ? slot2 : slot3;
+    const bool mk = on && slot >= 0;
+    const unsigned grp = run_peers(__ballot_sync(kFull, mk), (int)e);
+    if (mk) {
+      const unsigned lo = __reduce_min_sync(grp, (unsigned)r), hi = __reduce_max_sync(grp, (unsigned)r);
+      if (lane == __ffs(grp) - 1) {
+        uint32_t* u = slot == 0 ? &B.ent[e].lo : &B.ent[e].hi;
+        uint32_t old = lo == hi ? atomicCAS(u, kNoEnt, lo) : kMixedRoot;
+        if (old != kNoEnt && old != lo) atomicExch(u, kMixedRoot);
+      }
+    }
+  }
+}
+
+// The smallest core index of every component, kept at its root (compmin starts as
+// every core cell's own).  Roots are the cells of smallest index; most cells find a
+// smaller value already in place, so few atomics are left.
+__global__ void k_comp_min(const gdl::Bufs B) {
   const int64_t M = *B.M;
-  for (int64_t m = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; m < M;
-       m += (int64_t)gridDim.x * blockDim.x) {
-    if (B.cellcore[m] == 0) continue;
-    B.parent[m] = uf_find(B.parent, (int)m);
+  const int lane = threadIdx.x & 31;
+  for (int64_t m0 = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); m0 < M;
+       m0 += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t m = m0 + lane;
+    const bool on = m < M && B.cellcore[m] > 0;
+    int r = 0;
+    if (on) {
+      r = uf_find(B.parent, (int)m);
+      B.parent[m] = r;
+    }
+    const bool sub = on && r != (int)m;
+    const unsigned grp = run_peers(__ballot_sync(kFull, sub), r);
+    if (sub) {
+      const int mn = (int)__reduce_min_sync(grp, (unsigned)B.cellmin[m]);
+      if (lane == __ffs(grp) - 1 && mn < *reinterpret_cast<volatile int*>(B.compmin + r))
+        atomicMin(B.compmin + r, mn);
+    }
   }
 }
 
@@ -2572,9 +3125,11 @@ __global__ void k_roots(const gdl::Bufs B) {
   const int64_t M = *B.M;
   for (int64_t m = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; m < M;
        m += (int64_t)gridDim.x * blockDim.x) {
+    BlockEnt& E = B.ent[B.cellent[m]];
+    if (E.base == (uint32_t)m) E.lo = INT_MAX;  // smallest cluster id, set by k_cell_ids
     if (B.cellcore[m] == 0) continue;
     if (uf_find(B.parent, (int)m) == (int)m) {
-      const uint32_t cm = (uint32_t)B.cellmin[m];
+      const uint32_t cm = (uint32_t)B.compmin[m];
       atomicOr(B.fbits + (cm >> 5), 1u << (cm & 31));
     }
   }
@@ -2583,20 +3138,31 @@ __global__ void k_roots(const gdl::Bufs B) {
 // Per cell: the cluster id of its core points (the rank of its root's mark,
 // less the marks of the instances before it: cluster numbers restart at 0 in
 // every instance), INT_MAX without core points.
+// Each block's smallest id goes to its entry (one atomic per run of lanes of
+// one block).
 template <bool KEY64>
 __global__ void k_cell_ids(const gdl::Bufs B) {
   const int LB = B.Bi->LB;
   const int64_t M = *B.M;
-  for (int64_t m = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; m < M;
-       m += (int64_t)gridDim.x * blockDim.x) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t m0 = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); m0 < M;
+       m0 += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t m = m0 + lane;
     int cid = INT_MAX;
-    if (B.cellcore[m] > 0) {
-      const uint64_t key = key_at<KEY64>(B, B.reps[m]);
-      const DevParams& P = B.Pv[(int)(key >> LB)];
-      const int64_t root_min = B.cellmin[uf_find(B.parent, (int)m)];
+    uint32_t e = 0;
+    const bool on = m < M && B.cellcore[m] > 0;
+    if (on) {
+      const DevParams& P = B.Pv[inst_of(ckey_at<KEY64>(B, m), LB)];
+      const int64_t root_min = B.compmin[uf_find(B.parent, (int)m)];
       cid = (int)(bit_rank(B.fbits, B.fpre, root_min) - bit_rank(B.fbits, B.fpre, P.pt_off));
+      e = B.cellent[m];
     }
-    B.cellcid[m] = cid;
+    if (m < M) B.cellcid[m] = cid;
+    const unsigned grp = run_peers(__ballot_sync(kFull, on), (int)e);
+    if (on) {
+      const unsigned mn = __reduce_min_sync(grp, (unsigned)cid);
+      if (lane == __ffs(grp) - 1) atomicMin(&B.ent[e].lo, mn);
+    }
   }
 }
 
@@ -2641,8 +3207,6 @@ __global__ void __launch_bounds__(kCellThreads) k_border_heavy(const gdl::Bufs B
   dim_range<D>(B, mlo, mhi);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   WarpStage<D>& S = stage[w];
-  const double* __restrict__ X = B.X;
-  const float* __restrict__ Xf = B.Xf;
     const int64_t W = (int64_t)gridDim.x * kWarpsPerBlock;
   const OffTab& T = kFullSt[D - 2];
   Tally t;
@@ -2651,10 +3215,9 @@ __global__ void __launch_bounds__(kCellThreads) k_border_heavy(const gdl::Bufs B
     const int64_t m = B.hv_cell[h];
     if (m < mlo || m >= mhi) continue;
     const int b = B.reps[m], e = B.reps[m + 1];
-    const CellCtx cx = cell_ctx<KEY64>(B, b, LB);
+    const CellCtx cx = cell_ctx<KEY64>(B, m, LB);
     const DevParams& P = *cx.P;
     const PredParams Q = pred_params(P);
-    const GridView gv = view_of(B, P);
     const CellXYZ<D> cc = decompose<D>(cx.local, P);
     for (int c0 = b; c0 < e; c0 += 32) {
       // stage this chunk's non-core points
@@ -2666,11 +3229,8 @@ __global__ void __launch_bounds__(kCellThreads) k_border_heavy(const gdl::Bufs B
       if (nc) {
         const int slot = __popc(ncm & ((1u << lane) - 1u));
         sIdx[w][slot] = i;
-#pragma unroll
-        for (int k = 0; k < D; ++k) {
-          if (!F32) S.x[slot][k] = X[k * n + i];
-          if (F32) S.f[slot][k] = Xf[k * n + i];
-        }
+        if (F32) ld_f<D>(B, i, S.f[slot]);
+        else ld_x<D>(B, i, S.x[slot]);
       }
       __syncwarp();
       int best = INT_MAX;  // lane j < na: best cluster of staged point j
@@ -2679,15 +3239,14 @@ __global__ void __launch_bounds__(kCellThreads) k_border_heavy(const gdl::Bufs B
         bool has = false;
         int bB = 0, eB = 0, cid = INT_MAX;
         if (tt < T.n) {
-          const int64_t kb = offset_key<D>(cc, T.o[tt][0], T.o[tt][1], T.o[tt][2], P);
-          if (kb >= 0) {
-            const int2 cb = gv.cell(B, (uint64_t)kb);
-            bB = cb.x;
-            eB = cb.y;
-            if (bB < eB) {
-              cid = B.cellcid[cell_of(B, bB)];  // INT_MAX without core points
-              has = cid != INT_MAX;
-            }
+          const int c = find_cell<D, KEY64>(B, P, (int64_t)cc.c[0] + T.o[tt][0],
+                                            (int64_t)cc.c[1] + T.o[tt][1],
+                                            (int64_t)cc.c[2] + T.o[tt][2]);
+          if (c >= 0) {
+            bB = B.reps[c];
+            eB = B.reps[c + 1];
+            cid = B.cellcid[c];  // INT_MAX without core points
+            has = cid != INT_MAX;
           }
         }
         unsigned mask = __ballot_sync(kFull, has);
@@ -2702,12 +3261,12 @@ __global__ void __launch_bounds__(kCellThreads) k_border_heavy(const gdl::Bufs B
             const int q = qb + lane;
             const bool valid = q < ceB && B.core[q];
             Cand<D, F32> c;
-            if (valid) load_cand<D, F32>(c, X, Xf, n, q);
+            if (valid) load_cand<D, F32>(c, B, q);
             unsigned pending = wantm;
             while (pending) {
               const int j = __ffs(pending) - 1;
               pending &= pending - 1;
-              bool hit = valid && pair_test<D, F32>(S.x[j], S.f[j], c, X, n, q, sIdx[w][j], false, Q, t);
+              bool hit = valid && pair_test<D, F32>(S.x[j], S.f[j], c, B, P, q, sIdx[w][j], false, Q, t);
               if (__any_sync(kFull, hit)) {
                 if (lane == j) best = cB;
                 wantm &= ~(1u << j);
@@ -2798,10 +3357,11 @@ static int grid_for(int64_t work, int threads, int sms, int per_sm) {
 }
 
 int grids(const Bufs& B, int K, int nchunks, double mult2, double mult3, uint64_t dense_floor,
-          uint64_t dense_per_point, cudaStream_t s) {
+          uint64_t dense_per_point, uint64_t rows_floor, cudaStream_t s) {
   k_bbox_init<<<(K + 255) / 256, 256, 0, s>>>(B, K);
   if (nchunks > 0) k_bbox_chunk<<<nchunks, kBboxThreads, 0, s>>>(B);
-  k_params_inst<<<(K + 127) / 128, 128, 0, s>>>(B, K, mult2, mult3, dense_floor, dense_per_point);
+  k_params_inst<<<(K + 127) / 128, 128, 0, s>>>(B, K, mult2, mult3, dense_floor, dense_per_point,
+                                                rows_floor);
   k_layout<<<1, 1024, 0, s>>>(B, K);
   return 3 + (nchunks > 0 ? 1 : 0);
 }
@@ -2839,48 +3399,30 @@ static int scan_launches(int64_t nw) { return gdprim::scan_launches(nw); }
 
 // the set bits of B.lbits over [0, n) listed in order into B.blist, their
 // count in *B.lcount
-static int list_bits(const Bufs& B, int64_t n, int sms, void* scan_temp, cudaStream_t s) {
+static int list_bits(const Bufs& B, int64_t n, void* scan_temp, cudaStream_t s) {
   const int64_t nw = (n + 31) / 32;
-  gdprim::exclusive_scan_popc(B.lbits, B.lpre, nw, scan_temp, B.lcount, s, B.ctr + kCtrWaitTimeouts);
-  gdprim::compact_bits(B.lbits, B.lpre, nw, B.blist, sms, s);
-  return scan_launches(nw) + (nw > 0 ? 1 : 0);
+  gdprim::list_bits(B.lbits, B.lpre, nw, B.blist, scan_temp, B.lcount, s, B.ctr + kCtrWaitTimeouts);
+  return nw > 0 ? 1 : 0;
 }
 
-int runs(const Bufs& B, bool key64, int64_t n, bool mixed, int sms, void* scan_temp,
-         cudaStream_t s) {
-  const int g = grid_for(n, 256, sms, 8);
-  const int64_t nw = (n + 31) / 32;
-  if (key64) k_run_bits<unsigned long long><<<g, 256, 0, s>>>(
-      static_cast<const unsigned long long*>(B.keys), n, B.runbits);
-  else k_run_bits<uint32_t><<<g, 256, 0, s>>>(static_cast<const uint32_t*>(B.keys), n, B.runbits);
-  gdprim::exclusive_scan_popc(B.runbits, B.runpre, nw, scan_temp, B.M, s, B.ctr + kCtrWaitTimeouts);
-  gdprim::compact_bits(B.runbits, B.runpre, nw, reinterpret_cast<uint32_t*>(B.reps), sms, s);
-  if (key64) k_runs_finish<unsigned long long><<<1, 32, 0, s>>>(B, n, mixed ? 1 : 0);
-  else k_runs_finish<uint32_t><<<1, 32, 0, s>>>(B, n, mixed ? 1 : 0);
-  return 3 + scan_launches(nw);
-}
-
-int cell_counts(const Bufs& B, bool key64, int64_t n, int sms, cudaStream_t s) {
-  if (key64) k_cell_counts<unsigned long long><<<grid_for(n, 256, sms, 8), 256, 0, s>>>(B);
-  else k_cell_counts<uint32_t><<<grid_for(n, 256, sms, 8), 256, 0, s>>>(B);
+int runs(const Bufs& B, bool key64, int64_t n, void* scan_temp, cudaStream_t s) {
+  const int64_t T = (n + kRunTile - 1) / kRunTile;
+  using U64 = unsigned long long;
+  void* ck = const_cast<void*>(B.ckeys);
+  gdprim::LookbackCtl* ctl = gdprim::lb_ctl(scan_temp);
+  unsigned long long* st = gdprim::lb_status(scan_temp);
+  if (key64)
+    k_runs<U64><<<(unsigned)T, kRunThreads, 0, s>>>(B, n, static_cast<U64*>(ck), (unsigned)T, ctl, st);
+  else
+    k_runs<uint32_t><<<(unsigned)T, kRunThreads, 0, s>>>(B, n, static_cast<uint32_t*>(ck),
+                                                         (unsigned)T, ctl, st);
   return 1;
 }
 
-int start_fill(const Bufs& B, int K, cudaStream_t s) {
-  k_start_fill<<<(K + 127) / 128, 128, 0, s>>>(B, K);
-  return 1;
-}
-
-int occ_rank(const Bufs& B, int K, void* scan_temp, cudaStream_t s) {
-  if (!B.occ_words) return 0;
-  gdprim::exclusive_scan_popc(B.occ, B.wpre, (int64_t)B.occ_words, scan_temp, nullptr, s, B.ctr + kCtrWaitTimeouts);
-  k_rank_off<<<(K + 127) / 128, 128, 0, s>>>(B, K);
-  return scan_launches((int64_t)B.occ_words) + 1;
-}
-
-int hash_insert(const Bufs& B, bool key64, int64_t n, int sms, cudaStream_t s) {
-  if (key64) k_row_hash<unsigned long long><<<grid_for(n, 256, sms, 8), 256, 0, s>>>(B);
-  else k_row_hash<uint32_t><<<grid_for(n, 256, sms, 8), 256, 0, s>>>(B);
+int cells(const Bufs& B, bool key64, int64_t n, int sms, cudaStream_t s) {
+  const int g = grid_for(n, kCellsThreads * kCellsU, sms, 8);
+  if (key64) k_cells<unsigned long long><<<g, kCellsThreads, 0, s>>>(B);
+  else k_cells<uint32_t><<<g, kCellsThreads, 0, s>>>(B);
   return 1;
 }
 
@@ -2904,7 +3446,7 @@ int hash_insert(const Bufs& B, bool key64, int64_t n, int sms, cudaStream_t s) {
 
 static int per_dim(int dims) { return ((dims & 1) ? 1 : 0) + ((dims & 2) ? 1 : 0); }
 
-int core(const Bufs& B, int64_t n, int dims, bool f32, bool key64, bool one, int sms,
+int core(const Bufs& B, int64_t n, int dims, bool f32, bool key64, bool one, bool fresh, int sms,
          void* scan_temp, cudaStream_t s) {
   cudaMemsetAsync(B.ctr + kCtrHeavyCore, 0, 8, s);
   // per-cell core counts (0) and smallest core indices (0xffffffff as unsigned)
@@ -2912,28 +3454,39 @@ int core(const Bufs& B, int64_t n, int dims, bool f32, bool key64, bool one, int
   cudaMemsetAsync(B.cellmin, 0xff, (size_t)n * 4, s);
   // dense cells at once; the other points listed in sorted order for the walk
   const int g = grid_for(n, 256, sms, 8);
+  const int chunk = f32 ? kCoreChunk : 1;
   if (key64) {
-    if (one) k_core_split<true, true><<<g, 256, 0, s>>>(B, n);
-    else k_core_split<true, false><<<g, 256, 0, s>>>(B, n);
+    if (one) k_core_split<true, true><<<g, 256, 0, s>>>(B, n, chunk, fresh ? 0 : 1);
+    else k_core_split<true, false><<<g, 256, 0, s>>>(B, n, chunk, fresh ? 0 : 1);
   } else {
-    if (one) k_core_split<false, true><<<g, 256, 0, s>>>(B, n);
-    else k_core_split<false, false><<<g, 256, 0, s>>>(B, n);
+    if (one) k_core_split<false, true><<<g, 256, 0, s>>>(B, n, chunk, fresh ? 0 : 1);
+    else k_core_split<false, false><<<g, 256, 0, s>>>(B, n, chunk, fresh ? 0 : 1);
   }
-  int L = 1 + list_bits(B, n, sms, scan_temp, s);
+  int L = 1 + list_bits(B, n, scan_temp, s);
   cudaMemsetAsync(B.ctr + kCtrWalkCursor2, 0, 16, s);
-  // 3D walks split after the 3x3 near rows (the first nine of kRows)
-  const int rows2 = kRowsPerDim[0], rows3 = kRowsPerDim[1], near3 = kNearRows3;
+  // 3D walks split after pass 0 (the 3^3 shell)
   if (dims & 2) cudaMemsetAsync(B.fbits, 0, (size_t)B.nw * 4, s);
-  if (dims & 1) GD_L1(2, f32, key64, k_core_point, sms * 8, kScanThreadsPerBlock, B, n, 0, rows2);
+  auto walk = [&](auto dim, int q0, int q1) {
+    constexpr int D = decltype(dim)::value;
+    if (f32) {
+      const int grid = sms * kCoreCellMinBlocks;
+      if (key64) k_core_cell<D, true><<<grid, kCoreThreads, 0, s>>>(B, n, q0, q1);
+      else k_core_cell<D, false><<<grid, kCoreThreads, 0, s>>>(B, n, q0, q1);
+    } else {
+      const int grid = sms * kCoreMinBlocks;
+      if (key64) k_core_point<D, true><<<grid, kCoreThreads, 0, s>>>(B, n, q0, q1);
+      else k_core_point<D, false><<<grid, kCoreThreads, 0, s>>>(B, n, q0, q1);
+    }
+  };
+  if (dims & 1) walk(std::integral_constant<int, 2>{}, 0, 2);
   if (dims & 2) {
-    GD_L1(3, f32, key64, k_core_point, sms * 8, kScanThreadsPerBlock, B, n, 0, near3);
+    walk(std::integral_constant<int, 3>{}, 0, 1);
     // the undecided 3D points, listed in sorted order
-    gdprim::exclusive_scan_popc(B.fbits, B.fpre, B.nw, scan_temp, B.lcount, s,
-                                B.ctr + kCtrWaitTimeouts);
-    gdprim::compact_bits(B.fbits, B.fpre, B.nw, B.blist, sms, s);
+    gdprim::list_bits(B.fbits, B.fpre, B.nw, B.blist, scan_temp, B.lcount, s,
+                      B.ctr + kCtrWaitTimeouts);
     cudaMemsetAsync(B.ctr + kCtrWalkCursor3, 0, 8, s);
-    GD_L1(3, f32, key64, k_core_point, sms * 8, kScanThreadsPerBlock, B, n, near3, rows3);
-    L += scan_launches(B.nw) + 2;
+    walk(std::integral_constant<int, 3>{}, 1, 2);
+    L += 2;
   }
   GD_LAUNCH_DIMS(dims, f32, key64, k_core_heavy, sms * 8, kCellThreads, B, n);
   return L + 2 * per_dim(dims);
@@ -2941,11 +3494,14 @@ int core(const Bufs& B, int64_t n, int dims, bool f32, bool key64, bool one, int
 
 int unite(const Bufs& B, int64_t n, int dims, bool f32, bool key64, int sms, void* scan_temp,
           cudaStream_t s) {
-  if (B.occ_words) cudaMemsetAsync(B.cocc, 0, B.occ_words * 4, s);
   cudaMemsetAsync(B.lbits, 0, (size_t)B.nw * 4, s);
-  if (key64) k_parent_init<true><<<grid_for(n, 256, sms, 8), 256, 0, s>>>(B, n);
-  else k_parent_init<false><<<grid_for(n, 256, sms, 8), 256, 0, s>>>(B, n);
-  int L = 1 + list_bits(B, n, sms, scan_temp, s);
+  if (key64) k_core_cells<true><<<grid_for(n, 256, sms, 8), 256, 0, s>>>(B, n);
+  else k_core_cells<false><<<grid_for(n, 256, sms, 8), 256, 0, s>>>(B, n);
+  int L = 1 + list_bits(B, n, scan_temp, s);
+  const int lgrid = grid_for(n, 256, sms, 8);
+  GD_LAUNCH_DIMS(dims, f32, key64, k_links, lgrid, 256, B, n);
+  k_flood<<<grid_for(n, 128, sms, 16), 128, 0, s>>>(B);
+  L += per_dim(dims) + 1;
   int launched = 0;
   for (int pass = 0; pass < kUnionPasses; ++pass) {
     // the dimensions that have this pass
@@ -2961,11 +3517,15 @@ int unite(const Bufs& B, int64_t n, int dims, bool f32, bool key64, int sms, voi
     const bool last = pass == kUnionPasses - 1 ||
                       !(dims & ((pass + 1 < union_passes(2) ? 1 : 0) |
                                 (pass + 1 < union_passes(3) ? 2 : 0)));
-    if (!last) k_compress<<<grid_for(n, 256, sms, 8), 256, 0, s>>>(B);
+    // (the entries' word for pass 1 is lo, for pass 2 hi)
+    if (!last)
+      k_compress<<<grid_for(n, 256, sms, 8), 256, 0, s>>>(B, pass + 1 < union_passes(2) ? pass : -1,
+                                                          pass + 1 < union_passes(3) ? pass : -1);
     launched += 2 * per_dim(pd) + (last ? 0 : 1);
   }
+  k_comp_min<<<grid_for(n, 256, sms, 8), 256, 0, s>>>(B);
   k_asym_resolve<<<1, 32, 0, s>>>(B);
-  return L + launched + 1;
+  return L + launched + 2;
 }
 
 int roots(const Bufs& B, bool key64, int64_t n, int sms, void* scan_temp, cudaStream_t s) {
@@ -2980,13 +3540,13 @@ int roots(const Bufs& B, bool key64, int64_t n, int sms, void* scan_temp, cudaSt
 
 int label(const Bufs& B, int64_t n, int sms, void* scan_temp, cudaStream_t s) {
   k_label<<<grid_for(n, 256, sms, 8), 256, 0, s>>>(B, n);
-  return 1 + list_bits(B, n, sms, scan_temp, s);
+  return 1 + list_bits(B, n, scan_temp, s);
 }
 
 int border(const Bufs& B, int64_t n, int dims, bool f32, bool key64, int sms, cudaStream_t s) {
   cudaMemsetAsync(B.ctr + kCtrHeavyBorder, 0, 8, s);
   cudaMemsetAsync(B.ctr + kCtrWalkCursor2, 0, 16, s);
-  GD_LAUNCH_DIMS(dims, f32, key64, k_border_point, sms * 8, kScanThreadsPerBlock, B, n);
+  GD_LAUNCH_DIMS(dims, f32, key64, k_border_point, sms * kBorderMinBlocks, kBorderThreads, B, n);
   GD_LAUNCH_DIMS(dims, f32, key64, k_border_heavy, sms * 8, kCellThreads, B, n);
   return 2 * per_dim(dims);
 }

@@ -1,13 +1,6 @@
 // gd_prims.cu -- device primitives: exclusive scan and a stable LSD radix sort.
 //
-// The scan is a single-pass design with decoupled look-back: each tile
-// publishes its aggregate, reads its predecessors' published values back to the
-// nearest inclusive prefix, and publishes its own inclusive prefix.  Tiles take
-// their index from an atomic counter when their block starts, so a tile only
-// waits on tiles that running blocks hold and every wait ends; each wait is
-// still bounded (kWaitPolls polls), and a wait that gives up counts the
-// predecessor as 0 -- every offset then stays at or below its true value, so no
-// write leaves its array -- and is reported through the caller's counter.
+// Scans are single-pass, with decoupled look-back (gd_lookback.cuh).
 //
 // Scan (u32): tiles of 8192 elements (512 threads x 16 contiguous items), one
 // launch (k_scan_onepass): reads 4 B, writes 4 B/elem.  Against the earlier
@@ -25,13 +18,8 @@
 // ms): with about 760 tiles in flight the serial per-digit look-back chains
 // cost more than the upsweep and the histogram scan they replace.
 // This replaces thrust::sort_by_key (main.cu:332).
-//
-// The scan's state between launches lives in the caller's temp memory, which
-// must be zero when first used (the callers clear it when they allocate it): a
-// control block (tile counter, finished-block counter, launch epoch) that the
-// last block of each launch resets, and the status words, tagged with the
-// launch's epoch so that words left by earlier launches read as not ready.
 #include "gd_internal.cuh"
+#include "gd_lookback.cuh"
 
 namespace gdprim {
 
@@ -41,138 +29,11 @@ constexpr int kScanThreads = 512;
 constexpr int kScanItems = 16;
 constexpr int kScanTile = kScanThreads * kScanItems;
 
-__device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v, int lane) {
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    uint32_t t = __shfl_up_sync(gd::kFull, v, o);
-    if (lane >= o) v += t;
-  }
-  return v;
-}
-
-// exclusive scan of one value per thread across a block of NT threads
-template <int NT>
-__device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* s_warp,
-                                                    uint32_t* block_total) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  constexpr int NW = NT / 32;
-  uint32_t inc = warp_incl_scan(v, lane);
-  if (lane == 31) s_warp[w] = inc;
-  __syncthreads();
-  if (w == 0) {
-    uint32_t t = lane < NW ? s_warp[lane] : 0u;
-    uint32_t ti = warp_incl_scan(t, lane);
-    if (lane < NW) s_warp[lane] = ti - t;
-    if (lane == NW - 1 && block_total) *block_total = ti;
-  }
-  __syncthreads();
-  uint32_t r = s_warp[w] + inc - v;
-  __syncthreads();
-  return r;
-}
-
 // value of one scanned element: the element itself, or (POPC) the number of
 // set bits of a 32-bit word
 template <bool POPC>
 __device__ __forceinline__ uint32_t scan_val(uint32_t x) {
   return POPC ? (uint32_t)__popc(x) : x;
-}
-
-// ------------------------------------------------------------ look-back state
-struct LookbackCtl {
-  unsigned int tile;   // next tile index of the running launch
-  unsigned int done;   // blocks of the running launch that finished
-  unsigned int epoch;  // launches completed on this control block
-  unsigned int pad[13];
-};
-static_assert(sizeof(LookbackCtl) == 64, "control block is 64 bytes");
-
-// A predecessor tile's block is already running when its tile is waited on, so
-// its aggregate follows within microseconds; 2^14 polls (about 16 ms) only end
-// waits that could never succeed.
-constexpr unsigned kWaitPolls = 1u << 14;
-
-__device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long* p) {
-  unsigned long long v;
-  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return v;
-}
-
-__device__ __forceinline__ void st_relaxed_u64(unsigned long long* p, unsigned long long v) {
-  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-
-// status word: tag (bits 63..34), kind (33..32: 1 aggregate, 2 inclusive
-// prefix), value (31..0)
-__device__ __forceinline__ unsigned long long lb_word(uint32_t tag, uint32_t kind, uint32_t v) {
-  return ((unsigned long long)tag << 34) | ((unsigned long long)kind << 32) | v;
-}
-
-// A tile's status word once it carries this launch's tag: its kind (1 or 2)
-// and value; kind 0 (value 0) when kWaitPolls polls saw nothing.
-__device__ __forceinline__ uint32_t lb_wait(const unsigned long long* p, uint32_t tag,
-                                            uint32_t& v) {
-  for (unsigned it = 0; it < kWaitPolls; ++it) {
-    const unsigned long long w = ld_relaxed_u64(p);
-    const uint32_t kind = (uint32_t)(w >> 32) & 3u;
-    if ((uint32_t)(w >> 34) == tag && kind != 0u) {
-      v = (uint32_t)w;
-      return kind;
-    }
-    if (it >= 4) __nanosleep(64);
-  }
-  v = 0;
-  return 0;
-}
-
-// Block start: the tile index (from the counter) and the launch's tag.
-__device__ __forceinline__ void lb_begin(LookbackCtl* ctl, unsigned* s_tile, unsigned* s_epoch) {
-  if (threadIdx.x == 0) {
-    *s_tile = atomicAdd(&ctl->tile, 1u);
-    *s_epoch = *reinterpret_cast<volatile unsigned*>(&ctl->epoch);
-  }
-  __syncthreads();
-}
-
-__device__ __forceinline__ uint32_t lb_tag(unsigned epoch) { return (epoch & 0x3fffffffu) + 1u; }
-
-// Block end, after every thread is done with the status words: the last block
-// of the launch resets the counters and advances the epoch for the next one.
-__device__ __forceinline__ void lb_end(LookbackCtl* ctl, unsigned tiles, unsigned epoch) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    if (atomicAdd(&ctl->done, 1u) == tiles - 1u) {
-      ctl->tile = 0u;
-      ctl->done = 0u;
-      ctl->epoch = epoch + 1u;
-    }
-  }
-}
-
-// Exclusive prefix of tile `tile` from its predecessors' status words, by one
-// warp (32 predecessors per round, nearest first).  *gave_up: a wait ran out.
-__device__ __forceinline__ uint32_t lb_warp_prefix(const unsigned long long* status, int64_t tile,
-                                                   uint32_t tag, bool* gave_up) {
-  const int lane = threadIdx.x & 31;
-  uint32_t excl = 0;
-  bool lost = false;
-  for (int64_t top = tile - 1; top >= 0; top -= 32) {
-    const int64_t k = top - lane;
-    uint32_t v = 0, kind = 2;  // before tile 0: an inclusive prefix of 0
-    if (k >= 0) kind = lb_wait(status + k, tag, v);
-    lost |= __any_sync(gd::kFull, kind == 0u);
-    // nearest lane holding a prefix (or a wait that gave up): sum up to it
-    const unsigned stop = __ballot_sync(gd::kFull, kind != 1u);
-    const int last = stop ? __ffs(stop) - 1 : 31;
-    uint32_t add = lane <= last ? v : 0u;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) add += __shfl_xor_sync(gd::kFull, add, o);
-    excl += add;
-    if (stop) break;
-  }
-  *gave_up = lost;
-  return excl;
 }
 
 // Single-pass exclusive scan (decoupled look-back).
@@ -212,21 +73,9 @@ k_scan_onepass(const uint32_t* in, uint32_t* out, int64_t n, unsigned tiles, Loo
 #pragma unroll
   for (int i = 0; i < kScanItems; ++i) sum += v[i];
   uint32_t ex = block_excl_scan<kScanThreads>(sum, s_warp, &s_agg);
-  if (threadIdx.x < 32) {
-    const uint32_t agg = s_agg;
-    unsigned long long* my = status + tile;
-    if (threadIdx.x == 0) st_relaxed_u64(my, lb_word(tag, tile == 0 ? 2u : 1u, agg));
-    bool lost = false;
-    const uint32_t excl = tile == 0 ? 0u : lb_warp_prefix(status, (int64_t)tile, tag, &lost);
-    if (threadIdx.x == 0) {
-      if (tile != 0) st_relaxed_u64(my, lb_word(tag, 2u, excl + agg));
-      s_excl = excl;
-      if (lost && timeouts) atomicAdd(timeouts, 1ull);
-      if (tile == tiles - 1u && total_dev) *total_dev = excl + agg;
-    }
-  }
-  __syncthreads();
-  ex += s_excl;
+  const uint32_t excl = lb_tile_prefix(status, tile, tag, &s_agg, &s_excl, timeouts);
+  if (threadIdx.x == 0 && tile == tiles - 1u && total_dev) *total_dev = excl + s_agg;
+  ex += excl;
 #pragma unroll
   for (int i = 0; i < kScanItems; ++i) {
     uint32_t t = v[i];
@@ -385,30 +234,59 @@ k_rs_downsweep(const K* __restrict__ kin, const uint32_t* __restrict__ vin,
   }
 }
 
-// positions of the set bits, in order: out[pre[w] + r] = 32 w + (bit r of word
-// w).  A warp takes 32 words (one per lane), then writes them one word at a
-// time with a lane per bit, so each word's entries go out in one store.
-__global__ void k_compact_bits(const uint32_t* __restrict__ words,
-                               const uint32_t* __restrict__ pre, int64_t nw,
-                               uint32_t* __restrict__ out) {
-  const int lane = threadIdx.x & 31;
-  const unsigned below = (1u << lane) - 1u;
-  const int64_t step = (int64_t)gridDim.x * blockDim.x;  // 32 words per warp
-  for (int64_t w0 = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); w0 < nw;
-       w0 += step) {
-    const int64_t w = w0 + lane;
-    const uint32_t x = w < nw ? words[w] : 0u;
-    const uint32_t p = w < nw ? pre[w] : 0u;
-    unsigned busy = __ballot_sync(gd::kFull, x != 0u);
-    while (busy) {
-      const int src = __ffs(busy) - 1;
-      busy &= busy - 1;
-      const uint32_t xs = __shfl_sync(gd::kFull, x, src);
-      const uint32_t ps = __shfl_sync(gd::kFull, p, src);
-      if ((xs >> lane) & 1u)
-        out[ps + (uint32_t)__popc(xs & below)] = (uint32_t)((w0 + src) << 5) + (uint32_t)lane;
-    }
+// Set bits of a mask listed in one pass: per-word prefix counts (pre) and the
+// positions of the set bits in order (out[pre[w] + r] = 32 w + (bit r of word w)).
+// A tile is 2048 words (512 threads x 4): word counts are scanned in the block, the
+// tile's prefix comes by look-back, and each warp then writes its 128 words one at
+// a time with a lane per bit, so each word's entries go out in one store.  One
+// launch where a scan and a compaction took two.
+constexpr int kListThreads = 512, kListWords = 4, kListTile = kListThreads * kListWords;
+__global__ void __launch_bounds__(kListThreads)
+k_list_bits(const uint32_t* __restrict__ words, uint32_t* __restrict__ pre, int64_t nw,
+            uint32_t* __restrict__ out, unsigned tiles, LookbackCtl* ctl,
+            unsigned long long* status, uint32_t* total_dev, unsigned long long* timeouts) {
+  __shared__ uint32_t s_warp[32];
+  __shared__ unsigned s_tile, s_epoch;
+  __shared__ uint32_t s_agg, s_excl;
+  __shared__ uint32_t s_w[kListTile], s_p[kListTile];
+  lb_begin(ctl, &s_tile, &s_epoch);
+  const unsigned tile = s_tile, epoch = s_epoch;
+  if (tile >= tiles) {
+    // a counter left inconsistent (never expected): no tile, report it
+    if (threadIdx.x == 0 && timeouts) atomicAdd(timeouts, 1ull);
+    lb_end(ctl, tiles, epoch);
+    return;
   }
+  const int64_t base = (int64_t)tile * kListTile;
+  uint32_t v[kListWords], sum = 0;
+#pragma unroll
+  for (int i = 0; i < kListWords; ++i) {
+    const int64_t w = base + threadIdx.x * kListWords + i;
+    v[i] = w < nw ? words[w] : 0u;
+    sum += (uint32_t)__popc(v[i]);
+  }
+  uint32_t ex = block_excl_scan<kListThreads>(sum, s_warp, &s_agg);
+  const uint32_t excl = lb_tile_prefix(status, tile, lb_tag(epoch), &s_agg, &s_excl, timeouts);
+  if (threadIdx.x == 0 && tile == tiles - 1u && total_dev) *total_dev = excl + s_agg;
+  ex += excl;
+#pragma unroll
+  for (int i = 0; i < kListWords; ++i) {
+    const int k = threadIdx.x * kListWords + i;
+    if (base + k < nw) pre[base + k] = ex;
+    s_w[k] = v[i];
+    s_p[k] = ex;
+    ex += (uint32_t)__popc(v[i]);
+  }
+  __syncwarp();  // a warp's words were written by its own lanes
+  const int lane = threadIdx.x & 31, k0 = (threadIdx.x >> 5) * 32 * kListWords;
+  const unsigned below = (1u << lane) - 1u;
+#pragma unroll 4
+  for (int k = k0; k < k0 + 32 * kListWords; ++k) {
+    const uint32_t x = s_w[k];
+    if ((x >> lane) & 1u)
+      out[s_p[k] + (uint32_t)__popc(x & below)] = (uint32_t)((base + k) << 5) + (uint32_t)lane;
+  }
+  lb_end(ctl, tiles, epoch);
 }
 
 __global__ void k_iota(uint32_t* v, int64_t n) {
@@ -437,11 +315,8 @@ void scan_impl(const uint32_t* in, uint32_t* out, int64_t n, void* temp, uint32_
     return;
   }
   const int64_t T = (n + kScanTile - 1) / kScanTile;
-  LookbackCtl* ctl = static_cast<LookbackCtl*>(temp);
-  unsigned long long* status =
-      reinterpret_cast<unsigned long long*>(static_cast<char*>(temp) + sizeof(LookbackCtl));
-  k_scan_onepass<POPC><<<(unsigned)T, kScanThreads, 0, s>>>(in, out, n, (unsigned)T, ctl, status,
-                                                            total_dev, timeouts);
+  k_scan_onepass<POPC><<<(unsigned)T, kScanThreads, 0, s>>>(in, out, n, (unsigned)T, lb_ctl(temp),
+                                                            lb_status(temp), total_dev, timeouts);
 }
 
 void exclusive_scan_u32(const uint32_t* in, uint32_t* out, int64_t n, void* temp,
@@ -454,12 +329,15 @@ void exclusive_scan_popc(const uint32_t* words, uint32_t* pre, int64_t nw, void*
   scan_impl<true>(words, pre, nw, temp, total_dev, s, timeouts);
 }
 
-void compact_bits(const uint32_t* words, const uint32_t* pre, int64_t nw, uint32_t* out, int sms,
-                  cudaStream_t s) {
-  if (nw <= 0) return;
-  int64_t g = (nw + 255) / 256;
-  if (g > (int64_t)sms * 8) g = (int64_t)sms * 8;
-  k_compact_bits<<<(unsigned)g, 256, 0, s>>>(words, pre, nw, out);
+void list_bits(const uint32_t* words, uint32_t* pre, int64_t nw, uint32_t* out, void* temp,
+               uint32_t* total_dev, cudaStream_t s, unsigned long long* timeouts) {
+  if (nw <= 0) {
+    cudaMemsetAsync(total_dev, 0, sizeof(uint32_t), s);
+    return;
+  }
+  const int64_t T = (nw + kListTile - 1) / kListTile;
+  k_list_bits<<<(unsigned)T, kListThreads, 0, s>>>(words, pre, nw, out, (unsigned)T, lb_ctl(temp),
+                                                   lb_status(temp), total_dev, timeouts);
 }
 
 // sort temp: the [digit][tile] histogram.  Its scan keeps its state in the
