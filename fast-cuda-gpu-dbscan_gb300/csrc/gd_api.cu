@@ -112,6 +112,12 @@ struct gd_ctx {
   uint32_t* sids = nullptr;
   uint32_t hmask = 0;
   cudaEvent_t ev[8] = {};
+  bool times_due = false;  // the last run's events have not been read into st yet
+  // a small run (gd_small.cuh): its arguments, and the pinned mirror of the small block
+  bool is_small = false;
+  gd::SmallArgs sa{};
+  DevBuf asymwork;
+  unsigned char* mirror = nullptr;
   // CUDA graph of the expand launches, captured on the second gd_expand of one
   // index build and replayed by later ones (minpts sweeps)
   bool graphs = true;
@@ -157,7 +163,7 @@ struct gd_ctx {
                    &keys1,  &vals0,  &vals1,    &X,       &Xf,     &ent,      &links, &cellent, &blklist, &rowtab, &hkeys,
                    &hvals,  &reps,   &bits,     &core,    &cellcore, &cellmin, &cellrep,
                    &parent, &cellcid,  &lab,     &asym,   &hvcell,   &hvmask,
-                   &out,    &coreout, &sorttemp, &scantemp, &small, &kcount};
+                   &out,    &coreout, &sorttemp, &scantemp, &small, &kcount, &asymwork};
     for (DevBuf* b : a) {
       if (keep_small && b == &small) continue;
       if (b->p) cudaFree(b->p);
@@ -166,7 +172,9 @@ struct gd_ctx {
     }
   }
 
-  // small block: M | total clusters | counters
+  // small block (kSmallBlock bytes): M | total clusters | counters | (small runs:) run
+  // layout, barrier
+  static constexpr size_t kSmallBlock = 4096, kMirror = 2048, kBiAt = 1024, kBarAt = 2048;
   uint32_t* dM() { return static_cast<uint32_t*>(small.p); }
   uint32_t* dK() { return reinterpret_cast<uint32_t*>(static_cast<char*>(small.p) + 4); }
   unsigned long long* dCtr() {
@@ -217,9 +225,43 @@ struct gd_ctx {
     B.tn_border = tn_border;
     return B;
   }
+
+  // the buffers of a small run
+  gdl::Bufs small_bufs() {
+    gdl::Bufs B;
+    char* sm = static_cast<char*>(small.p);
+    B.coords = coords_ptr;
+    B.Pv = static_cast<gd::DevParams*>(Pv.p);
+    B.Bi = reinterpret_cast<gd::BatchInfo*>(sm + kBiAt);
+    B.ids = static_cast<uint32_t*>(vals1.p);
+    gdl::set_bits(B, static_cast<uint32_t*>(bits.p), n);
+    B.M = dM();
+    B.K = dK();
+    B.ent = static_cast<gd::BlockEnt*>(ent.p);
+    B.hkeys = static_cast<unsigned long long*>(hkeys.p);
+    B.hmask = sa.hash_slots - 1;
+    B.X = static_cast<double*>(X.p);
+    B.Xf = static_cast<float*>(Xf.p);
+    B.core = static_cast<uint8_t*>(core.p);
+    B.cellcore = static_cast<int*>(cellcore.p);
+    B.cellmin = static_cast<int*>(cellmin.p);
+    B.parent = static_cast<int*>(parent.p);
+    B.cellcid = static_cast<int*>(cellcid.p);
+    B.lab = static_cast<int*>(lab.p);
+    B.compmin = B.lab;
+    B.asym = static_cast<int*>(asym.p);
+    B.ctr = dCtr();
+    B.tn_link = INT32_MAX;  // links are searched to the end
+    return B;
+  }
 };
 
 namespace {
+
+gd_status grid_too_large() {
+  return fail(GD_ERANGE, "eps-cell grid too large (extent/eps beyond 2^31 cells per axis, or "
+                         "cell keys and instance ids beyond 62 bits)");
+}
 
 // Point runs of at most kChunkPoints points, one instance each.
 void make_chunks(const std::vector<gd::InstDesc>& desc, std::vector<gd::Chunk>& out) {
@@ -235,10 +277,93 @@ void make_chunks(const std::vector<gd::InstDesc>& desc, std::vector<gd::Chunk>& 
     }
 }
 
+// Build stage of a small run (one instance, at most small_points of its dimension).  Returns
+// with ctx->is_small false when its grid is for the general path.
+gd_status build_small(gd_ctx* ctx) {
+  ctx->drop_graph();
+  cudaStream_t s = ctx->stream;
+  const gd::InstDesc& I = ctx->hdesc[0];
+  const int64_t n = I.n;
+  ctx->K = 1;
+  ctx->n = n;
+  const uint64_t dmax = gd::small_direct_max(n);
+  const uint32_t slots = gd::small_hash_slots(n);
+  GD_TRY(ctx->ensure(ctx->Pv, sizeof(gd::DevParams), "instance parameters"));
+  GD_TRY(ctx->ensure(ctx->keys0, n * 8, "point keys"));
+  GD_TRY(ctx->ensure(ctx->keys1, n * 8, "cell keys"));
+  GD_TRY(ctx->ensure(ctx->vals0, n * 4, "point cells"));
+  GD_TRY(ctx->ensure(ctx->vals1, n * 4, "ids"));
+  GD_TRY(ctx->ensure(ctx->bbox, (size_t)ctx->sms * 64, "bounds"));
+  GD_TRY(ctx->ensure(ctx->X, (size_t)n * I.dim * 8, "sorted coordinates"));
+  GD_TRY(ctx->ensure(ctx->Xf, (size_t)n * (I.dim == 3 ? 16 : 8), "f32 coordinates"));
+  GD_TRY(ctx->ensure(ctx->ent, std::max<uint64_t>(dmax, slots) * sizeof(gd::BlockEnt), "block entries"));
+  GD_TRY(ctx->ensure(ctx->hkeys, (uint64_t)slots * 8, "block hash"));
+  GD_TRY(ctx->ensure(ctx->cellent, n * 4, "point places"));
+  GD_TRY(ctx->ensure(ctx->blklist, n * 4, "position cells"));
+  GD_TRY(ctx->ensure(ctx->hvmask, n * 8, "cell ranges"));
+  GD_TRY(ctx->ensure(ctx->hvcell, n * 4, "walk list"));
+  GD_TRY(ctx->ensure(ctx->bits, gdl::bit_layout(n).words * 4, "bit masks"));
+  GD_TRY(ctx->ensure(ctx->core, n, "core flags"));
+  GD_TRY(ctx->ensure(ctx->cellcore, n * 4, "cell core counts"));
+  GD_TRY(ctx->ensure(ctx->cellmin, n * 4, "cell min index"));
+  GD_TRY(ctx->ensure(ctx->cellrep, n * 4, "cell representatives"));
+  GD_TRY(ctx->ensure(ctx->parent, n * 4, "union-find parents"));
+  GD_TRY(ctx->ensure(ctx->cellcid, n * 4, "cell cluster ids"));
+  GD_TRY(ctx->ensure(ctx->lab, n * 4, "labels"));
+  GD_TRY(ctx->ensure(ctx->asym, gd::kAsymCap * 8, "one-directional links"));
+  GD_TRY(ctx->ensure(ctx->asymwork, sizeof(gd::AsymWork), "merge replay"));
+  ctx->is_small = true;
+  ctx->x64 = true;
+  char* sm = static_cast<char*>(ctx->small.p);
+  gd::SmallArgs& A = ctx->sa;
+  A.coords = ctx->coords_ptr + I.co_off;
+  A.n = (int)n;
+  A.dim = I.dim;
+  A.eps = I.eps;
+  A.mult = I.dim == 2 ? ctx->mult2 : ctx->mult3;
+  A.direct_max = dmax;
+  A.hash_slots = slots;
+  A.bar = reinterpret_cast<unsigned*>(sm + gd_ctx::kBarAt);
+  A.part = static_cast<long long*>(ctx->bbox.p);
+  A.ptkey = static_cast<uint64_t*>(ctx->keys0.p);
+  A.cellkey = static_cast<uint64_t*>(ctx->keys1.p);
+  A.ptcell = static_cast<uint32_t*>(ctx->vals0.p);
+  A.ptpos = static_cast<uint32_t*>(ctx->cellent.p);
+  A.pcell = static_cast<uint32_t*>(ctx->blklist.p);
+  A.crange = static_cast<uint2*>(ctx->hvmask.p);
+  A.list = static_cast<uint32_t*>(ctx->hvcell.p);
+  A.cellrep = static_cast<uint32_t*>(ctx->cellrep.p);
+  A.asym = static_cast<gd::AsymWork*>(ctx->asymwork.p);
+  GD_CUDA(cudaMemsetAsync(sm, 0, gd_ctx::kSmallBlock, s), "clear counters");
+  GD_CUDA(gdl::small_index(ctx->small_bufs(), A, ctx->sms, s), "small index launch");
+  GD_CUDA(cudaMemcpyAsync(ctx->mirror, sm, gd_ctx::kMirror, cudaMemcpyDeviceToHost, s),
+          "read run layout");
+  GD_CUDA(cudaStreamSynchronize(s), "small index");
+  std::memcpy(&ctx->bi, ctx->mirror + gd_ctx::kBiAt, sizeof(gd::BatchInfo));
+  const gd::BatchInfo& bi = ctx->bi;
+  const unsigned long long* ctr = reinterpret_cast<const unsigned long long*>(ctx->mirror + 128);
+  if (ctr[gd::kCtrWaitTimeouts]) return fail(GD_ECUDA, "a grid barrier wait gave up");
+  if (bi.flags & gd::kFlagNonFinite) return fail(GD_EINVAL, "input has NaN or Inf coordinates");
+  if (bi.flags & gd::kFlagGridTooLarge) return grid_too_large();
+  if (bi.flags & gd::kFlagNotSmall) {
+    ctx->is_small = false;
+    return GD_OK;
+  }
+  ctx->f32 = ctx->precision == GD_PREC_FP32_BAND && !bi.band_off;
+  ctx->dims = I.dim == 2 ? 1 : 2;
+  ctx->launches = 1;
+  ctx->st.grid_cells = (int64_t)bi.grid_cells;
+  ctx->st.key_bits = bi.LB;
+  ctx->fresh_index = true;
+  ctx->stage = 1;
+  return GD_OK;
+}
+
 // Build stage of a run: ctx->hdesc (internal order, 2D instances first) and
 // ctx->coords_ptr (device) are set by the caller.
 gd_status build_run(gd_ctx* ctx, uint64_t dense_floor, uint64_t rows_floor) {
   ctx->drop_graph();
+  ctx->is_small = false;
   cudaStream_t s = ctx->stream;
   const int K = (int)ctx->hdesc.size();
   ctx->K = K;
@@ -267,9 +392,7 @@ gd_status build_run(gd_ctx* ctx, uint64_t dense_floor, uint64_t rows_floor) {
   GD_CUDA(cudaStreamSynchronize(s), "grid parameters");
   const gd::BatchInfo& bi = ctx->bi;
   if (bi.flags & gd::kFlagNonFinite) return fail(GD_EINVAL, "input has NaN or Inf coordinates");
-  if (bi.flags & gd::kFlagGridTooLarge)
-    return fail(GD_ERANGE, "eps-cell grid too large (extent/eps beyond 2^31 cells per axis, or "
-                           "cell keys and instance ids beyond 62 bits)");
+  if (bi.flags & gd::kFlagGridTooLarge) return grid_too_large();
   ctx->key64 = bi.key64 != 0;
   // float32 filter when asked for; a single instance without a valid band
   // runs the float64 kernels (a batch keeps the filter: such instances send
@@ -378,6 +501,19 @@ cudaError_t launch_expand(gd_ctx* ctx, bool capturing) {
 gd_status expand_run(gd_ctx* ctx) {
   cudaStream_t s = ctx->stream;
   const int64_t n = ctx->n;
+  if (ctx->is_small) {
+    if (!ctx->fresh_index)
+      GD_CUDA(cudaMemsetAsync(ctx->dCtr() + gd::kCtrTests64, 0,
+                              (gd::kCtrWalkCursor3 - gd::kCtrTests64 + 1) * 8, s), "clear counters");
+    ctx->fresh_index = false;
+    cudaEventRecord(ctx->ev[3], s);
+    GD_CUDA(gdl::small_expand(ctx->small_bufs(), ctx->sa, ctx->f32, ctx->hdesc[0].minpts, nullptr,
+                              ctx->sms, s), "small expand launch");
+    cudaEventRecord(ctx->ev[4], s);
+    ctx->expand_launches = 1;
+    ctx->stage = 2;
+    return GD_OK;
+  }
   GD_TRY(ctx->ensure(ctx->core, n, "core flags"));
   GD_TRY(ctx->ensure(ctx->cellcore, n * 4, "cell core counts"));
   GD_TRY(ctx->ensure(ctx->cellmin, n * 4, "cell min index"));
@@ -447,9 +583,13 @@ gd_status finish_run(gd_ctx* ctx, int32_t* labels, uint8_t* is_core, int32_t on_
       cout = static_cast<uint8_t*>(ctx->coreout.p);
     }
   }
-  GD_CUDA(cudaMemsetAsync(ctx->dCtr() + gd::kCtrCore, 0, 2 * 8, s), "clear counters");
-  gdl::Bufs B = ctx->bufs();
-  int fin = gdl::scatter_labels(B, n, out, cout, ctx->sms, s);
+  int fin;
+  if (ctx->is_small) {
+    fin = gdl::small_scatter(ctx->small_bufs(), (int)n, out, cout, ctx->sms, s);
+  } else {
+    GD_CUDA(cudaMemsetAsync(ctx->dCtr() + gd::kCtrCore, 0, 2 * 8, s), "clear counters");
+    fin = gdl::scatter_labels(ctx->bufs(), n, out, cout, ctx->sms, s);
+  }
   cudaEventRecord(ctx->ev[6], s);
   if (!on_device) {
     GD_CUDA(cudaMemcpyAsync(labels, out, n * 4, cudaMemcpyDeviceToHost, s), "copy labels");
@@ -463,12 +603,14 @@ gd_status finish_run(gd_ctx* ctx, int32_t* labels, uint8_t* is_core, int32_t on_
             "copy cluster counts");
   }
   cudaEventRecord(ctx->ev[7], s);
-  unsigned long long ctr[gd::kCtrCount];
-  uint32_t K = 0;
-  GD_CUDA(cudaMemcpyAsync(ctr, ctx->dCtr(), sizeof ctr, cudaMemcpyDeviceToHost, s), "counters");
-  GD_CUDA(cudaMemcpyAsync(&K, ctx->dK(), 4, cudaMemcpyDeviceToHost, s), "cluster count");
+  GD_CUDA(cudaMemcpyAsync(ctx->mirror, ctx->small.p, gd_ctx::kBiAt, cudaMemcpyDeviceToHost, s),
+          "counters");
   cudaError_t e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return cuda_fail(e, "DBSCAN pipeline");
+  uint32_t K;
+  unsigned long long ctr[gd::kCtrCount];
+  std::memcpy(&K, ctx->mirror + 4, 4);
+  std::memcpy(ctr, ctx->mirror + 128, sizeof ctr);
   S.n_points = n;
   S.n_clusters = K;
   S.n_noise = (int64_t)ctr[gd::kCtrNoise];
@@ -494,21 +636,29 @@ gd_status finish_run(gd_ctx* ctx, int32_t* labels, uint8_t* is_core, int32_t on_
     return fail(GD_ERANGE, "more one-directional core neighbour pairs than the merge replay "
                            "holds (2048)");
   }
-  float ms = 0;
-  cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);
-  S.ms_h2d = ms;
-  cudaEventElapsedTime(&ms, ctx->ev[1], ctx->ev[2]);
-  S.ms_index = ms;
-  cudaEventElapsedTime(&ms, ctx->ev[3], ctx->ev[4]);
-  S.ms_core = ms;
-  cudaEventElapsedTime(&ms, ctx->ev[4], ctx->ev[5]);
-  S.ms_union = ms;
-  cudaEventElapsedTime(&ms, ctx->ev[5], ctx->ev[6]);
-  S.ms_label = ms;
-  cudaEventElapsedTime(&ms, ctx->ev[6], ctx->ev[7]);
-  S.ms_d2h = ms;
-  S.ms_total = S.ms_index + S.ms_core + S.ms_union + S.ms_label;
+  ctx->times_due = true;
   return GD_OK;
+}
+
+// The last run's statistics, its phase times read from the events when first asked
+// for.  A small run expands in one kernel, whose time is reported as ms_core.
+const gd_stats& read_stats(gd_ctx* ctx) {
+  gd_stats& S = ctx->st;
+  if (!ctx->times_due) return S;
+  ctx->times_due = false;
+  auto span = [&](int a, int b) {
+    float ms = 0;
+    cudaEventElapsedTime(&ms, ctx->ev[a], ctx->ev[b]);
+    return (double)ms;
+  };
+  S.ms_h2d = span(0, 1);
+  S.ms_index = span(1, 2);
+  S.ms_core = span(3, 4);
+  S.ms_union = ctx->is_small ? 0.0 : span(4, 5);
+  S.ms_label = ctx->is_small ? span(4, 6) : span(5, 6);
+  S.ms_d2h = span(6, 7);
+  S.ms_total = S.ms_index + S.ms_core + S.ms_union + S.ms_label;
+  return S;
 }
 
 // Points of a run on the device: the caller's device pointer, or a copy of
@@ -574,7 +724,12 @@ gd_status gd_ctx_create(int32_t device, gd_ctx** out) {
   }
   c->stream = c->own;
   for (auto& ev : c->ev) cudaEventCreate(&ev);
-  gd_status s = c->ensure(c->small, 4096, "small buffer");
+  gd_status s = c->ensure(c->small, gd_ctx::kSmallBlock, "small buffer");
+  if (s == GD_OK && cudaHostAlloc(reinterpret_cast<void**>(&c->mirror), gd_ctx::kMirror,
+                                  cudaHostAllocDefault) != cudaSuccess) {
+    cudaGetLastError();
+    s = fail(GD_ENOMEM, "pinned counters");
+  }
   if (s != GD_OK) {
     gd_ctx_destroy(c);
     return s;
@@ -589,6 +744,7 @@ void gd_ctx_destroy(gd_ctx* ctx) {
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   ctx->drop_graph();
   ctx->free_all(false);
+  if (ctx->mirror) cudaFreeHost(ctx->mirror);
   for (auto& ev : ctx->ev)
     if (ev) cudaEventDestroy(ev);
   if (ctx->own) cudaStreamDestroy(ctx->own);
@@ -742,6 +898,7 @@ gd_status gd_index_build(gd_ctx* ctx, const gd_points* pts, double eps) {
   ctx->st = gd_stats{};
   ctx->st.n_points = pts->n;
   ctx->launches = 0;
+  ctx->times_due = false;
   cudaEventRecord(ctx->ev[0], ctx->stream);
   GD_TRY(stage_points(ctx, pts->coords, pts->n * pts->dim, pts->on_device));
   cudaEventRecord(ctx->ev[1], ctx->stream);
@@ -751,6 +908,14 @@ gd_status gd_index_build(gd_ctx* ctx, const gd_points* pts, double eps) {
     ctx->n = 0;
     ctx->stage = 1;
     return GD_OK;
+  }
+  // small runs take their own kernels
+  if (pts->n <= gd::small_points(pts->dim)) {
+    GD_TRY(build_small(ctx));
+    if (ctx->is_small) {
+      cudaEventRecord(ctx->ev[2], ctx->stream);
+      return GD_OK;
+    }
   }
   GD_TRY(build_run(ctx, kBlockFloor, kRowFloor));
   cudaEventRecord(ctx->ev[2], ctx->stream);
@@ -766,7 +931,9 @@ gd_status gd_expand(gd_ctx* ctx, int32_t minpts) {
     ctx->stage = 2;
     return GD_OK;
   }
-  if (ctx->K == 1) {
+  if (ctx->is_small) {
+    ctx->hdesc[0].minpts = minpts;
+  } else if (ctx->K == 1) {
     // minpts does not shape the grid: set it in the instance's parameters
     gd::DevParams* P0 = static_cast<gd::DevParams*>(ctx->Pv.p);
     ctx->hdesc[0].minpts = minpts;
@@ -801,7 +968,7 @@ gd_status gd_dbscan(gd_ctx* ctx, const gd_points* pts, double eps, int32_t minpt
   GD_TRY(gd_index_build(ctx, pts, eps));
   GD_TRY(gd_expand(ctx, minpts));
   GD_TRY(gd_get_result(ctx, labels, nullptr, pts->on_device, nullptr, nullptr));
-  if (stats) *stats = ctx->st;
+  if (stats) *stats = read_stats(ctx);
   return GD_OK;
 }
 
@@ -814,6 +981,7 @@ gd_status gd_batch_dbscan(gd_ctx* ctx, int32_t count, const gd_instance* inst,
   ctx->stage = 0;
   ctx->st = gd_stats{};
   ctx->launches = 0;
+  ctx->times_due = false;
   // validate; caller layout offsets; internal order puts 2D instances first
   std::vector<gd::InstDesc> user(count);
   int64_t pt = 0, co = 0;
@@ -856,13 +1024,13 @@ gd_status gd_batch_dbscan(gd_ctx* ctx, int32_t count, const gd_instance* inst,
   GD_TRY(finish_run(ctx, labels, nullptr, on_device, kc.data(), (int)kc.size()));
   if (cluster_counts)
     for (int j = 0; j < count; ++j) cluster_counts[order[j]] = kc[j];
-  if (stats) *stats = ctx->st;
+  if (stats) *stats = read_stats(ctx);
   return GD_OK;
 }
 
 gd_status gd_get_stats(gd_ctx* ctx, gd_stats* stats) {
   if (!ctx || !stats) return fail(GD_EINVAL, "gd_get_stats: NULL argument");
-  *stats = ctx->st;
+  *stats = read_stats(ctx);
   return GD_OK;
 }
 

@@ -217,6 +217,7 @@ constexpr uint64_t kRowsPerPoint = 8;
 
 constexpr int kFlagNonFinite = 1;     // NaN or Inf coordinate
 constexpr int kFlagGridTooLarge = 2;  // cell counts and instance ids beyond 62 bits
+constexpr int kFlagNotSmall = 8;      // the grid is not for the small kernels
 constexpr int kFlagNoShortcut = 4;    // |x| too large relative to eps for the
                                       // box-test shortcut / float32 filter
 
@@ -245,6 +246,50 @@ enum Counter {
 
 // Capacity of the list of one-directional core-core pairs (see k_asym_resolve).
 constexpr int kAsymCap = 2048;
+
+// Work space of the merge replay (k_asym_resolve).
+struct AsymWork {
+  int from[kAsymCap], to[kAsymCap];
+  int node[2 * kAsymCap], assigned[2 * kAsymCap];
+};
+
+// A small run's arguments beside its buffers (gd_small.cuh).
+struct SmallArgs {
+  const double* coords;
+  int n, dim;
+  double eps, mult;
+  uint64_t direct_max;       // blocks a direct table may have
+  uint32_t hash_slots;       // slots of the block hash (power of two); 0: direct grids only
+  unsigned* bar;             // barrier: arrivals, generation (zero when first used)
+  long long* part;           // 8 words per block: bounds of its points, non-finite flag
+  uint64_t* ptkey;           // per point: entry << 6 | place in the block
+  uint32_t* ptcell;          // per point: its cell
+  uint32_t* ptpos;           // per point: its place in the cell
+  uint32_t* pcell;           // per position: its cell
+  uint64_t* cellkey;         // per cell: entry << 6 | place in the block
+  uint2* crange;             // per cell: its positions [x, y)
+  uint32_t* list;            // positions outside dense cells (per expand)
+  uint32_t* cellrep;         // per core cell: its first core point (position)
+  AsymWork* asym;
+};
+
+constexpr int kSmallThreads = 512;
+// Single runs of at most this many points take the small kernels when their grid has
+// a direct block table.  The lines lie where the general pipeline's launches stop
+// dominating: 2D 482 -> 341 us at 128k points, 510 -> 398 at 256k (blobs, float64); 3D
+// 756 -> 648 at 128k, but 789 -> 960 at 256k.  With a block hash at most
+// kSmallHashPoints: larger sparse sets are the general path's row tables'.
+constexpr int64_t small_points(int dim) { return dim == 2 ? 262144 : 131072; }
+constexpr int64_t kSmallHashPoints = 16384;
+__host__ __device__ constexpr uint64_t small_direct_max(int64_t n) {
+  return n < 4096 ? 8192 : 2 * (uint64_t)n;
+}
+__host__ __device__ constexpr uint32_t small_hash_slots(int64_t n) {
+  if (n > kSmallHashPoints) return 0;
+  uint32_t h = 1024;
+  while (h < 2 * (uint64_t)n) h <<= 1;
+  return h;
+}
 
 // Hash of occupied block rows (sparse grids): open addressing, linear probing.
 constexpr unsigned long long kHashEmpty = ~0ull;

@@ -140,6 +140,12 @@ int label(const Bufs& B, int64_t n, int sms, void* scan_temp, cudaStream_t s);
 int border(const Bufs& B, int64_t n, int dims, bool f32, bool key64, int sms, cudaStream_t s);
 int scatter_labels(const Bufs& B, int64_t n, int* out, uint8_t* core_out, int sms,
                    cudaStream_t s);
+// small runs: index build, expand (out: labels in the caller's order, or null: kept in
+// lab for small_scatter); cooperative launches
+cudaError_t small_index(const Bufs& B, const gd::SmallArgs& A, int sms, cudaStream_t s);
+cudaError_t small_expand(const Bufs& B, const gd::SmallArgs& A, bool f32, int minpts, int* out,
+                         int sms, cudaStream_t s);
+int small_scatter(const Bufs& B, int n, int* out, uint8_t* core_out, int sms, cudaStream_t s);
 // per-instance cluster counts (K entries) from the cluster marks
 int cluster_counts(const Bufs& B, int K, int64_t* out, cudaStream_t s);
 

@@ -25,9 +25,10 @@
 //     cell table or hash) is cleared inside each call.  Calls whose work
 //     overlaps on the GPU (two host threads, or two streams) race on the array
 //     and must be serialised by the caller.
-//   * The call synchronises its stream twice: once in the middle, to read the
-//     grid layout back to the host, and once at the end.  It uses the same
-//     kernels as gd_dbscan, so the labels are identical.
+//   * The call synchronises its stream once, at the end; where the grid is not for
+//     the small kernels (too many blocks for a direct table or, up to 16384 points,
+//     a block hash) three times, the general pipeline's layout read among them.  It
+//     uses the same kernels as gd_dbscan, so the labels are identical.
 #include <algorithm>
 #include <cstring>
 #include <mutex>
@@ -59,7 +60,8 @@ constexpr size_t kOffChunks = kOffInst + up(sizeof(gd::InstDesc));
 constexpr size_t kOffPv = kOffChunks + up(kMaxChunks * sizeof(gd::Chunk));
 constexpr size_t kOffBi = kOffPv + up(sizeof(gd::DevParams));
 constexpr size_t kOffBbox = kOffBi + up(sizeof(gd::BatchInfo));
-constexpr size_t kOffKeys0 = kOffBbox + up(6 * 8);
+constexpr size_t kMaxSms = 512;  // bounds of one block per SM (small kernels)
+constexpr size_t kOffKeys0 = kOffBbox + up(kMaxSms * 64);
 constexpr size_t kOffKeys1 = kOffKeys0 + up(kMaxPoints * 8);
 constexpr size_t kOffVals0 = kOffKeys1 + up(kMaxPoints * 8);
 constexpr size_t kOffVals1 = kOffVals0 + up(kMaxPoints * 4);
@@ -193,7 +195,10 @@ extern "C" gd_status gd_dbscan_noalloc(const double* coords_dev, int64_t n, int3
   if (n == 0) return GD_OK;
   if (gdprim::sort_temp_bytes(kMaxPoints) > kSortTempBytes ||
       gdprim::scan_temp_bytes(gdprim::sort_scan_elems(kMaxPoints)) > kScanTempBytes ||
-      gdprim::scan_temp_bytes(kMaxPoints + 1) > kScanTempBytes)
+      gdprim::scan_temp_bytes(kMaxPoints + 1) > kScanTempBytes ||
+      sizeof(gd::AsymWork) > kSortTempBytes ||
+      gd::small_hash_slots(gd::kSmallHashPoints) > kTableBlocks + kMaxPoints ||
+      gd::small_hash_slots(gd::kSmallHashPoints) > kHashSlots)
     return fail(GD_EINVAL, "gd_dbscan_noalloc: scratch layout inconsistent (build error)");
 
   int dev = 0;
@@ -209,6 +214,79 @@ extern "C" gd_status gd_dbscan_noalloc(const double* coords_dev, int64_t n, int3
   uint32_t* dM = reinterpret_cast<uint32_t*>(base + kOffSmall);
   uint32_t* dK = reinterpret_cast<uint32_t*>(base + kOffSmall + 4);
   unsigned long long* dCtr = reinterpret_cast<unsigned long long*>(base + kOffSmall + 128);
+
+  // the small kernels first (gd_small.cuh): they leave at once, and say so, when the
+  // grid is not for them
+  {
+    gd::SmallArgs A;
+    A.coords = coords_dev;
+    A.n = (int)n;
+    A.dim = dim;
+    A.eps = eps;
+    A.mult = 0.5 * (1.0 + 1.0 / 65536.0);
+    A.direct_max = std::min<uint64_t>(gd::small_direct_max(n), kTableBlocks + kMaxPoints);
+    A.hash_slots = gd::small_hash_slots(n);
+    A.bar = reinterpret_cast<unsigned*>(base + kOffSmall + 2048);
+    A.part = reinterpret_cast<long long*>(base + kOffBbox);
+    A.ptkey = reinterpret_cast<uint64_t*>(base + kOffKeys0);
+    A.cellkey = reinterpret_cast<uint64_t*>(base + kOffKeys1);
+    A.ptcell = reinterpret_cast<uint32_t*>(base + kOffVals0);
+    A.ptpos = reinterpret_cast<uint32_t*>(base + kOffCellent);
+    A.pcell = reinterpret_cast<uint32_t*>(base + kOffBlklist);
+    A.crange = reinterpret_cast<uint2*>(base + kOffHvMask);
+    A.list = reinterpret_cast<uint32_t*>(base + kOffHvCell);
+    A.cellrep = reinterpret_cast<uint32_t*>(base + kOffCellrep);
+    A.asym = reinterpret_cast<gd::AsymWork*>(base + kOffSortTemp);
+    gdl::Bufs B;
+    B.coords = coords_dev;
+    B.Pv = reinterpret_cast<gd::DevParams*>(base + kOffPv);
+    B.Bi = reinterpret_cast<gd::BatchInfo*>(base + kOffSmall + 1024);
+    B.ids = reinterpret_cast<uint32_t*>(base + kOffVals1);
+    gdl::set_bits(B, reinterpret_cast<uint32_t*>(base + kOffBits), n);
+    B.M = dM;
+    B.K = dK;
+    B.ent = reinterpret_cast<gd::BlockEnt*>(base + kOffEnt);
+    B.hkeys = reinterpret_cast<unsigned long long*>(base + kOffHkeys);
+    B.hmask = A.hash_slots - 1;
+    B.X = reinterpret_cast<double*>(base + kOffX);
+    B.Xf = reinterpret_cast<float*>(base + kOffXf);
+    B.core = base + kOffCore;
+    B.cellcore = reinterpret_cast<int*>(base + kOffCellcore);
+    B.cellmin = reinterpret_cast<int*>(base + kOffCellmin);
+    B.parent = reinterpret_cast<int*>(base + kOffParent);
+    B.cellcid = reinterpret_cast<int*>(base + kOffCellcid);
+    B.lab = reinterpret_cast<int*>(base + kOffLab);
+    B.compmin = B.lab;
+    B.asym = reinterpret_cast<int*>(base + kOffAsym);
+    B.ctr = dCtr;
+    B.tn_link = INT32_MAX;
+    const int nb = std::min(sms, (int)kMaxSms);
+    NA_CUDA(cudaMemsetAsync(base + kOffSmall, 0, 4096, s), "clear counters");
+    NA_CUDA(gdl::small_index(B, A, nb, s), "small index launch");
+    NA_CUDA(gdl::small_expand(B, A, precision == GD_PREC_FP32_BAND, minpts, labels_dev, nb, s),
+            "small expand launch");
+    alignas(8) unsigned char back[1024 + sizeof(gd::BatchInfo)];
+    NA_CUDA(cudaMemcpyAsync(back, base + kOffSmall, sizeof back, cudaMemcpyDeviceToHost, s),
+            "read counters");
+    NA_CUDA(cudaStreamSynchronize(s), "DBSCAN pipeline");
+    gd::BatchInfo bi;
+    std::memcpy(&bi, back + 1024, sizeof bi);
+    const unsigned long long* ctr = reinterpret_cast<const unsigned long long*>(back + 128);
+    if (ctr[gd::kCtrWaitTimeouts])
+      return fail(GD_ECUDA, "gd_dbscan_noalloc: a grid barrier wait gave up");
+    if (bi.flags & gd::kFlagNonFinite)
+      return fail(GD_EINVAL, "gd_dbscan_noalloc: input has NaN or Inf coordinates");
+    if (bi.flags & gd::kFlagGridTooLarge)
+      return fail(GD_ERANGE, "gd_dbscan_noalloc: eps-cell grid too large");
+    if (!(bi.flags & gd::kFlagNotSmall)) {
+      if (ctr[gd::kCtrAsymEdges] > (unsigned long long)gd::kAsymCap)
+        return fail(GD_ERANGE, "gd_dbscan_noalloc: too many one-directional core neighbour pairs");
+      uint32_t K;
+      std::memcpy(&K, back + 4, 4);
+      if (n_clusters) *n_clusters = K;
+      return GD_OK;
+    }
+  }
 
   // the run description: one instance, chunks of kChunkPoints points
   gd::InstDesc desc{0, n, 0, eps, dim, minpts};

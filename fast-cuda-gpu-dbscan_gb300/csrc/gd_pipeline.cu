@@ -173,34 +173,31 @@ __global__ void __launch_bounds__(kBboxThreads) k_bbox_chunk(const gdl::Bufs B) 
   }
 }
 
-// One thread per instance: its grid and float32 band from its bounding box.
-__global__ void k_params_inst(const gdl::Bufs B, int K, double mult2, double mult3,
-                              uint64_t dense_floor, uint64_t dense_per_point,
-                              uint64_t rows_floor) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= K) return;
-  const InstDesc I = B.inst[i];
+// An instance's grid and float32 band from its bounding box [lo, hi] (its points'
+// least and greatest coordinates; not read when it has none).
+__device__ void fill_params(DevParams& p, const InstDesc& I, int inst, const double* lo,
+                            const double* hi, double mult, uint64_t dense_floor,
+                            uint64_t dense_per_point, uint64_t rows_floor) {
   const int D = I.dim;
   const double eps = I.eps;
-  DevParams p;
   int fl = 0;
-  for (int k = 0; k < 3; ++k) { p.lo[k] = 0; p.hi[k] = 0; p.centre[k] = 0; p.G[k] = 1; }
-  if (I.n > 0)
-    for (int k = 0; k < D; ++k) {
-      p.lo[k] = dbl_of(B.bbox[i * 6 + k]);
-      p.hi[k] = dbl_of(B.bbox[i * 6 + 3 + k]);
-      p.centre[k] = 0.5 * p.lo[k] + 0.5 * p.hi[k];
-    }
+  for (int k = 0; k < 3; ++k) {
+    const bool on = k < D && I.n > 0;
+    p.lo[k] = on ? lo[k] : 0.0;
+    p.hi[k] = on ? hi[k] : 0.0;
+    p.centre[k] = on ? 0.5 * lo[k] + 0.5 * hi[k] : 0.0;
+    p.G[k] = 1;
+  }
   p.dim = D;
   p.minpts = I.minpts;
   p.eps = eps;
   p.eps2 = __dmul_rn(eps, eps);
-  p.f = __dmul_rn(eps, D == 2 ? mult2 : mult3);
+  p.f = __dmul_rn(eps, mult);
   p.inv_f = 1.0 / p.f;
   p.pt_off = I.pt_off;
   p.n = I.n;
   p.co_off = I.co_off;
-  p.inst = i;
+  p.inst = inst;
   double cells = 1.0;
   uint64_t C = 1;
   uint64_t NB = 1;
@@ -348,6 +345,22 @@ __global__ void k_params_inst(const gdl::Bufs B, int K, double mult2, double mul
   p.row_off = 0;
   p.kmask = 0;
   p.LB = 0;
+}
+
+// One thread per instance.
+__global__ void k_params_inst(const gdl::Bufs B, int K, double mult2, double mult3,
+                              uint64_t dense_floor, uint64_t dense_per_point,
+                              uint64_t rows_floor) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= K) return;
+  const InstDesc I = B.inst[i];
+  double lo[3], hi[3];
+  for (int k = 0; k < 3; ++k) {
+    lo[k] = dbl_of(B.bbox[i * 6 + k]);
+    hi[k] = dbl_of(B.bbox[i * 6 + 3 + k]);
+  }
+  DevParams p;
+  fill_params(p, I, i, lo, hi, I.dim == 2 ? mult2 : mult3, dense_floor, dense_per_point, rows_floor);
   B.Pv[i] = p;
 }
 
@@ -501,6 +514,55 @@ __device__ __forceinline__ int cell_index_f64(double x, double lo, double inv_f)
   return __double2int_rd(__dmul_rn(__dsub_rn(x, lo), inv_f));
 }
 
+// Cell along one axis: kfast, lo32, inv32 and band as in DevParams::key_*.
+__device__ __forceinline__ int cell_of_coord(double x, bool kfast, double lo, double inv_f,
+                                             float lo32, float inv32, float band, int64_t G) {
+  // 32-bit cell index: conversions to 64-bit integers run on this GPU's
+  // narrow float64 pipe; every cell index is below 2^31 (grids are checked)
+  int q;
+  bool fast = false;
+  if (kfast) {
+    // float32 cell position (no float64 instruction), used when it is
+    // farther than key_band from a cell boundary
+    const unsigned long long bits = (unsigned long long)__double_as_longlong(x);
+    const int fe = (int)((bits >> 52) & 0x7ff) - 1023 + 127;
+    const bool zero = (bits << 1) == 0;
+    if (zero || (fe > 0 && fe < 255)) {
+      const unsigned sgn = (unsigned)(bits >> 63) << 31;
+      const float x32 = zero ? 0.0f
+                             : __uint_as_float(sgn | ((unsigned)fe << 23) |
+                                               (unsigned)((bits >> 29) & 0x7fffffu));
+      const float t = __fmul_rn(__fsub_rn(x32, lo32), inv32);
+      if (fabsf(t) < 4194304.0f) {
+        // floor without a conversion instruction: for |t| < 2^22,
+        // t + 1.5 * 2^23 rounded down lies in [2^23, 2^24), where floats are
+        // the integers, so it is floor(t) + 1.5 * 2^23 exactly and its
+        // mantissa bits hold floor(t) + 2^22
+        const float s = __fadd_rd(t, 12582912.0f);
+        const float fl = __fsub_rn(s, 12582912.0f);
+        const float fr = __fsub_rn(t, fl);
+        if (fr > band && fr < 1.0f - band) {
+          q = (int)(__float_as_uint(s) - 0x4b400000u);
+          fast = true;
+        }
+      }
+    }
+  }
+  // the float64 formula for the few coordinates near a cell boundary
+  if (!fast) q = cell_index_f64(x, lo, inv_f);
+  q = q < 0 ? 0 : ((int64_t)q >= G ? (int)(G - 1) : q);
+  return q;
+}
+
+// Local key from the cells along each axis.
+__device__ __forceinline__ uint64_t key_of_cell(int D, const int* c, int B1, int B2) {
+  return D == 2 ? ((uint64_t)(unsigned)(c[0] >> 3) * (unsigned)B1 + (unsigned)(c[1] >> 3)) << kBlockBits |
+                      (unsigned)((c[0] & 7) << 3 | (c[1] & 7))
+                : (((uint64_t)(unsigned)(c[0] >> 2) * (unsigned)B1 + (unsigned)(c[1] >> 2)) * (unsigned)B2 +
+                   (unsigned)(c[2] >> 2)) << kBlockBits |
+                      (unsigned)((c[0] & 3) << 4 | (c[1] & 3) << 2 | (c[2] & 3));
+}
+
 // One block per chunk: cell key of every point, instance id above the local key.
 template <class Key>
 __global__ void __launch_bounds__(256) k_keys(const gdl::Bufs B, Key* __restrict__ keys) {
@@ -524,49 +586,9 @@ __global__ void __launch_bounds__(256) k_keys(const gdl::Bufs B, Key* __restrict
     for (int k = 0; k < 3; ++k) {
       if (k >= D) break;
       const double x = xs[k];
-      // 32-bit cell index: conversions to 64-bit integers run on this GPU's
-      // narrow float64 pipe; every cell index is below 2^31 (grids are checked)
-      int q;
-      bool fast = false;
-      if (kfast) {
-        // float32 cell position (no float64 instruction), used when it is
-        // farther than key_band from a cell boundary
-        const unsigned long long bits = (unsigned long long)__double_as_longlong(x);
-        const int fe = (int)((bits >> 52) & 0x7ff) - 1023 + 127;
-        const bool zero = (bits << 1) == 0;
-        if (zero || (fe > 0 && fe < 255)) {
-          const unsigned sgn = (unsigned)(bits >> 63) << 31;
-          const float x32 = zero ? 0.0f
-                                 : __uint_as_float(sgn | ((unsigned)fe << 23) |
-                                                   (unsigned)((bits >> 29) & 0x7fffffu));
-          const float t = __fmul_rn(__fsub_rn(x32, lo32[k]), inv32);
-          if (fabsf(t) < 4194304.0f) {
-            // floor without a conversion instruction: for |t| < 2^22,
-            // t + 1.5 * 2^23 rounded down lies in [2^23, 2^24), where floats are
-            // the integers, so it is floor(t) + 1.5 * 2^23 exactly and its
-            // mantissa bits hold floor(t) + 2^22
-            const float s = __fadd_rd(t, 12582912.0f);
-            const float fl = __fsub_rn(s, 12582912.0f);
-            const float fr = __fsub_rn(t, fl);
-            if (fr > band && fr < 1.0f - band) {
-              q = (int)(__float_as_uint(s) - 0x4b400000u);
-              fast = true;
-            }
-          }
-        }
-      }
-      // the float64 formula for the few coordinates near a cell boundary
-      if (!fast) q = cell_index_f64(x, lo[k], inv_f);
-      q = q < 0 ? 0 : ((int64_t)q >= G[k] ? (int)(G[k] - 1) : q);
-      c[k] = q;
+      c[k] = cell_of_coord(x, kfast, lo[k], inv_f, lo32[k], inv32, band, G[k]);
     }
-    const uint64_t key =
-        D == 2 ? ((uint64_t)(unsigned)(c[0] >> 3) * (unsigned)B1 + (unsigned)(c[1] >> 3)) << kBlockBits |
-                     (unsigned)((c[0] & 7) << 3 | (c[1] & 7))
-               : (((uint64_t)(unsigned)(c[0] >> 2) * (unsigned)B1 + (unsigned)(c[1] >> 2)) * (unsigned)B2 +
-                  (unsigned)(c[2] >> 2)) << kBlockBits |
-                     (unsigned)((c[0] & 3) << 4 | (c[1] & 3) << 2 | (c[2] & 3));
-    out[l] = (Key)(hi + key);
+    out[l] = (Key)(hi + key_of_cell(D, c, B1, B2));
   };
   if (D == 2) for_points<2>(pts, c.begin - P.pt_off, c.end - P.pt_off, key_of);
   else for_points<3>(pts, c.begin - P.pt_off, c.end - P.pt_off, key_of);
@@ -2999,22 +3021,21 @@ __global__ void __launch_bounds__(kCellThreads) k_union_heavy(const gdl::Bufs B,
 // a cluster that absorbs every unassigned component reachable along directed
 // links.  Absorbed roots are re-parented under the opening root.  One thread;
 // the list holds at most kAsymCap links (more is reported as an error).
-__global__ void k_asym_resolve(const gdl::Bufs B) {
+// cell(q): the cell of sorted position q.
+template <class F>
+__device__ void asym_resolve(const gdl::Bufs& B, AsymWork& W, F&& cell) {
   const int* __restrict__ cellmin = B.compmin;  // per root: the component's smallest core index
   int* parent = B.parent;
   const int* __restrict__ asym_list = B.asym;
-  unsigned long long* ctr = B.ctr;
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  unsigned long long E = ctr[kCtrAsymEdges];
+  unsigned long long E = B.ctr[kCtrAsymEdges];
   if (E == 0) return;
   if (E > (unsigned long long)kAsymCap) return;  // reported by the host
-  __shared__ int from[kAsymCap], to[kAsymCap];
-  __shared__ int node[2 * kAsymCap], assigned[2 * kAsymCap];
+  int *from = W.from, *to = W.to, *node = W.node, *assigned = W.assigned;
   int ne = 0, nv = 0;
   for (unsigned long long i = 0; i < E; ++i) {
     int a = asym_list[2 * i], b = asym_list[2 * i + 1];
-    int ra = uf_find(parent, cell_of(B, a));
-    int rb = uf_find(parent, cell_of(B, b));
+    int ra = uf_find(parent, cell(a));
+    int rb = uf_find(parent, cell(b));
     if (ra == rb) continue;
     from[ne] = ra;
     to[ne] = rb;
@@ -3060,6 +3081,12 @@ __global__ void k_asym_resolve(const gdl::Bufs B) {
   }
   for (int v = 0; v < nv; ++v)
     if (assigned[v] != node[v]) parent[node[v]] = assigned[v];
+}
+
+__global__ void k_asym_resolve(const gdl::Bufs B) {
+  __shared__ AsymWork W;
+  if (threadIdx.x == 0 && blockIdx.x == 0)
+    asym_resolve(B, W, [&](int q) { return cell_of(B, q); });
 }
 
 // parent[m] <- root (full path compression).  slot[D] (for the cells of that
@@ -3342,6 +3369,8 @@ __global__ void k_cluster_counts(const gdl::Bufs B, int K, int64_t* out) {
   }
 }
 
+#include "gd_small.cuh"
+
 }  // namespace gd
 // ------------------------------------------------------------------ launchers
 namespace gdl {
@@ -3554,6 +3583,34 @@ int border(const Bufs& B, int64_t n, int dims, bool f32, bool key64, int sms, cu
 int scatter_labels(const Bufs& B, int64_t n, int* out, uint8_t* core_out, int sms,
                    cudaStream_t s) {
   k_scatter_labels<<<grid_for(n, 256, sms, 8), 256, 0, s>>>(B, n, out, core_out);
+  return 1;
+}
+
+// blocks of a small run's kernels: one resident block per SM at most
+static int small_grid(int64_t lanes, int sms) {
+  const int64_t g = (lanes + kSmallThreads - 1) / kSmallThreads;
+  return (int)(g < 1 ? 1 : (g > sms ? sms : g));
+}
+
+cudaError_t small_index(const Bufs& B, const SmallArgs& A, int sms, cudaStream_t s) {
+  void* args[] = {const_cast<Bufs*>(&B), const_cast<SmallArgs*>(&A)};
+  const void* f = A.dim == 2 ? (const void*)k_small_index<2> : (const void*)k_small_index<3>;
+  return cudaLaunchCooperativeKernel(f, dim3(small_grid(A.n, sms)), dim3(kSmallThreads), args, 0, s);
+}
+
+cudaError_t small_expand(const Bufs& B, const SmallArgs& A, bool f32, int minpts, int* out, int sms,
+                         cudaStream_t s) {
+  void* args[] = {const_cast<Bufs*>(&B), const_cast<SmallArgs*>(&A), &minpts, &out};
+  const void* f = A.dim == 2
+                      ? (f32 ? (const void*)k_small_expand<2, true> : (const void*)k_small_expand<2, false>)
+                      : (f32 ? (const void*)k_small_expand<3, true> : (const void*)k_small_expand<3, false>);
+  const int G = A.dim == 2 ? SmallWalk<2>::G : SmallWalk<3>::G;
+  return cudaLaunchCooperativeKernel(f, dim3(small_grid((int64_t)A.n * G, sms)), dim3(kSmallThreads),
+                                     args, (size_t)B.nwf * 4, s);
+}
+
+int small_scatter(const Bufs& B, int n, int* out, uint8_t* core_out, int sms, cudaStream_t s) {
+  k_small_scatter<<<grid_for(n, 256, sms, 8), 256, 0, s>>>(B, n, out, core_out);
   return 1;
 }
 

@@ -1,0 +1,683 @@
+// gd_small.cuh -- one small instance in two cooperative kernels (included by
+// gd_pipeline.cu, namespace gd).
+//
+// A small instance spends its time in launches and in dependent loads, not in work:
+// the general pipeline's 40 launches took 0.33 of the 0.39 ms of a 1,000-point run.
+// Here the index build is one kernel and the expand another, their phases separated
+// by grid-wide barriers (about 1 us each), and every stencil walk takes a group of
+// lanes -- one lane per block of the stencil, 4 in 2D and 8 in 3D -- so that a walk's
+// chain of loads is a quarter or an eighth as long.
+//
+// The index needs no sort: points set their cell's bit in their block's occupancy
+// word, each occupied block then takes a run of cell numbers from a counter, points
+// take their place in their cell from the cell's counter, and each cell takes a run
+// of positions from another.  Cells of a block are consecutive and in bit order, as
+// the walks need; the order of blocks, and of points in a cell, is whatever the
+// counters gave, which no label depends on.  Blocks are found directly (one entry per
+// block) where there are few, else by a hash of block keys.
+//
+// Both kernels are launched cooperatively (every block resident), so the barrier's
+// waits end; they are still bounded, and one that gives up makes its block leave and
+// is reported (kCtrWaitTimeouts).
+
+
+constexpr unsigned kBarrierPolls = 1u << 25;  // 2 s and more
+
+// All blocks of the launch; false when the wait gave up (the block must leave).
+__device__ __forceinline__ bool grid_barrier(const SmallArgs& A, unsigned long long* timeouts) {
+  if (gridDim.x == 1) {
+    __syncthreads();
+    return true;
+  }
+  __shared__ int s_ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int ok = 1;
+    unsigned gen;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(gen) : "l"(A.bar + 1) : "memory");
+    __threadfence();
+    if (atomicAdd(A.bar, 1u) == gridDim.x - 1u) {
+      A.bar[0] = 0;
+      __threadfence();
+      asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(A.bar + 1), "r"(gen + 1u) : "memory");
+    } else {
+      ok = 0;
+      for (unsigned it = 0; it < kBarrierPolls; ++it) {
+        unsigned g;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(g) : "l"(A.bar + 1) : "memory");
+        if (g != gen) {
+          ok = 1;
+          break;
+        }
+        if (it > 64) __nanosleep(64);
+      }
+      if (!ok) atomicAdd(timeouts, 1ull);
+    }
+    __threadfence();
+    s_ok = ok;
+  }
+  __syncthreads();
+  return s_ok != 0;
+}
+
+// One lane's share of a counter that the warp's lanes draw on together.
+__device__ __forceinline__ uint32_t warp_draw(unsigned long long* c, uint32_t want) {
+  const int lane = threadIdx.x & 31;
+  uint32_t inc = want;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t v = __shfl_up_sync(kFull, inc, o);
+    if (lane >= o) inc += v;
+  }
+  const uint32_t total = __shfl_sync(kFull, inc, 31);
+  unsigned long long at = 0;
+  if (lane == 0 && total) at = atomicAdd(c, (unsigned long long)total);
+  return (uint32_t)__shfl_sync(kFull, at, 0) + inc - want;
+}
+
+// Entry of a block, kNoEnt when outside the grid or (hash) not occupied.
+template <int D>
+__device__ __forceinline__ uint32_t small_ent(const gdl::Bufs& B, const DevParams& P, int x, int y,
+                                              int z) {
+  if (x < 0 || x >= P.Bk[0] || y < 0 || y >= P.Bk[1]) return kNoEnt;
+  if (D == 3 && (z < 0 || z >= P.Bk[2])) return kNoEnt;
+  uint64_t blk = (uint64_t)(unsigned)x * (unsigned)P.Bk[1] + (unsigned)y;
+  if (D == 3) blk = blk * (unsigned)P.Bk[2] + (unsigned)z;
+  if (P.sparse == 0) return (uint32_t)blk;
+  const uint32_t mask = B.hmask;
+  uint32_t h = hash_key(blk) & mask;
+  for (uint32_t probe = 0; probe <= mask; ++probe) {
+    const unsigned long long k = B.hkeys[h];
+    if (k == blk) return h;
+    if (k == kHashEmpty) break;
+    h = (h + 1) & mask;
+  }
+  return kNoEnt;
+}
+
+// ---------------------------------------------------------------- index build
+template <int D>
+__global__ void __launch_bounds__(kSmallThreads) k_small_index(const gdl::Bufs B, const SmallArgs A) {
+  __shared__ DevParams P;
+  __shared__ long long s_b[7][kSmallThreads / 32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int n = A.n, T = gridDim.x * kSmallThreads, t0 = blockIdx.x * kSmallThreads + threadIdx.x;
+  unsigned long long* timeouts = B.ctr + kCtrWaitTimeouts;
+  {
+    // bounds of the block's points
+    long long lo[D], hi[D], bad = 0;
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
+      lo[k] = LLONG_MAX;
+      hi[k] = LLONG_MIN;
+    }
+    for (int l = t0; l < n; l += T)
+#pragma unroll
+      for (int k = 0; k < D; ++k) {
+        const double x = A.coords[(int64_t)l * D + k];
+        bad |= (__double_as_longlong(x) & 0x7ff0000000000000LL) == 0x7ff0000000000000LL;
+        const long long o = ord_of(x);
+        lo[k] = min(lo[k], o);
+        hi[k] = max(hi[k], o);
+      }
+    bad = __any_sync(kFull, bad != 0);
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        lo[k] = min(lo[k], __shfl_xor_sync(kFull, lo[k], o));
+        hi[k] = max(hi[k], __shfl_xor_sync(kFull, hi[k], o));
+      }
+      if (lane == 0) {
+        s_b[k][w] = lo[k];
+        s_b[3 + k][w] = hi[k];
+      }
+    }
+    if (lane == 0) s_b[6][w] = bad;
+    __syncthreads();
+    if (threadIdx.x < 7 && (threadIdx.x == 6 || threadIdx.x % 3 < D)) {
+      const int k = threadIdx.x;
+      long long v = s_b[k][0];
+      for (int j = 1; j < kSmallThreads / 32; ++j)
+        v = k < 3 ? min(v, s_b[k][j]) : max(v, s_b[k][j]);
+      A.part[blockIdx.x * 8 + k] = v;
+    }
+  }
+  if (!grid_barrier(A, timeouts)) return;
+  // every block: the same bounds, the same grid
+  if (w < 7 && (w == 6 || w % 3 < D)) {
+    long long v = w < 3 ? LLONG_MAX : LLONG_MIN;
+    for (int j = lane; j < (int)gridDim.x; j += 32) {
+      const long long x = A.part[j * 8 + w];
+      v = w < 3 ? min(v, x) : max(v, x);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const long long x = __shfl_xor_sync(kFull, v, o);
+      v = w < 3 ? min(v, x) : max(v, x);
+    }
+    if (lane == 0) s_b[w][0] = v;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
+    for (int k = 0; k < D; ++k) {
+      lo[k] = dbl_of(s_b[k][0]);
+      hi[k] = dbl_of(s_b[3 + k][0]);
+    }
+    const InstDesc I{0, n, 0, A.eps, D, 1};
+    fill_params(P, I, 0, lo, hi, A.mult, A.direct_max, 0, 0);
+    int fl = P.flags | (s_b[6][0] > 0 ? kFlagNonFinite : 0) |
+             (P.cell_bits > 62 ? kFlagGridTooLarge : 0);
+    if (P.sparse != 0) {
+      P.sparse = 1;
+      if (A.hash_slots == 0) fl |= kFlagNotSmall;
+    }
+    P.flags = fl;
+    P.LB = P.key_bits;
+    P.kmask = P.LB >= 64 ? ~0ull : (1ull << P.LB) - 1ull;
+    if (blockIdx.x == 0) {
+      B.Pv[0] = P;
+      BatchInfo bi{};
+      bi.K = 1;
+      bi.LB = P.LB;
+      bi.flags = fl;
+      bi.max_dim = D;
+      bi.K2 = D == 2 ? 1 : 0;
+      bi.any_xf = 1;
+      bi.band_off = !(P.eps2_lo32 > 0.0f);
+      bi.grid_cells = P.sparse == 0 ? P.NB << kBlockBits : 0;
+      bi.any_sparse = P.sparse == 1;
+      *B.Bi = bi;
+    }
+  }
+  __syncthreads();
+  if (P.flags & (kFlagNonFinite | kFlagGridTooLarge | kFlagNotSmall)) return;  // (every block)
+  const uint32_t ents = P.sparse == 0 ? (uint32_t)P.NB : A.hash_slots;
+  for (uint32_t e = t0; e < ents; e += T) {
+    B.ent[e] = BlockEnt{};
+    if (P.sparse) B.hkeys[e] = kHashEmpty;
+  }
+  if (!grid_barrier(A, timeouts)) return;
+  // cells: occupancy bits
+  for (int l = t0; l < n; l += T) {
+    int c[3] = {0, 0, 0};
+#pragma unroll
+    for (int k = 0; k < D; ++k)
+      c[k] = cell_of_coord(A.coords[(int64_t)l * D + k], P.key_fast != 0, P.lo[k], P.inv_f,
+                           P.key_lo32[k], P.key_inv32, P.key_band, P.G[k]);
+    const uint64_t key = key_of_cell(D, c, P.Bk[1], P.Bk[2]);
+    const uint64_t blk = key >> kBlockBits;
+    uint32_t e = (uint32_t)blk;
+    if (P.sparse) {
+      const uint32_t mask = B.hmask;
+      uint32_t h = hash_key(blk) & mask;
+      e = 0;
+      for (uint32_t probe = 0; probe <= mask; ++probe) {  // more slots than points: one is free
+        const unsigned long long prev = atomicCAS(B.hkeys + h, kHashEmpty, (unsigned long long)blk);
+        if (prev == kHashEmpty || prev == blk) {
+          e = h;
+          break;
+        }
+        h = (h + 1) & mask;
+      }
+    }
+    const unsigned long long bit = 1ull << (key & 63);
+    if (!(*reinterpret_cast<volatile unsigned long long*>(&B.ent[e].occ) & bit))
+      atomicOr(&B.ent[e].occ, bit);
+    A.ptkey[l] = (uint64_t)e << kBlockBits | (key & 63);
+  }
+  if (!grid_barrier(A, timeouts)) return;
+  // cell numbers: a run per block
+  for (uint32_t e0 = t0 - lane; e0 < ents; e0 += T) {
+    const uint32_t e = e0 + lane;
+    unsigned long long occ = e < ents ? B.ent[e].occ : 0ull;
+    uint32_t m = warp_draw(B.ctr + kCtrCells, (uint32_t)__popcll(occ));
+    if (!occ) continue;
+    BlockEnt E{};
+    E.occ = occ;
+    E.base = m;
+    B.ent[e] = E;
+    for (; occ; occ &= occ - 1, ++m) {
+      A.cellkey[m] = (uint64_t)e << kBlockBits | (unsigned)(__ffsll((long long)occ) - 1);
+      B.cellcore[m] = 0;
+    }
+  }
+  if (!grid_barrier(A, timeouts)) return;
+  // places in the cells
+  for (int l = t0; l < n; l += T) {
+    const uint64_t k = A.ptkey[l];
+    const EntHead h = ent_head(B, (uint32_t)(k >> kBlockBits));
+    const int m = ent_cell(h.occ, h.base, (int)(k & 63));
+    A.ptcell[l] = (uint32_t)m;
+    A.ptpos[l] = (uint32_t)atomicAdd(B.cellcore + m, 1);
+  }
+  if (!grid_barrier(A, timeouts)) return;
+  // positions: a run per cell
+  const int M = (int)*reinterpret_cast<volatile unsigned long long*>(B.ctr + kCtrCells);
+  for (int m0 = t0 - lane; m0 < M; m0 += T) {
+    const int m = m0 + lane;
+    const uint32_t len = m < M ? (uint32_t)B.cellcore[m] : 0u;
+    const uint32_t at = warp_draw(B.ctr + kCtrBlocks, len);
+    if (m < M) A.crange[m] = make_uint2(at, at + len);
+  }
+  if (!grid_barrier(A, timeouts)) return;
+  // sorted points
+  for (int l = t0; l < n; l += T) {
+    const uint32_t m = A.ptcell[l];
+    const int64_t i = A.crange[m].x + A.ptpos[l];
+    B.ids[i] = (uint32_t)l;
+    A.pcell[i] = m;
+    double x[3];
+    float f[3];
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
+      x[k] = A.coords[(int64_t)l * D + k];
+      B.X[i * D + k] = x[k];
+      f[k] = __double2float_rn(__dsub_rn(x[k], P.centre[k]));
+    }
+    if (D == 2) reinterpret_cast<float2*>(B.Xf)[i] = make_float2(f[0], f[1]);
+    else reinterpret_cast<float4*>(B.Xf)[i] = make_float4(f[0], f[1], f[2], 0.0f);
+  }
+}
+
+// --------------------------------------------------------------------- expand
+// A lane's part of a cell's stencil: one block (first-axis half, [middle-axis half,]
+// last-axis half by lane).
+template <int D>
+struct SmallWalk {
+  using St = Stencil<D>;
+  static constexpr int G = D == 3 ? 8 : 4;  // lanes per group
+  CellXYZ<D> cc;
+  int half[D];
+  St st;
+  uint32_t e;
+  // cell given by its key (entry << 6 | place) and its entry's block coordinates
+  __device__ __forceinline__ void init(const gdl::Bufs& B, const DevParams& P, uint64_t ck, int g) {
+    const uint32_t own = (uint32_t)(ck >> kBlockBits);
+    const uint64_t blk = P.sparse == 0 ? own : B.hkeys[own];
+    cc = decompose<D>(blk << kBlockBits | (ck & 63), P);
+    st.init(cc);
+    half[0] = D == 3 ? g >> 2 : g >> 1;
+    if (D == 3) half[1] = (g >> 1) & 1;
+    half[D - 1] = g & 1;
+    e = small_ent<D>(B, P, st.b0[0] + half[0], st.b0[1] + half[1], D == 3 ? st.b0[D - 1] + half[D - 1] : 0);
+  }
+  // this block's cells of the stencil w[] (per-axis sets as Stencil::w5)
+  __device__ __forceinline__ unsigned long long mask(const uint32_t* w) const {
+    StencilWords<D> W;
+    W.init(w);
+    const uint32_t yz = (D == 3 ? (half[1] ? W.y[1] : W.y[0]) : ~0u) & (half[D - 1] ? W.z[1] : W.z[0]);
+    return (unsigned long long)((half[0] ? W.xh[1] : W.xh[0]) & yz) << 32 |
+           ((half[0] ? W.xl[1] : W.xl[0]) & yz);
+  }
+  // offset along axis k of the block's cell at `bit` from the cell
+  __device__ __forceinline__ int off(int bit, int k) const {
+    return st.off0(cc, k) + (half[k] << St::S) + St::bit_off(bit, k);
+  }
+  // mask of this group's lanes
+  static __device__ __forceinline__ unsigned group() {
+    return (G == 8 ? 0xffu : 0xfu) << ((threadIdx.x & 31) & ~(G - 1));
+  }
+};
+
+// point-to-cell classification as in the walks (classify), from in-cell position u
+template <int D, bool F32>
+__global__ void __launch_bounds__(kSmallThreads) k_small_expand(const gdl::Bufs B, const SmallArgs A,
+                                                                int minpts, int* __restrict__ out) {
+  using W = SmallWalk<D>;
+  __shared__ DevParams P;
+  extern __shared__ uint32_t s_pre[];  // prefix counts of the cluster marks
+  __shared__ uint32_t s_warp[32];
+  const int lane = threadIdx.x & 31, g = lane & (W::G - 1);
+  const unsigned grp = W::group();
+  const int n = A.n, T = gridDim.x * kSmallThreads, t0 = blockIdx.x * kSmallThreads + threadIdx.x;
+  const int gT = T / W::G, g0 = t0 / W::G;
+  unsigned long long* timeouts = B.ctr + kCtrWaitTimeouts;
+  for (int k = threadIdx.x; k < (int)(sizeof(DevParams) / 4); k += kSmallThreads)
+    reinterpret_cast<uint32_t*>(&P)[k] = reinterpret_cast<const uint32_t*>(B.Pv)[k];
+  __syncthreads();
+  if (P.flags & (kFlagNonFinite | kFlagGridTooLarge | kFlagNotSmall)) return;  // (every block)
+  if (threadIdx.x == 0) P.minpts = minpts;
+  __syncthreads();
+  const PredParams Q = pred_params(P);
+  const bool prune = Q.prune != 0;
+  const int M = (int)B.ctr[kCtrCells];
+  const int nwf = (int)B.nwf;
+  Tally t;
+  // ---- cells and marks cleared; the points outside dense cells listed
+  for (int m = t0; m < M; m += T) {
+    const uint2 r = A.crange[m];
+    B.cellcore[m] = (int)(r.y - r.x) >= minpts ? (int)(r.y - r.x) : 0;
+    B.cellmin[m] = INT_MAX;
+    B.parent[m] = m;
+    B.ent[A.cellkey[m] >> kBlockBits].core = 0;
+  }
+  for (int k = t0; k < nwf; k += T) B.fbits[k] = 0;
+  for (int i0 = t0 - lane; i0 < n; i0 += T) {
+    const int i = i0 + lane;
+    bool walk = false;
+    if (i < n) {
+      const uint2 r = A.crange[A.pcell[i]];
+      walk = (int)(r.y - r.x) < minpts;
+    }
+    const uint32_t at = warp_draw(B.ctr + kCtrWalkCursor2, walk ? 1u : 0u);
+    if (walk) A.list[at] = (uint32_t)i;
+  }
+  if (!grid_barrier(A, timeouts)) return;
+  const int L = (int)*reinterpret_cast<volatile unsigned long long*>(B.ctr + kCtrWalkCursor2);
+  // ---- core flags: dense cells' points at once, then a group per listed point.
+  // Each lane classifies its block's cells; where the group's sure neighbours and
+  // open candidates leave the decision open, the lanes test their candidates one
+  // per step, the warp's groups in step together, until the group's count or its
+  // candidates decide.
+  for (int i = t0; i < n; i += T) {
+    const int m = (int)A.pcell[i];
+    const uint2 r = A.crange[m];
+    if ((int)(r.y - r.x) < minpts) continue;
+    B.core[i] = 1;
+    if (i == (int)r.x) atomicAdd(B.ctr + kCtrDenseCells, 1ull);
+    const int id = (int)B.ids[i];
+    if (id < *reinterpret_cast<volatile int*>(B.cellmin + m)) atomicMin(B.cellmin + m, id);
+  }
+  for (int j0 = (t0 - lane) / W::G; j0 < L; j0 += gT) {
+    const int j = j0 + lane / W::G;
+    const bool valid = j < L;
+    const int i = valid ? (int)A.list[j] : 0;
+    int m = 0, add = 0, open = 0;
+    double px[D];
+    float pf[D];
+    unsigned long long w = 0;  // open cells
+    EntHead h{0, 0, 0};
+    int own = 0;
+    if (valid) {
+      m = (int)A.pcell[i];
+      const uint2 r = A.crange[m];
+      own = (int)(r.y - r.x);
+      W wk;
+      wk.init(B, P, A.cellkey[m], g);
+      float u[D];
+      load_point<D, F32>(px, pf, B, i, prune);
+      if (prune) {
+        float o[D];
+        cell_origin32<D>(wk.cc, P, o);
+        frac_pos<D>(pf, o, Q, u);
+      }
+      h = ent_head(B, wk.e);
+      for (unsigned long long v = h.occ & wk.mask(wk.st.w5); v; v &= v - 1) {
+        const int bit = __ffsll((long long)v) - 1;
+        const int c = ent_cell(h.occ, h.base, bit);
+        if (c == m) continue;
+        const int cls = prune ? classify<D>(u, wk.off(bit, 0), wk.off(bit, 1),
+                                            D == 3 ? wk.off(bit, D - 1) : 0, Q) : 0;
+        if (cls < 0) continue;
+        const uint2 q = A.crange[c];
+        if (cls > 0) {
+          add += (int)(q.y - q.x);
+        } else {
+          w |= 1ull << bit;
+          open += (int)(q.y - q.x);
+        }
+      }
+    }
+#pragma unroll
+    for (int o = W::G / 2; o > 0; o >>= 1) {
+      add += __shfl_xor_sync(kFull, add, o);
+      open += __shfl_xor_sync(kFull, open, o);
+    }
+    int cnt = own + add;
+    bool more = valid && cnt < minpts && cnt + open >= minpts && w != 0;
+    uint32_t q = 0, qe = 0;
+    while (true) {
+      bool hit = false;
+      if (more) {
+        if (q == qe) {
+          const uint2 r = A.crange[ent_cell(h.occ, h.base, __ffsll((long long)w) - 1)];
+          w &= w - 1;
+          q = r.x;
+          qe = r.y;
+        }
+        Cand<D, F32> cd;
+        load_cand<D, F32>(cd, B, q);
+        hit = pair_test<D, F32>(px, pf, cd, B, P, q, i, true, Q, t);
+        ++q;
+      }
+      cnt += __popc(__ballot_sync(kFull, hit) & grp);
+      more = more && cnt < minpts && (q < qe || w != 0);
+      if (!__any_sync(kFull, more)) break;
+    }
+    if (valid && g == 0) {
+      const bool isc = cnt >= minpts;
+      B.core[i] = isc ? 1 : 0;
+      if (isc) {
+        atomicAdd(B.cellcore + m, 1);
+        const int id = (int)B.ids[i];
+        if (id < *reinterpret_cast<volatile int*>(B.cellmin + m)) atomicMin(B.cellmin + m, id);
+      }
+    }
+  }
+  if (!grid_barrier(A, timeouts)) return;
+  // ---- core words, each core cell's representative (its first core point)
+  for (int m = t0; m < M; m += T) {
+    if (B.cellcore[m] == 0) continue;
+    B.compmin[m] = B.cellmin[m];
+    uint32_t q = A.crange[m].x;
+    while (!B.core[q]) ++q;
+    A.cellrep[m] = q;
+    const uint64_t k = A.cellkey[m];
+    atomicOr(&B.ent[k >> kBlockBits].core, 1ull << (k & 63));
+  }
+  if (!grid_barrier(A, timeouts)) return;
+  // ---- union, a group per core cell: first the near neighbours (pass 0 of the
+  // half stencil), then, from compressed parents, the others, most of which settle
+  // from one parent load
+  for (int step = 0; step < 2; ++step) {
+    for (int m = g0; m < M; m += gT) {
+      if (B.cellcore[m] == 0) continue;  // (the whole group)
+      const uint64_t ck = A.cellkey[m];
+      unsigned long long w = kPassMasks[D - 2].m[0][ck & 63][g];
+      if (step > 0) {
+        w = 0;
+        for (int ps = 1; ps < union_passes(D); ++ps) w |= kPassMasks[D - 2].m[ps][ck & 63][g];
+      }
+      if (!w) continue;
+      W wk;
+      wk.init(B, P, ck, g);
+      if (wk.e == kNoEnt) continue;
+      w &= ent_tail(B, wk.e).core;
+      if (!w) continue;
+      const EntHead h = ent_head(B, wk.e);
+      const int ra0 = *reinterpret_cast<volatile int*>(B.parent + m);
+      if (step > 0) {
+        // parents four at a time; one equal to A's settles the cell
+        unsigned long long slow = 0;
+        while (w) {
+          int bit[4], pr[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            bit[k] = w ? __ffsll((long long)w) - 1 : -1;
+            w &= w - 1;
+            pr[k] = bit[k] >= 0
+                        ? *reinterpret_cast<volatile int*>(B.parent + ent_cell(h.occ, h.base, bit[k]))
+                        : ra0;
+          }
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            if (pr[k] != ra0) slow |= 1ull << bit[k];
+        }
+        w = slow;
+        if (!w) continue;
+      }
+      const uint2 r = A.crange[m];
+      Cand<D, F32> ca;
+      load_cand<D, F32>(ca, B, A.cellrep[m]);
+      const bool single = B.cellcore[m] == 1;
+      float oA[D];
+      if (prune) cell_origin32<D>(wk.cc, P, oA);
+      while (w) {
+        const int bit = __ffsll((long long)w) - 1;
+        w &= w - 1;
+        const int c = ent_cell(h.occ, h.base, bit);
+        if (step > 0 && uf_find(B.parent, m) == uf_find(B.parent, c)) continue;
+        // the representatives first, then the search
+        Cand<D, F32> cd;
+        load_cand<D, F32>(cd, B, A.cellrep[c]);
+        bool linked, apart;
+        if (F32) {
+          ++t.t32;
+          const float s2 = dist2_f32<D>(ca.f, cd.f);
+          linked = s2 < Q.eps2_lo32;
+          apart = s2 > Q.eps2_hi32;
+        } else {
+          ++t.t64;
+          const double d2 = dist2_f64<D>(ca.x, cd.x);
+          linked = d2_le(d2, Q.eps2_in);
+          apart = !d2_le(d2, Q.eps2);
+        }
+        if (!linked && !(apart && single && B.cellcore[c] == 1)) {
+          const uint2 q = A.crange[c];
+          linked = inline_link<D, F32>(B, n, (int)r.x, (int)r.y, (int)q.x, (int)q.y, oA,
+                                       wk.off(bit, 0), wk.off(bit, 1),
+                                       D == 3 ? wk.off(bit, D - 1) : 0, P, Q, t) > 0;
+        }
+        if (linked) uf_union(B.parent, m, c);
+      }
+    }
+    if (!grid_barrier(A, timeouts)) return;
+    if (step == 0) {
+      for (int m = t0; m < M; m += T)
+        if (B.cellcore[m] > 0) B.parent[m] = uf_find(B.parent, m);
+      if (!grid_barrier(A, timeouts)) return;
+    }
+  }
+  // ---- components: smallest core index at the root
+  for (int m = t0; m < M; m += T) {
+    if (B.cellcore[m] == 0) continue;
+    const int r = uf_find(B.parent, m), mn = B.cellmin[m];
+    if (r != m && mn < *reinterpret_cast<volatile int*>(B.compmin + r)) atomicMin(B.compmin + r, mn);
+  }
+  if (!grid_barrier(A, timeouts)) return;
+  if (*reinterpret_cast<volatile unsigned long long*>(B.ctr + kCtrAsymEdges) != 0) {
+    if (t0 == 0) asym_resolve(B, *A.asym, [&](int q) { return (int)A.pcell[q]; });
+    if (!grid_barrier(A, timeouts)) return;
+  }
+  // ---- cluster marks
+  for (int m = t0; m < M; m += T) {
+    if (B.cellcore[m] == 0) continue;
+    if (uf_find(B.parent, m) == m) {
+      const uint32_t cm = (uint32_t)B.compmin[m];
+      atomicOr(B.fbits + (cm >> 5), 1u << (cm & 31));
+    }
+  }
+  if (!grid_barrier(A, timeouts)) return;
+  // ---- cluster numbers: every block ranks the marks for itself
+  {
+    const int per = (nwf + kSmallThreads - 1) / kSmallThreads;
+    const int k0 = threadIdx.x * per, k1 = min(k0 + per, nwf);
+    uint32_t sum = 0;
+    for (int k = k0; k < k1; ++k) sum += (uint32_t)__popc(B.fbits[k]);
+    __shared__ uint32_t s_total;
+    uint32_t ex = gdprim::block_excl_scan<kSmallThreads>(sum, s_warp, &s_total);
+    for (int k = k0; k < k1; ++k) {
+      s_pre[k] = ex;
+      ex += (uint32_t)__popc(B.fbits[k]);
+    }
+    __syncthreads();
+    if (t0 == 0) *B.K = s_total;
+  }
+  for (int m = t0; m < M; m += T) {
+    int cid = INT_MAX;
+    if (B.cellcore[m] > 0) {
+      const uint32_t rm = (uint32_t)B.compmin[uf_find(B.parent, m)];
+      cid = (int)(s_pre[rm >> 5] + (uint32_t)__popc(B.fbits[rm >> 5] & ((1u << (rm & 31)) - 1u)));
+    }
+    B.cellcid[m] = cid;
+  }
+  if (!grid_barrier(A, timeouts)) return;
+  // ---- labels: core points their cell's, the others a border search
+  uint32_t noise = 0, ncore = 0;
+  for (int i = t0; i < n; i += T) {
+    if (!B.core[i]) continue;
+    const int best = B.cellcid[A.pcell[i]];
+    ++ncore;
+    if (out) out[B.ids[i]] = best;
+    else B.lab[i] = best;
+  }
+  for (int j = g0; j < L; j += gT) {
+    const int i = (int)A.list[j];
+    if (B.core[i]) continue;  // (the whole group)
+    const int m = (int)A.pcell[i];
+    int best = INT_MAX;
+    {
+      W wk;
+      wk.init(B, P, A.cellkey[m], g);
+      unsigned long long w = 0;
+      EntHead h{0, 0, 0};
+      if (wk.e != kNoEnt) w = ent_tail(B, wk.e).core & wk.mask(wk.st.w5);
+      if (w) {
+        h = ent_head(B, wk.e);
+        double px[D];
+        float pf[D], u[D];
+        load_point<D, F32>(px, pf, B, i, prune);
+        if (prune) {
+          float o[D];
+          cell_origin32<D>(wk.cc, P, o);
+          frac_pos<D>(pf, o, Q, u);
+        }
+        while (w) {
+          const int bit = __ffsll((long long)w) - 1;
+          w &= w - 1;
+          const int c = ent_cell(h.occ, h.base, bit);
+          const int cB = B.cellcid[c];
+          if (cB >= best) continue;
+          const int cls = prune ? classify<D>(u, wk.off(bit, 0), wk.off(bit, 1),
+                                              D == 3 ? wk.off(bit, D - 1) : 0, Q) : 0;
+          if (cls < 0) continue;
+          if (cls > 0) {
+            best = cB;
+            continue;
+          }
+          const uint2 q = A.crange[c];
+          for (uint32_t qq = q.x; qq < q.y; ++qq) {
+            if (!B.core[qq]) continue;
+            Cand<D, F32> cd;
+            load_cand<D, F32>(cd, B, qq);
+            if (pair_test<D, F32>(px, pf, cd, B, P, qq, i, false, Q, t)) {
+              best = cB;
+              break;
+            }
+          }
+        }
+      }
+#pragma unroll
+      for (int o = W::G / 2; o > 0; o >>= 1) best = min(best, __shfl_xor_sync(grp, best, o));
+      if (best == INT_MAX) best = kNoise;
+      noise += g == 0 && best == kNoise;
+    }
+    if (g == 0) {
+      if (out) out[B.ids[i]] = best;
+      else B.lab[i] = best;
+    }
+  }
+  flush_tally(t, B.ctr);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    noise += __shfl_xor_sync(kFull, noise, o);
+    ncore += __shfl_xor_sync(kFull, ncore, o);
+  }
+  if (lane == 0) {
+    if (noise) atomicAdd(B.ctr + kCtrNoise, (unsigned long long)noise);
+    if (ncore) atomicAdd(B.ctr + kCtrCore, (unsigned long long)ncore);
+  }
+}
+
+// labels (and core flags) back to the caller's order, where the expand did not
+// write them itself
+__global__ void k_small_scatter(const gdl::Bufs B, int n, int* __restrict__ out,
+                                uint8_t* __restrict__ core_out) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const uint32_t j = B.ids[i];
+    out[j] = B.lab[i];
+    if (core_out) core_out[j] = B.core[i];
+  }
+}

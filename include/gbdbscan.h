@@ -81,14 +81,15 @@ typedef struct gd_stats {
   int64_t asym_pairs;       /* core pairs that are neighbours in one direction only
                                (the box test and the distance test disagree at the
                                last bit; their merges are replayed in order) */
-  int64_t grid_cells;       /* occupancy-table entries: cells of cell tables, rows of
-                               row tables (a hashed grid has none) */
+  int64_t grid_cells;       /* cells that direct block tables cover, and rows of block-row
+                               tables (a hashed grid has none) */
   int32_t precision_used;   /* gd_precision actually run */
   int32_t key_bits;         /* radix-sort key width */
   int32_t launches;         /* kernel launches of the last pipeline run */
   int32_t reserved;
   double ms_index;          /* device time: bbox, keys, sort, cell table */
-  double ms_core;           /* device time: core flags */
+  double ms_core;           /* device time: core flags (small runs, which expand in one
+                               kernel: the whole expand) */
   double ms_union;          /* device time: union-find */
   double ms_label;          /* device time: cluster ids, borders, output order */
   double ms_total;          /* device time of the whole pipeline (without host copies) */
@@ -116,7 +117,7 @@ gd_status gd_ctx_trim(gd_ctx* ctx);
 /* No counterpart in the reference.  With graphs enabled (the default), the
    second gd_expand on one index build captures the expand launches into a CUDA
    graph and later gd_expand calls on that index (other minpts) replay it with
-   one launch.  A new index build, a tuning change or gd_ctx_trim drops it. */
+   one launch.  (Small runs expand in one kernel anyway and capture nothing.)  A new index build, a tuning change or gd_ctx_trim drops it. */
 gd_status gd_ctx_set_graphs(gd_ctx* ctx, int32_t enable);
 
 /* ---- the pipeline, stage by stage ---------------------------------------- */
@@ -262,8 +263,8 @@ gd_status gd_server_get_stats(gd_server* srv, gd_server_stats* stats);
    nothing is allocated or freed.  The first call in a CUDA context of a device
    does a one-time set-up (it looks up that array's device address); make that
    first call before any stream capture begins.  The call synchronises its
-   stream twice: in the middle, to read the grid layout back to the host, and
-   at the end.  Calls share the array and it keeps the last call's contents;
+   stream once, at the end; where the grid needs the general pipeline (more than
+   16384 points spread too far for a direct block table) three times.  Calls share the array and it keeps the last call's contents;
    calls that overlap on the GPU race and must be serialised by the caller.
    labels_dev is undefined when the call fails.  n_clusters may be NULL. */
 #define GD_NOALLOC_MAX_POINTS 32768
