@@ -93,7 +93,7 @@ struct gd_ctx {
   double mult2 = kDefaultCellMult2, mult3 = kDefaultCellMult3;
   int tn_core = kDefaultCoreTests, tn_link = kDefaultLinkTests, tn_border = kDefaultBorderTests;
 
-  DevBuf coords, inst, chunks, Pv, Bi, bbox, keys0, keys1, vals0, vals1, X, Xf, ent, links, cellent, blklist,
+  DevBuf coords, inst, chunks, Pv, Bi, bbox, keys0, keys1, vals0, vals1, X, Xf, ent, links, pop, cellent, blklist,
       rowtab, hkeys, hvals, reps, bits, core, cellcore, cellmin, cellrep, parent, cellcid, lab, asym,
       hvcell, hvmask, out, coreout, sorttemp, scantemp, small, kcount;
 
@@ -160,7 +160,7 @@ struct gd_ctx {
 
   void free_all(bool keep_small) {
     DevBuf* a[] = {&coords, &inst,   &chunks,   &Pv,      &Bi,     &bbox,     &keys0,
-                   &keys1,  &vals0,  &vals1,    &X,       &Xf,     &ent,      &links, &cellent, &blklist, &rowtab, &hkeys,
+                   &keys1,  &vals0,  &vals1,    &X,       &Xf,     &ent,      &links, &pop, &cellent, &blklist, &rowtab, &hkeys,
                    &hvals,  &reps,   &bits,     &core,    &cellcore, &cellmin, &cellrep,
                    &parent, &cellcid,  &lab,     &asym,   &hvcell,   &hvmask,
                    &out,    &coreout, &sorttemp, &scantemp, &small, &kcount, &asymwork};
@@ -199,6 +199,7 @@ struct gd_ctx {
     B.ckeys = skeys == keys0.p ? keys1.p : keys0.p;
     B.ent = static_cast<gd::BlockEnt*>(ent.p);
     B.links = static_cast<gd::BlockLinks*>(links.p);
+    B.pop = f32 ? static_cast<gd::BlockPop*>(pop.p) : nullptr;
     B.ent_base = (uint32_t)bi.ent_total;
     B.cellent = static_cast<uint32_t*>(cellent.p);
     B.blklist = static_cast<uint32_t*>(blklist.p);
@@ -416,6 +417,9 @@ gd_status build_run(gd_ctx* ctx, uint64_t dense_floor, uint64_t rows_floor) {
   GD_TRY(ctx->ensure(ctx->links,
                      (bi.ent_total + (direct_only ? 0 : (uint64_t)n)) * sizeof(gd::BlockLinks),
                      "block links"));
+  if (ctx->f32)
+    GD_TRY(ctx->ensure(ctx->pop, (bi.ent_total + (direct_only ? 0 : (uint64_t)n)) * sizeof(gd::BlockPop),
+                       "block populations"));
   GD_TRY(ctx->ensure(ctx->cellent, n * 4, "cell entries"));
   GD_TRY(ctx->ensure(ctx->blklist, n * 4, "block list"));
   GD_TRY(ctx->ensure(ctx->rowtab, bi.row_total * 8, "row tables"));

@@ -211,6 +211,11 @@ struct alignas(8) BlockLinks {
   uint32_t w[3][2];
 };
 
+// Cells of a block holding two points and more, three and more.
+struct alignas(16) BlockPop {
+  uint32_t two[2], three[2];
+};
+
 // A grid with too many blocks for a direct table takes a table of its block
 // rows when it has at most this many rows per point (or the table floor).
 constexpr uint64_t kRowsPerPoint = 8;
@@ -240,7 +245,7 @@ enum Counter {
   kCtrWalkCursor2,      // walk-list entries handed out (2D, 3D); cleared before each walk launch
   kCtrWalkCursor3,
   kCtrWaitTimeouts,     // scan / sort launches whose look-back wait gave up (never expected)
-  kCtrBlocks,           // occupied blocks of the index
+  kCtrBlocks,           // blocks holding a core point (small runs: positions handed out)
   kCtrCount = 18
 };
 

@@ -41,10 +41,11 @@ struct Bufs {
   int64_t nw = 0;               // words of runbits / lbits
   int64_t nwf = 0;              // words of fbits
   const void* ckeys = nullptr;  // per non-empty cell: its key (same width as keys)
-  uint32_t* blklist = nullptr;  // first cell of every occupied block
+  uint32_t* blklist = nullptr;  // a core cell of every block holding one
   uint32_t* cellent = nullptr;  // per non-empty cell: its block's entry
   gd::BlockEnt* ent = nullptr;  // block entries: direct tables first, then (from ent_base)
   gd::BlockLinks* links = nullptr;  // per entry, as ent
+  gd::BlockPop* pop = nullptr;      // per entry, as ent; null in float64 mode
   uint32_t ent_base = 0;        // one slot per cell, used at each block's first cell
   uint2* rowtab = nullptr;      // row tables: cells [x, y) of every block row
   unsigned long long* hkeys = nullptr;  // row hash slots: key of the block row's start

@@ -70,7 +70,8 @@ constexpr size_t kOffXf = kOffX + up(kMaxPoints * 3 * 8);
 constexpr size_t kOffTable = kOffXf + up(kMaxPoints * 4 * 4);
 constexpr size_t kOffEnt = kOffTable + up(kTableRows * 8);
 constexpr size_t kOffLinks = kOffEnt + up((kTableBlocks + kMaxPoints) * sizeof(gd::BlockEnt));
-constexpr size_t kOffHkeys = kOffLinks + up((kTableBlocks + kMaxPoints) * sizeof(gd::BlockLinks));
+constexpr size_t kOffPop = kOffLinks + up((kTableBlocks + kMaxPoints) * sizeof(gd::BlockLinks));
+constexpr size_t kOffHkeys = kOffPop + up((kTableBlocks + kMaxPoints) * sizeof(gd::BlockPop));
 constexpr size_t kOffHvals = kOffHkeys + up(kHashSlots * 8);
 constexpr size_t kOffReps = kOffHvals + up(kHashSlots * 8);
 constexpr size_t kOffCellent = kOffReps + up((kMaxPoints + 1) * 4);
@@ -356,6 +357,7 @@ extern "C" gd_status gd_dbscan_noalloc(const double* coords_dev, int64_t n, int3
   B.ckeys = skeys == base + kOffKeys0 ? base + kOffKeys1 : base + kOffKeys0;
   B.ent = reinterpret_cast<gd::BlockEnt*>(base + kOffEnt);
   B.links = reinterpret_cast<gd::BlockLinks*>(base + kOffLinks);
+  B.pop = f32 ? reinterpret_cast<gd::BlockPop*>(base + kOffPop) : nullptr;
   B.ent_base = (uint32_t)bi.ent_total;
   B.rowtab = reinterpret_cast<uint2*>(base + kOffTable);
   B.hkeys = reinterpret_cast<unsigned long long*>(base + kOffHkeys);

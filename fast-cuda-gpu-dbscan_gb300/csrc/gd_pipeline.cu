@@ -783,59 +783,25 @@ k_runs(const gdl::Bufs B, int64_t n, Key* __restrict__ ckeys, unsigned tiles,
 // consecutive in key order, mostly within one warp: the run of lanes of one block
 // forms its occupancy word together; the lane of the block's first cell reads on
 // where the block goes past the warp's end (at most 63 cells), and writes the
-// entry (core word and roots empty) and its empty link words.  Every cell notes
+// entry (core word and roots empty).  Every cell notes
 // where its block's entry is.  The first and last cell of a block row write the
 // row's cell range (row table or hash slot).
-constexpr int kCellsThreads = 256, kCellsU = 4;
 template <class Key>
-__global__ void __launch_bounds__(kCellsThreads) k_cells(const gdl::Bufs B) {
+__global__ void __launch_bounds__(256) k_cells(const gdl::Bufs B) {
   const Key* __restrict__ ckeys = static_cast<const Key*>(B.ckeys);
   const int LB = B.Bi->LB;
   const int64_t M = *B.M;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  // kCellsU groups of 32 cells per warp and round; the round's block list entries
-  // take one atomic (an atomic per warp had bound the kernel: C3 159 us)
-  __shared__ uint32_t s_cnt[32];
-  __shared__ unsigned long long s_at;
-  const int64_t per = (int64_t)kCellsThreads * kCellsU;
-  for (int64_t r0 = blockIdx.x * per; r0 < M; r0 += gridDim.x * per) {
-    uint64_t kk[kCellsU];
-    unsigned ff[kCellsU];
-#pragma unroll
-    for (int u = 0; u < kCellsU; ++u) {
-      const int64_t m0 = r0 + (w * kCellsU + u) * 32, m = m0 + lane;
-      const uint64_t key = (uint64_t)ckeys[m < M ? m : M - 1];
-      const uint64_t blk = key >> kBlockBits;  // with the instance id
-      uint64_t pb = __shfl_up_sync(kFull, blk, 1);
-      if (lane == 0) pb = m > 0 && m < M ? (uint64_t)ckeys[m - 1] >> kBlockBits : ~0ull;
-      kk[u] = key;
-      ff[u] = __ballot_sync(kFull, m < M && (m == 0 || pb != blk));
-      if (lane == 0) s_cnt[w * kCellsU + u] = (uint32_t)__popc(ff[u]);
-    }
-    __syncthreads();
-    if (w == 0) {
-      const uint32_t c = s_cnt[lane];
-      uint32_t inc = c;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(kFull, inc, o);
-        if (lane >= o) inc += v;
-      }
-      s_cnt[lane] = inc - c;
-      if (lane == 31) s_at = atomicAdd(B.ctr + kCtrBlocks, (unsigned long long)inc);
-    }
-    __syncthreads();
-    const unsigned long long at0 = s_at;
-#pragma unroll
-    for (int u = 0; u < kCellsU; ++u) {
-    const int64_t m0 = r0 + (w * kCellsU + u) * 32, m = m0 + lane;
+  const int lane = threadIdx.x & 31;
+  for (int64_t m0 = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); m0 < M;
+       m0 += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t m = m0 + lane;
+    const uint64_t key = (uint64_t)ckeys[m < M ? m : M - 1];
+    const uint64_t blk = key >> kBlockBits;  // with the instance id
+    uint64_t pb = __shfl_up_sync(kFull, blk, 1);
+    if (lane == 0) pb = m > 0 ? (uint64_t)ckeys[m - 1] >> kBlockBits : ~0ull;
+    const bool first = m < M && (m == 0 || pb != blk);
+    const unsigned firsts = __ballot_sync(kFull, first);
     if (m >= M) continue;
-    const uint64_t key = kk[u], blk = key >> kBlockBits;
-    const unsigned firsts = ff[u];
-    const bool first = (firsts >> lane) & 1u;
-    // the block list, in no particular order
-    if (first)
-      B.blklist[at0 + s_cnt[w * kCellsU + u] + __popc(firsts & ((1u << lane) - 1u))] = (uint32_t)m;
     const DevParams& P = B.Pv[inst_of(key, LB)];
     const uint64_t lblk = (key & P.kmask) >> kBlockBits;
     const int mode = P.sparse;
@@ -847,9 +813,45 @@ __global__ void __launch_bounds__(kCellsThreads) k_cells(const gdl::Bufs B) {
     const int nv = M - m0 < 32 ? (int)(M - m0) : 32;
     const int re = after ? __ffs(after) - 1 : nv;
     const unsigned run = (unsigned)((1ull << re) - (1ull << rs));
-    const uint32_t b = 1u << (key & 31);
-    uint32_t lo = __reduce_or_sync(run, (key & 32) ? 0u : b);
-    uint32_t hi = __reduce_or_sync(run, (key & 32) ? b : 0u);
+    // the run's occupancy word, its cells of two points and more, of three and more:
+    // by reductions over the run where the warp holds few runs, else gathered by each
+    // run's first lane, a step per lane of the longest run
+    const int len = B.pop ? B.reps[m + 1] - B.reps[m] : 1;
+    const uint32_t code = (uint32_t)(key & 63) | (len > 2 ? 0x80u : len > 1 ? 0x40u : 0u);
+    const unsigned valid = __activemask();
+    uint32_t lo = 0, hi = 0;
+    BlockPop pop{};
+    auto add = [&](uint32_t c) {
+      const uint32_t b = 1u << (c & 31);
+      const bool up = (c & 32) != 0;
+      lo |= up ? 0u : b;
+      hi |= up ? b : 0u;
+      if (c & 0xc0u) {
+        pop.two[0] |= up ? 0u : b;
+        pop.two[1] |= up ? b : 0u;
+        if (c & 0x80u) {
+          pop.three[0] |= up ? 0u : b;
+          pop.three[1] |= up ? b : 0u;
+        }
+      }
+    };
+    add(code);
+    if (__popc(heads & valid) <= 5) {
+      lo = __reduce_or_sync(run, lo);
+      hi = __reduce_or_sync(run, hi);
+      if (B.pop) {
+        pop.two[0] = __reduce_or_sync(run, pop.two[0]);
+        pop.two[1] = __reduce_or_sync(run, pop.two[1]);
+        pop.three[0] = __reduce_or_sync(run, pop.three[0]);
+        pop.three[1] = __reduce_or_sync(run, pop.three[1]);
+      }
+    } else {
+      const int longest = (int)__reduce_max_sync(valid, (unsigned)(re - rs));
+      for (int k = 1; k < longest; ++k) {
+        const uint32_t c = __shfl_down_sync(valid, code, k);
+        if (lane == rs && k < re - rs) add(c);
+      }
+    }
     uint32_t e = P.ent_off + (uint32_t)lblk;
     if (mode != 0) {
       // the block's first cell: the run's first lane, or cells before the warp
@@ -864,8 +866,12 @@ __global__ void __launch_bounds__(kCellsThreads) k_cells(const gdl::Bufs B) {
         for (int64_t c = m0 + 32; c < M; ++c) {
           const uint64_t k = (uint64_t)ckeys[c];
           if (k >> kBlockBits != blk) break;
-          if (k & 32) hi |= 1u << (k & 31);
-          else lo |= 1u << (k & 31);
+          const int h = (k & 32) ? 1 : 0, cl = B.pop ? B.reps[c + 1] - B.reps[c] : 1;
+          const uint32_t cb = 1u << (k & 31);
+          if (h) hi |= cb;
+          else lo |= cb;
+          if (cl > 1) pop.two[h] |= cb;
+          if (cl > 2) pop.three[h] |= cb;
         }
       BlockEnt E;
       E.occ = (unsigned long long)hi << 32 | lo;
@@ -875,7 +881,7 @@ __global__ void __launch_bounds__(kCellsThreads) k_cells(const gdl::Bufs B) {
       E.hi = kNoEnt;
       E.uni = kNoEnt;
       B.ent[e] = E;
-      B.links[e] = BlockLinks{};
+      if (B.pop) B.pop[e] = pop;
     }
     if (mode == 0) continue;
     // the row's first key and the first key past it (no key of the run lies
@@ -907,8 +913,6 @@ __global__ void __launch_bounds__(kCellsThreads) k_cells(const gdl::Bufs B) {
       if (rfirst) slot->x = (uint32_t)m;
       if (rlast) slot->y = (uint32_t)(m + 1);
     }
-    }
-    __syncthreads();
   }
 }
 
@@ -1709,6 +1713,73 @@ __host__ __device__ constexpr int core_axes(int d) { return d == 3 ? 1 : d; }
 constexpr int kCoreThreads = 128;
 constexpr int kCoreWarps = kCoreThreads / 32;
 
+// Points in the stencil of a cell, counted up to `enough`: occupied cells, cells of
+// two and more, and the rest of the cells of three and more one by one.
+template <int D, bool KEY64>
+__device__ __forceinline__ int stencil_points(const gdl::Bufs& B, const DevParams& P,
+                                              uint64_t local, int enough) {
+  using St = Stencil<D>;
+  const CellXYZ<D> cc = decompose<D>(local, P);
+  St st;
+  st.init(cc);
+  StencilWords<D> W5;
+  W5.init(st.w5);
+  int pts = 0;
+  for (int r = 0; r < St::ROWS && pts < enough; ++r) {
+    const int64_t row = st.row(r, P);
+    if (row < 0) continue;
+    uint2 m[2];
+    W5.row(r, m[0], m[1]);
+    uint32_t e[2];
+    block_pair<D, KEY64>(B, P, (uint64_t)row, st.b0[D - 1], (m[0].x | m[0].y) != 0,
+                         (m[1].x | m[1].y) != 0, e[0], e[1]);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (e[h] == kNoEnt) continue;
+      const EntHead a = ent_head(B, e[h]);
+      const unsigned long long M = u64_of(m[h]), o = a.occ & M;
+      if (!o) continue;
+      const BlockPop p = B.pop[e[h]];
+      pts += __popcll(o) + __popcll((p.two[0] | (unsigned long long)p.two[1] << 32) & M);
+      for (unsigned long long w = (p.three[0] | (unsigned long long)p.three[1] << 32) & M;
+           w && pts < enough; w &= w - 1) {
+        const int c = ent_cell(a.occ, a.base, __ffsll((long long)w) - 1);
+        pts += B.reps[c + 1] - B.reps[c] - 2;
+      }
+    }
+  }
+  return pts;
+}
+
+// Cells whose stencil holds fewer than minpts points: no point of theirs is a core
+// point, and none needs a walk (a bit per cell in fbits).  A thread per cell.
+// Float32-band mode only: there it saves the batch workload, three of whose points in
+// four are noise, a quarter of the core phase (32.5 -> 25.1 ms) and costs a
+// single-instance run nothing (C3: core 1.85 -> 1.73 ms, index 1.58 -> 1.70).  The
+// float64 walk drops such points before it tests them; there the extra pass cost more
+// than it saved (2D tracks 1.03 -> 1.09 ms).
+template <bool KEY64>
+__global__ void __launch_bounds__(256) k_core_filter(const gdl::Bufs B) {
+  const int LB = B.Bi->LB;
+  const int64_t M = *B.M;
+  const int lane = threadIdx.x & 31;
+  for (int64_t m0 = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); m0 < M;
+       m0 += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t m = m0 + lane;
+    bool skip = false;
+    if (m < M) {
+      const uint64_t key = ckey_at<KEY64>(B, m);
+      const DevParams& P = B.Pv[inst_of(key, LB)];
+      const int minpts = P.minpts;
+      if (B.reps[m + 1] - B.reps[m] < minpts)
+        skip = (P.dim == 2 ? stencil_points<2, KEY64>(B, P, key & P.kmask, minpts)
+                           : stencil_points<3, KEY64>(B, P, key & P.kmask, minpts)) < minpts;
+    }
+    const unsigned b = __ballot_sync(kFull, skip);
+    if (lane == 0) B.fbits[m0 >> 5] = b;
+  }
+}
+
 // Core flags of points in dense cells (at least minpts points: all core, no
 // test), with their cells' core counts and smallest core indices.  Every other
 // point gets its bit in the walk list's mask (listed in sorted order
@@ -1720,12 +1791,12 @@ __global__ void k_core_split(const gdl::Bufs B, int64_t n, int chunk, int clear)
   const int LB = B.Bi->LB;
   const int lane = threadIdx.x & 31;
   unsigned long long dense = 0;
-  // a later expand of the index: the blocks' words start empty again (their link
-  // words do already)
-  const int64_t NBk = clear ? (int64_t)B.ctr[kCtrBlocks] : 0;
-  for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < NBk;
-       j += (int64_t)gridDim.x * blockDim.x) {
-    BlockEnt& E = B.ent[B.cellent[B.blklist[j]]];
+  // a later expand of the index: the blocks' words start empty again
+  const int64_t Mc = clear ? (int64_t)*B.M : 0;
+  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < Mc;
+       c += (int64_t)gridDim.x * blockDim.x) {
+    BlockEnt& E = B.ent[B.cellent[c]];
+    if (E.base != (uint32_t)c) continue;
     E.lo = kNoEnt;
     E.core = 0;
     E.hi = kNoEnt;
@@ -1760,8 +1831,11 @@ __global__ void k_core_split(const gdl::Bufs B, int64_t n, int chunk, int clear)
         B.core[i] = 1;
         if (i == b[u]) ++dense;
       }
-      // the walk list: the chunk starts among the points outside dense cells
-      const unsigned wl = __ballot_sync(kFull, i < n && !dn && ((int)i - b[u]) % chunk == 0);
+      // the walk list: the chunk starts among the points outside dense cells, but for
+      // the cells that k_core_filter settled
+      const bool out = B.pop && i < n && !dn && ((B.fbits[m[u] >> 5] >> (m[u] & 31)) & 1u);
+      if (out) B.core[i] = 0;
+      const unsigned wl = __ballot_sync(kFull, i < n && !dn && !out && ((int)i - b[u]) % chunk == 0);
       if (lane == 0) B.lbits[i0 >> 5] = wl;
       const unsigned cm = __ballot_sync(kFull, dn);
       const unsigned grp = run_peers(cm, m[u]);
@@ -2783,25 +2857,60 @@ __global__ void __launch_bounds__(kCellThreads) k_core_heavy(const gdl::Bufs B, 
 // ------------------------------------------------------------- union-find
 // Each core cell's representative (its first core point) and its bit in its
 // block's core word, and the mask of the core-cell list (listed in order for the
-// union; a word per warp over [0, n)).
+// union; a word per warp over [0, n)).  The cell whose bit is the block's first
+// lists the block (blklist, in no particular order) and clears its link words.
+// A round of a thread block takes kCoreCellsU x 256 cells and one atomic for its list
+// entries (an atomic per warp, all at one address, bounds such a kernel: about 0.7 ns
+// each).
+constexpr int kCoreCellsU = 4;
 template <bool KEY64>
-__global__ void k_core_cells(const gdl::Bufs B, int64_t n) {
+__global__ void __launch_bounds__(256) k_core_cells(const gdl::Bufs B, int64_t n) {
   const int64_t M = *B.M;
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  __shared__ uint32_t s_cnt[32];
+  __shared__ unsigned long long s_at;
+  const int64_t per = 256 * kCoreCellsU;
   // words of the mask beyond the cells are cleared before the launch
-  for (int64_t m0 = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); m0 < M;
-       m0 += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t m = m0 + lane;
-    const bool f = m < M && B.cellcore[m] > 0;
-    if (f) {
-      int q = B.reps[m];
-      while (!B.core[q]) ++q;
-      B.cellrep[m] = q;
-      B.compmin[m] = B.cellmin[m];
-      atomicOr(&B.ent[B.cellent[m]].core, 1ull << ((unsigned)ckey_at<KEY64>(B, m) & 63u));
+  for (int64_t r0 = blockIdx.x * per; r0 < M; r0 += gridDim.x * per) {
+    unsigned news[kCoreCellsU];
+#pragma unroll
+    for (int u = 0; u < kCoreCellsU; ++u) {
+      const int64_t m0 = r0 + (w * kCoreCellsU + u) * 32, m = m0 + lane;
+      const bool f = m < M && B.cellcore[m] > 0;
+      bool fresh = false;
+      if (f) {
+        int q = B.reps[m];
+        while (!B.core[q]) ++q;
+        B.cellrep[m] = q;
+        B.compmin[m] = B.cellmin[m];
+        const uint32_t e = B.cellent[m];
+        fresh = atomicOr(&B.ent[e].core, 1ull << ((unsigned)ckey_at<KEY64>(B, m) & 63u)) == 0;
+        if (fresh) B.links[e] = BlockLinks{};
+      }
+      const unsigned bl = __ballot_sync(kFull, f);
+      if (lane == 0 && m0 < M) B.lbits[m0 >> 5] = bl;
+      news[u] = __ballot_sync(kFull, fresh);
+      if (lane == 0) s_cnt[w * kCoreCellsU + u] = (uint32_t)__popc(news[u]);
     }
-    const unsigned bl = __ballot_sync(kFull, f);
-    if (lane == 0) B.lbits[m0 >> 5] = bl;
+    __syncthreads();
+    if (w == 0) {
+      const uint32_t c = s_cnt[lane];
+      uint32_t inc = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(kFull, inc, o);
+        if (lane >= o) inc += v;
+      }
+      s_cnt[lane] = inc - c;
+      if (lane == 31 && inc) s_at = atomicAdd(B.ctr + kCtrBlocks, (unsigned long long)inc);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kCoreCellsU; ++u)
+      if ((news[u] >> lane) & 1u)
+        B.blklist[s_at + s_cnt[w * kCoreCellsU + u] + __popc(news[u] & ((1u << lane) - 1u))] =
+            (uint32_t)(r0 + (w * kCoreCellsU + u) * 32 + lane);
+    __syncthreads();
   }
 }
 
@@ -2905,13 +3014,13 @@ __global__ void k_flood(const gdl::Bufs B) {
   const int64_t NBk = (int64_t)B.ctr[kCtrBlocks];
   for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < NBk;
        j += (int64_t)gridDim.x * blockDim.x) {
-    const int m0 = (int)B.blklist[j];
-    const uint32_t e = B.cellent[m0];
+    const int mc = (int)B.blklist[j];  // a cell of the block
+    const uint32_t e = B.cellent[mc];
+    const EntHead hd = ent_head(B, e);
     unsigned long long left = B.ent[e].core;
-    if (!left) continue;
-    const unsigned long long occ = B.ent[e].occ;
+    const unsigned long long occ = hd.occ;
+    const int m0 = (int)hd.base;
     const BlockLinks lk = B.links[e];
-    B.links[e] = BlockLinks{};  // for the next expand
     uint32_t uni = kNoEnt;
     unsigned long long l[3];
 #pragma unroll
@@ -3449,9 +3558,9 @@ int runs(const Bufs& B, bool key64, int64_t n, void* scan_temp, cudaStream_t s) 
 }
 
 int cells(const Bufs& B, bool key64, int64_t n, int sms, cudaStream_t s) {
-  const int g = grid_for(n, kCellsThreads * kCellsU, sms, 8);
-  if (key64) k_cells<unsigned long long><<<g, kCellsThreads, 0, s>>>(B);
-  else k_cells<uint32_t><<<g, kCellsThreads, 0, s>>>(B);
+  const int g = grid_for(n, 256, sms, 8);
+  if (key64) k_cells<unsigned long long><<<g, 256, 0, s>>>(B);
+  else k_cells<uint32_t><<<g, 256, 0, s>>>(B);
   return 1;
 }
 
@@ -3484,6 +3593,10 @@ int core(const Bufs& B, int64_t n, int dims, bool f32, bool key64, bool one, boo
   // dense cells at once; the other points listed in sorted order for the walk
   const int g = grid_for(n, 256, sms, 8);
   const int chunk = f32 ? kCoreChunk : 1;
+  if (B.pop) {
+    if (key64) k_core_filter<true><<<g, 256, 0, s>>>(B);
+    else k_core_filter<false><<<g, 256, 0, s>>>(B);
+  }
   if (key64) {
     if (one) k_core_split<true, true><<<g, 256, 0, s>>>(B, n, chunk, fresh ? 0 : 1);
     else k_core_split<true, false><<<g, 256, 0, s>>>(B, n, chunk, fresh ? 0 : 1);
@@ -3491,7 +3604,7 @@ int core(const Bufs& B, int64_t n, int dims, bool f32, bool key64, bool one, boo
     if (one) k_core_split<false, true><<<g, 256, 0, s>>>(B, n, chunk, fresh ? 0 : 1);
     else k_core_split<false, false><<<g, 256, 0, s>>>(B, n, chunk, fresh ? 0 : 1);
   }
-  int L = 1 + list_bits(B, n, scan_temp, s);
+  int L = (B.pop ? 2 : 1) + list_bits(B, n, scan_temp, s);
   cudaMemsetAsync(B.ctr + kCtrWalkCursor2, 0, 16, s);
   // 3D walks split after pass 0 (the 3^3 shell)
   if (dims & 2) cudaMemsetAsync(B.fbits, 0, (size_t)B.nw * 4, s);
@@ -3524,8 +3637,9 @@ int core(const Bufs& B, int64_t n, int dims, bool f32, bool key64, bool one, boo
 int unite(const Bufs& B, int64_t n, int dims, bool f32, bool key64, int sms, void* scan_temp,
           cudaStream_t s) {
   cudaMemsetAsync(B.lbits, 0, (size_t)B.nw * 4, s);
-  if (key64) k_core_cells<true><<<grid_for(n, 256, sms, 8), 256, 0, s>>>(B, n);
-  else k_core_cells<false><<<grid_for(n, 256, sms, 8), 256, 0, s>>>(B, n);
+  cudaMemsetAsync(B.ctr + kCtrBlocks, 0, 8, s);
+  if (key64) k_core_cells<true><<<grid_for(n, 256 * kCoreCellsU, sms, 8), 256, 0, s>>>(B, n);
+  else k_core_cells<false><<<grid_for(n, 256 * kCoreCellsU, sms, 8), 256, 0, s>>>(B, n);
   int L = 1 + list_bits(B, n, scan_temp, s);
   const int lgrid = grid_for(n, 256, sms, 8);
   GD_LAUNCH_DIMS(dims, f32, key64, k_links, lgrid, 256, B, n);

@@ -236,11 +236,11 @@ k_rs_downsweep(const K* __restrict__ kin, const uint32_t* __restrict__ vin,
 
 // Set bits of a mask listed in one pass: per-word prefix counts (pre) and the
 // positions of the set bits in order (out[pre[w] + r] = 32 w + (bit r of word w)).
-// A tile is 2048 words (512 threads x 4): word counts are scanned in the block, the
-// tile's prefix comes by look-back, and each warp then writes its 128 words one at
+// A tile is 512 words, one per thread: word counts are scanned in the block, the
+// tile's prefix comes by look-back, and each warp then writes its 32 words one at
 // a time with a lane per bit, so each word's entries go out in one store.  One
 // launch where a scan and a compaction took two.
-constexpr int kListThreads = 512, kListWords = 4, kListTile = kListThreads * kListWords;
+constexpr int kListThreads = 512, kListWords = 1, kListTile = kListThreads * kListWords;
 __global__ void __launch_bounds__(kListThreads)
 k_list_bits(const uint32_t* __restrict__ words, uint32_t* __restrict__ pre, int64_t nw,
             uint32_t* __restrict__ out, unsigned tiles, LookbackCtl* ctl,
