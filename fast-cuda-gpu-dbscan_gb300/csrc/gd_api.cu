@@ -93,7 +93,7 @@ struct gd_ctx {
   double mult2 = kDefaultCellMult2, mult3 = kDefaultCellMult3;
   int tn_core = kDefaultCoreTests, tn_link = kDefaultLinkTests, tn_border = kDefaultBorderTests;
 
-  DevBuf coords, inst, chunks, Pv, Bi, bbox, keys0, keys1, vals0, vals1, X, Xf, ent, links, pop, cellent, blklist,
+  DevBuf coords, inst, chunks, Pv, Bi, bbox, keys0, keys1, vals0, vals1, X, Xf, ent, links, pop, cellent, blklist, nbr,
       rowtab, hkeys, hvals, reps, bits, core, cellcore, cellmin, cellrep, parent, cellcid, lab, asym,
       hvcell, hvmask, out, coreout, sorttemp, scantemp, small, kcount;
 
@@ -160,7 +160,7 @@ struct gd_ctx {
 
   void free_all(bool keep_small) {
     DevBuf* a[] = {&coords, &inst,   &chunks,   &Pv,      &Bi,     &bbox,     &keys0,
-                   &keys1,  &vals0,  &vals1,    &X,       &Xf,     &ent,      &links, &pop, &cellent, &blklist, &rowtab, &hkeys,
+                   &keys1,  &vals0,  &vals1,    &X,       &Xf,     &ent,      &links, &pop, &cellent, &blklist, &nbr, &rowtab, &hkeys,
                    &hvals,  &reps,   &bits,     &core,    &cellcore, &cellmin, &cellrep,
                    &parent, &cellcid,  &lab,     &asym,   &hvcell,   &hvmask,
                    &out,    &coreout, &sorttemp, &scantemp, &small, &kcount, &asymwork};
@@ -203,6 +203,7 @@ struct gd_ctx {
     B.ent_base = (uint32_t)bi.ent_total;
     B.cellent = static_cast<uint32_t*>(cellent.p);
     B.blklist = static_cast<uint32_t*>(blklist.p);
+    B.nbr = bi.row_total || bi.any_sparse ? static_cast<uint2*>(nbr.p) : nullptr;
     B.rowtab = static_cast<uint2*>(rowtab.p);
     B.hkeys = static_cast<unsigned long long*>(hkeys.p);
     B.hvals = static_cast<uint2*>(hvals.p);
@@ -422,6 +423,7 @@ gd_status build_run(gd_ctx* ctx, uint64_t dense_floor, uint64_t rows_floor) {
                        "block populations"));
   GD_TRY(ctx->ensure(ctx->cellent, n * 4, "cell entries"));
   GD_TRY(ctx->ensure(ctx->blklist, n * 4, "block list"));
+  if (!direct_only) GD_TRY(ctx->ensure(ctx->nbr, n * 4 * sizeof(uint2), "neighbour entries"));
   GD_TRY(ctx->ensure(ctx->rowtab, bi.row_total * 8, "row tables"));
   uint64_t hcap = 1024;
   if (bi.any_sparse) {

@@ -47,6 +47,8 @@ struct Bufs {
   gd::BlockLinks* links = nullptr;  // per entry, as ent
   gd::BlockPop* pop = nullptr;      // per entry, as ent; null in float64 mode
   uint32_t ent_base = 0;        // one slot per cell, used at each block's first cell
+  uint2* nbr = nullptr;         // 4 per cell: neighbour entries by stencil row (k_neighbors);
+                                // null when every instance has a direct table
   uint2* rowtab = nullptr;      // row tables: cells [x, y) of every block row
   unsigned long long* hkeys = nullptr;  // row hash slots: key of the block row's start
   uint2* hvals = nullptr;               // row hash slots: cells [x, y) of the row

@@ -76,7 +76,8 @@ constexpr size_t kOffHvals = kOffHkeys + up(kHashSlots * 8);
 constexpr size_t kOffReps = kOffHvals + up(kHashSlots * 8);
 constexpr size_t kOffCellent = kOffReps + up((kMaxPoints + 1) * 4);
 constexpr size_t kOffBlklist = kOffCellent + up(kMaxPoints * 4);
-constexpr size_t kOffBits = kOffBlklist + up(kMaxPoints * 4);  // cell starts, lists, marks
+constexpr size_t kOffNbr = kOffBlklist + up(kMaxPoints * 4);
+constexpr size_t kOffBits = kOffNbr + up(kMaxPoints * 32);  // cell starts, lists, marks
 constexpr size_t kOffCore = kOffBits + up(gdl::bit_layout(kMaxPoints).words * 4);
 constexpr size_t kOffCellcore = kOffCore + up(kMaxPoints);
 constexpr size_t kOffCellmin = kOffCellcore + up(kMaxPoints * 4);
@@ -354,6 +355,7 @@ extern "C" gd_status gd_dbscan_noalloc(const double* coords_dev, int64_t n, int3
   B.reps = reinterpret_cast<int*>(base + kOffReps);
   B.cellent = reinterpret_cast<uint32_t*>(base + kOffCellent);
   B.blklist = reinterpret_cast<uint32_t*>(base + kOffBlklist);
+  B.nbr = bi.row_total || bi.any_sparse ? reinterpret_cast<uint2*>(base + kOffNbr) : nullptr;
   B.ckeys = skeys == base + kOffKeys0 ? base + kOffKeys1 : base + kOffKeys0;
   B.ent = reinterpret_cast<gd::BlockEnt*>(base + kOffEnt);
   B.links = reinterpret_cast<gd::BlockLinks*>(base + kOffLinks);
