@@ -1599,7 +1599,7 @@ __device__ __forceinline__ WalkCursor walk_cursor(const gdl::Bufs& B, int64_t jl
 #define GD_CORE_MIN_BLOCKS 8
 #endif
 #ifndef GD_CORE_CELL_MIN_BLOCKS
-#define GD_CORE_CELL_MIN_BLOCKS 8
+#define GD_CORE_CELL_MIN_BLOCKS 7
 #endif
 #ifndef GD_UNION_MIN_BLOCKS
 #define GD_UNION_MIN_BLOCKS 6
@@ -1913,12 +1913,14 @@ __global__ void k_core_split(const gdl::Bufs B, int64_t n, int chunk, int clear)
 // one stencil walk: the stencil comes as a few 64-cell occupancy words (4 block
 // lookups in 2D, 8 in 3D, two at a time; home row first), masked to the cells
 // within one (pass 0) and then two (pass 1) of the own cell, whose points count at
-// once; slabs and cells out of reach of the chunk's bounding box leave the walk.
+// once; slabs out of reach of the chunk's bounding box leave the masks.
 // Every candidate of an occupied cell is loaded once and tested against all the
 // chunk's points in registers -- a float32 test is about nine instructions, less
 // than the steps that reach a candidate, so sharing those pays more than any
 // finer rule on what to test.  Only cells of more than kCoreBigCell points are
-// classified per point first (wholly inside eps: count, wholly outside: skip).
+// classified first, as a whole and per point (wholly inside eps: count, wholly
+// outside: skip; from 1, 2, 5 points on the batch's core phase took 20.7, 20.1 and 18.7
+// ms, from 8 on 18.4, and no less beyond).
 // A chunk whose tests pass the budget sends its cell to the warp kernel, which
 // recomputes the whole cell.  Per-cell core counts and smallest core indices are
 // warp-aggregated atomics (cleared before the launch).
@@ -2007,25 +2009,20 @@ k_core_cell(const gdl::Bufs B, int64_t n, int p0, int p1) {
       int budget = B.tn_core * present;
       bool done = present == 0;
       // one occupied cell: place `bit` of block (row r, half h) of the stencil
-      auto visit = [&](int c, int bit, int r, int h) {
-        int off[3] = {0, 0, 0};
-#pragma unroll
-        for (int k = 0; k < D; ++k) {
-          const int half = k == D - 1 ? h : (D == 3 ? (k == 0 ? r >> 1 : r & 1) : r);
-          off[k] = st.off0(cc, k) + (half << St::S) + St::bit_off(bit, k);
-        }
-        if (prune) {
+      auto visit = [&](int q0, int qe, int bit, int r, int h) {
+        if (prune && qe - q0 > kCoreBigCell) {
+          // out of reach of all the points, or settled for each of them?
+          int off[3] = {0, 0, 0};
           float smin = 0.0f;
 #pragma unroll
           for (int k = 0; k < D; ++k) {
+            const int half = k == D - 1 ? h : (D == 3 ? (k == 0 ? r >> 1 : r & 1) : r);
+            off[k] = st.off0(cc, k) + (half << St::S) + St::bit_off(bit, k);
             const float d = (float)off[k];
             const float mn = fmaxf(fmaxf(d - uhi[k], ulo[k] - 1.0f - d), 0.0f);
             smin = fmaf(mn, mn, smin);
           }
           if (smin >= Q.thr_out) return;
-        }
-        const int q0 = B.reps[c], qe = B.reps[c + 1];
-        if (prune && qe - q0 > kCoreBigCell) {
           int cl[C];
           bool open = false;
 #pragma unroll
@@ -2135,7 +2132,8 @@ k_core_cell(const gdl::Bufs B, int64_t n, int p0, int p1) {
             }
             const int bit = __ffsll((long long)w) - 1;
             w &= w - 1;
-            visit(ent_cell(a.occ, a.base, bit), bit, r, h);
+            const int c = ent_cell(a.occ, a.base, bit);
+            visit(B.reps[c], B.reps[c + 1], bit, r, h);
           }
         }
       }
