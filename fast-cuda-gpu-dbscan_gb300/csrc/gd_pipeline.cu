@@ -781,9 +781,9 @@ k_runs(const gdl::Bufs B, int64_t n, Key* __restrict__ ckeys, unsigned tiles,
 
 // Block entries and row lookups, a lane per cell.  A block's cells are
 // consecutive in key order, mostly within one warp: the run of lanes of one block
-// forms its occupancy word together; the lane of the block's first cell reads on
-// where the block goes past the warp's end (at most 63 cells), and writes the
-// entry (core word and roots empty).  Every cell notes
+// forms its occupancy word together; where the block of the last lane goes past the
+// warp's end the warp reads on (at most 63 cells), and the lane of the block's first
+// cell writes the entry (core word and roots empty).  Every cell notes
 // where its block's entry is.  The first and last cell of a block row write the
 // row's cell range (row table or hash slot).
 template <class Key>
@@ -801,10 +801,6 @@ __global__ void __launch_bounds__(256) k_cells(const gdl::Bufs B) {
     if (lane == 0) pb = m > 0 ? (uint64_t)ckeys[m - 1] >> kBlockBits : ~0ull;
     const bool first = m < M && (m == 0 || pb != blk);
     const unsigned firsts = __ballot_sync(kFull, first);
-    if (m >= M) continue;
-    const DevParams& P = B.Pv[inst_of(key, LB)];
-    const uint64_t lblk = (key & P.kmask) >> kBlockBits;
-    const int mode = P.sparse;
     // this lane's run: lanes [rs, re) hold cells of its block
     const unsigned heads = firsts | 1u;
     const unsigned upto = (unsigned)((2ull << lane) - 1ull);
@@ -812,46 +808,69 @@ __global__ void __launch_bounds__(256) k_cells(const gdl::Bufs B) {
     const unsigned after = heads & ~upto;
     const int nv = M - m0 < 32 ? (int)(M - m0) : 32;
     const int re = after ? __ffs(after) - 1 : nv;
-    const unsigned run = (unsigned)((1ull << re) - (1ull << rs));
-    // the run's occupancy word, its cells of two points and more, of three and more:
-    // by reductions over the run where the warp holds few runs, else gathered by each
-    // run's first lane, a step per lane of the longest run
-    const int len = B.pop ? B.reps[m + 1] - B.reps[m] : 1;
-    const uint32_t code = (uint32_t)(key & 63) | (len > 2 ? 0x80u : len > 1 ? 0x40u : 0u);
-    const unsigned valid = __activemask();
-    uint32_t lo = 0, hi = 0;
-    BlockPop pop{};
-    auto add = [&](uint32_t c) {
-      const uint32_t b = 1u << (c & 31);
-      const bool up = (c & 32) != 0;
-      lo |= up ? 0u : b;
-      hi |= up ? b : 0u;
-      if (c & 0xc0u) {
-        pop.two[0] |= up ? 0u : b;
-        pop.two[1] |= up ? b : 0u;
-        if (c & 0x80u) {
-          pop.three[0] |= up ? 0u : b;
-          pop.three[1] |= up ? b : 0u;
-        }
+    // the run's occupancy word, its cells of two points and more, of three and more,
+    // gathered at its first lane: a segmented OR over the lanes that follow
+    const int len = B.pop && m < M ? B.reps[m + 1] - B.reps[m] : 1;
+    const uint32_t b = 1u << (key & 31);
+    const bool up = (key & 32) != 0;
+    uint32_t lo = up ? 0u : b, hi = up ? b : 0u;
+    BlockPop pop;
+    pop.two[0] = len > 1 ? lo : 0u;
+    pop.two[1] = len > 1 ? hi : 0u;
+    pop.three[0] = len > 2 ? lo : 0u;
+    pop.three[1] = len > 2 ? hi : 0u;
+    auto gather = [&](uint32_t& x) {
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_down_sync(kFull, x, o);
+        if (lane + o < re) x |= y;
       }
     };
-    add(code);
-    if (__popc(heads & valid) <= 5) {
-      lo = __reduce_or_sync(run, lo);
-      hi = __reduce_or_sync(run, hi);
-      if (B.pop) {
-        pop.two[0] = __reduce_or_sync(run, pop.two[0]);
-        pop.two[1] = __reduce_or_sync(run, pop.two[1]);
-        pop.three[0] = __reduce_or_sync(run, pop.three[0]);
-        pop.three[1] = __reduce_or_sync(run, pop.three[1]);
-      }
-    } else {
-      const int longest = (int)__reduce_max_sync(valid, (unsigned)(re - rs));
-      for (int k = 1; k < longest; ++k) {
-        const uint32_t c = __shfl_down_sync(valid, code, k);
-        if (lane == rs && k < re - rs) add(c);
+    gather(lo);
+    gather(hi);
+    if (B.pop) {
+      gather(pop.two[0]);
+      gather(pop.two[1]);
+      gather(pop.three[0]);
+      gather(pop.three[1]);
+    }
+    // the block of the warp's last lane goes on past it: the warp reads on together
+    const int rl = 31 - __clz(heads);
+    if (m0 + 32 < M && ((firsts >> rl) & 1u)) {
+      const uint64_t bl = __shfl_sync(kFull, blk, 31);
+      for (int64_t c0 = m0 + 32;; c0 += 32) {
+        const int64_t c = c0 + lane;
+        const uint64_t k = c < M ? (uint64_t)ckeys[c] : 0;
+        const bool same = c < M && k >> kBlockBits == bl;
+        if (!__any_sync(kFull, same)) break;
+        const uint32_t cb = same ? 1u << (k & 31) : 0u;
+        const bool cu = (k & 32) != 0;
+        const int cl = B.pop && same ? B.reps[c + 1] - B.reps[c] : 1;
+        const uint32_t l0 = cu ? 0u : cb, h0 = cu ? cb : 0u;
+        const uint32_t a0 = __reduce_or_sync(kFull, l0), a1 = __reduce_or_sync(kFull, h0);
+        if (lane == rl) {
+          lo |= a0;
+          hi |= a1;
+        }
+        if (B.pop) {
+          const uint32_t t0 = __reduce_or_sync(kFull, cl > 1 ? l0 : 0u);
+          const uint32_t t1 = __reduce_or_sync(kFull, cl > 1 ? h0 : 0u);
+          const uint32_t u0 = __reduce_or_sync(kFull, cl > 2 ? l0 : 0u);
+          const uint32_t u1 = __reduce_or_sync(kFull, cl > 2 ? h0 : 0u);
+          if (lane == rl) {
+            pop.two[0] |= t0;
+            pop.two[1] |= t1;
+            pop.three[0] |= u0;
+            pop.three[1] |= u1;
+          }
+        }
+        if (!__all_sync(kFull, same)) break;
       }
     }
+    if (m >= M) continue;
+    const DevParams& P = B.Pv[inst_of(key, LB)];
+    const uint64_t lblk = (key & P.kmask) >> kBlockBits;
+    const int mode = P.sparse;
     uint32_t e = P.ent_off + (uint32_t)lblk;
     if (mode != 0) {
       // the block's first cell: the run's first lane, or cells before the warp
@@ -862,17 +881,6 @@ __global__ void __launch_bounds__(256) k_cells(const gdl::Bufs B) {
     }
     B.cellent[m] = e;
     if (first) {
-      if (re == 32)
-        for (int64_t c = m0 + 32; c < M; ++c) {
-          const uint64_t k = (uint64_t)ckeys[c];
-          if (k >> kBlockBits != blk) break;
-          const int h = (k & 32) ? 1 : 0, cl = B.pop ? B.reps[c + 1] - B.reps[c] : 1;
-          const uint32_t cb = 1u << (k & 31);
-          if (h) hi |= cb;
-          else lo |= cb;
-          if (cl > 1) pop.two[h] |= cb;
-          if (cl > 2) pop.three[h] |= cb;
-        }
       BlockEnt E;
       E.occ = (unsigned long long)hi << 32 | lo;
       E.base = (uint32_t)m;
@@ -2307,7 +2315,7 @@ k_core_point(const gdl::Bufs B, int64_t n, int p0, int p1) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           unsigned long long w = hd[h].occ & M[h], open = 0;
-          while (w) {
+          while (w && cnt < minpts) {
             const int bit = __ffsll((long long)w) - 1;
             w &= w - 1;
             int cls = 0;
