@@ -522,7 +522,6 @@ gd_status expand_run(gd_ctx* ctx) {
   }
   GD_TRY(ctx->ensure(ctx->core, n, "core flags"));
   GD_TRY(ctx->ensure(ctx->cellcore, n * 4, "cell core counts"));
-  GD_TRY(ctx->ensure(ctx->cellmin, n * 4, "cell min index"));
   GD_TRY(ctx->ensure(ctx->cellrep, n * 4, "cell representatives"));
   GD_TRY(ctx->ensure(ctx->parent, n * 4, "union-find parents"));
   GD_TRY(ctx->ensure(ctx->cellcid, n * 4, "cell cluster ids"));

@@ -14,7 +14,8 @@
 // Per non-empty cell, indexed by its cell index m (0..M-1, key order; the
 // walks reach it from a block entry's occupancy word without loading reps):
 //   cellcore[m]  number of core points in the cell
-//   cellmin[m]   smallest original index among the cell's core points
+//   compmin[m]   smallest original index among the cell's core points (general path: that of
+//                its first core position, ids ascend within a cell; small path: cellmin[m])
 //   parent[m]    union-find parent (a cell index)
 //   cellcid[m]   cluster id of the cell's core points (INT_MAX: none)
 #pragma once

@@ -58,8 +58,9 @@ struct Bufs {
   float* Xf = nullptr;          // sorted centred float32 points (2 or 4 floats each)
   uint8_t* core = nullptr;      // core flag per sorted position
   int* cellcore = nullptr;      // per cell m: number of core points
-  int* cellmin = nullptr;       // per cell m: smallest global index of a core point
-  int* compmin = nullptr;       // per root: smallest core index of its component (in lab's
+  int* cellmin = nullptr;       // small runs, per cell m: smallest index of a core point
+  int* compmin = nullptr;       // per core cell: its smallest core index; per root, in the
+                                // end, its component's (in lab's
                                 // memory, which holds no labels before the border search)
   int* cellrep = nullptr;       // per core cell m: its first core point (sorted position)
   int* parent = nullptr;        // per cell m: union-find parent (a cell index)

@@ -377,7 +377,6 @@ extern "C" gd_status gd_dbscan_noalloc(const double* coords_dev, int64_t n, int3
   // expansion (the same stages as gd_expand)
   B.core = base + kOffCore;
   B.cellcore = reinterpret_cast<int*>(base + kOffCellcore);
-  B.cellmin = reinterpret_cast<int*>(base + kOffCellmin);
   B.cellrep = reinterpret_cast<int*>(base + kOffCellrep);
   B.parent = reinterpret_cast<int*>(base + kOffParent);
   B.cellcid = reinterpret_cast<int*>(base + kOffCellcid);

@@ -1131,12 +1131,6 @@ __device__ __forceinline__ void flush_tally(const Tally& t, unsigned long long* 
   }
 }
 
-__device__ __forceinline__ int warp_min_i32(int v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(kFull, v, o));
-  return v;
-}
-
 // The lanes sharing this lane's value v, for values that sit in runs of
 // consecutive lanes (lanes holding sorted points: a cell's points are
 // neighbours).  act: the lanes taking part; the result is the run of
@@ -1843,7 +1837,7 @@ __global__ void __launch_bounds__(256) k_core_filter(const gdl::Bufs B) {
 }
 
 // Core flags of points in dense cells (at least minpts points: all core, no
-// test), with their cells' core counts and smallest core indices.  Every other
+// test), with their cells' core counts.  Every other
 // point gets its bit in the walk list's mask (listed in sorted order
 // afterwards), so that k_core_point's warps hold only neighbouring points that
 // walk.  ONE: a single instance (its parameters are Pv[0]).
@@ -1869,13 +1863,11 @@ __global__ void k_core_split(const gdl::Bufs B, int64_t n, int chunk, int clear)
   for (int64_t g0 = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); g0 < n;
        g0 += U * stride) {
     int m[U], b[U], e[U], mp[U];
-    uint32_t id[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int64_t i = g0 + u * stride + lane;
       const int64_t ic = i < n ? i : n - 1;
       m[u] = cell_of(B, ic);
-      id[u] = B.ids[ic];
       mp[u] = B.Pv[ONE ? 0 : (int)(key_at<KEY64>(B, ic) >> LB)].minpts;
     }
 #pragma unroll
@@ -1891,23 +1883,17 @@ __global__ void k_core_split(const gdl::Bufs B, int64_t n, int chunk, int clear)
       const bool dn = i < n && e[u] - b[u] >= mp[u];
       if (dn) {
         B.core[i] = 1;
-        if (i == b[u]) ++dense;
+        if (i == b[u]) {
+          B.cellcore[m[u]] = e[u] - b[u];
+          ++dense;
+        }
       }
       // the walk list: the chunk starts among the points outside dense cells, but for
       // the cells that k_core_filter settled
       const bool out = B.pop && i < n && !dn && ((B.fbits[m[u] >> 5] >> (m[u] & 31)) & 1u);
       if (out) B.core[i] = 0;
-      const unsigned wl = __ballot_sync(kFull, i < n && !dn && !out && ((int)i - b[u]) % chunk == 0);
+      const unsigned wl = __ballot_sync(kFull, i < n && !dn && !out && (((int)i - b[u]) & (chunk - 1)) == 0);
       if (lane == 0) B.lbits[i0 >> 5] = wl;
-      const unsigned cm = __ballot_sync(kFull, dn);
-      const unsigned grp = run_peers(cm, m[u]);
-      if (dn) {
-        const unsigned mn = __reduce_min_sync(grp, id[u]);
-        if (lane == __ffs(grp) - 1) {
-          atomicAdd(B.cellcore + m[u], __popc(grp));
-          atomicMin(reinterpret_cast<unsigned*>(B.cellmin) + m[u], mn);
-        }
-      }
     }
   }
 #pragma unroll
@@ -1930,8 +1916,8 @@ __global__ void k_core_split(const gdl::Bufs B, int64_t n, int chunk, int clear)
 // outside: skip; from 1, 2, 5 points on the batch's core phase took 20.7, 20.1 and 18.7
 // ms, from 8 on 18.4, and no less beyond).
 // A chunk whose tests pass the budget sends its cell to the warp kernel, which
-// recomputes the whole cell.  Per-cell core counts and smallest core indices are
-// warp-aggregated atomics (cleared before the launch).
+// recomputes the whole cell.  Per-cell core counts are atomics (cleared before the
+// launch).
 //
 // Passes [p0, p1).  3D runs pass 0 for every listed chunk first: a chunk with an
 // undecided point keeps its points' counts in lab[] (kDecided for decided ones)
@@ -2148,7 +2134,6 @@ k_core_cell(const gdl::Bufs B, int64_t n, int p0, int p1) {
     }
     // results: core flags; in a first launch the undecided chunks go on
     int ncore = 0;
-    unsigned mn = 0xffffffffu;
     if (valid && !over) {
       bool go_on = false;
 #pragma unroll
@@ -2160,25 +2145,12 @@ k_core_cell(const gdl::Bufs B, int64_t n, int p0, int p1) {
           go_on |= !isc;
         }
         if (isc || !split) B.core[i + a] = isc ? 1 : 0;
-        if (isc) {
-          ++ncore;
-          mn = min(mn, B.ids[i + a]);
-        }
+        ncore += isc;
       }
       if (go_on) atomicOr(B.fbits + (i >> 5), 1u << (i & 31));
     }
-    // per-cell core count and smallest core index, one atomic pair per cell
-    // and warp
-    const unsigned cm = __ballot_sync(kFull, ncore > 0);
-    const unsigned grp = run_peers(cm, m);
-    if (ncore > 0) {
-      const unsigned mm = __reduce_min_sync(grp, mn);
-      const unsigned nn = __reduce_add_sync(grp, (unsigned)ncore);
-      if (lane == __ffs(grp) - 1) {
-        atomicAdd(B.cellcore + m, (int)nn);
-        atomicMin(reinterpret_cast<unsigned*>(B.cellmin) + m, mm);
-      }
-    }
+    // per-cell core count
+    if (ncore > 0) atomicAdd(B.cellcore + m, ncore);
     // cells with an undecided chunk, once per warp
     const unsigned om = __ballot_sync(kFull, over);
     bool lead = false;
@@ -2430,17 +2402,9 @@ k_core_point(const gdl::Bufs B, int64_t n, int p0, int p1) {
       atomicOr(B.fbits + (i >> 5), 1u << (i & 31));
     }
     if (valid && !over && !go_on) B.core[i] = isc ? 1 : 0;
-    // per-cell core count and smallest core index, one atomic pair per cell
-    // and warp
-    const unsigned cm = __ballot_sync(kFull, isc);
-    const unsigned grp = run_peers(cm, m);
-    if (isc) {
-      const unsigned mn = __reduce_min_sync(grp, (unsigned)B.ids[i]);
-      if (lane == __ffs(grp) - 1) {
-        atomicAdd(B.cellcore + m, __popc(grp));
-        atomicMin(reinterpret_cast<unsigned*>(B.cellmin) + m, mn);
-      }
-    }
+    // per-cell core count, one atomic per cell and warp
+    const unsigned grp = run_peers(__ballot_sync(kFull, isc), m);
+    if (isc && lane == __ffs(grp) - 1) atomicAdd(B.cellcore + m, __popc(grp));
     // cells with an undecided point, once per warp
     const unsigned om = __ballot_sync(kFull, over);
     bool lead = false;
@@ -2863,19 +2827,14 @@ __global__ void __launch_bounds__(kCellThreads) k_core_heavy(const gdl::Bufs B, 
     const DevParams& P = *cx.P;
     const PredParams Q = pred_params(P);
     if (sz >= Q.minpts) {
-      int mn = INT_MAX;
-      for (int i = b + lane; i < e; i += 32) {
-        B.core[i] = 1;
-        mn = min(mn, (int)B.ids[i]);
-      }
-      mn = warp_min_i32(mn);
-      if (lane == 0) { B.cellcore[m] = sz; B.cellmin[m] = mn; ++dense; }
+      for (int i = b + lane; i < e; i += 32) B.core[i] = 1;
+      if (lane == 0) { B.cellcore[m] = sz; ++dense; }
       continue;
     }
     const CellXYZ<D> cc = decompose<D>(cx.local, P);
     int ncells = 0;
     const int total = build_cells<D, KEY64>(B, CL, cc, P, lane, ncells);
-    int ncore = 0, mn = INT_MAX;
+    int ncore = 0;
     for (int c0 = 0; c0 < sz; c0 += 32) {
       const int na = min(32, sz - c0);
       if (lane < na) {
@@ -2903,12 +2862,10 @@ __global__ void __launch_bounds__(kCellThreads) k_core_heavy(const gdl::Bufs B, 
       }
       const bool isc = lane < na && mycnt >= Q.minpts;
       if (lane < na) B.core[b + c0 + lane] = isc ? 1 : 0;
-      if (isc) mn = min(mn, (int)B.ids[b + c0 + lane]);
       ncore += __popc(__ballot_sync(kFull, isc));
       __syncwarp();
     }
-    mn = warp_min_i32(mn);
-    if (lane == 0) { B.cellcore[m] = ncore; B.cellmin[m] = mn; }
+    if (lane == 0) B.cellcore[m] = ncore;
   }
   flush_tally(t, B.ctr);
   if (lane == 0 && dense) atomicAdd(B.ctr + kCtrDenseCells, dense);
@@ -2942,7 +2899,7 @@ __global__ void __launch_bounds__(256) k_core_cells(const gdl::Bufs B, int64_t n
         int q = B.reps[m];
         while (!B.core[q]) ++q;
         B.cellrep[m] = q;
-        B.compmin[m] = B.cellmin[m];
+        B.compmin[m] = (int)B.ids[q];  // the sort is stable: its smallest core index
         const uint32_t e = B.cellent[m];
         fresh = atomicOr(&B.ent[e].core, 1ull << ((unsigned)ckey_at<KEY64>(B, m) & 63u)) == 0;
         if (fresh) B.links[e] = BlockLinks{};
@@ -3308,7 +3265,7 @@ __global__ void k_comp_min(const gdl::Bufs B) {
     const bool sub = on && r != (int)m;
     const unsigned grp = run_peers(__ballot_sync(kFull, sub), r);
     if (sub) {
-      const int mn = (int)__reduce_min_sync(grp, (unsigned)B.cellmin[m]);
+      const int mn = (int)__reduce_min_sync(grp, (unsigned)B.compmin[m]);
       if (lane == __ffs(grp) - 1 && mn < *reinterpret_cast<volatile int*>(B.compmin + r))
         atomicMin(B.compmin + r, mn);
     }
@@ -3650,9 +3607,7 @@ static int per_dim(int dims) { return ((dims & 1) ? 1 : 0) + ((dims & 2) ? 1 : 0
 int core(const Bufs& B, int64_t n, int dims, bool f32, bool key64, bool one, bool fresh, int sms,
          void* scan_temp, cudaStream_t s) {
   cudaMemsetAsync(B.ctr + kCtrHeavyCore, 0, 8, s);
-  // per-cell core counts (0) and smallest core indices (0xffffffff as unsigned)
-  cudaMemsetAsync(B.cellcore, 0, (size_t)n * 4, s);
-  cudaMemsetAsync(B.cellmin, 0xff, (size_t)n * 4, s);
+  cudaMemsetAsync(B.cellcore, 0, (size_t)n * 4, s);  // per-cell core counts
   // dense cells at once; the other points listed in sorted order for the walk
   const int g = grid_for(n, 256, sms, 8);
   const int chunk = f32 ? kCoreChunk : 1;
