@@ -16,6 +16,7 @@
 #include <cstddef>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <string>
 #include <vector>
 
@@ -54,6 +55,10 @@ gd_status cuda_fail(cudaError_t e, const char* what) {
 struct DevBuf {
   void* p = nullptr;
   size_t bytes = 0;
+};
+struct Want {
+  DevBuf* b;
+  size_t bytes;
 };
 
 constexpr double kDefaultCellMult = 0.5 * (1.0 + 1.0 / 65536.0);
@@ -148,28 +153,75 @@ struct gd_ctx {
     return GD_OK;
   }
 
-  // ensure() for temp memory that must be zero when first used (the scan
-  // state): cleared on the stream whenever it is (re)allocated
-  gd_status ensure_zeroed(DevBuf& b, size_t bytes, const char* what) {
-    void* before = b.p;
-    const size_t had = b.bytes;
-    GD_TRY(ensure(b, bytes, what));
-    if (b.p != before || b.bytes != had) GD_CUDA(cudaMemsetAsync(b.p, 0, b.bytes, stream), what);
+  // The buffers of a run and, apart from them, those of its tables (needed before the
+  // run's sizes are known): each set is one allocation, cut into its buffers.  A
+  // buffer that has to grow moves the whole set (nothing in it outlives an index build),
+  // every buffer keeping at least the size it had.  cudaMalloc and cudaFree take 30 us
+  // each and more by their number than by their size (1 GB: in 32 buffers 1065 and
+  // 1408 us, in one 122 and 415 us): the first run of a context on 10M 2D points took
+  // 2541 us with an allocation per buffer and takes 2098 (2M 3D points: 2496, 1952).
+  static constexpr int kRunBufs = 30, kTableBufs = 5;
+  DevBuf* const run_set[kRunBufs] = {
+      &keys0, &keys1, &vals0,  &vals1,    &X,       &Xf,      &ent,      &links,    &pop,
+      &cellent, &blklist, &nbr, &rowtab,  &hkeys,   &hvals,   &reps,     &bits,     &core,
+      &cellcore, &cellmin, &cellrep, &parent, &cellcid, &lab, &asym,     &asymwork, &hvcell,
+      &hvmask, &sorttemp, &scantemp};
+  DevBuf* const table_set[kTableBufs] = {&inst, &chunks, &Pv, &Bi, &bbox};
+  void* run_slab = nullptr;
+  void* table_slab = nullptr;
+
+  static void drop_set(void*& slab, DevBuf* const* set, int k) {
+    if (slab) cudaFree(slab);
+    slab = nullptr;
+    for (int i = 0; i < k; ++i) *set[i] = DevBuf{};
+  }
+
+  gd_status ensure_set(void*& slab, DevBuf* const* set, int k, std::initializer_list<Want> wants,
+                       const char* what) {
+    bool grow = false;
+    for (const Want& w : wants) grow |= w.b->bytes < up256(w.bytes);
+    if (!grow) return GD_OK;
+    size_t size[kRunBufs], total = 0;
+    for (int i = 0; i < k; ++i) {
+      size[i] = set[i]->bytes;
+      for (const Want& w : wants)
+        if (w.b == set[i]) size[i] = std::max(size[i], up256(w.bytes));
+      total += size[i];
+    }
+    drop_set(slab, set, k);
+    const cudaError_t e = cudaMalloc(&slab, total);
+    if (e != cudaSuccess) {
+      slab = nullptr;
+      return cuda_fail(e, what);
+    }
+    char* at = static_cast<char*>(slab);
+    for (int i = 0; i < k; ++i) {
+      if (!size[i]) continue;
+      set[i]->p = at;
+      set[i]->bytes = size[i];
+      at += size[i];
+    }
+    // the scans' state is zero when first used
+    if (set == run_set && scantemp.p)
+      GD_CUDA(cudaMemsetAsync(scantemp.p, 0, scantemp.bytes, stream), what);
     return GD_OK;
+  }
+  gd_status ensure_run(std::initializer_list<Want> w) {
+    return ensure_set(run_slab, run_set, kRunBufs, w, "run buffers");
+  }
+  gd_status ensure_tables(std::initializer_list<Want> w) {
+    return ensure_set(table_slab, table_set, kTableBufs, w, "run tables");
   }
 
   void free_all(bool keep_small) {
-    DevBuf* a[] = {&coords, &inst,   &chunks,   &Pv,      &Bi,     &bbox,     &keys0,
-                   &keys1,  &vals0,  &vals1,    &X,       &Xf,     &ent,      &links, &pop, &cellent, &blklist, &nbr, &rowtab, &hkeys,
-                   &hvals,  &reps,   &bits,     &core,    &cellcore, &cellmin, &cellrep,
-                   &parent, &cellcid,  &lab,     &asym,   &hvcell,   &hvmask,
-                   &out,    &coreout, &sorttemp, &scantemp, &small, &kcount, &asymwork};
+    DevBuf* a[] = {&coords, &out, &coreout, &kcount, &small};
     for (DevBuf* b : a) {
       if (keep_small && b == &small) continue;
       if (b->p) cudaFree(b->p);
-      b->p = nullptr;
-      b->bytes = 0;
+      *b = DevBuf{};
     }
+    drop_set(run_slab, run_set, kRunBufs);
+    drop_set(table_slab, table_set, kTableBufs);
   }
 
   // small block (kSmallBlock bytes): M | total clusters | counters | (small runs:) run
@@ -290,30 +342,32 @@ gd_status build_small(gd_ctx* ctx) {
   ctx->n = n;
   const uint64_t dmax = gd::small_direct_max(n);
   const uint32_t slots = gd::small_hash_slots(n);
-  GD_TRY(ctx->ensure(ctx->Pv, sizeof(gd::DevParams), "instance parameters"));
-  GD_TRY(ctx->ensure(ctx->keys0, n * 8, "point keys"));
-  GD_TRY(ctx->ensure(ctx->keys1, n * 8, "cell keys"));
-  GD_TRY(ctx->ensure(ctx->vals0, n * 4, "point cells"));
-  GD_TRY(ctx->ensure(ctx->vals1, n * 4, "ids"));
-  GD_TRY(ctx->ensure(ctx->bbox, (size_t)ctx->sms * 64, "bounds"));
-  GD_TRY(ctx->ensure(ctx->X, (size_t)n * I.dim * 8, "sorted coordinates"));
-  GD_TRY(ctx->ensure(ctx->Xf, (size_t)n * (I.dim == 3 ? 16 : 8), "f32 coordinates"));
-  GD_TRY(ctx->ensure(ctx->ent, std::max<uint64_t>(dmax, slots) * sizeof(gd::BlockEnt), "block entries"));
-  GD_TRY(ctx->ensure(ctx->hkeys, (uint64_t)slots * 8, "block hash"));
-  GD_TRY(ctx->ensure(ctx->cellent, n * 4, "point places"));
-  GD_TRY(ctx->ensure(ctx->blklist, n * 4, "position cells"));
-  GD_TRY(ctx->ensure(ctx->hvmask, n * 8, "cell ranges"));
-  GD_TRY(ctx->ensure(ctx->hvcell, n * 4, "walk list"));
-  GD_TRY(ctx->ensure(ctx->bits, gdl::bit_layout(n).words * 4, "bit masks"));
-  GD_TRY(ctx->ensure(ctx->core, n, "core flags"));
-  GD_TRY(ctx->ensure(ctx->cellcore, n * 4, "cell core counts"));
-  GD_TRY(ctx->ensure(ctx->cellmin, n * 4, "cell min index"));
-  GD_TRY(ctx->ensure(ctx->cellrep, n * 4, "cell representatives"));
-  GD_TRY(ctx->ensure(ctx->parent, n * 4, "union-find parents"));
-  GD_TRY(ctx->ensure(ctx->cellcid, n * 4, "cell cluster ids"));
-  GD_TRY(ctx->ensure(ctx->lab, n * 4, "labels"));
-  GD_TRY(ctx->ensure(ctx->asym, gd::kAsymCap * 8, "one-directional links"));
-  GD_TRY(ctx->ensure(ctx->asymwork, sizeof(gd::AsymWork), "merge replay"));
+  const size_t N = (size_t)n;
+  GD_TRY(ctx->ensure_tables({{&ctx->Pv, sizeof(gd::DevParams)}, {&ctx->bbox, (size_t)ctx->sms * 64}}));
+  GD_TRY(ctx->ensure_run({
+      {&ctx->keys0, N * 8},     // point keys
+      {&ctx->keys1, N * 8},     // cell keys
+      {&ctx->vals0, N * 4},     // point cells
+      {&ctx->vals1, N * 4},     // ids
+      {&ctx->X, N * I.dim * 8},
+      {&ctx->Xf, N * (I.dim == 3 ? 16 : 8)},
+      {&ctx->ent, std::max<uint64_t>(dmax, slots) * sizeof(gd::BlockEnt)},
+      {&ctx->hkeys, (uint64_t)slots * 8},
+      {&ctx->cellent, N * 4},   // point places
+      {&ctx->blklist, N * 4},   // position cells
+      {&ctx->hvmask, N * 8},    // cell ranges
+      {&ctx->hvcell, N * 4},    // walk list
+      {&ctx->bits, gdl::bit_layout(n).words * 4},
+      {&ctx->core, N},
+      {&ctx->cellcore, N * 4},
+      {&ctx->cellmin, N * 4},
+      {&ctx->cellrep, N * 4},
+      {&ctx->parent, N * 4},
+      {&ctx->cellcid, N * 4},
+      {&ctx->lab, N * 4},
+      {&ctx->asym, gd::kAsymCap * 8},
+      {&ctx->asymwork, sizeof(gd::AsymWork)},
+  }));
   ctx->is_small = true;
   ctx->x64 = true;
   char* sm = static_cast<char*>(ctx->small.p);
@@ -374,11 +428,11 @@ gd_status build_run(gd_ctx* ctx, uint64_t dense_floor, uint64_t rows_floor) {
   ctx->n = n;
   make_chunks(ctx->hdesc, ctx->hchunk);
   const int nch = (int)ctx->hchunk.size();
-  GD_TRY(ctx->ensure(ctx->inst, K * sizeof(gd::InstDesc), "instance table"));
-  GD_TRY(ctx->ensure(ctx->chunks, std::max(1, nch) * sizeof(gd::Chunk), "chunk table"));
-  GD_TRY(ctx->ensure(ctx->Pv, K * sizeof(gd::DevParams), "instance parameters"));
-  GD_TRY(ctx->ensure(ctx->Bi, sizeof(gd::BatchInfo), "run layout"));
-  GD_TRY(ctx->ensure(ctx->bbox, K * 6 * 8, "bounding boxes"));
+  GD_TRY(ctx->ensure_tables({{&ctx->inst, K * sizeof(gd::InstDesc)},
+                             {&ctx->chunks, std::max(1, nch) * sizeof(gd::Chunk)},
+                             {&ctx->Pv, K * sizeof(gd::DevParams)},
+                             {&ctx->Bi, sizeof(gd::BatchInfo)},
+                             {&ctx->bbox, (size_t)K * 6 * 8}}));
   GD_CUDA(cudaMemcpyAsync(ctx->inst.p, ctx->hdesc.data(), K * sizeof(gd::InstDesc),
                           cudaMemcpyHostToDevice, s), "upload instances");
   if (nch)
@@ -404,40 +458,45 @@ gd_status build_run(gd_ctx* ctx, uint64_t dense_floor, uint64_t rows_floor) {
   ctx->dims = (bi.K2 > 0 ? 1 : 0) | (bi.K2 < K ? 2 : 0);
   const size_t kw = ctx->key64 ? 8 : 4;
   const int maxd = bi.max_dim;
-  GD_TRY(ctx->ensure(ctx->keys0, n * kw, "keys"));
-  GD_TRY(ctx->ensure(ctx->keys1, n * kw, "keys"));
-  GD_TRY(ctx->ensure(ctx->vals0, n * 4, "ids"));
-  GD_TRY(ctx->ensure(ctx->vals1, n * 4, "ids"));
   ctx->x64 = !ctx->f32 || bi.band_off;
-  if (ctx->x64) GD_TRY(ctx->ensure(ctx->X, (size_t)n * maxd * 8, "sorted coordinates"));
-  if (ctx->xf) GD_TRY(ctx->ensure(ctx->Xf, (size_t)n * (maxd == 3 ? 16 : 8), "f32 coordinates"));
   // block entries: direct tables, then one slot per cell if some instance has none
   const bool direct_only = bi.row_total == 0 && !bi.any_sparse;
-  GD_TRY(ctx->ensure(ctx->ent, (bi.ent_total + (direct_only ? 0 : (uint64_t)n)) * sizeof(gd::BlockEnt),
-                     "block entries"));
-  GD_TRY(ctx->ensure(ctx->links,
-                     (bi.ent_total + (direct_only ? 0 : (uint64_t)n)) * sizeof(gd::BlockLinks),
-                     "block links"));
-  if (ctx->f32)
-    GD_TRY(ctx->ensure(ctx->pop, (bi.ent_total + (direct_only ? 0 : (uint64_t)n)) * sizeof(gd::BlockPop),
-                       "block populations"));
-  GD_TRY(ctx->ensure(ctx->cellent, n * 4, "cell entries"));
-  GD_TRY(ctx->ensure(ctx->blklist, n * 4, "block list"));
-  if (!direct_only) GD_TRY(ctx->ensure(ctx->nbr, n * 4 * sizeof(uint2), "neighbour entries"));
-  GD_TRY(ctx->ensure(ctx->rowtab, bi.row_total * 8, "row tables"));
+  const size_t N = (size_t)n, nent = bi.ent_total + (direct_only ? 0 : N);
   uint64_t hcap = 1024;
-  if (bi.any_sparse) {
-    while (hcap < 2 * (uint64_t)n) hcap <<= 1;
-    GD_TRY(ctx->ensure(ctx->hkeys, hcap * 8, "row hash keys"));
-    GD_TRY(ctx->ensure(ctx->hvals, hcap * 8, "row hash values"));
-  }
+  while (bi.any_sparse && hcap < 2 * (uint64_t)n) hcap <<= 1;
   ctx->hmask = (uint32_t)(hcap - 1);
-  GD_TRY(ctx->ensure(ctx->reps, (n + 1) * 4, "cell reps"));
-  GD_TRY(ctx->ensure(ctx->bits, gdl::bit_layout(n).words * 4, "bit masks"));
-  GD_TRY(ctx->ensure(ctx->sorttemp, gdprim::sort_temp_bytes(n), "sort temp"));
-  const size_t sc = std::max(gdprim::scan_temp_bytes(n + 1),
-                             gdprim::scan_temp_bytes(gdprim::sort_scan_elems(n)));
-  GD_TRY(ctx->ensure_zeroed(ctx->scantemp, sc, "scan temp"));
+  GD_TRY(ctx->ensure_run({
+      {&ctx->keys0, N * kw},
+      {&ctx->keys1, N * kw},
+      {&ctx->vals0, N * 4},
+      {&ctx->vals1, N * 4},
+      {&ctx->X, ctx->x64 ? N * maxd * 8 : 0},
+      {&ctx->Xf, ctx->xf ? N * (maxd == 3 ? 16 : 8) : 0},
+      {&ctx->ent, nent * sizeof(gd::BlockEnt)},
+      {&ctx->links, nent * sizeof(gd::BlockLinks)},
+      {&ctx->pop, ctx->f32 ? nent * sizeof(gd::BlockPop) : 0},
+      {&ctx->cellent, N * 4},
+      {&ctx->blklist, N * 4},
+      {&ctx->nbr, direct_only ? 0 : N * 4 * sizeof(uint2)},
+      {&ctx->rowtab, std::max<uint64_t>(1, bi.row_total) * 8},
+      {&ctx->hkeys, bi.any_sparse ? hcap * 8 : 0},
+      {&ctx->hvals, bi.any_sparse ? hcap * 8 : 0},
+      {&ctx->reps, (N + 1) * 4},
+      {&ctx->bits, gdl::bit_layout(n).words * 4},
+      {&ctx->sorttemp, gdprim::sort_temp_bytes(n)},
+      {&ctx->scantemp, std::max(gdprim::scan_temp_bytes(n + 1),
+                                gdprim::scan_temp_bytes(gdprim::sort_scan_elems(n)))},
+      // the expand stage's
+      {&ctx->core, N},
+      {&ctx->cellcore, N * 4},
+      {&ctx->cellrep, N * 4},
+      {&ctx->parent, N * 4},
+      {&ctx->cellcid, N * 4},
+      {&ctx->lab, N * 4},
+      {&ctx->asym, gd::kAsymCap * 8},
+      {&ctx->hvcell, N * 4},  // heavy work
+      {&ctx->hvmask, N * 8},
+  }));
   const int key_bits = bi.LB + bi.IB;
   int r;
   uint32_t* vb[2] = {static_cast<uint32_t*>(ctx->vals0.p), static_cast<uint32_t*>(ctx->vals1.p)};
@@ -506,7 +565,6 @@ cudaError_t launch_expand(gd_ctx* ctx, bool capturing) {
 
 gd_status expand_run(gd_ctx* ctx) {
   cudaStream_t s = ctx->stream;
-  const int64_t n = ctx->n;
   if (ctx->is_small) {
     if (!ctx->fresh_index)
       GD_CUDA(cudaMemsetAsync(ctx->dCtr() + gd::kCtrTests64, 0,
@@ -520,18 +578,6 @@ gd_status expand_run(gd_ctx* ctx) {
     ctx->stage = 2;
     return GD_OK;
   }
-  GD_TRY(ctx->ensure(ctx->core, n, "core flags"));
-  GD_TRY(ctx->ensure(ctx->cellcore, n * 4, "cell core counts"));
-  GD_TRY(ctx->ensure(ctx->cellrep, n * 4, "cell representatives"));
-  GD_TRY(ctx->ensure(ctx->parent, n * 4, "union-find parents"));
-  GD_TRY(ctx->ensure(ctx->cellcid, n * 4, "cell cluster ids"));
-  GD_TRY(ctx->ensure(ctx->lab, n * 4, "labels"));
-  GD_TRY(ctx->ensure(ctx->asym, gd::kAsymCap * 8, "one-directional links"));
-  GD_TRY(ctx->ensure(ctx->hvcell, n * 4, "heavy-work list"));
-  GD_TRY(ctx->ensure(ctx->hvmask, n * 8, "heavy-work masks"));
-  GD_TRY(ctx->ensure_zeroed(ctx->scantemp,
-                            std::max(gdprim::scan_temp_bytes(n + 1), ctx->scantemp.bytes),
-                            "scan temp"));
   ctx->stage = 2;
   if (ctx->graphs && ctx->xgraph) {
     GD_CUDA(cudaGraphLaunch(ctx->xgraph, s), "expand graph launch");
