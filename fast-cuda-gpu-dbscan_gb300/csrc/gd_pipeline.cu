@@ -514,44 +514,37 @@ __device__ __forceinline__ int cell_index_f64(double x, double lo, double inv_f)
   return __double2int_rd(__dmul_rn(__dsub_rn(x, lo), inv_f));
 }
 
-// Cell along one axis: kfast, lo32, inv32 and band as in DevParams::key_*.
+// Cell along one axis: kfast, lo32, inv32 and band as in DevParams::key_*; G1: the
+// axis' last cell.
 __device__ __forceinline__ int cell_of_coord(double x, bool kfast, double lo, double inv_f,
-                                             float lo32, float inv32, float band, int64_t G) {
+                                             float lo32, float inv32, float band, int G1) {
   // 32-bit cell index: conversions to 64-bit integers run on this GPU's
   // narrow float64 pipe; every cell index is below 2^31 (grids are checked)
   int q;
   bool fast = false;
   if (kfast) {
     // float32 cell position (no float64 instruction), used when it is
-    // farther than key_band from a cell boundary
+    // farther than key_band from a cell boundary.  key_fast means |x| < 2^100 and
+    // positions in [-1, 2^21 + 1].
     const unsigned long long bits = (unsigned long long)__double_as_longlong(x);
-    const int fe = (int)((bits >> 52) & 0x7ff) - 1023 + 127;
-    const bool zero = (bits << 1) == 0;
-    if (zero || (fe > 0 && fe < 255)) {
-      const unsigned sgn = (unsigned)(bits >> 63) << 31;
-      const float x32 = zero ? 0.0f
-                             : __uint_as_float(sgn | ((unsigned)fe << 23) |
-                                               (unsigned)((bits >> 29) & 0x7fffffu));
-      const float t = __fmul_rn(__fsub_rn(x32, lo32), inv32);
-      if (fabsf(t) < 4194304.0f) {
-        // floor without a conversion instruction: for |t| < 2^22,
-        // t + 1.5 * 2^23 rounded down lies in [2^23, 2^24), where floats are
-        // the integers, so it is floor(t) + 1.5 * 2^23 exactly and its
-        // mantissa bits hold floor(t) + 2^22
-        const float s = __fadd_rd(t, 12582912.0f);
-        const float fl = __fsub_rn(s, 12582912.0f);
-        const float fr = __fsub_rn(t, fl);
-        if (fr > band && fr < 1.0f - band) {
-          q = (int)(__float_as_uint(s) - 0x4b400000u);
-          fast = true;
-        }
-      }
-    }
+    const unsigned hw = (unsigned)(bits >> 32);
+    // sign, the exponent's low 8 bits with the bias moved by 896 (a flip of the
+    // highest), 23 mantissa bits; below 2^-126: 0, off by less than 2^-26 cells
+    const unsigned m = (__funnelshift_l((unsigned)bits, hw, 3) ^ 0x40000000u) & 0x7fffffffu;
+    const float x32 = __uint_as_float((hw & 0x80000000u) | ((hw & 0x7fffffffu) < 0x38100000u ? 0u : m));
+    const float t = __fmul_rn(__fsub_rn(x32, lo32), inv32);
+    // floor without a conversion instruction: for |t| < 2^22,
+    // t + 1.5 * 2^23 rounded down lies in [2^23, 2^24), where floats are
+    // the integers, so it is floor(t) + 1.5 * 2^23 exactly and its
+    // mantissa bits hold floor(t) + 2^22
+    const float s = __fadd_rd(t, 12582912.0f);
+    const float fr = __fsub_rn(t, __fsub_rn(s, 12582912.0f));
+    q = (int)(__float_as_uint(s) - 0x4b400000u);
+    fast = fr > band && fr < 1.0f - band;
   }
   // the float64 formula for the few coordinates near a cell boundary
   if (!fast) q = cell_index_f64(x, lo, inv_f);
-  q = q < 0 ? 0 : ((int64_t)q >= G ? (int)(G - 1) : q);
-  return q;
+  return min(max(q, 0), G1);
 }
 
 // Local key from the cells along each axis.
@@ -564,34 +557,41 @@ __device__ __forceinline__ uint64_t key_of_cell(int D, const int* c, int B1, int
 }
 
 // One block per chunk: cell key of every point, instance id above the local key.
+// Memory bound if the instructions per coordinate stay few (10M 2D / 20M 3D points: 42
+// and 91 us, floors 30 and 83; with the range checks and the select over a run-time
+// dimension that the host's key_fast conditions make needless, 71 and 140 us).
 template <class Key>
 __global__ void __launch_bounds__(256) k_keys(const gdl::Bufs B, Key* __restrict__ keys) {
   const Chunk c = B.chunks[blockIdx.x];
   const DevParams& P = B.Pv[c.inst];
-  const int D = P.dim;
-  double lo[3], inv_f = P.inv_f;
-  int64_t G[3];
-  for (int k = 0; k < 3; ++k) { lo[k] = P.lo[k]; G[k] = P.G[k]; }
+  const double inv_f = P.inv_f;
+  double lo[3];
+  int G1[3];
+  float lo32[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    lo[k] = P.lo[k];
+    G1[k] = (int)(P.G[k] - 1);
+    lo32[k] = P.key_lo32[k];
+  }
   const uint64_t hi = inst_key(P.inst, P.LB);
   const int B1 = P.Bk[1], B2 = P.Bk[2];
   const bool kfast = P.key_fast != 0;
   const float band = P.key_band, inv32 = P.key_inv32;
-  float lo32[3];
-  for (int k = 0; k < 3; ++k) lo32[k] = P.key_lo32[k];
   const double* __restrict__ pts = B.coords + P.co_off;
   Key* __restrict__ out = keys + P.pt_off;
-  auto key_of = [&](int64_t l, const double* xs) {
-    int c[3] = {0, 0, 0};
+  auto points = [&](auto dim) {
+    constexpr int D = decltype(dim)::value;
+    for_points<D>(pts, c.begin - P.pt_off, c.end - P.pt_off, [&](int64_t l, const double* xs) {
+      int q[3] = {0, 0, 0};
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      if (k >= D) break;
-      const double x = xs[k];
-      c[k] = cell_of_coord(x, kfast, lo[k], inv_f, lo32[k], inv32, band, G[k]);
-    }
-    out[l] = (Key)(hi + key_of_cell(D, c, B1, B2));
+      for (int k = 0; k < D; ++k)
+        q[k] = cell_of_coord(xs[k], kfast, lo[k], inv_f, lo32[k], inv32, band, G1[k]);
+      out[l] = (Key)(hi + key_of_cell(D, q, B1, B2));
+    });
   };
-  if (D == 2) for_points<2>(pts, c.begin - P.pt_off, c.end - P.pt_off, key_of);
-  else for_points<3>(pts, c.begin - P.pt_off, c.end - P.pt_off, key_of);
+  if (P.dim == 2) points(std::integral_constant<int, 2>{});
+  else points(std::integral_constant<int, 3>{});
 }
 
 // Coordinates of one point in 16-byte loads where the address allows (a 2D

@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_small_index(const gdl::Bufs B
 #pragma unroll
     for (int k = 0; k < D; ++k)
       c[k] = cell_of_coord(A.coords[(int64_t)l * D + k], P.key_fast != 0, P.lo[k], P.inv_f,
-                           P.key_lo32[k], P.key_inv32, P.key_band, P.G[k]);
+                           P.key_lo32[k], P.key_inv32, P.key_band, (int)(P.G[k] - 1));
     const uint64_t key = key_of_cell(D, c, P.Bk[1], P.Bk[2]);
     const uint64_t blk = key >> kBlockBits;
     uint32_t e = (uint32_t)blk;
