@@ -98,17 +98,31 @@ k_scan_onepass(const uint32_t* in, uint32_t* out, int64_t n, unsigned tiles, Loo
 // ---------------------------------------------------------------- radix sort
 constexpr int kRsThreads = 256;
 constexpr int kRsWarps = kRsThreads / 32;
+// tiles from which an upsweep block takes four (a chip's worth of blocks stays: 256)
+constexpr int64_t kRsFour = 1024;
 constexpr int kRsMaxBins = 512;  // digits of 8 or 9 bits
 // items per thread: 16 for 32-bit keys (4096-pair tiles), 8 for 64-bit keys
 template <class K>
 constexpr int rs_items() { return sizeof(K) == 4 ? 16 : 8; }
+// Blocks per SM that the downsweep's registers leave room for, and when it loads its
+// values.  32-bit keys: three blocks, the values loaded after the ranking so that they
+// arrive during the tile scan (10M pairs, three passes: 193 us; loaded with the keys 202;
+// four blocks 198).  64-bit keys, half as many items per thread: five blocks, values
+// loaded with the keys (131M pairs, whole index: 16.57 ms; four blocks 16.66, three
+// 17.0, late loads 17.2).
+template <class K>
+constexpr int rs_min_blocks() { return sizeof(K) == 4 ? 3 : 5; }
 constexpr int kRsMinTile = kRsThreads * 8;
 
-template <class K, int ITEMS, int RB>
+// A block counts the digits of G consecutive tiles (G | T), so that a digit's counts,
+// T apart from the next digit's, leave in one store of G (20M keys, three passes: a
+// tile per block 90 us, four 75; 2M keys: 17, but four tiles leave too few blocks, 50).
+template <class K, int ITEMS, int RB, int G>
 __global__ void __launch_bounds__(kRsThreads)
 k_rs_upsweep(const K* __restrict__ keys, int64_t n, int shift, uint32_t* __restrict__ hist,
              int64_t T) {
   constexpr int SEG = 32 * ITEMS, TILE = kRsThreads * ITEMS, BINS = 1 << RB;
+  constexpr int BPT = BINS / kRsThreads;
   constexpr uint32_t MASK = BINS - 1;
   // warp-private digit counts (shared-memory atomics), summed at the end
   __shared__ uint32_t h[kRsWarps][BINS];
@@ -117,34 +131,53 @@ k_rs_upsweep(const K* __restrict__ keys, int64_t n, int shift, uint32_t* __restr
   for (int ww = 0; ww < kRsWarps; ++ww)
     for (int d = threadIdx.x; d < BINS; d += kRsThreads) h[ww][d] = 0;
   __syncthreads();
-  const int64_t seg = (int64_t)blockIdx.x * TILE + w * SEG;
-  // every item's key in flight at once, then the counts
-  uint32_t d[ITEMS];
+  uint32_t tot[BPT][G];
 #pragma unroll
-  for (int i = 0; i < ITEMS; ++i) {
-    const int64_t e = seg + i * 32 + lane;
-    d[i] = e < n ? (uint32_t)(__ldg(keys + e) >> shift) & MASK : 0xffffffffu;
+  for (int g = 0; g < G; ++g) {
+    const int64_t seg = ((int64_t)blockIdx.x * G + g) * TILE + w * SEG;
+    // every item's key in flight at once, then the counts
+    uint32_t d[ITEMS];
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+      const int64_t e = seg + i * 32 + lane;
+      d[i] = e < n ? (uint32_t)(__ldg(keys + e) >> shift) & MASK : 0xffffffffu;
+    }
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i)
+      if (d[i] != 0xffffffffu) atomicAdd(&h[w][d[i]], 1u);
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < BPT; ++q) {
+      tot[q][g] = 0;
+#pragma unroll
+      for (int ww = 0; ww < kRsWarps; ++ww) {
+        uint32_t& c = h[ww][q * kRsThreads + threadIdx.x];
+        tot[q][g] += c;
+        if (g + 1 < G) c = 0;
+      }
+    }
+    if (g + 1 < G) __syncthreads();
   }
 #pragma unroll
-  for (int i = 0; i < ITEMS; ++i)
-    if (d[i] != 0xffffffffu) atomicAdd(&h[w][d[i]], 1u);
-  __syncthreads();
-  for (int d = threadIdx.x; d < BINS; d += kRsThreads) {
-    uint32_t tot = 0;
+  for (int q = 0; q < BPT; ++q) {
+    uint32_t* out = hist + (int64_t)(q * kRsThreads + threadIdx.x) * T + (int64_t)blockIdx.x * G;
+    if constexpr (G == 4)
+      *reinterpret_cast<uint4*>(out) = make_uint4(tot[q][0], tot[q][1], tot[q][2], tot[q][3]);
+    else
 #pragma unroll
-    for (int ww = 0; ww < kRsWarps; ++ww) tot += h[ww][d];
-    hist[(int64_t)d * T + blockIdx.x] = tot;
+      for (int g = 0; g < G; ++g) out[g] = tot[q][g];
   }
 }
 
 template <class K, int ITEMS, int RB>
-__global__ void __launch_bounds__(kRsThreads)
+__global__ void __launch_bounds__(kRsThreads, rs_min_blocks<K>())
 k_rs_downsweep(const K* __restrict__ kin, const uint32_t* __restrict__ vin,
                K* __restrict__ kout, uint32_t* __restrict__ vout, int64_t n,
                int shift, const uint32_t* __restrict__ goff, int64_t T) {
   constexpr int SEG = 32 * ITEMS, TILE = kRsThreads * ITEMS, BINS = 1 << RB;
   constexpr int BPT = BINS / kRsThreads;  // digits per thread in the tile scan
   constexpr uint32_t MASK = BINS - 1;
+  constexpr bool LATE = sizeof(K) == 4;
   static_assert(TILE <= 65535, "per-warp digit offsets are 16-bit");
   __shared__ K s_keys[TILE];
   __shared__ uint32_t s_vals[TILE];
@@ -164,13 +197,8 @@ k_rs_downsweep(const K* __restrict__ kin, const uint32_t* __restrict__ vin,
 #pragma unroll
   for (int i = 0; i < ITEMS; ++i) {
     int64_t e = seg + i * 32 + lane;
-    if (e < n) {
-      k[i] = __ldg(kin + e);
-      v[i] = vin ? __ldg(vin + e) : (uint32_t)e;
-    } else {
-      k[i] = ~(K)0;
-      v[i] = 0;
-    }
+    k[i] = e < n ? __ldg(kin + e) : ~(K)0;
+    if (!LATE) v[i] = vin && e < n ? __ldg(vin + e) : (uint32_t)e;
   }
 #pragma unroll
   for (int i = 0; i < ITEMS; ++i) {
@@ -188,6 +216,12 @@ k_rs_downsweep(const K* __restrict__ kin, const uint32_t* __restrict__ vin,
     if (lane == __ffs(peers) - 1) s_cnt[w][d] = (uint16_t)(b + (uint32_t)__popc(peers));
     __syncwarp();
     r[i] = b + (uint32_t)__popc(peers & lt_mask);
+  }
+  if constexpr (LATE)  // the values, on their way during the tile scan
+#pragma unroll
+  for (int i = 0; i < ITEMS; ++i) {
+    const int64_t e = seg + i * 32 + lane;
+    v[i] = vin && e < n ? __ldg(vin + e) : (uint32_t)e;
   }
   __syncthreads();
   {
@@ -345,7 +379,7 @@ void list_bits(const uint32_t* words, uint32_t* pre, int64_t nw, uint32_t* out, 
 // buffer, a larger sort's status words would lie where a smaller sort left its
 // histogram, and a count that looks like a tagged word would pass for a prefix.
 int64_t sort_scan_elems(int64_t n) {
-  return (n + kRsMinTile - 1) / kRsMinTile * kRsMaxBins;
+  return ((n + kRsMinTile - 1) / kRsMinTile + 3) / 4 * 4 * kRsMaxBins;
 }
 
 size_t sort_temp_bytes(int64_t n) {
@@ -357,16 +391,24 @@ int sort_passes(K* keys[2], uint32_t* vals[2], int64_t n, int passes, bool vals_
                 void* temp, void* scan_temp, cudaStream_t s, unsigned long long* timeouts) {
   constexpr int ITEMS = rs_items<K>();
   constexpr int TILE = kRsThreads * ITEMS;
-  const int64_t T = (n + TILE - 1) / TILE;
+  // four tiles per upsweep block where that leaves enough blocks; the histogram is then
+  // for a multiple of four tiles, the last ones perhaps empty
+  int64_t T = (n + TILE - 1) / TILE;
+  const bool four = T >= kRsFour;
+  const int64_t tiles = T;
+  if (four) T = (T + 3) & ~(int64_t)3;
   const int64_t h = T << RB;
   uint32_t* hist = static_cast<uint32_t*>(temp);
   int cur = 0;
   for (int p = 0; p < passes; ++p) {
     int shift = RB * p;
-    k_rs_upsweep<K, ITEMS, RB><<<(unsigned)T, kRsThreads, 0, s>>>(keys[cur], n, shift, hist, T);
+    if (four)
+      k_rs_upsweep<K, ITEMS, RB, 4><<<(unsigned)(T / 4), kRsThreads, 0, s>>>(keys[cur], n, shift, hist, T);
+    else
+      k_rs_upsweep<K, ITEMS, RB, 1><<<(unsigned)T, kRsThreads, 0, s>>>(keys[cur], n, shift, hist, T);
     exclusive_scan_u32(hist, hist, h, scan_temp, nullptr, s, timeouts);
     const uint32_t* vin = (p == 0 && vals_in_is_iota) ? nullptr : vals[cur];
-    k_rs_downsweep<K, ITEMS, RB><<<(unsigned)T, kRsThreads, 0, s>>>(
+    k_rs_downsweep<K, ITEMS, RB><<<(unsigned)tiles, kRsThreads, 0, s>>>(
         keys[cur], vin, keys[cur ^ 1], vals[cur ^ 1], n, shift, hist, T);
     cur ^= 1;
   }
