@@ -7,7 +7,7 @@
 // device; plug-ins that run inside a host process whose memory manager owns
 // the GPU's memory may not allocate behind its back.  They pass device
 // pointers for the points and the labels; every other buffer of the pipeline
-// lives in one file-scope __device__ array (kScratchBytes, about 5 MiB) that
+// lives in one file-scope __device__ array (kScratchBytes, about 8.7 MiB) that
 // the module holds on every GPU that loads this library until the process
 // exits.
 //

@@ -259,13 +259,14 @@ gd_status gd_server_get_stats(gd_server* srv, gd_server_stats* stats);
    is rejected with GD_ERANGE.  coords_dev (n x dim float64) and labels_dev
    (n int32) are device pointers on the current device; stream may be NULL
    (default stream).  All scratch is one fixed static device array of about
-   5 MiB that every GPU which loads the library keeps until the process exits;
+   8.7 MiB that every GPU which loads the library keeps until the process exits;
    nothing is allocated or freed.  The first call in a CUDA context of a device
    does a one-time set-up (it looks up that array's device address); make that
    first call before any stream capture begins.  The call synchronises its
    stream once, at the end; where the grid needs the general pipeline (more than
-   16384 points spread too far for a direct block table) three times.  Calls share the array and it keeps the last call's contents;
-   calls that overlap on the GPU race and must be serialised by the caller.
+   16384 points spread too far for a direct block table) three times.  Calls
+   share the array and it keeps the last call's contents; calls that overlap on
+   the GPU race and must be serialised by the caller.
    labels_dev is undefined when the call fails.  n_clusters may be NULL. */
 #define GD_NOALLOC_MAX_POINTS 32768
 gd_status gd_dbscan_noalloc(const double* coords_dev, int64_t n, int32_t dim, double eps,
