@@ -320,11 +320,12 @@ gd_status grid_too_large() {
 // Point runs of at most kChunkPoints points, one instance each.
 void make_chunks(const std::vector<gd::InstDesc>& desc, std::vector<gd::Chunk>& out) {
   out.clear();
-  for (size_t i = 0; i < desc.size(); ++i)
+  int64_t before = 0;  // points of the instances before
+  for (size_t i = 0; i < desc.size(); before += desc[i].n, ++i)
     for (int64_t b = 0; b < desc[i].n; b += gd::kChunkPoints) {
       gd::Chunk c;
       c.inst = (int32_t)i;
-      c.pad = 0;
+      c.sorted = (int32_t)(before + b);
       c.begin = desc[i].pt_off + b;
       c.end = desc[i].pt_off + std::min<int64_t>(desc[i].n, b + gd::kChunkPoints);
       out.push_back(c);
@@ -461,6 +462,9 @@ gd_status build_run(gd_ctx* ctx, uint64_t dense_floor, uint64_t rows_floor) {
   ctx->x64 = !ctx->f32 || bi.band_off;
   // block entries: direct tables, then one slot per cell if some instance has none
   const bool direct_only = bi.row_total == 0 && !bi.any_sparse;
+  const int key_bits = bi.LB + bi.IB;
+  gdprim::SortChunks sc;
+  if (K > 1 && gdprim::sort_by_instance(n, nch, bi.LB, key_bits)) sc.count = nch;
   const size_t N = (size_t)n, nent = bi.ent_total + (direct_only ? 0 : N);
   uint64_t hcap = 1024;
   while (bi.any_sparse && hcap < 2 * (uint64_t)n) hcap <<= 1;
@@ -483,9 +487,9 @@ gd_status build_run(gd_ctx* ctx, uint64_t dense_floor, uint64_t rows_floor) {
       {&ctx->hvals, bi.any_sparse ? hcap * 8 : 0},
       {&ctx->reps, (N + 1) * 4},
       {&ctx->bits, gdl::bit_layout(n).words * 4},
-      {&ctx->sorttemp, gdprim::sort_temp_bytes(n)},
+      {&ctx->sorttemp, gdprim::sort_temp_bytes(n, sc.count)},
       {&ctx->scantemp, std::max(gdprim::scan_temp_bytes(n + 1),
-                                gdprim::scan_temp_bytes(gdprim::sort_scan_elems(n)))},
+                                gdprim::scan_temp_bytes(gdprim::sort_scan_elems(n, sc.count)))},
       // the expand stage's
       {&ctx->core, N},
       {&ctx->cellcore, N * 4},
@@ -497,7 +501,11 @@ gd_status build_run(gd_ctx* ctx, uint64_t dense_floor, uint64_t rows_floor) {
       {&ctx->hvcell, N * 4},  // heavy work
       {&ctx->hvmask, N * 8},
   }));
-  const int key_bits = bi.LB + bi.IB;
+  const int sort_bits = sc.count ? bi.LB : key_bits;
+  if (sc.count) {
+    sc.chunks = static_cast<const gd::Chunk*>(ctx->chunks.p);
+    sc.Pv = static_cast<const gd::DevParams*>(ctx->Pv.p);
+  }
   int r;
   uint32_t* vb[2] = {static_cast<uint32_t*>(ctx->vals0.p), static_cast<uint32_t*>(ctx->vals1.p)};
   B = ctx->bufs();
@@ -505,16 +513,16 @@ gd_status build_run(gd_ctx* ctx, uint64_t dense_floor, uint64_t rows_floor) {
   if (ctx->key64) {
     using U64 = unsigned long long;
     U64* kb[2] = {static_cast<U64*>(ctx->keys0.p), static_cast<U64*>(ctx->keys1.p)};
-    r = gdprim::radix_sort_pairs<U64>(kb, vb, n, key_bits, true, ctx->sorttemp.p,
-                                      ctx->scantemp.p, s, ctx->dCtr() + gd::kCtrWaitTimeouts);
+    r = gdprim::radix_sort_pairs<U64>(kb, vb, n, sort_bits, true, ctx->sorttemp.p,
+                                      ctx->scantemp.p, s, ctx->dCtr() + gd::kCtrWaitTimeouts, sc);
     ctx->skeys = kb[r];
   } else {
     uint32_t* kb[2] = {static_cast<uint32_t*>(ctx->keys0.p), static_cast<uint32_t*>(ctx->keys1.p)};
-    r = gdprim::radix_sort_pairs<uint32_t>(kb, vb, n, key_bits, true, ctx->sorttemp.p,
-                                           ctx->scantemp.p, s, ctx->dCtr() + gd::kCtrWaitTimeouts);
+    r = gdprim::radix_sort_pairs<uint32_t>(kb, vb, n, sort_bits, true, ctx->sorttemp.p,
+                                           ctx->scantemp.p, s, ctx->dCtr() + gd::kCtrWaitTimeouts, sc);
     ctx->skeys = kb[r];
   }
-  L += gdprim::sort_launches(n, key_bits);
+  L += gdprim::sort_launches(n, sort_bits);
   ctx->sids = vb[r];
   B = ctx->bufs();
   L += gdl::gather(B, ctx->key64, n, ctx->xf, K == 1, ctx->sms, s);

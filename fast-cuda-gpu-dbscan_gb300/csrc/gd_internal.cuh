@@ -42,7 +42,7 @@ struct InstDesc {
 // A run of points of one instance (bbox and key kernels take one block each).
 struct Chunk {
   int32_t inst;
-  int32_t pad;
+  int32_t sorted;      // its first position with the instances in their own order
   int64_t begin;       // global point indices [begin, end)
   int64_t end;
 };
@@ -405,17 +405,29 @@ void list_bits(const uint32_t* words, uint32_t* pre, int64_t nw, uint32_t* out, 
                uint32_t* total_dev, cudaStream_t s, unsigned long long* timeouts = nullptr);
 // temp bytes needed by radix_sort_pairs for n elements (either key width), and
 // the elements its scan temp must allow for (scan_temp_bytes of that many)
-size_t sort_temp_bytes(int64_t n);
-int64_t sort_scan_elems(int64_t n);
+// (chunks: as for radix_sort_pairs, 0 without)
+size_t sort_temp_bytes(int64_t n, int chunks = 0);
+int64_t sort_scan_elems(int64_t n, int chunks = 0);
+// The chunks of a run of several instances, for a sort instance by instance.
+struct SortChunks {
+  const gd::Chunk* chunks = nullptr;
+  const gd::DevParams* Pv = nullptr;
+  int count = 0;
+};
+// Whether a run of n points in `chunks` chunks, with keys of `local` bits below the
+// instance id's, is sorted instance by instance on the local bits alone.
+bool sort_by_instance(int64_t n, int chunks, int local, int bits);
 // Stable LSD radix sort of (key, value) pairs on the low `bits` key bits,
 // K = uint32_t or unsigned long long.  keys/vals: ping-pong buffers [0] and
 // [1]; input in [0].  If vals_in_is_iota, vals[0] is not read and the values
-// are taken as 0..n-1.  Returns the index (0 or 1) of the buffer that holds the
+// are taken as 0..n-1.  With chunks: the pairs of each instance by themselves, on the
+// low `bits` bits, the instances in their own order (input: in that of the points).
+// Returns the index (0 or 1) of the buffer that holds the
 // result.  timeouts as for the scan.
 template <class K>
 int radix_sort_pairs(K* keys[2], uint32_t* vals[2], int64_t n, int bits, bool vals_in_is_iota,
                      void* temp, void* scan_temp, cudaStream_t s,
-                     unsigned long long* timeouts = nullptr);
+                     unsigned long long* timeouts = nullptr, const SortChunks& sc = {});
 // kernels one radix_sort_pairs call launches
 int sort_launches(int64_t n, int bits);
 // digit width radix_sort_pairs uses for a `bits`-bit key (8 or 9)

@@ -18,6 +18,8 @@
 // ms): with about 760 tiles in flight the serial per-digit look-back chains
 // cost more than the upsweep and the histogram scan they replace.
 // This replaces thrust::sort_by_key (main.cu:332).
+#include <algorithm>
+
 #include "gd_internal.cuh"
 #include "gd_lookback.cuh"
 
@@ -114,14 +116,46 @@ template <class K>
 constexpr int rs_min_blocks() { return sizeof(K) == 4 ? 3 : 5; }
 constexpr int kRsMinTile = kRsThreads * 8;
 
+// A tile's place.  Plain: tile t of T, counts at [digit][tile].  By instance: a chunk of
+// one instance holds kChunkPoints / TILE tiles (the last chunk's perhaps empty), and the
+// counts lie [instance][digit][tile of the instance], so that their one scan gives every
+// instance's pairs their place among its own.
+struct RsPlace {
+  int64_t base, end;      // pairs [base, end) (the tile's, or more)
+  int64_t hist, stride;   // counts of digit d at hist + d * stride
+};
+template <int TILE, int BINS, bool SEG>
+__device__ __forceinline__ RsPlace rs_place(const SortChunks& sc, int64_t tile, int64_t n, int64_t T,
+                                            bool first) {
+  RsPlace p;
+  if constexpr (!SEG) {
+    p.base = tile * TILE;
+    p.end = n;
+    p.hist = tile;
+    p.stride = T;
+  } else {
+    constexpr int TPC = (int)(gd::kChunkPoints / TILE);
+    const int64_t ci = tile / TPC;
+    const gd::Chunk c = sc.chunks[ci];
+    const int64_t sub = tile % TPC, off = c.begin - sc.Pv[c.inst].pt_off;
+    const int64_t c0 = ci - off / gd::kChunkPoints;  // the instance's first chunk
+    const int64_t b = first ? c.begin : (int64_t)c.sorted;
+    p.base = b + sub * TILE;
+    p.end = b + (c.end - c.begin);
+    p.stride = (sc.Pv[c.inst].n + gd::kChunkPoints - 1) / gd::kChunkPoints * TPC;
+    p.hist = c0 * TPC * BINS + (ci - c0) * TPC + sub;
+  }
+  return p;
+}
+
 // A block counts the digits of G consecutive tiles (G | T), so that a digit's counts,
 // T apart from the next digit's, leave in one store of G (20M keys, three passes: a
 // tile per block 90 us, four 75; 2M keys: 17, but four tiles leave too few blocks, 50).
-template <class K, int ITEMS, int RB, int G>
+template <class K, int ITEMS, int RB, int G, bool SEG>
 __global__ void __launch_bounds__(kRsThreads)
 k_rs_upsweep(const K* __restrict__ keys, int64_t n, int shift, uint32_t* __restrict__ hist,
-             int64_t T) {
-  constexpr int SEG = 32 * ITEMS, TILE = kRsThreads * ITEMS, BINS = 1 << RB;
+             int64_t T, const SortChunks sc, bool first) {
+  constexpr int WSEG = 32 * ITEMS, TILE = kRsThreads * ITEMS, BINS = 1 << RB;
   constexpr int BPT = BINS / kRsThreads;
   constexpr uint32_t MASK = BINS - 1;
   // warp-private digit counts (shared-memory atomics), summed at the end
@@ -132,15 +166,16 @@ k_rs_upsweep(const K* __restrict__ keys, int64_t n, int shift, uint32_t* __restr
     for (int d = threadIdx.x; d < BINS; d += kRsThreads) h[ww][d] = 0;
   __syncthreads();
   uint32_t tot[BPT][G];
+  const RsPlace at = rs_place<TILE, BINS, SEG>(sc, (int64_t)blockIdx.x * G, n, T, first);
 #pragma unroll
   for (int g = 0; g < G; ++g) {
-    const int64_t seg = ((int64_t)blockIdx.x * G + g) * TILE + w * SEG;
+    const int64_t seg = at.base + g * TILE + w * WSEG;
     // every item's key in flight at once, then the counts
     uint32_t d[ITEMS];
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) {
       const int64_t e = seg + i * 32 + lane;
-      d[i] = e < n ? (uint32_t)(__ldg(keys + e) >> shift) & MASK : 0xffffffffu;
+      d[i] = e < at.end ? (uint32_t)(__ldg(keys + e) >> shift) & MASK : 0xffffffffu;
     }
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i)
@@ -160,21 +195,24 @@ k_rs_upsweep(const K* __restrict__ keys, int64_t n, int shift, uint32_t* __restr
   }
 #pragma unroll
   for (int q = 0; q < BPT; ++q) {
-    uint32_t* out = hist + (int64_t)(q * kRsThreads + threadIdx.x) * T + (int64_t)blockIdx.x * G;
+    uint32_t* out = hist + at.hist + (int64_t)(q * kRsThreads + threadIdx.x) * at.stride;
     if constexpr (G == 4)
       *reinterpret_cast<uint4*>(out) = make_uint4(tot[q][0], tot[q][1], tot[q][2], tot[q][3]);
+    else if constexpr (G == 2)
+      *reinterpret_cast<uint2*>(out) = make_uint2(tot[q][0], tot[q][1]);
     else
 #pragma unroll
       for (int g = 0; g < G; ++g) out[g] = tot[q][g];
   }
 }
 
-template <class K, int ITEMS, int RB>
+template <class K, int ITEMS, int RB, bool SEG>
 __global__ void __launch_bounds__(kRsThreads, rs_min_blocks<K>())
 k_rs_downsweep(const K* __restrict__ kin, const uint32_t* __restrict__ vin,
                K* __restrict__ kout, uint32_t* __restrict__ vout, int64_t n,
-               int shift, const uint32_t* __restrict__ goff, int64_t T) {
-  constexpr int SEG = 32 * ITEMS, TILE = kRsThreads * ITEMS, BINS = 1 << RB;
+               int shift, const uint32_t* __restrict__ goff, int64_t T, const SortChunks sc,
+               bool first) {
+  constexpr int WSEG = 32 * ITEMS, TILE = kRsThreads * ITEMS, BINS = 1 << RB;
   constexpr int BPT = BINS / kRsThreads;  // digits per thread in the tile scan
   constexpr uint32_t MASK = BINS - 1;
   constexpr bool LATE = sizeof(K) == 4;
@@ -186,19 +224,21 @@ k_rs_downsweep(const K* __restrict__ kin, const uint32_t* __restrict__ vin,
   __shared__ int32_t s_gbase[BINS];
   __shared__ uint32_t s_warp[32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int64_t base = (int64_t)blockIdx.x * TILE;
-  const int valid_count = (int)min((int64_t)TILE, n - base);
+  const RsPlace at = rs_place<TILE, BINS, SEG>(sc, blockIdx.x, n, T, first);
+  const int64_t base = at.base, end = at.end;
+  if (base >= end) return;  // an empty tile of a last chunk
+  const int valid_count = (int)min((int64_t)TILE, end - base);
   for (int i = lane; i < BINS; i += 32) s_cnt[w][i] = 0;
   __syncwarp();
   const unsigned lt_mask = (1u << lane) - 1u;
   K k[ITEMS];
   uint32_t v[ITEMS], r[ITEMS];
-  const int64_t seg = base + w * SEG;
+  const int64_t seg = base + w * WSEG;
 #pragma unroll
   for (int i = 0; i < ITEMS; ++i) {
     int64_t e = seg + i * 32 + lane;
-    k[i] = e < n ? __ldg(kin + e) : ~(K)0;
-    if (!LATE) v[i] = vin && e < n ? __ldg(vin + e) : (uint32_t)e;
+    k[i] = e < end ? __ldg(kin + e) : ~(K)0;
+    if (!LATE) v[i] = vin && e < end ? __ldg(vin + e) : (uint32_t)e;
   }
 #pragma unroll
   for (int i = 0; i < ITEMS; ++i) {
@@ -221,7 +261,7 @@ k_rs_downsweep(const K* __restrict__ kin, const uint32_t* __restrict__ vin,
 #pragma unroll
   for (int i = 0; i < ITEMS; ++i) {
     const int64_t e = seg + i * 32 + lane;
-    v[i] = vin && e < n ? __ldg(vin + e) : (uint32_t)e;
+    v[i] = vin && e < end ? __ldg(vin + e) : (uint32_t)e;
   }
   __syncthreads();
   {
@@ -246,7 +286,7 @@ k_rs_downsweep(const K* __restrict__ kin, const uint32_t* __restrict__ vin,
     for (int q = 0; q < BPT; ++q) {
       const int d = threadIdx.x * BPT + q;
       s_dstart[d] = ex;
-      s_gbase[d] = (int32_t)goff[(int64_t)d * T + blockIdx.x] - (int32_t)ex;
+      s_gbase[d] = (int32_t)goff[at.hist + (int64_t)d * at.stride] - (int32_t)ex;
       ex += tots[q];
     }
   }
@@ -378,23 +418,35 @@ void list_bits(const uint32_t* words, uint32_t* pre, int64_t nw, uint32_t* out, 
 // caller's scan temp, which holds nothing but scan state: were the two in one
 // buffer, a larger sort's status words would lie where a smaller sort left its
 // histogram, and a count that looks like a tagged word would pass for a prefix.
-int64_t sort_scan_elems(int64_t n) {
-  return ((n + kRsMinTile - 1) / kRsMinTile + 3) / 4 * 4 * kRsMaxBins;
+int64_t sort_scan_elems(int64_t n, int chunks) {
+  const int64_t plain = ((n + kRsMinTile - 1) / kRsMinTile + 3) / 4 * 4;
+  return std::max(plain, chunks * (gd::kChunkPoints / kRsMinTile)) * kRsMaxBins;
 }
 
-size_t sort_temp_bytes(int64_t n) {
-  return align_up((size_t)sort_scan_elems(n) * sizeof(uint32_t));
+size_t sort_temp_bytes(int64_t n, int chunks) {
+  return align_up((size_t)sort_scan_elems(n, chunks) * sizeof(uint32_t));
 }
 
-template <class K, int RB>
+// The points lie instance by instance already, so the id's bits need no pass (120M points
+// in 4096 instances, 48-bit keys of 36 local bits: six passes and 49.8 ms a run, by
+// instance four and 48.5); chunks that are half empty or more would cost more in empty
+// tiles' counts.
+bool sort_by_instance(int64_t n, int chunks, int local, int bits) {
+  auto passes = [](int b) { return (b + sort_digit_bits(b) - 1) / sort_digit_bits(b); };
+  return local > 0 && passes(local) < passes(bits) && chunks * gd::kChunkPoints <= 2 * n;
+}
+
+template <class K, int RB, bool SEG>
 int sort_passes(K* keys[2], uint32_t* vals[2], int64_t n, int passes, bool vals_in_is_iota,
-                void* temp, void* scan_temp, cudaStream_t s, unsigned long long* timeouts) {
+                void* temp, void* scan_temp, cudaStream_t s, unsigned long long* timeouts,
+                const SortChunks& sc) {
   constexpr int ITEMS = rs_items<K>();
   constexpr int TILE = kRsThreads * ITEMS;
   // four tiles per upsweep block where that leaves enough blocks; the histogram is then
   // for a multiple of four tiles, the last ones perhaps empty
-  int64_t T = (n + TILE - 1) / TILE;
-  const bool four = T >= kRsFour;
+  constexpr int TPC = (int)(gd::kChunkPoints / TILE);  // (by instance: a chunk's)
+  int64_t T = SEG ? (int64_t)sc.count * TPC : (n + TILE - 1) / TILE;
+  const bool four = !SEG && T >= kRsFour;
   const int64_t tiles = T;
   if (four) T = (T + 3) & ~(int64_t)3;
   const int64_t h = T << RB;
@@ -402,14 +454,20 @@ int sort_passes(K* keys[2], uint32_t* vals[2], int64_t n, int passes, bool vals_
   int cur = 0;
   for (int p = 0; p < passes; ++p) {
     int shift = RB * p;
-    if (four)
-      k_rs_upsweep<K, ITEMS, RB, 4><<<(unsigned)(T / 4), kRsThreads, 0, s>>>(keys[cur], n, shift, hist, T);
+    const bool first = p == 0;
+    if constexpr (SEG)
+      k_rs_upsweep<K, ITEMS, RB, TPC, true><<<(unsigned)sc.count, kRsThreads, 0, s>>>(
+          keys[cur], n, shift, hist, T, sc, first);
+    else if (four)
+      k_rs_upsweep<K, ITEMS, RB, 4, false><<<(unsigned)(T / 4), kRsThreads, 0, s>>>(keys[cur], n, shift, hist,
+                                                                           T, sc, first);
     else
-      k_rs_upsweep<K, ITEMS, RB, 1><<<(unsigned)T, kRsThreads, 0, s>>>(keys[cur], n, shift, hist, T);
+      k_rs_upsweep<K, ITEMS, RB, 1, false><<<(unsigned)T, kRsThreads, 0, s>>>(keys[cur], n, shift, hist, T, sc,
+                                                                       first);
     exclusive_scan_u32(hist, hist, h, scan_temp, nullptr, s, timeouts);
     const uint32_t* vin = (p == 0 && vals_in_is_iota) ? nullptr : vals[cur];
-    k_rs_downsweep<K, ITEMS, RB><<<(unsigned)tiles, kRsThreads, 0, s>>>(
-        keys[cur], vin, keys[cur ^ 1], vals[cur ^ 1], n, shift, hist, T);
+    k_rs_downsweep<K, ITEMS, RB, SEG><<<(unsigned)tiles, kRsThreads, 0, s>>>(
+        keys[cur], vin, keys[cur ^ 1], vals[cur ^ 1], n, shift, hist, T, sc, first);
     cur ^= 1;
   }
   return cur;
@@ -428,7 +486,8 @@ int sort_launches(int64_t n, int bits) {
 // else of 8 bits.
 template <class K>
 int radix_sort_pairs(K* keys[2], uint32_t* vals[2], int64_t n, int bits, bool vals_in_is_iota,
-                     void* temp, void* scan_temp, cudaStream_t s, unsigned long long* timeouts) {
+                     void* temp, void* scan_temp, cudaStream_t s, unsigned long long* timeouts,
+                     const SortChunks& sc) {
   if (n <= 0) return 0;
   const int rb = sort_digit_bits(bits);
   const int passes = (bits + rb - 1) / rb;
@@ -436,16 +495,15 @@ int radix_sort_pairs(K* keys[2], uint32_t* vals[2], int64_t n, int bits, bool va
     if (vals_in_is_iota) k_iota<<<1024, 256, 0, s>>>(vals[0], n);
     return 0;
   }
-  return rb == 9 ? sort_passes<K, 9>(keys, vals, n, passes, vals_in_is_iota, temp, scan_temp, s,
-                                     timeouts)
-                 : sort_passes<K, 8>(keys, vals, n, passes, vals_in_is_iota, temp, scan_temp, s,
-                                     timeouts);
+  auto* f = sc.chunks ? (rb == 9 ? sort_passes<K, 9, true> : sort_passes<K, 8, true>)
+                      : (rb == 9 ? sort_passes<K, 9, false> : sort_passes<K, 8, false>);
+  return f(keys, vals, n, passes, vals_in_is_iota, temp, scan_temp, s, timeouts, sc);
 }
 
 template int radix_sort_pairs<uint32_t>(uint32_t* [2], uint32_t* [2], int64_t, int, bool, void*,
-                                        void*, cudaStream_t, unsigned long long*);
+                                        void*, cudaStream_t, unsigned long long*, const SortChunks&);
 template int radix_sort_pairs<unsigned long long>(unsigned long long* [2], uint32_t* [2], int64_t,
                                                   int, bool, void*, void*, cudaStream_t,
-                                                  unsigned long long*);
+                                                  unsigned long long*, const SortChunks&);
 
 }  // namespace gdprim
