@@ -108,7 +108,6 @@ struct gd_ctx {
   int64_t n = 0;
   int dims = 0;   // bit 0: 2D instances present, bit 1: 3D
   bool f32 = false, key64 = false, xf = false;
-  bool x64 = true;  // the run keeps sorted float64 points
   gd::BatchInfo bi{};
   std::vector<gd::InstDesc> hdesc;
   std::vector<gd::Chunk> hchunk;
@@ -260,7 +259,7 @@ struct gd_ctx {
     B.hkeys = static_cast<unsigned long long*>(hkeys.p);
     B.hvals = static_cast<uint2*>(hvals.p);
     B.hmask = hmask;
-    B.X = x64 ? static_cast<double*>(X.p) : nullptr;
+    B.X = static_cast<double*>(X.p);
     B.Xf = static_cast<float*>(Xf.p);
     B.core = static_cast<uint8_t*>(core.p);
     B.cellcore = static_cast<int*>(cellcore.p);
@@ -370,7 +369,6 @@ gd_status build_small(gd_ctx* ctx) {
       {&ctx->asymwork, sizeof(gd::AsymWork)},
   }));
   ctx->is_small = true;
-  ctx->x64 = true;
   char* sm = static_cast<char*>(ctx->small.p);
   gd::SmallArgs& A = ctx->sa;
   A.coords = ctx->coords_ptr + I.co_off;
@@ -459,7 +457,6 @@ gd_status build_run(gd_ctx* ctx, uint64_t dense_floor, uint64_t rows_floor) {
   ctx->dims = (bi.K2 > 0 ? 1 : 0) | (bi.K2 < K ? 2 : 0);
   const size_t kw = ctx->key64 ? 8 : 4;
   const int maxd = bi.max_dim;
-  ctx->x64 = !ctx->f32 || bi.band_off;
   // block entries: direct tables, then one slot per cell if some instance has none
   const bool direct_only = bi.row_total == 0 && !bi.any_sparse;
   const int key_bits = bi.LB + bi.IB;
@@ -474,7 +471,7 @@ gd_status build_run(gd_ctx* ctx, uint64_t dense_floor, uint64_t rows_floor) {
       {&ctx->keys1, N * kw},
       {&ctx->vals0, N * 4},
       {&ctx->vals1, N * 4},
-      {&ctx->X, ctx->x64 ? N * maxd * 8 : 0},
+      {&ctx->X, N * maxd * 8},
       {&ctx->Xf, ctx->xf ? N * (maxd == 3 ? 16 : 8) : 0},
       {&ctx->ent, nent * sizeof(gd::BlockEnt)},
       {&ctx->links, nent * sizeof(gd::BlockLinks)},

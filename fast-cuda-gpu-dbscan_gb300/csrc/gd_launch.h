@@ -53,8 +53,7 @@ struct Bufs {
   unsigned long long* hkeys = nullptr;  // row hash slots: key of the block row's start
   uint2* hvals = nullptr;               // row hash slots: cells [x, y) of the row
   uint32_t hmask = 0;                   // row hash: slots - 1
-  double* X = nullptr;          // sorted float64 points (2 or 3 doubles each); null in a
-                                // float32-band run whose instances all have a band
+  double* X = nullptr;          // sorted float64 points (2 or 3 doubles each)
   float* Xf = nullptr;          // sorted centred float32 points (2 or 4 floats each)
   uint8_t* core = nullptr;      // core flag per sorted position
   int* cellcore = nullptr;      // per cell m: number of core points

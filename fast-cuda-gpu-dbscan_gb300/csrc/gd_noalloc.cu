@@ -350,7 +350,7 @@ extern "C" gd_status gd_dbscan_noalloc(const double* coords_dev, int64_t n, int3
   B.blist = vb[1 - r];  // the sort's other id and key buffers are free after the sort
   gdl::set_bits(B, reinterpret_cast<uint32_t*>(base + kOffBits), n);
   B.K = dK;
-  B.X = f32 ? nullptr : reinterpret_cast<double*>(base + kOffX);
+  B.X = reinterpret_cast<double*>(base + kOffX);
   B.Xf = reinterpret_cast<float*>(base + kOffXf);
   B.reps = reinterpret_cast<int*>(base + kOffReps);
   B.cellent = reinterpret_cast<uint32_t*>(base + kOffCellent);

@@ -624,8 +624,10 @@ __device__ __forceinline__ void load_coords(const double* __restrict__ src, doub
   }
 }
 
-// Sorted copies: float64 points (16 or 24 bytes each; X null: none wanted) and
-// centred float32 ones (8 or 16 bytes).  2D positions come first in a mixed run,
+// Sorted copies: float64 points (16 or 24 bytes each) and centred float32 ones (8 or 16
+// bytes).  The float64 ones are written in every mode: the points are the caller's, who may
+// change or free them once the first expand has returned, and later expands of the index
+// re-test the float32 band's pairs.  2D positions come first in a mixed run,
 // so each point lies at its position times its own size.  ONE: a single
 // instance (its parameters are Pv[0], no key is read).  kGatherU points per
 // thread and pass, so that as many random loads are in flight.
@@ -660,13 +662,11 @@ __global__ void k_gather(const gdl::Bufs B, int64_t n) {
       if (i >= n) continue;
       const DevParams& P = *Pp[u];
       const int D = P.dim;
-      if (B.X) {
-        if (D == 2) {
-          reinterpret_cast<double2*>(B.X)[i] = make_double2(v[u][0], v[u][1]);
-        } else {
+      if (D == 2) {
+        reinterpret_cast<double2*>(B.X)[i] = make_double2(v[u][0], v[u][1]);
+      } else {
 #pragma unroll
-          for (int k = 0; k < 3; ++k) B.X[3 * i + k] = v[u][k];
-        }
+        for (int k = 0; k < 3; ++k) B.X[3 * i + k] = v[u][k];
       }
       if (XF) {
         const float f0 = __double2float_rn(__dsub_rn(v[u][0], P.centre[0]));
@@ -1000,20 +1000,6 @@ __device__ __forceinline__ void ld_f(const gdl::Bufs& B, int64_t i, float* v) {
     v[D - 1] = t.z;
   }
 }
-// Float64 coordinates for a band re-test: the sorted copy, or (float32-band runs
-// keep none when every instance has a band) the caller's point.
-template <int D>
-__device__ __forceinline__ void exact_x(const gdl::Bufs& B, const DevParams& P, int64_t i,
-                                        double* v) {
-  if (B.X) {
-    ld_x<D>(B, i, v);
-    return;
-  }
-  const double* src = B.coords + P.co_off + ((int64_t)B.ids[i] - P.pt_off) * D;
-#pragma unroll
-  for (int k = 0; k < D; ++k) v[k] = src[k];
-}
-
 // One candidate (sorted position q) in the layout the mode tests with.
 template <int D, bool F32>
 struct Cand {
@@ -1059,9 +1045,8 @@ __device__ __forceinline__ float dist2_f32(const float* a, const float* b) {
 // float64 coordinates of both are loaded only for a band re-test.
 template <int D, bool F32, class PP>
 __device__ __forceinline__ bool pair_test(const double* sx, const float* sf, const Cand<D, F32>& c,
-                                          const gdl::Bufs& B, const DevParams& I, int64_t q,
-                                          int64_t si, bool stage_is_centre, const PP& P,
-                                          Tally& t) {
+                                          const gdl::Bufs& B, int64_t q, int64_t si,
+                                          bool stage_is_centre, const PP& P, Tally& t) {
   if (F32) {
     ++t.t32;
     float s = dist2_f32<D>(sf, c.f);
@@ -1069,8 +1054,8 @@ __device__ __forceinline__ bool pair_test(const double* sx, const float* sf, con
     if (s > P.eps2_hi32) return false;
     ++t.band;
     double qx[D], px[D];
-    exact_x<D>(B, I, q, qx);
-    exact_x<D>(B, I, si, px);
+    ld_x<D>(B, q, qx);
+    ld_x<D>(B, si, px);
     ++t.t64;
     double d2 = dist2_f64<D>(px, qx);
     return stage_is_centre ? pred_from_d2<D>(d2, px, qx, P) : pred_from_d2<D>(d2, qx, px, P);
@@ -1085,8 +1070,8 @@ __device__ __forceinline__ bool pair_test(const double* sx, const float* sf, con
 // directions; counts pairs that are neighbours in exactly one direction.
 template <int D, bool F32, class PP>
 __device__ __forceinline__ bool link_test(const double* sx, const float* sf, const Cand<D, F32>& c,
-                                          const gdl::Bufs& B, const DevParams& I, int a, int q,
-                                          const PP& P, Tally& t) {
+                                          const gdl::Bufs& B, int a, int q, const PP& P,
+                                          Tally& t) {
   double qx[D], ax[D];
   if (F32) {
     ++t.t32;
@@ -1095,8 +1080,8 @@ __device__ __forceinline__ bool link_test(const double* sx, const float* sf, con
     if (s > P.eps2_hi32) return false;
     ++t.band;
     // float64 coordinates of both, for the band re-test only
-    exact_x<D>(B, I, q, qx);
-    exact_x<D>(B, I, a, ax);
+    ld_x<D>(B, q, qx);
+    ld_x<D>(B, a, ax);
   } else {
 #pragma unroll
     for (int k = 0; k < D; ++k) {
@@ -2069,14 +2054,14 @@ k_core_cell(const gdl::Bufs B, int64_t n, int p0, int p1) {
           if (band) {
             // the float64 predicate for the points whose float32 test cannot say
             double qx[D];
-            exact_x<D>(B, P, q, qx);
+            ld_x<D>(B, q, qx);
 #pragma unroll
             for (int a = 0; a < C; ++a) {
               if (a >= na) continue;
               const float s2 = dist2_f32<D>(pf[a], f);
               if (s2 < Q.eps2_lo32 || s2 > Q.eps2_hi32) continue;
               double px[D];
-              exact_x<D>(B, P, i + a, px);
+              ld_x<D>(B, i + a, px);
               ++t.band;
               ++t.t64;
               cnt[a] += pred_from_d2<D>(dist2_f64<D>(px, qx), px, qx, Q) ? 1 : 0;
@@ -2451,7 +2436,7 @@ __device__ __forceinline__ int inline_link(const gdl::Bufs& B, int64_t n, int bA
       if (budget-- == 0) return -1;
       Cand<D, F32> cd;
       load_cand<D, F32>(cd, B, q);
-      if (link_test<D, F32>(ax, af, cd, B, P, a, q, Q, t)) return 1;
+      if (link_test<D, F32>(ax, af, cd, B, a, q, Q, t)) return 1;
     }
   }
   return 0;
@@ -2790,7 +2775,7 @@ __global__ void __launch_bounds__(kBorderThreads, kBorderMinBlocks) k_border_poi
             }
             Cand<D, F32> cd;
             load_cand<D, F32>(cd, B, qq);
-            if (pair_test<D, F32>(px, pf, cd, B, P, qq, i, false, Q, t)) {
+            if (pair_test<D, F32>(px, pf, cd, B, qq, i, false, Q, t)) {
               best = cB;
               break;
             }
@@ -2864,7 +2849,7 @@ __global__ void __launch_bounds__(kCellThreads) k_core_heavy(const gdl::Bufs B, 
           load_cand<D, F32>(cd, B, q);
         }
         for (int j = 0; j < na; ++j) {
-          bool hit = valid && pair_test<D, F32>(S.x[j], S.f[j], cd, B, P, q, b + c0 + j, true, Q, t);
+          bool hit = valid && pair_test<D, F32>(S.x[j], S.f[j], cd, B, q, b + c0 + j, true, Q, t);
           unsigned bal = __ballot_sync(kFull, hit);
           if (lane == j) mycnt += __popc(bal);
         }
@@ -3133,7 +3118,7 @@ __global__ void __launch_bounds__(kCellThreads) k_union_heavy(const gdl::Bufs B,
             float af[D];
             if (F32) ld_f<D>(B, a, af);
             else ld_x<D>(B, a, ax);
-            bool hit = valid && link_test<D, F32>(ax, af, c, B, P, a, q, Q, t);
+            bool hit = valid && link_test<D, F32>(ax, af, c, B, a, q, Q, t);
             found = __any_sync(kFull, hit);
           }
         }
@@ -3429,7 +3414,7 @@ __global__ void __launch_bounds__(kCellThreads) k_border_heavy(const gdl::Bufs B
             while (pending) {
               const int j = __ffs(pending) - 1;
               pending &= pending - 1;
-              bool hit = valid && pair_test<D, F32>(S.x[j], S.f[j], c, B, P, q, sIdx[w][j], false, Q, t);
+              bool hit = valid && pair_test<D, F32>(S.x[j], S.f[j], c, B, q, sIdx[w][j], false, Q, t);
               if (__any_sync(kFull, hit)) {
                 if (lane == j) best = cB;
                 wantm &= ~(1u << j);

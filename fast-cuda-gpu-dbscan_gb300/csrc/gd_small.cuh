@@ -439,7 +439,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_small_expand(const gdl::Bufs 
         }
         Cand<D, F32> cd;
         load_cand<D, F32>(cd, B, q);
-        hit = pair_test<D, F32>(px, pf, cd, B, P, q, i, true, Q, t);
+        hit = pair_test<D, F32>(px, pf, cd, B, q, i, true, Q, t);
         ++q;
       }
       cnt += __popc(__ballot_sync(kFull, hit) & grp);
@@ -642,7 +642,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_small_expand(const gdl::Bufs 
             if (!B.core[qq]) continue;
             Cand<D, F32> cd;
             load_cand<D, F32>(cd, B, qq);
-            if (pair_test<D, F32>(px, pf, cd, B, P, qq, i, false, Q, t)) {
+            if (pair_test<D, F32>(px, pf, cd, B, qq, i, false, Q, t)) {
               best = cB;
               break;
             }

@@ -125,7 +125,9 @@ gd_status gd_ctx_set_graphs(gd_ctx* ctx, int32_t enable);
    per-node tree allocation (main.cu:264-305), INDEXING_STRUCTURE
    (indexing.cu:54-118), thrust::sort_by_key (main.cu:332) and
    INDEXING_ADJUSTMENT (indexing.cu:23-51).  Builds the eps-cell grid of the
-   points on the device; the points must stay valid until gd_expand returns. */
+   points on the device; the points must stay valid until gd_expand returns.  (The
+   index keeps its own copy of them: later gd_expand calls on it do not read the
+   caller's.) */
 gd_status gd_index_build(gd_ctx* ctx, const gd_points* pts, double eps);
 
 /* Replaces the expansion loop main.cu:369-403: MonitorSeedPoints
