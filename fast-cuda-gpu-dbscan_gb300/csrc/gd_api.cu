@@ -304,7 +304,7 @@ struct gd_ctx {
     B.compmin = B.lab;
     B.asym = static_cast<int*>(asym.p);
     B.ctr = dCtr();
-    B.tn_link = INT32_MAX;  // links are searched to the end
+    B.tn_link = gd::kSmallLinkTests;
     return B;
   }
 };
@@ -380,7 +380,7 @@ gd_status build_small(gd_ctx* ctx) {
   A.hash_slots = slots;
   A.bar = reinterpret_cast<unsigned*>(sm + gd_ctx::kBarAt);
   A.part = static_cast<long long*>(ctx->bbox.p);
-  A.ptkey = static_cast<uint64_t*>(ctx->keys0.p);
+  A.ptkey = static_cast<unsigned long long*>(ctx->keys0.p);
   A.cellkey = static_cast<uint64_t*>(ctx->keys1.p);
   A.ptcell = static_cast<uint32_t*>(ctx->vals0.p);
   A.ptpos = static_cast<uint32_t*>(ctx->cellent.p);

@@ -268,7 +268,8 @@ struct SmallArgs {
   uint32_t hash_slots;       // slots of the block hash (power of two); 0: direct grids only
   unsigned* bar;             // barrier: arrivals, generation (zero when first used)
   long long* part;           // 8 words per block: bounds of its points, non-finite flag
-  uint64_t* ptkey;           // per point: entry << 6 | place in the block
+  // (index; in the expand these three hold the lists of open link searches)
+  unsigned long long* ptkey; // per point: entry << 6 | place in the block
   uint32_t* ptcell;          // per point: its cell
   uint32_t* ptpos;           // per point: its place in the cell
   uint32_t* pcell;           // per position: its cell
@@ -280,6 +281,8 @@ struct SmallArgs {
 };
 
 constexpr int kSmallThreads = 512;
+// pair tests one lane of a small run spends on a cell pair before the pair goes to a warp
+constexpr int kSmallLinkTests = 256;
 // Single runs of at most this many points take the small kernels when their grid has
 // a direct block table.  The lines lie where the general pipeline's launches stop
 // dominating: 2D 482 -> 341 us at 128k points, 510 -> 398 at 256k (blobs, float64); 3D

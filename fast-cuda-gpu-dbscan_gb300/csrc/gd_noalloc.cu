@@ -230,7 +230,7 @@ extern "C" gd_status gd_dbscan_noalloc(const double* coords_dev, int64_t n, int3
     A.hash_slots = gd::small_hash_slots(n);
     A.bar = reinterpret_cast<unsigned*>(base + kOffSmall + 2048);
     A.part = reinterpret_cast<long long*>(base + kOffBbox);
-    A.ptkey = reinterpret_cast<uint64_t*>(base + kOffKeys0);
+    A.ptkey = reinterpret_cast<unsigned long long*>(base + kOffKeys0);
     A.cellkey = reinterpret_cast<uint64_t*>(base + kOffKeys1);
     A.ptcell = reinterpret_cast<uint32_t*>(base + kOffVals0);
     A.ptpos = reinterpret_cast<uint32_t*>(base + kOffCellent);
@@ -261,7 +261,7 @@ extern "C" gd_status gd_dbscan_noalloc(const double* coords_dev, int64_t n, int3
     B.compmin = B.lab;
     B.asym = reinterpret_cast<int*>(base + kOffAsym);
     B.ctr = dCtr;
-    B.tn_link = INT32_MAX;
+    B.tn_link = gd::kSmallLinkTests;
     const int nb = std::min(sms, (int)kMaxSms);
     NA_CUDA(cudaMemsetAsync(base + kOffSmall, 0, 4096, s), "clear counters");
     NA_CUDA(gdl::small_index(B, A, nb, s), "small index launch");

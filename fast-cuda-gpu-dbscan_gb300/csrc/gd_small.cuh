@@ -321,10 +321,183 @@ struct SmallWalk {
   }
 };
 
-// point-to-cell classification as in the walks (classify), from in-cell position u
+// ---- link searches that a lane does not finish.  A lane of the union spends at most
+// kSmallLinkTests tests on a cell pair, and none on a pair of more than kSmallLanePairs point
+// pairs: a pair of crowded cells that are apart by a little more than eps would otherwise keep
+// one lane busy for |A| |B| tests while every other block waits at the barrier.  The cells with
+// open pairs are listed with those pairs as a mask (offsets of the step's half stencil) and
+// searched after the barrier, a warp per cell; pairs of more than kSmallWarpPairs point pairs
+// then by the whole grid, one after the other.  (Two crowds of 5,000 points each, 1.1 eps
+// apart, float64, whole call: 0.70 ms in 2D and 0.79 in 3D; 20,000 each: 6.4 and 8.6.  The
+// general path's warp per pair: 234 and 304 ms; 4.5 and 5.5 s.)
+// The lists lie in buffers of the index build that are free by now: each cell's mask in ptkey,
+// the listed cells in ptcell (each once per step), large pairs in ptpos: a pair of more than 2^17 point
+// pairs has a cell of more than 362 points, there are at most n / 363 of those, each in at
+// most 124 pairs (62 in each half of the 3D stencil), which is below n / 2.
+constexpr long long kSmallLanePairs = 1ll << 16, kSmallWarpPairs = 1ll << 17;
+__host__ __device__ constexpr int small_big_cap(int n) { return n / 2; }
+
+constexpr int kShell3 = make_half(3, 1).n;
+static_assert(kShell3 + make_half(3, 2).n <= 64 && make_half(2, 1).n <= 64, "a mask per step");
+
+// Index of an offset among the step's half stencil (step 0: pass 0; step 1: the others).
+template <int D>
+__device__ __forceinline__ int small_open_bit(int step, int ox, int oy, int oz) {
+  const int ax = max(abs(ox), max(abs(oy), abs(oz)));
+  if (step == 0) return half_bit<D>(0, ox, oy, oz);
+  return D == 3 && ax > 1 ? kShell3 + half_bit<D>(2, ox, oy, oz) : half_bit<D>(1, ox, oy, oz);
+}
+
+// Core point a of one cell against the core points [b0, b1) of another: whether one is its
+// neighbour both ways.  A warp, a lane per candidate.
 template <int D, bool F32>
-__global__ void __launch_bounds__(kSmallThreads) k_small_expand(const gdl::Bufs B, const SmallArgs A,
-                                                                int minpts, int* __restrict__ out) {
+__device__ __forceinline__ bool small_warp_row(const gdl::Bufs& B, int a, int b0, int b1,
+                                               const PredParams& Q, Tally& t) {
+  const int lane = threadIdx.x & 31;
+  double ax[D];
+  float af[D];
+  if (F32) ld_f<D>(B, a, af);
+  else ld_x<D>(B, a, ax);
+  for (int qb = b0; qb < b1; qb += 32) {
+    const int q = qb + lane;
+    bool hit = false;
+    if (q < b1 && B.core[q]) {
+      Cand<D, F32> c;
+      load_cand<D, F32>(c, B, q);
+      hit = link_test<D, F32>(ax, af, c, B, a, q, Q, t);
+    }
+    if (__any_sync(kFull, hit)) return true;
+  }
+  return false;
+}
+
+// The same for core points [a0, a0 + na), na <= 32, of the cell with origin oA: those that
+// have the other cell (at offset o) wholly inside or outside their reach need no tests.
+template <int D, bool F32>
+__device__ __forceinline__ bool small_warp_rows(const gdl::Bufs& B, int a0, int na, int b0, int b1,
+                                                const float* oA, const int* o, const PredParams& Q,
+                                                Tally& t) {
+  const int lane = threadIdx.x & 31;
+  int cls = -1;
+  if (lane < na && B.core[a0 + lane]) {
+    cls = 0;
+    if (Q.prune) {
+      float f[D], u[D];
+      ld_f<D>(B, a0 + lane, f);
+      frac_pos<D>(f, oA, Q, u);
+      cls = classify<D>(u, o[0], o[1], o[2], Q);
+    }
+  }
+  if (__any_sync(kFull, cls > 0)) return true;  // (the other cell holds a core point)
+  for (unsigned w = __ballot_sync(kFull, cls == 0); w; w &= w - 1)
+    if (small_warp_row<D, F32>(B, a0 + __ffs(w) - 1, b0, b1, Q, t)) return true;
+  return false;
+}
+
+// two cells' roots equal (one answer for the warp)
+__device__ __forceinline__ bool small_same(const gdl::Bufs& B, int a, int b) {
+  int same = 0;
+  if ((threadIdx.x & 31) == 0) same = uf_find(B.parent, a) == uf_find(B.parent, b);
+  return __shfl_sync(kFull, same, 0) != 0;
+}
+
+// The listed cells' open pairs, a warp per cell.
+template <int D, bool F32>
+__device__ __noinline__ void small_link_cells(const gdl::Bufs& B, const SmallArgs& A,
+                                              const DevParams& P, int step, int listed,
+                                              unsigned long long* nbig) {
+  constexpr int S = block_shift<D>(), SM = (1 << S) - 1;
+  const int lane = threadIdx.x & 31;
+  const int W = gridDim.x * (kSmallThreads / 32);
+  const PredParams Q = pred_params(P);
+  uint2* big = reinterpret_cast<uint2*>(A.ptpos);
+  const int n0 = kHalf[D - 2][step].n, n1 = step == 0 ? 0 : kHalf[D - 2][2].n;
+  Tally t;
+  for (int h = blockIdx.x * (kSmallThreads / 32) + (threadIdx.x >> 5); h < listed; h += W) {
+    const int m = (int)A.ptcell[h];
+    const unsigned long long open = A.ptkey[m];
+    __syncwarp();
+    if (lane == 0) A.ptkey[m] = 0;  // for the next step
+    const uint64_t ck = A.cellkey[m];
+    const uint32_t own = (uint32_t)(ck >> kBlockBits);
+    const uint64_t blk = P.sparse == 0 ? own : B.hkeys[own];
+    const CellXYZ<D> cc = decompose<D>(blk << kBlockBits | (ck & 63), P);
+    const uint2 ra = A.crange[m];
+    float oA[D];
+    if (Q.prune) cell_origin32<D>(cc, P, oA);
+    for (int t0 = 0; t0 < n0 + n1; t0 += 32) {
+      const int tt = t0 + lane;
+      int c = -1;
+      uint2 rb = make_uint2(0, 0);
+      if (tt < n0 + n1 && ((open >> tt) & 1ull)) {
+        const signed char* o = tt < n0 ? kHalf[D - 2][step].o[tt] : kHalf[D - 2][2].o[tt - n0];
+        const int x = cc.c[0] + o[0], y = cc.c[1] + o[1], z = cc.c[2] + o[2];
+        const EntHead e = ent_head(B, small_ent<D>(B, P, x >> S, y >> S, D == 3 ? z >> S : 0));
+        const int bit = D == 3 ? (x & SM) << (2 * S) | (y & SM) << S | (z & SM)
+                               : (x & SM) << S | (y & SM);
+        if ((e.occ >> bit) & 1ull) {
+          c = ent_cell(e.occ, e.base, bit);
+          rb = A.crange[c];
+        }
+      }
+      for (unsigned mask = __ballot_sync(kFull, c >= 0); mask; mask &= mask - 1) {
+        const int src = __ffs(mask) - 1, k = t0 + src;
+        const int cb = __shfl_sync(kFull, c, src);
+        const int b0 = (int)__shfl_sync(kFull, rb.x, src), b1 = (int)__shfl_sync(kFull, rb.y, src);
+        if (small_same(B, m, cb)) continue;
+        if ((long long)(ra.y - ra.x) * (b1 - b0) > kSmallWarpPairs) {
+          if (lane == 0) {
+            const unsigned long long at = atomicAdd(nbig, 1ull);
+            if (at < (unsigned long long)small_big_cap(A.n))
+              big[at] = make_uint2((uint32_t)m, (uint32_t)cb);
+          }
+          continue;
+        }
+        const signed char* ob = k < n0 ? kHalf[D - 2][step].o[k] : kHalf[D - 2][2].o[k - n0];
+        const int o[3] = {ob[0], ob[1], ob[2]};
+        bool found = false;
+        for (int a = (int)ra.x; a < (int)ra.y && !found; a += 32)
+          found = small_warp_rows<D, F32>(B, a, min(32, (int)ra.y - a), b0, b1, oA, o, Q, t);
+        if (found && lane == 0) uf_union(B.parent, m, cb);
+        __syncwarp();
+      }
+    }
+  }
+  flush_tally(t, B.ctr);
+}
+
+// The large pairs, each by the whole grid: a warp per point of the first cell.
+template <int D, bool F32>
+__device__ __noinline__ void small_link_big(const gdl::Bufs& B, const SmallArgs& A,
+                                            const DevParams& P, int pairs) {
+  const int W = gridDim.x * (kSmallThreads / 32);
+  const int w = blockIdx.x * (kSmallThreads / 32) + (threadIdx.x >> 5);
+  const PredParams Q = pred_params(P);
+  const uint2* big = reinterpret_cast<const uint2*>(A.ptpos);
+  pairs = min(pairs, small_big_cap(A.n));
+  Tally t;
+  for (int p = 0; p < pairs; ++p) {
+    const int m = (int)big[p].x, c = (int)big[p].y;
+    const uint2 ra = A.crange[m], rb = A.crange[c];
+    for (int a = (int)ra.x + w; a < (int)ra.y; a += W) {
+      if (!B.core[a]) continue;
+      if (small_same(B, m, c)) break;
+      if (small_warp_row<D, F32>(B, a, (int)rb.x, (int)rb.y, Q, t)) {
+        if ((threadIdx.x & 31) == 0) uf_union(B.parent, m, c);
+        __syncwarp();
+        break;
+      }
+    }
+  }
+  flush_tally(t, B.ctr);
+}
+
+// Two blocks' registers fit an SM, so that two runs on different streams do not wait for each
+// other's end (one block per SM: 118 registers, no spills, and within 1 % of the time).
+template <int D, bool F32>
+__global__ void __launch_bounds__(kSmallThreads, 2)
+k_small_expand(const __grid_constant__ gdl::Bufs B, const __grid_constant__ SmallArgs A, int minpts,
+               int* __restrict__ out) {
   using W = SmallWalk<D>;
   __shared__ DevParams P;
   extern __shared__ uint32_t s_pre[];  // prefix counts of the cluster marks
@@ -351,6 +524,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_small_expand(const gdl::Bufs 
     B.cellcore[m] = (int)(r.y - r.x) >= minpts ? (int)(r.y - r.x) : 0;
     B.cellmin[m] = INT_MAX;
     B.parent[m] = m;
+    A.ptkey[m] = 0;  // no link search open
     B.ent[A.cellkey[m] >> kBlockBits].core = 0;
   }
   for (int k = t0; k < nwf; k += T) B.fbits[k] = 0;
@@ -470,8 +644,10 @@ __global__ void __launch_bounds__(kSmallThreads) k_small_expand(const gdl::Bufs 
   if (!grid_barrier(A, timeouts)) return;
   // ---- union, a group per core cell: first the near neighbours (pass 0 of the
   // half stencil), then, from compressed parents, the others, most of which settle
-  // from one parent load
+  // from one parent load.  Pairs that pass a lane's budget follow after the barrier.
   for (int step = 0; step < 2; ++step) {
+    unsigned long long* nopen = B.ctr + (step == 0 ? kCtrHeavyCore : kCtrHeavyUnion);
+    unsigned long long* nbig = B.ctr + (step == 0 ? kCtrHeavyBorder : kCtrWalkCursor3);
     for (int m = g0; m < M; m += gT) {
       if (B.cellcore[m] == 0) continue;  // (the whole group)
       const uint64_t ck = A.cellkey[m];
@@ -536,14 +712,29 @@ __global__ void __launch_bounds__(kSmallThreads) k_small_expand(const gdl::Bufs 
         }
         if (!linked && !(apart && single && B.cellcore[c] == 1)) {
           const uint2 q = A.crange[c];
-          linked = inline_link<D, F32>(B, n, (int)r.x, (int)r.y, (int)q.x, (int)q.y, oA,
-                                       wk.off(bit, 0), wk.off(bit, 1),
-                                       D == 3 ? wk.off(bit, D - 1) : 0, P, Q, t) > 0;
+          const int ox = wk.off(bit, 0), oy = wk.off(bit, 1), oz = D == 3 ? wk.off(bit, D - 1) : 0;
+          const int res = (long long)(r.y - r.x) * (q.y - q.x) > kSmallLanePairs
+                              ? -1
+                              : inline_link<D, F32>(B, n, (int)r.x, (int)r.y, (int)q.x, (int)q.y,
+                                                    oA, ox, oy, oz, P, Q, t);
+          linked = res > 0;
+          if (res < 0 && atomicOr(A.ptkey + m, 1ull << small_open_bit<D>(step, ox, oy, oz)) == 0)
+            A.ptcell[atomicAdd(nopen, 1ull)] = (uint32_t)m;
         }
         if (linked) uf_union(B.parent, m, c);
       }
     }
     if (!grid_barrier(A, timeouts)) return;
+    const int listed = (int)*reinterpret_cast<volatile unsigned long long*>(nopen);
+    if (listed) {
+      small_link_cells<D, F32>(B, A, P, step, listed, nbig);
+      if (!grid_barrier(A, timeouts)) return;
+      const int pairs = (int)*reinterpret_cast<volatile unsigned long long*>(nbig);
+      if (pairs) {
+        small_link_big<D, F32>(B, A, P, pairs);
+        if (!grid_barrier(A, timeouts)) return;
+      }
+    }
     if (step == 0) {
       for (int m = t0; m < M; m += T)
         if (B.cellcore[m] > 0) B.parent[m] = uf_find(B.parent, m);
