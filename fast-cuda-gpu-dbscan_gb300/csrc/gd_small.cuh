@@ -511,8 +511,14 @@ k_small_expand(const __grid_constant__ gdl::Bufs B, const __grid_constant__ Smal
     reinterpret_cast<uint32_t*>(&P)[k] = reinterpret_cast<const uint32_t*>(B.Pv)[k];
   __syncthreads();
   if (P.flags & (kFlagNonFinite | kFlagGridTooLarge | kFlagNotSmall)) return;  // (every block)
-  if (threadIdx.x == 0) P.minpts = minpts;
+  // a wait of the index build gave up: cells, ids and places may be an earlier call's
+  __shared__ int s_off;
+  if (threadIdx.x == 0) {
+    s_off = *reinterpret_cast<volatile unsigned long long*>(timeouts) != 0;
+    P.minpts = minpts;
+  }
   __syncthreads();
+  if (s_off) return;
   const PredParams Q = pred_params(P);
   const bool prune = Q.prune != 0;
   const int M = (int)B.ctr[kCtrCells];
