@@ -397,7 +397,10 @@ gd_status build_small(gd_ctx* ctx) {
   std::memcpy(&ctx->bi, ctx->mirror + gd_ctx::kBiAt, sizeof(gd::BatchInfo));
   const gd::BatchInfo& bi = ctx->bi;
   const unsigned long long* ctr = reinterpret_cast<const unsigned long long*>(ctx->mirror + 128);
-  if (ctr[gd::kCtrWaitTimeouts]) return fail(GD_ECUDA, "a grid barrier wait gave up");
+  if (ctr[gd::kCtrWaitTimeouts]) {  // a barrier wait gave up: the general path has none
+    ctx->is_small = false;
+    return GD_OK;
+  }
   if (bi.flags & gd::kFlagNonFinite) return fail(GD_EINVAL, "input has NaN or Inf coordinates");
   if (bi.flags & gd::kFlagGridTooLarge) return grid_too_large();
   if (bi.flags & gd::kFlagNotSmall) {
@@ -618,8 +621,23 @@ gd_status expand_run(gd_ctx* ctx) {
   return GD_OK;
 }
 
-// Scatter labels (and core flags) to the caller's point order, copy them out,
-// read the counters into ctx->st.
+// A small run whose expand gave up at a barrier (other streams' kernels kept SMs busy all the
+// while) goes through the general path instead, from the index's own copy of the points: the
+// caller's may be gone by now.
+gd_status redo_general(gd_ctx* ctx) {
+  const gd::InstDesc& I = ctx->hdesc[0];
+  if (ctx->coords_ptr != ctx->coords.p) {
+    GD_TRY(ctx->ensure(ctx->coords, (size_t)I.n * I.dim * 8, "points"));
+    gdl::small_points(ctx->small_bufs(), (int)I.n, I.dim, static_cast<double*>(ctx->coords.p),
+                      ctx->sms, ctx->stream);
+    ctx->coords_ptr = static_cast<const double*>(ctx->coords.p);
+  }
+  ctx->stage = 0;
+  GD_TRY(build_run(ctx, kBlockFloor, kRowFloor));
+  cudaEventRecord(ctx->ev[2], ctx->stream);
+  return expand_run(ctx);
+}
+
 // Scatter labels (and core flags) to the caller's order, copy them out, read the
 // counters, all behind one stream synchronisation.  A batch also passes its
 // per-instance cluster-count array (kc, kc_count entries in sorted-instance
@@ -680,6 +698,10 @@ gd_status finish_run(gd_ctx* ctx, int32_t* labels, uint8_t* is_core, int32_t on_
   S.asym_pairs = (int64_t)ctr[gd::kCtrAsym];
   S.precision_used = ctx->f32 ? GD_PREC_FP32_BAND : GD_PREC_FP64;
   S.launches = ctx->launches + ctx->expand_launches + fin;
+  if (ctr[gd::kCtrWaitTimeouts] && ctx->is_small) {
+    GD_TRY(redo_general(ctx));
+    return finish_run(ctx, labels, is_core, on_device, kc, kc_count);
+  }
   if (ctr[gd::kCtrWaitTimeouts]) {
     // start the scan state afresh for the next run
     if (ctx->scantemp.p) cudaMemsetAsync(ctx->scantemp.p, 0, ctx->scantemp.bytes, s);

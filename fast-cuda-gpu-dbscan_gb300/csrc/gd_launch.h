@@ -148,6 +148,8 @@ int scatter_labels(const Bufs& B, int64_t n, int* out, uint8_t* core_out, int sm
 cudaError_t small_index(const Bufs& B, const gd::SmallArgs& A, int sms, cudaStream_t s);
 cudaError_t small_expand(const Bufs& B, const gd::SmallArgs& A, bool f32, int minpts, int* out,
                          int sms, cudaStream_t s);
+// the points in the caller's order, from the sorted copy
+int small_points(const Bufs& B, int n, int dim, double* out, int sms, cudaStream_t s);
 int small_scatter(const Bufs& B, int n, int* out, uint8_t* core_out, int sms, cudaStream_t s);
 // per-instance cluster counts (K entries) from the cluster marks
 int cluster_counts(const Bufs& B, int K, int64_t* out, cudaStream_t s);

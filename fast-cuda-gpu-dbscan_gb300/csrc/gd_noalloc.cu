@@ -274,13 +274,13 @@ extern "C" gd_status gd_dbscan_noalloc(const double* coords_dev, int64_t n, int3
     gd::BatchInfo bi;
     std::memcpy(&bi, back + 1024, sizeof bi);
     const unsigned long long* ctr = reinterpret_cast<const unsigned long long*>(back + 128);
-    if (ctr[gd::kCtrWaitTimeouts])
-      return fail(GD_ECUDA, "gd_dbscan_noalloc: a grid barrier wait gave up");
-    if (bi.flags & gd::kFlagNonFinite)
+    // (where a barrier wait gave up: the general pipeline, which has none)
+    const bool gave_up = ctr[gd::kCtrWaitTimeouts] != 0;
+    if (!gave_up && (bi.flags & gd::kFlagNonFinite))
       return fail(GD_EINVAL, "gd_dbscan_noalloc: input has NaN or Inf coordinates");
-    if (bi.flags & gd::kFlagGridTooLarge)
+    if (!gave_up && (bi.flags & gd::kFlagGridTooLarge))
       return fail(GD_ERANGE, "gd_dbscan_noalloc: eps-cell grid too large");
-    if (!(bi.flags & gd::kFlagNotSmall)) {
+    if (!gave_up && !(bi.flags & gd::kFlagNotSmall)) {
       if (ctr[gd::kCtrAsymEdges] > (unsigned long long)gd::kAsymCap)
         return fail(GD_ERANGE, "gd_dbscan_noalloc: too many one-directional core neighbour pairs");
       uint32_t K;

@@ -3736,6 +3736,11 @@ cudaError_t small_expand(const Bufs& B, const SmallArgs& A, bool f32, int minpts
                                      args, (size_t)B.nwf * 4, s);
 }
 
+int small_points(const Bufs& B, int n, int dim, double* out, int sms, cudaStream_t s) {
+  k_small_points<<<grid_for(n, 256, sms, 8), 256, 0, s>>>(B, n, dim, out);
+  return 1;
+}
+
 int small_scatter(const Bufs& B, int n, int* out, uint8_t* core_out, int sms, cudaStream_t s) {
   k_small_scatter<<<grid_for(n, 256, sms, 8), 256, 0, s>>>(B, n, out, core_out);
   return 1;

@@ -18,7 +18,7 @@
 //
 // Both kernels are launched cooperatively (every block resident), so the barrier's
 // waits end; they are still bounded, and one that gives up makes its block leave and
-// is reported (kCtrWaitTimeouts).
+// is reported (kCtrWaitTimeouts): the host then takes the general path.
 
 
 constexpr unsigned kBarrierPolls = 1u << 25;  // 2 s and more
@@ -876,5 +876,13 @@ __global__ void k_small_scatter(const gdl::Bufs B, int n, int* __restrict__ out,
     const uint32_t j = B.ids[i];
     out[j] = B.lab[i];
     if (core_out) core_out[j] = B.core[i];
+  }
+}
+
+// the points back in the caller's order
+__global__ void k_small_points(const gdl::Bufs B, int n, int dim, double* __restrict__ out) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const int64_t j = B.ids[i];
+    for (int k = 0; k < dim; ++k) out[j * dim + k] = B.X[(int64_t)i * dim + k];
   }
 }

@@ -10,6 +10,16 @@
 
 #include "gd_launch.h"
 
+// a small index build after which the wait counter is set, where asked for
+namespace gdl {
+int index_gives_up = 0;
+cudaError_t small_index_checked(const Bufs& B, const gd::SmallArgs& A, int sms, cudaStream_t s) {
+  const cudaError_t e = small_index(B, A, sms, s);
+  if (index_gives_up) cudaMemsetAsync(B.ctr + gd::kCtrWaitTimeouts, 1, 1, s);
+  return e;
+}
+}  // namespace gdl
+#define small_index small_index_checked
 #include "gd_api.cu"
 
 namespace {
@@ -76,11 +86,52 @@ void expand_after_a_failed_index() {
   gd_ctx_destroy(c);
 }
 
+std::vector<int32_t> result(gd_ctx* c, int64_t n) {
+  std::vector<int32_t> lab(n);
+  CHECK(gd_get_result(c, lab.data(), nullptr, 0, nullptr, nullptr) == GD_OK);
+  return lab;
+}
+
+// A small run that gives up in its index build or in an expand gets its labels from the
+// general path, and the context goes on working: further expands, then another small run.
+void a_small_run_gives_up() {
+  for (int dim = 2; dim <= 3; ++dim)
+    for (int prec = 0; prec < 2; ++prec) {
+      const int64_t n = 5000;
+      const std::vector<double> p = points(n, dim, dim == 2 ? 40 : 12, 7 + dim);
+      const std::vector<int32_t> w5 = general(p, dim, 0.3, 5), w9 = general(p, dim, 0.3, 9);
+      double* d = static_cast<double*>(on_device(p.data(), p.size() * 8));
+      const gd_points host{p.data(), n, dim, 0}, dev{d, n, dim, 1};
+      gd_ctx* c = nullptr;
+      CHECK(gd_ctx_create(0, &c) == GD_OK);
+      CHECK(gd_ctx_set_precision(c, prec) == GD_OK);
+      gdl::index_gives_up = 1;
+      CHECK(gd_index_build(c, &host, 0.3) == GD_OK && !c->is_small);
+      gdl::index_gives_up = 0;
+      CHECK(gd_expand(c, 5) == GD_OK && result(c, n) == w5);
+      for (const gd_points* g : {&host, &dev}) {
+        CHECK(gd_index_build(c, g, 0.3) == GD_OK && c->is_small);
+        CHECK(gd_expand(c, 9) == GD_OK && result(c, n) == w9 && c->is_small);
+        CHECK(gd_expand(c, 5) == GD_OK);
+        set_counter(c, gd::kCtrWaitTimeouts, 1);
+        if (g->on_device) CHECK(cudaMemset(d, 0, p.size() * 8) == cudaSuccess);
+        CHECK(result(c, n) == w5 && !c->is_small);
+        CHECK(gd_expand(c, 9) == GD_OK && result(c, n) == w9);
+        CHECK(gd_expand(c, 5) == GD_OK && result(c, n) == w5);
+      }
+      std::vector<int32_t> lab(n);
+      CHECK(gd_dbscan(c, &host, 0.3, 9, lab.data(), nullptr) == GD_OK && lab == w9 && c->is_small);
+      cudaFree(d);
+      gd_ctx_destroy(c);
+    }
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
   const std::string name = argc > 1 ? argv[1] : "";
   if (name == "expand_after_a_failed_index") expand_after_a_failed_index();
+  else if (name == "a_small_run_gives_up") a_small_run_gives_up();
   else return 2;
   return bad;
 }
