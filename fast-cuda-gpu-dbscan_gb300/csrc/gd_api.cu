@@ -571,8 +571,32 @@ cudaError_t launch_expand(gd_ctx* ctx, bool capturing) {
   return e;
 }
 
+// The last finished run's statistics, its phase times read from the events when first asked
+// for, or before an expand records the events again.  A small run expands in one kernel, whose
+// time is reported as ms_core.
+const gd_stats& read_stats(gd_ctx* ctx) {
+  gd_stats& S = ctx->st;
+  if (!ctx->times_due) return S;
+  ctx->times_due = false;
+  auto span = [&](int a, int b) {
+    float ms = 0;
+    if (cudaEventElapsedTime(&ms, ctx->ev[a], ctx->ev[b]) == cudaSuccess) return (double)ms;
+    cudaGetLastError();
+    return 0.0;
+  };
+  S.ms_h2d = span(0, 1);
+  S.ms_index = span(1, 2);
+  S.ms_core = span(3, 4);
+  S.ms_union = ctx->is_small ? 0.0 : span(4, 5);
+  S.ms_label = ctx->is_small ? span(4, 6) : span(5, 6);
+  S.ms_d2h = span(6, 7);
+  S.ms_total = S.ms_index + S.ms_core + S.ms_union + S.ms_label;
+  return S;
+}
+
 gd_status expand_run(gd_ctx* ctx) {
   cudaStream_t s = ctx->stream;
+  read_stats(ctx);
   if (ctx->is_small) {
     if (!ctx->fresh_index)
       GD_CUDA(cudaMemsetAsync(ctx->dCtr() + gd::kCtrTests64, 0,
@@ -716,27 +740,6 @@ gd_status finish_run(gd_ctx* ctx, int32_t* labels, uint8_t* is_core, int32_t on_
   }
   ctx->times_due = true;
   return GD_OK;
-}
-
-// The last run's statistics, its phase times read from the events when first asked
-// for.  A small run expands in one kernel, whose time is reported as ms_core.
-const gd_stats& read_stats(gd_ctx* ctx) {
-  gd_stats& S = ctx->st;
-  if (!ctx->times_due) return S;
-  ctx->times_due = false;
-  auto span = [&](int a, int b) {
-    float ms = 0;
-    cudaEventElapsedTime(&ms, ctx->ev[a], ctx->ev[b]);
-    return (double)ms;
-  };
-  S.ms_h2d = span(0, 1);
-  S.ms_index = span(1, 2);
-  S.ms_core = span(3, 4);
-  S.ms_union = ctx->is_small ? 0.0 : span(4, 5);
-  S.ms_label = ctx->is_small ? span(4, 6) : span(5, 6);
-  S.ms_d2h = span(6, 7);
-  S.ms_total = S.ms_index + S.ms_core + S.ms_union + S.ms_label;
-  return S;
 }
 
 // Points of a run on the device: the caller's device pointer, or a copy of
