@@ -99,8 +99,13 @@ struct gd_ctx {
   int tn_core = kDefaultCoreTests, tn_link = kDefaultLinkTests, tn_border = kDefaultBorderTests;
 
   DevBuf coords, inst, chunks, Pv, Bi, bbox, keys0, keys1, vals0, vals1, X, Xf, ent, links, pop, cellent, blklist, nbr,
-      rowtab, hkeys, hvals, reps, bits, core, cellcore, cellmin, cellrep, parent, cellcid, lab, asym,
+      rowtab, hkeys, hvals, reps, bits, core, cellcore, cellrep, parent, cellcid, lab, asym,
       hvcell, hvmask, out, coreout, sorttemp, scantemp, small, kcount;
+  // a small run's
+  struct {
+    DevBuf ptkey, cellkey, ptcell, ids, X, Xf, ent, hkeys, ptpos, pcell, crange, list, bits, core,
+        cellcore, cellmin, cellrep, parent, cellcid, lab, asym, asymwork;
+  } sm;
 
   // the current run
   int stage = 0;  // 0: nothing, 1: indexed, 2: expanded
@@ -120,7 +125,6 @@ struct gd_ctx {
   // a small run (gd_small.cuh): its arguments, and the pinned mirror of the small block
   bool is_small = false;
   gd::SmallArgs sa{};
-  DevBuf asymwork;
   unsigned char* mirror = nullptr;
   // CUDA graph of the expand launches, captured on the second gd_expand of one
   // index build and replayed by later ones (minpts sweeps)
@@ -152,22 +156,29 @@ struct gd_ctx {
     return GD_OK;
   }
 
-  // The buffers of a run and, apart from them, those of its tables (needed before the
-  // run's sizes are known): each set is one allocation, cut into its buffers.  A
-  // buffer that has to grow moves the whole set (nothing in it outlives an index build),
-  // every buffer keeping at least the size it had.  cudaMalloc and cudaFree take 30 us
-  // each and more by their number than by their size (1 GB: in 32 buffers 1065 and
-  // 1408 us, in one 122 and 415 us): the first run of a context on 10M 2D points took
-  // 2541 us with an allocation per buffer and takes 2098 (2M 3D points: 2496, 1952).
-  static constexpr int kRunBufs = 30, kTableBufs = 5;
+  // The buffers of a run, those of its tables (needed before the run's sizes are known) and
+  // those of a small run: each set is one allocation, cut into its buffers.  A buffer that has
+  // to grow moves the whole set (nothing in it outlives an index build), every buffer keeping
+  // at least the size it had.  Small runs have their own set:
+  // a 1,000-point call after a run of 100M points must not move gigabytes for the few buffers
+  // that only small runs ask for.  cudaMalloc and cudaFree take 30 us each and more by their
+  // number than by their size (1 GB: in 32 buffers 1065 and 1408 us, in one 122 and 415 us):
+  // the first run of a context on 10M 2D points took 2541 us with an allocation per buffer and
+  // takes 2098 (2M 3D points: 2496, 1952).
+  static constexpr int kRunBufs = 28, kTableBufs = 5, kSmallBufs = 22;
   DevBuf* const run_set[kRunBufs] = {
       &keys0, &keys1, &vals0,  &vals1,    &X,       &Xf,      &ent,      &links,    &pop,
       &cellent, &blklist, &nbr, &rowtab,  &hkeys,   &hvals,   &reps,     &bits,     &core,
-      &cellcore, &cellmin, &cellrep, &parent, &cellcid, &lab, &asym,     &asymwork, &hvcell,
-      &hvmask, &sorttemp, &scantemp};
+      &cellcore, &cellrep, &parent, &cellcid, &lab, &asym,    &hvcell,   &hvmask,   &sorttemp,
+      &scantemp};
   DevBuf* const table_set[kTableBufs] = {&inst, &chunks, &Pv, &Bi, &bbox};
+  DevBuf* const small_set[kSmallBufs] = {
+      &sm.ptkey, &sm.cellkey, &sm.ptcell, &sm.ids,  &sm.X,        &sm.Xf,      &sm.ent,     &sm.hkeys,
+      &sm.ptpos, &sm.pcell,   &sm.crange, &sm.list, &sm.bits,     &sm.core,    &sm.cellcore, &sm.cellmin,
+      &sm.cellrep, &sm.parent, &sm.cellcid, &sm.lab, &sm.asym,    &sm.asymwork};
   void* run_slab = nullptr;
   void* table_slab = nullptr;
+  void* small_slab = nullptr;
 
   static void drop_set(void*& slab, DevBuf* const* set, int k) {
     if (slab) cudaFree(slab);
@@ -211,6 +222,9 @@ struct gd_ctx {
   gd_status ensure_tables(std::initializer_list<Want> w) {
     return ensure_set(table_slab, table_set, kTableBufs, w, "run tables");
   }
+  gd_status ensure_small(std::initializer_list<Want> w) {
+    return ensure_set(small_slab, small_set, kSmallBufs, w, "small-run buffers");
+  }
 
   void free_all(bool keep_small) {
     DevBuf* a[] = {&coords, &out, &coreout, &kcount, &small};
@@ -221,6 +235,7 @@ struct gd_ctx {
     }
     drop_set(run_slab, run_set, kRunBufs);
     drop_set(table_slab, table_set, kTableBufs);
+    drop_set(small_slab, small_set, kSmallBufs);
   }
 
   // small block (kSmallBlock bytes): M | total clusters | counters | (small runs:) run
@@ -263,7 +278,6 @@ struct gd_ctx {
     B.Xf = static_cast<float*>(Xf.p);
     B.core = static_cast<uint8_t*>(core.p);
     B.cellcore = static_cast<int*>(cellcore.p);
-    B.cellmin = static_cast<int*>(cellmin.p);
     B.cellrep = static_cast<int*>(cellrep.p);
     B.parent = static_cast<int*>(parent.p);
     B.cellcid = static_cast<int*>(cellcid.p);
@@ -282,27 +296,27 @@ struct gd_ctx {
   // the buffers of a small run
   gdl::Bufs small_bufs() {
     gdl::Bufs B;
-    char* sm = static_cast<char*>(small.p);
+    char* blk = static_cast<char*>(small.p);
     B.coords = coords_ptr;
     B.Pv = static_cast<gd::DevParams*>(Pv.p);
-    B.Bi = reinterpret_cast<gd::BatchInfo*>(sm + kBiAt);
-    B.ids = static_cast<uint32_t*>(vals1.p);
-    gdl::set_bits(B, static_cast<uint32_t*>(bits.p), n);
+    B.Bi = reinterpret_cast<gd::BatchInfo*>(blk + kBiAt);
+    B.ids = static_cast<uint32_t*>(sm.ids.p);
+    gdl::set_bits(B, static_cast<uint32_t*>(sm.bits.p), n);
     B.M = dM();
     B.K = dK();
-    B.ent = static_cast<gd::BlockEnt*>(ent.p);
-    B.hkeys = static_cast<unsigned long long*>(hkeys.p);
+    B.ent = static_cast<gd::BlockEnt*>(sm.ent.p);
+    B.hkeys = static_cast<unsigned long long*>(sm.hkeys.p);
     B.hmask = sa.hash_slots - 1;
-    B.X = static_cast<double*>(X.p);
-    B.Xf = static_cast<float*>(Xf.p);
-    B.core = static_cast<uint8_t*>(core.p);
-    B.cellcore = static_cast<int*>(cellcore.p);
-    B.cellmin = static_cast<int*>(cellmin.p);
-    B.parent = static_cast<int*>(parent.p);
-    B.cellcid = static_cast<int*>(cellcid.p);
-    B.lab = static_cast<int*>(lab.p);
+    B.X = static_cast<double*>(sm.X.p);
+    B.Xf = static_cast<float*>(sm.Xf.p);
+    B.core = static_cast<uint8_t*>(sm.core.p);
+    B.cellcore = static_cast<int*>(sm.cellcore.p);
+    B.cellmin = static_cast<int*>(sm.cellmin.p);
+    B.parent = static_cast<int*>(sm.parent.p);
+    B.cellcid = static_cast<int*>(sm.cellcid.p);
+    B.lab = static_cast<int*>(sm.lab.p);
     B.compmin = B.lab;
-    B.asym = static_cast<int*>(asym.p);
+    B.asym = static_cast<int*>(sm.asym.p);
     B.ctr = dCtr();
     B.tn_link = gd::kSmallLinkTests;
     return B;
@@ -344,29 +358,30 @@ gd_status build_small(gd_ctx* ctx) {
   const uint32_t slots = gd::small_hash_slots(n);
   const size_t N = (size_t)n;
   GD_TRY(ctx->ensure_tables({{&ctx->Pv, sizeof(gd::DevParams)}, {&ctx->bbox, (size_t)ctx->sms * 64}}));
-  GD_TRY(ctx->ensure_run({
-      {&ctx->keys0, N * 8},     // point keys
-      {&ctx->keys1, N * 8},     // cell keys
-      {&ctx->vals0, N * 4},     // point cells
-      {&ctx->vals1, N * 4},     // ids
-      {&ctx->X, N * I.dim * 8},
-      {&ctx->Xf, N * (I.dim == 3 ? 16 : 8)},
-      {&ctx->ent, std::max<uint64_t>(dmax, slots) * sizeof(gd::BlockEnt)},
-      {&ctx->hkeys, (uint64_t)slots * 8},
-      {&ctx->cellent, N * 4},   // point places
-      {&ctx->blklist, N * 4},   // position cells
-      {&ctx->hvmask, N * 8},    // cell ranges
-      {&ctx->hvcell, N * 4},    // walk list
-      {&ctx->bits, gdl::bit_layout(n).words * 4},
-      {&ctx->core, N},
-      {&ctx->cellcore, N * 4},
-      {&ctx->cellmin, N * 4},
-      {&ctx->cellrep, N * 4},
-      {&ctx->parent, N * 4},
-      {&ctx->cellcid, N * 4},
-      {&ctx->lab, N * 4},
-      {&ctx->asym, gd::kAsymCap * 8},
-      {&ctx->asymwork, sizeof(gd::AsymWork)},
+  auto& b = ctx->sm;
+  GD_TRY(ctx->ensure_small({
+      {&b.ptkey, N * 8},
+      {&b.cellkey, N * 8},
+      {&b.ptcell, N * 4},
+      {&b.ids, N * 4},
+      {&b.X, N * I.dim * 8},
+      {&b.Xf, N * (I.dim == 3 ? 16 : 8)},
+      {&b.ent, std::max<uint64_t>(dmax, slots) * sizeof(gd::BlockEnt)},
+      {&b.hkeys, (uint64_t)slots * 8},
+      {&b.ptpos, N * 4},
+      {&b.pcell, N * 4},
+      {&b.crange, N * 8},
+      {&b.list, N * 4},
+      {&b.bits, gdl::bit_layout(n).words * 4},
+      {&b.core, N},
+      {&b.cellcore, N * 4},
+      {&b.cellmin, N * 4},
+      {&b.cellrep, N * 4},
+      {&b.parent, N * 4},
+      {&b.cellcid, N * 4},
+      {&b.lab, N * 4},
+      {&b.asym, gd::kAsymCap * 8},
+      {&b.asymwork, sizeof(gd::AsymWork)},
   }));
   ctx->is_small = true;
   char* sm = static_cast<char*>(ctx->small.p);
@@ -380,15 +395,15 @@ gd_status build_small(gd_ctx* ctx) {
   A.hash_slots = slots;
   A.bar = reinterpret_cast<unsigned*>(sm + gd_ctx::kBarAt);
   A.part = static_cast<long long*>(ctx->bbox.p);
-  A.ptkey = static_cast<unsigned long long*>(ctx->keys0.p);
-  A.cellkey = static_cast<uint64_t*>(ctx->keys1.p);
-  A.ptcell = static_cast<uint32_t*>(ctx->vals0.p);
-  A.ptpos = static_cast<uint32_t*>(ctx->cellent.p);
-  A.pcell = static_cast<uint32_t*>(ctx->blklist.p);
-  A.crange = static_cast<uint2*>(ctx->hvmask.p);
-  A.list = static_cast<uint32_t*>(ctx->hvcell.p);
-  A.cellrep = static_cast<uint32_t*>(ctx->cellrep.p);
-  A.asym = static_cast<gd::AsymWork*>(ctx->asymwork.p);
+  A.ptkey = static_cast<unsigned long long*>(b.ptkey.p);
+  A.cellkey = static_cast<uint64_t*>(b.cellkey.p);
+  A.ptcell = static_cast<uint32_t*>(b.ptcell.p);
+  A.ptpos = static_cast<uint32_t*>(b.ptpos.p);
+  A.pcell = static_cast<uint32_t*>(b.pcell.p);
+  A.crange = static_cast<uint2*>(b.crange.p);
+  A.list = static_cast<uint32_t*>(b.list.p);
+  A.cellrep = static_cast<uint32_t*>(b.cellrep.p);
+  A.asym = static_cast<gd::AsymWork*>(b.asymwork.p);
   GD_CUDA(cudaMemsetAsync(sm, 0, gd_ctx::kSmallBlock, s), "clear counters");
   GD_CUDA(gdl::small_index(ctx->small_bufs(), A, ctx->sms, s), "small index launch");
   GD_CUDA(cudaMemcpyAsync(ctx->mirror, sm, gd_ctx::kMirror, cudaMemcpyDeviceToHost, s),

@@ -20,7 +20,16 @@ cudaError_t small_index_checked(const Bufs& B, const gd::SmallArgs& A, int sms, 
 }
 }  // namespace gdl
 #define small_index small_index_checked
+
+// device allocations of more than malloc_limit bytes are refused
+size_t malloc_limit = ~(size_t)0, malloc_calls = 0;
+cudaError_t limited_malloc(void** p, size_t bytes) {
+  ++malloc_calls;
+  return bytes > malloc_limit ? cudaErrorMemoryAllocation : cudaMalloc(p, bytes);
+}
+#define cudaMalloc limited_malloc
 #include "gd_api.cu"
+#undef cudaMalloc
 
 namespace {
 
@@ -126,12 +135,43 @@ void a_small_run_gives_up() {
     }
 }
 
+gd_status batch(gd_ctx* c, const std::vector<double>& p, int dim, double eps, int minpts,
+                std::vector<int32_t>& lab) {
+  lab.assign(p.size() / dim, 0);
+  const gd_instance I{(int64_t)lab.size(), dim, minpts, eps};
+  return gd_batch_dbscan(c, 1, &I, p.data(), 0, lab.data(), nullptr, nullptr);
+}
+
+// A small run leaves a large run's buffers where they are.
+void a_small_run_after_a_large_one() {
+  const std::vector<double> large = points(300000, 3, 60, 3), small = points(1000, 2, 20, 4);
+  gd_ctx* c = nullptr;
+  CHECK(gd_ctx_create(0, &c) == GD_OK);
+  std::vector<int32_t> lab;
+  CHECK(batch(c, large, 3, 0.3, 8, lab) == GD_OK);
+  const void* slab = c->run_slab;
+  const size_t bytes = c->X.bytes;
+  std::vector<int32_t> got(1000);
+  const gd_points g{small.data(), 1000, 2, 0};
+  malloc_calls = 0;
+  malloc_limit = 4 << 20;  // the buffers of 1,000 points
+  CHECK(gd_dbscan(c, &g, 0.3, 5, got.data(), nullptr) == GD_OK && c->is_small);
+  malloc_limit = ~(size_t)0;
+  CHECK(got == general(small, 2, 0.3, 5));
+  CHECK(c->run_slab == slab && c->X.bytes == bytes);
+  malloc_calls = 0;
+  CHECK(batch(c, large, 3, 0.3, 8, lab) == GD_OK && malloc_calls == 0);
+  CHECK(gd_dbscan(c, &g, 0.3, 5, got.data(), nullptr) == GD_OK && malloc_calls == 0);
+  gd_ctx_destroy(c);
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
   const std::string name = argc > 1 ? argv[1] : "";
   if (name == "expand_after_a_failed_index") expand_after_a_failed_index();
   else if (name == "a_small_run_gives_up") a_small_run_gives_up();
+  else if (name == "a_small_run_after_a_large_one") a_small_run_after_a_large_one();
   else return 2;
   return bad;
 }

@@ -31,7 +31,8 @@ def checks(built_lib):
     return run
 
 
-@pytest.mark.parametrize("name", ["expand_after_a_failed_index", "a_small_run_gives_up"])
+@pytest.mark.parametrize("name", ["expand_after_a_failed_index", "a_small_run_gives_up",
+                                  "a_small_run_after_a_large_one"])
 def test_context(checks, name):
     checks("ctx_checks", name)
 
