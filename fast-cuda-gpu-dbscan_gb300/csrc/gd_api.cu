@@ -159,7 +159,7 @@ struct gd_ctx {
   // The buffers of a run, those of its tables (needed before the run's sizes are known) and
   // those of a small run: each set is one allocation, cut into its buffers.  A buffer that has
   // to grow moves the whole set (nothing in it outlives an index build), every buffer keeping
-  // at least the size it had.  Small runs have their own set:
+  // at least the size it had where that still fits the device.  Small runs have their own set:
   // a 1,000-point call after a run of 100M points must not move gigabytes for the few buffers
   // that only small runs ask for.  cudaMalloc and cudaFree take 30 us each and more by their
   // number than by their size (1 GB: in 32 buffers 1065 and 1408 us, in one 122 and 415 us):
@@ -191,15 +191,22 @@ struct gd_ctx {
     bool grow = false;
     for (const Want& w : wants) grow |= w.b->bytes < up256(w.bytes);
     if (!grow) return GD_OK;
-    size_t size[kRunBufs], total = 0;
-    for (int i = 0; i < k; ++i) {
-      size[i] = set[i]->bytes;
-      for (const Want& w : wants)
-        if (w.b == set[i]) size[i] = std::max(size[i], up256(w.bytes));
-      total += size[i];
-    }
+    size_t size[kRunBufs], had[kRunBufs];
+    for (int i = 0; i < k; ++i) had[i] = set[i]->bytes;
     drop_set(slab, set, k);
-    const cudaError_t e = cudaMalloc(&slab, total);
+    cudaError_t e = cudaErrorMemoryAllocation;
+    // where the kept sizes do not fit, the wanted ones alone
+    for (int keep = 1; keep >= 0 && e == cudaErrorMemoryAllocation; --keep) {
+      size_t total = 0;
+      for (int i = 0; i < k; ++i) {
+        size[i] = keep ? had[i] : 0;
+        for (const Want& w : wants)
+          if (w.b == set[i]) size[i] = std::max(size[i], up256(w.bytes));
+        total += size[i];
+      }
+      cudaGetLastError();
+      e = cudaMalloc(&slab, total);
+    }
     if (e != cudaSuccess) {
       slab = nullptr;
       return cuda_fail(e, what);

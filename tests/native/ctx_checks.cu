@@ -165,6 +165,28 @@ void a_small_run_after_a_large_one() {
   gd_ctx_destroy(c);
 }
 
+// A run that fits the device is not refused for the sizes that earlier runs left.
+void kept_sizes_do_not_refuse_a_run() {
+  gd_ctx* c = nullptr;
+  CHECK(gd_ctx_create(0, &c) == GD_OK);
+  std::vector<int32_t> lab;
+  // a hashed 3D grid, then a larger set on a direct 2D grid
+  const std::vector<double> wide = points(200000, 3, 1e5, 5), dense = points(260000, 2, 40, 6);
+  const std::vector<int32_t> want = general(dense, 2, 0.3, 8);
+  gd_ctx* own = nullptr;  // what the second run takes by itself
+  CHECK(gd_ctx_create(0, &own) == GD_OK && batch(own, dense, 2, 0.3, 8, lab) == GD_OK);
+  size_t alone = 0, both = 0;
+  for (DevBuf* b : own->run_set) alone += b->bytes;
+  gd_ctx_destroy(own);
+  CHECK(batch(c, wide, 3, 0.3, 8, lab) == GD_OK);
+  for (DevBuf* b : c->run_set) both += b->bytes;
+  CHECK(both > alone);
+  malloc_limit = alone;
+  CHECK(batch(c, dense, 2, 0.3, 8, lab) == GD_OK && lab == want);
+  malloc_limit = ~(size_t)0;
+  gd_ctx_destroy(c);
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -172,6 +194,7 @@ int main(int argc, char** argv) {
   if (name == "expand_after_a_failed_index") expand_after_a_failed_index();
   else if (name == "a_small_run_gives_up") a_small_run_gives_up();
   else if (name == "a_small_run_after_a_large_one") a_small_run_after_a_large_one();
+  else if (name == "kept_sizes_do_not_refuse_a_run") kept_sizes_do_not_refuse_a_run();
   else return 2;
   return bad;
 }
