@@ -16,7 +16,6 @@
 #include <cstddef>
 #include <cstdio>
 #include <cstring>
-#include <initializer_list>
 #include <string>
 #include <vector>
 
@@ -100,7 +99,7 @@ struct gd_ctx {
 
   DevBuf coords, inst, chunks, Pv, Bi, bbox, keys0, keys1, vals0, vals1, X, Xf, ent, links, pop, cellent, blklist, nbr,
       rowtab, hkeys, hvals, reps, bits, core, cellcore, cellrep, parent, cellcid, lab, asym,
-      hvcell, hvmask, out, coreout, sorttemp, scantemp, small, kcount;
+      out, coreout, sorttemp, scantemp, small, kcount;
   // a small run's
   struct {
     DevBuf ptkey, cellkey, ptcell, ids, X, Xf, ent, hkeys, ptpos, pcell, crange, list, bits, core,
@@ -113,6 +112,7 @@ struct gd_ctx {
   int64_t n = 0;
   int dims = 0;   // bit 0: 2D instances present, bit 1: 3D
   bool f32 = false, key64 = false, xf = false;
+  bool lean = false;  // buffers per cell by the counted cells
   gd::BatchInfo bi{};
   std::vector<gd::InstDesc> hdesc;
   std::vector<gd::Chunk> hchunk;
@@ -165,12 +165,13 @@ struct gd_ctx {
   // number than by their size (1 GB: in 32 buffers 1065 and 1408 us, in one 122 and 415 us):
   // the first run of a context on 10M 2D points took 2541 us with an allocation per buffer and
   // takes 2098 (2M 3D points: 2496, 1952).
-  static constexpr int kRunBufs = 28, kTableBufs = 5, kSmallBufs = 22;
+  // A run whose buffers per cell do not fit the device at one per point gets them after its
+  // cells are counted (lean), in a fourth allocation.
+  static constexpr int kRunBufs = 26, kTableBufs = 5, kSmallBufs = 22;
   DevBuf* const run_set[kRunBufs] = {
       &keys0, &keys1, &vals0,  &vals1,    &X,       &Xf,      &ent,      &links,    &pop,
       &cellent, &blklist, &nbr, &rowtab,  &hkeys,   &hvals,   &reps,     &bits,     &core,
-      &cellcore, &cellrep, &parent, &cellcid, &lab, &asym,    &hvcell,   &hvmask,   &sorttemp,
-      &scantemp};
+      &cellcore, &cellrep, &parent, &cellcid, &lab, &asym,    &sorttemp, &scantemp};
   DevBuf* const table_set[kTableBufs] = {&inst, &chunks, &Pv, &Bi, &bbox};
   DevBuf* const small_set[kSmallBufs] = {
       &sm.ptkey, &sm.cellkey, &sm.ptcell, &sm.ids,  &sm.X,        &sm.Xf,      &sm.ent,     &sm.hkeys,
@@ -179,6 +180,8 @@ struct gd_ctx {
   void* run_slab = nullptr;
   void* table_slab = nullptr;
   void* small_slab = nullptr;
+  void* cell_slab = nullptr;  // a lean run's buffers per cell
+  int64_t cells_cap = 0, heavy_cap = 0;  // cells / heavy-list entries the run's buffers hold
 
   static void drop_set(void*& slab, DevBuf* const* set, int k) {
     if (slab) cudaFree(slab);
@@ -186,7 +189,7 @@ struct gd_ctx {
     for (int i = 0; i < k; ++i) *set[i] = DevBuf{};
   }
 
-  gd_status ensure_set(void*& slab, DevBuf* const* set, int k, std::initializer_list<Want> wants,
+  gd_status ensure_set(void*& slab, DevBuf* const* set, int k, const std::vector<Want>& wants,
                        const char* what) {
     bool grow = false;
     for (const Want& w : wants) grow |= w.b->bytes < up256(w.bytes);
@@ -194,6 +197,8 @@ struct gd_ctx {
     size_t size[kRunBufs], had[kRunBufs];
     for (int i = 0; i < k; ++i) had[i] = set[i]->bytes;
     drop_set(slab, set, k);
+    if (set == run_set && cell_slab) cudaFree(cell_slab);
+    if (set == run_set) cell_slab = nullptr;
     cudaError_t e = cudaErrorMemoryAllocation;
     // where the kept sizes do not fit, the wanted ones alone
     for (int keep = 1; keep >= 0 && e == cudaErrorMemoryAllocation; --keep) {
@@ -223,13 +228,31 @@ struct gd_ctx {
       GD_CUDA(cudaMemsetAsync(scantemp.p, 0, scantemp.bytes, stream), what);
     return GD_OK;
   }
-  gd_status ensure_run(std::initializer_list<Want> w) {
+  gd_status ensure_run(const std::vector<Want>& w) {
     return ensure_set(run_slab, run_set, kRunBufs, w, "run buffers");
   }
-  gd_status ensure_tables(std::initializer_list<Want> w) {
+  // buffers of run_set that it left out
+  gd_status ensure_cells(const std::vector<Want>& wants) {
+    size_t total = 0;
+    for (const Want& w : wants) total += up256(w.bytes);
+    if (cell_slab) cudaFree(cell_slab);
+    cell_slab = nullptr;
+    const cudaError_t e = cudaMalloc(&cell_slab, total);
+    if (e != cudaSuccess) {
+      cell_slab = nullptr;
+      return cuda_fail(e, "cell buffers");
+    }
+    char* at = static_cast<char*>(cell_slab);
+    for (const Want& w : wants) {
+      *w.b = DevBuf{up256(w.bytes) ? at : nullptr, up256(w.bytes)};
+      at += up256(w.bytes);
+    }
+    return GD_OK;
+  }
+  gd_status ensure_tables(const std::vector<Want>& w) {
     return ensure_set(table_slab, table_set, kTableBufs, w, "run tables");
   }
-  gd_status ensure_small(std::initializer_list<Want> w) {
+  gd_status ensure_small(const std::vector<Want>& w) {
     return ensure_set(small_slab, small_set, kSmallBufs, w, "small-run buffers");
   }
 
@@ -241,6 +264,8 @@ struct gd_ctx {
       *b = DevBuf{};
     }
     drop_set(run_slab, run_set, kRunBufs);
+    if (cell_slab) cudaFree(cell_slab);
+    cell_slab = nullptr;
     drop_set(table_slab, table_set, kTableBufs);
     drop_set(small_slab, small_set, kSmallBufs);
   }
@@ -272,7 +297,7 @@ struct gd_ctx {
     B.ckeys = skeys == keys0.p ? keys1.p : keys0.p;
     B.ent = static_cast<gd::BlockEnt*>(ent.p);
     B.links = static_cast<gd::BlockLinks*>(links.p);
-    B.pop = f32 ? static_cast<gd::BlockPop*>(pop.p) : nullptr;
+    B.pop = f32 && !lean ? static_cast<gd::BlockPop*>(pop.p) : nullptr;
     B.ent_base = (uint32_t)bi.ent_total;
     B.cellent = static_cast<uint32_t*>(cellent.p);
     B.blklist = static_cast<uint32_t*>(blklist.p);
@@ -290,9 +315,11 @@ struct gd_ctx {
     B.cellcid = static_cast<int*>(cellcid.p);
     B.lab = static_cast<int*>(lab.p);
     B.asym = static_cast<int*>(asym.p);
-    B.hv_cell = static_cast<int*>(hvcell.p);
     B.compmin = B.lab;
-    B.hv_mask = static_cast<unsigned long long*>(hvmask.p);
+    // the links between k_core_cells and k_flood, the heavy lists before and after
+    B.hv_mask = static_cast<unsigned long long*>(links.p);
+    B.hv_cell = reinterpret_cast<int*>(B.hv_mask + heavy_cap);
+    B.cells = cells_cap;
     B.ctr = dCtr();
     B.tn_core = tn_core;
     B.tn_link = tn_link;
@@ -487,23 +514,17 @@ gd_status build_run(gd_ctx* ctx, uint64_t dense_floor, uint64_t rows_floor) {
   const int key_bits = bi.LB + bi.IB;
   gdprim::SortChunks sc;
   if (K > 1 && gdprim::sort_by_instance(n, nch, bi.LB, key_bits)) sc.count = nch;
-  const size_t N = (size_t)n, nent = bi.ent_total + (direct_only ? 0 : N);
+  const size_t N = (size_t)n;
   uint64_t hcap = 1024;
   while (bi.any_sparse && hcap < 2 * (uint64_t)n) hcap <<= 1;
   ctx->hmask = (uint32_t)(hcap - 1);
-  GD_TRY(ctx->ensure_run({
+  std::vector<Want> wants = {
       {&ctx->keys0, N * kw},
       {&ctx->keys1, N * kw},
       {&ctx->vals0, N * 4},
       {&ctx->vals1, N * 4},
       {&ctx->X, N * maxd * 8},
       {&ctx->Xf, ctx->xf ? N * (maxd == 3 ? 16 : 8) : 0},
-      {&ctx->ent, nent * sizeof(gd::BlockEnt)},
-      {&ctx->links, nent * sizeof(gd::BlockLinks)},
-      {&ctx->pop, ctx->f32 ? nent * sizeof(gd::BlockPop) : 0},
-      {&ctx->cellent, N * 4},
-      {&ctx->blklist, N * 4},
-      {&ctx->nbr, direct_only ? 0 : N * 4 * sizeof(uint2)},
       {&ctx->rowtab, std::max<uint64_t>(1, bi.row_total) * 8},
       {&ctx->hkeys, bi.any_sparse ? hcap * 8 : 0},
       {&ctx->hvals, bi.any_sparse ? hcap * 8 : 0},
@@ -514,15 +535,43 @@ gd_status build_run(gd_ctx* ctx, uint64_t dense_floor, uint64_t rows_floor) {
                                 gdprim::scan_temp_bytes(gdprim::sort_scan_elems(n, sc.count)))},
       // the expand stage's
       {&ctx->core, N},
-      {&ctx->cellcore, N * 4},
-      {&ctx->cellrep, N * 4},
-      {&ctx->parent, N * 4},
-      {&ctx->cellcid, N * 4},
       {&ctx->lab, N * 4},
       {&ctx->asym, gd::kAsymCap * 8},
-      {&ctx->hvcell, N * 4},  // heavy work
-      {&ctx->hvmask, N * 8},
-  }));
+  };
+  // The buffers per cell, for up to C cells.  A heavy list takes a cell once per 32 entries of
+  // a walk list that hold it: a point's each at most, and no more than two launches' (3D core
+  // walk) passes and cells.
+  auto per_cell = [&](int64_t C) {
+    ctx->cells_cap = C;
+    ctx->heavy_cap = std::min<int64_t>(n, 2 * C + n / 16 + 128);
+    const size_t c = (size_t)C, nent = bi.ent_total + (direct_only ? 0 : c);
+    return std::vector<Want>{
+        {&ctx->ent, nent * sizeof(gd::BlockEnt)},
+        {&ctx->links, std::max(nent * sizeof(gd::BlockLinks), (size_t)ctx->heavy_cap * 12)},
+        {&ctx->pop, ctx->f32 && !ctx->lean ? nent * sizeof(gd::BlockPop) : 0},
+        {&ctx->nbr, direct_only ? 0 : c * 4 * sizeof(uint2)},
+        {&ctx->cellent, c * 4},
+        {&ctx->blklist, c * 4},
+        {&ctx->cellcore, c * 4},
+        {&ctx->cellrep, c * 4},
+        {&ctx->parent, c * 4},
+        {&ctx->cellcid, c * 4},
+    };
+  };
+  ctx->lean = false;
+  {
+    // room for a cell per point, where it fits the device (counting the cells first would
+    // cost a synchronisation)
+    std::vector<Want> all = wants;
+    for (const Want& w : per_cell(n)) all.push_back(w);
+    const gd_status st = ctx->ensure_run(all);
+    if (st == GD_ENOMEM) {
+      ctx->lean = true;
+      GD_TRY(ctx->ensure_run(wants));
+    } else if (st != GD_OK) {
+      return st;
+    }
+  }
   const int sort_bits = sc.count ? bi.LB : key_bits;
   if (sc.count) {
     sc.chunks = static_cast<const gd::Chunk*>(ctx->chunks.p);
@@ -549,6 +598,19 @@ gd_status build_run(gd_ctx* ctx, uint64_t dense_floor, uint64_t rows_floor) {
   B = ctx->bufs();
   L += gdl::gather(B, ctx->key64, n, ctx->xf, K == 1, ctx->sms, s);
   L += gdl::runs(B, ctx->key64, n, ctx->scantemp.p, s);
+  if (ctx->lean) {
+    GD_CUDA(cudaMemcpyAsync(ctx->mirror, ctx->small.p, gd_ctx::kBiAt, cudaMemcpyDeviceToHost, s),
+            "count cells");
+    GD_CUDA(cudaStreamSynchronize(s), "count cells");
+    const unsigned long long* ctr = reinterpret_cast<const unsigned long long*>(ctx->mirror + 128);
+    if (ctr[gd::kCtrWaitTimeouts]) {
+      cudaMemsetAsync(ctx->scantemp.p, 0, ctx->scantemp.bytes, s);
+      cudaStreamSynchronize(s);
+      return fail(GD_ECUDA, "a scan or sort look-back wait gave up (results discarded)");
+    }
+    GD_TRY(ctx->ensure_cells(per_cell((int64_t)ctr[gd::kCtrCells])));
+    B = ctx->bufs();
+  }
   // block entries and row lookups
   if (bi.ent_total)
     GD_CUDA(cudaMemsetAsync(ctx->ent.p, 0, bi.ent_total * sizeof(gd::BlockEnt), s), "clear blocks");

@@ -42,6 +42,7 @@ struct Bufs {
   int64_t nwf = 0;              // words of fbits
   const void* ckeys = nullptr;  // per non-empty cell: its key (same width as keys)
   uint32_t* blklist = nullptr;  // a core cell of every block holding one
+  int64_t cells = 0;            // cells that the buffers per cell hold
   uint32_t* cellent = nullptr;  // per non-empty cell: its block's entry
   gd::BlockEnt* ent = nullptr;  // block entries: direct tables first, then (from ent_base)
   gd::BlockLinks* links = nullptr;  // per entry, as ent
@@ -70,7 +71,7 @@ struct Bufs {
                                 // positions or cells, 2D instances' first), capacity n
   uint32_t* lcount = nullptr;   // device scalar: list length (lpre[nw])
   uint32_t* K = nullptr;        // device scalar: clusters of the run
-  int* hv_cell = nullptr;       // heavy-work list: cell index m (capacity n)
+  int* hv_cell = nullptr;       // heavy-work list: cell index m
   unsigned long long* hv_mask = nullptr;  // heavy-work list: stencil offsets still open
   unsigned long long* ctr = nullptr;      // gd::Counter
   // pair-test budgets of one thread before its work goes to a warp kernel

@@ -353,6 +353,7 @@ extern "C" gd_status gd_dbscan_noalloc(const double* coords_dev, int64_t n, int3
   B.X = reinterpret_cast<double*>(base + kOffX);
   B.Xf = reinterpret_cast<float*>(base + kOffXf);
   B.reps = reinterpret_cast<int*>(base + kOffReps);
+  B.cells = n;
   B.cellent = reinterpret_cast<uint32_t*>(base + kOffCellent);
   B.blklist = reinterpret_cast<uint32_t*>(base + kOffBlklist);
   B.nbr = bi.row_total || bi.any_sparse ? reinterpret_cast<uint2*>(base + kOffNbr) : nullptr;

@@ -3602,7 +3602,7 @@ static int per_dim(int dims) { return ((dims & 1) ? 1 : 0) + ((dims & 2) ? 1 : 0
 int core(const Bufs& B, int64_t n, int dims, bool f32, bool key64, bool one, bool fresh, int sms,
          void* scan_temp, cudaStream_t s) {
   cudaMemsetAsync(B.ctr + kCtrHeavyCore, 0, 8, s);
-  cudaMemsetAsync(B.cellcore, 0, (size_t)n * 4, s);  // per-cell core counts
+  cudaMemsetAsync(B.cellcore, 0, (size_t)B.cells * 4, s);  // per-cell core counts
   // dense cells at once; the other points listed in sorted order for the walk
   const int g = grid_for(n, 256, sms, 8);
   const int chunk = f32 ? kCoreChunk : 1;

@@ -187,6 +187,76 @@ void kept_sizes_do_not_refuse_a_run() {
   gd_ctx_destroy(c);
 }
 
+// A run whose buffers do not fit at a cell per point gets them by the counted cells: same
+// labels over direct, row-table and hashed grids and a mixed batch, for repeated expands, and
+// with every walk handed to the warp kernels (the heavy lists' size).
+void buffers_by_the_counted_cells() {
+  struct Case { int64_t n; int dim; double side; };
+  for (int prec = 0; prec < 2; ++prec)
+    for (const Case& k : {Case{300000, 2, 100}, Case{300000, 2, 3e6}, Case{150000, 3, 40},
+                          Case{150000, 3, 3e3}, Case{150000, 3, 1e5}})
+      for (int warps = 0; warps < 2; ++warps) {
+        const std::vector<double> p = points(k.n, k.dim, k.side, 11);
+        const gd_points g{p.data(), k.n, k.dim, 0};
+        gd_ctx* c = nullptr;
+        CHECK(gd_ctx_create(0, &c) == GD_OK && gd_ctx_set_precision(c, prec) == GD_OK);
+        if (warps) {
+          const gd_tuning t{0, 0, 0, 0, 0, 0};
+          CHECK(gd_ctx_set_tuning(c, &t) == GD_OK);
+        }
+        std::vector<int32_t> want[3];
+        const int mp[3] = {8, 4, 20};
+        CHECK(gd_index_build(c, &g, 0.3) == GD_OK && !c->is_small && !c->lean);
+        for (int e = 0; e < 3; ++e) {
+          CHECK(gd_expand(c, mp[e]) == GD_OK);
+          want[e] = result(c, k.n);
+        }
+        size_t all = 0;
+        for (DevBuf* b : c->run_set) all += b->bytes;
+        CHECK(gd_ctx_trim(c) == GD_OK);
+        malloc_limit = all - 1;
+        CHECK(gd_index_build(c, &g, 0.3) == GD_OK && c->lean && c->cells_cap < k.n);
+        for (int e = 0; e < 3; ++e) {
+          CHECK(gd_expand(c, mp[e]) == GD_OK);
+          CHECK(result(c, k.n) == want[e]);
+        }
+        // the room is there again
+        malloc_limit = ~(size_t)0;
+        CHECK(gd_index_build(c, &g, 0.3) == GD_OK && (!c->lean || prec == 0));
+        CHECK(gd_expand(c, 8) == GD_OK && result(c, k.n) == want[0]);
+        gd_ctx_destroy(c);
+      }
+  // a batch of both dimensions and all three lookups
+  std::vector<double> p;
+  std::vector<gd_instance> inst;
+  for (int i = 0; i < 24; ++i) {
+    const int dim = 2 + i % 2;
+    const double side[2][3] = {{30, 2e4, 3e6}, {30, 150, 2e4}};
+    const std::vector<double> q = points(3000 + 997 * i, dim, side[dim - 2][i / 2 % 3], i);
+    inst.push_back({(int64_t)q.size() / dim, dim, 5 + i % 3, 0.3});
+    p.insert(p.end(), q.begin(), q.end());
+  }
+  int64_t n = 0;
+  for (const gd_instance& i : inst) n += i.n;
+  for (int prec = 0; prec < 2; ++prec) {
+    gd_ctx* c = nullptr;
+    CHECK(gd_ctx_create(0, &c) == GD_OK && gd_ctx_set_precision(c, prec) == GD_OK);
+    std::vector<int32_t> want(n), lab(n);
+    auto run = [&](std::vector<int32_t>& out) {
+      return gd_batch_dbscan(c, (int)inst.size(), inst.data(), p.data(), 0, out.data(), nullptr,
+                             nullptr);
+    };
+    CHECK(run(want) == GD_OK && !c->lean);
+    size_t all = 0;
+    for (DevBuf* b : c->run_set) all += b->bytes;
+    CHECK(gd_ctx_trim(c) == GD_OK);
+    malloc_limit = all - 1;
+    CHECK(run(lab) == GD_OK && c->lean && lab == want);
+    malloc_limit = ~(size_t)0;
+    gd_ctx_destroy(c);
+  }
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -195,6 +265,7 @@ int main(int argc, char** argv) {
   else if (name == "a_small_run_gives_up") a_small_run_gives_up();
   else if (name == "a_small_run_after_a_large_one") a_small_run_after_a_large_one();
   else if (name == "kept_sizes_do_not_refuse_a_run") kept_sizes_do_not_refuse_a_run();
+  else if (name == "buffers_by_the_counted_cells") buffers_by_the_counted_cells();
   else return 2;
   return bad;
 }
