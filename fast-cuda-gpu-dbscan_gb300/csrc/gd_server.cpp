@@ -39,9 +39,10 @@ double ms_since(Clock::time_point t0, Clock::time_point t) {
   return std::chrono::duration<double, std::milli>(t - t0).count();
 }
 
-// device bytes one point of a request may need during a run (buffers of the
-// build and expand stages, cell tables and row hash, generously rounded)
-constexpr int64_t kBytesPerPoint = 320;
+// device bytes one point of a request may need during a run: coordinates and label 28, sort,
+// sorted copies and per-point state 76, a cell slot 24 + 104, its block of a direct table 72 or
+// its rows 64, the row hash that the batch shares 64 (3D, float32 mode, 64-bit keys: 368)
+constexpr int64_t kBytesPerPoint = 384;
 constexpr int64_t kBytesPerRequest = 1 << 16;
 
 struct Request {

@@ -30,6 +30,7 @@ cudaError_t limited_malloc(void** p, size_t bytes) {
 #define cudaMalloc limited_malloc
 #include "gd_api.cu"
 #undef cudaMalloc
+#include "gd_server.cpp"
 
 namespace {
 
@@ -257,6 +258,44 @@ void buffers_by_the_counted_cells() {
   }
 }
 
+// The server admits requests by an estimate of their device memory, which a batch's buffers
+// must not pass: every lookup alone, and mixed so that most instances have a direct table and
+// the batch still holds slots and a row hash.
+void server_estimate() {
+  for (int prec = 0; prec < 2; ++prec)
+    for (int mix = 0; mix < 5; ++mix) {
+      std::vector<double> p;
+      std::vector<gd_instance> inst;
+      for (int i = 0; i < 40; ++i) {
+        const int dim = 3, n = 13200;  // (the row hash has almost four slots per point)
+        // blocks of just below one per point: direct; rows below 8 per point: table; else hash
+        const double block = 4 * 0.3 / std::sqrt(3.0), direct = 22.9 * block, rows = 323 * block;
+        const double side = mix == 0   ? direct
+                            : mix == 1 ? rows
+                            : mix == 2 ? 2e4
+                            : mix == 3 ? (i ? direct : 2e4)
+                                       : (i ? rows : 2e4);
+        std::mt19937_64 g(i);
+        std::uniform_real_distribution<double> u(0, side);
+        for (int k = 0; k < n * dim; ++k) p.push_back(u(g));
+        inst.push_back({n, dim, 5, 0.3});
+      }
+      const int64_t n = (int64_t)p.size() / 3;
+      std::vector<int32_t> lab(n);
+      gd_ctx* c = nullptr;
+      CHECK(gd_ctx_create(0, &c) == GD_OK && gd_ctx_set_precision(c, prec) == GD_OK);
+      CHECK(gd_batch_dbscan(c, (int)inst.size(), inst.data(), p.data(), 0, lab.data(), nullptr,
+                            nullptr) == GD_OK);
+      size_t bytes = c->coords.bytes + c->out.bytes;
+      for (DevBuf* b : c->run_set) bytes += b->bytes;
+      for (DevBuf* b : c->table_set) bytes += b->bytes;
+      std::printf("precision %d mix %d: %.1f bytes per point\n", prec, mix, (double)bytes / n);
+      CHECK((int64_t)bytes <= n * kBytesPerPoint + (int64_t)inst.size() * kBytesPerRequest);
+      CHECK((mix == 0) == (c->bi.row_total == 0 && !c->bi.any_sparse));
+      gd_ctx_destroy(c);
+    }
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -266,6 +305,7 @@ int main(int argc, char** argv) {
   else if (name == "a_small_run_after_a_large_one") a_small_run_after_a_large_one();
   else if (name == "kept_sizes_do_not_refuse_a_run") kept_sizes_do_not_refuse_a_run();
   else if (name == "buffers_by_the_counted_cells") buffers_by_the_counted_cells();
+  else if (name == "server_estimate") server_estimate();
   else return 2;
   return bad;
 }

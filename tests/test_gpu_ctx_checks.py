@@ -34,7 +34,8 @@ def checks(built_lib):
 @pytest.mark.parametrize("name", ["expand_after_a_failed_index", "a_small_run_gives_up",
                                   "a_small_run_after_a_large_one",
                                   "kept_sizes_do_not_refuse_a_run",
-                                  "buffers_by_the_counted_cells"])
+                                  "buffers_by_the_counted_cells",
+                                  "server_estimate"])
 def test_context(checks, name):
     checks("ctx_checks", name)
 
