@@ -369,7 +369,7 @@ __global__ void k_params_inst(const gdl::Bufs B, int K, double mult2, double mul
 __global__ void __launch_bounds__(1024) k_layout(const gdl::Bufs B, int K) {
   __shared__ unsigned long long s_part[32], s_part2[32];
   __shared__ int s_red[5][32];
-  __shared__ unsigned long long s_carry, s_carry2, s_cells;
+  __shared__ unsigned long long s_carry, s_carry2;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   int lb = 0, cb = 0, fl = 0, sp = 0, xf = 0, md = 2, k2 = 0;
   for (int i = threadIdx.x; i < K; i += blockDim.x) {
@@ -430,13 +430,14 @@ __global__ void __launch_bounds__(1024) k_layout(const gdl::Bufs B, int K) {
     *B.Bi = bi;
     s_carry = 0;
     s_carry2 = 0;
-    s_cells = 0;
   }
   __syncthreads();
   const int LB = B.Bi->LB;
   const uint64_t kmask = LB >= 64 ? ~0ull : ((1ull << LB) - 1ull);
   // exclusive scans of the table sizes, 1024 instances at a time: block entries
-  // of direct tables, rows of row tables (none for the hash)
+  // of direct tables, rows of row tables (none for the hash).  Their totals give the grid's
+  // cells too (20,000 instances: 114 us; with a shared 64-bit atomic per instance for those
+  // cells 805).
   for (int base = 0; base < K; base += 1024) {
     const int i = base + threadIdx.x;
     unsigned long long vo = 0, vs = 0;
@@ -444,7 +445,6 @@ __global__ void __launch_bounds__(1024) k_layout(const gdl::Bufs B, int K) {
       const DevParams& p = B.Pv[i];
       vo = p.sparse == 0 ? p.NB : 0;
       vs = p.sparse == 2 ? p.rows : 0;
-      if (p.sparse != 1) atomicAdd(&s_cells, (vo << kBlockBits) + vs);
     }
     unsigned long long io = vo, is = vs;
 #pragma unroll
@@ -493,7 +493,7 @@ __global__ void __launch_bounds__(1024) k_layout(const gdl::Bufs B, int K) {
   if (threadIdx.x == 0) {
     B.Bi->ent_total = s_carry;
     B.Bi->row_total = s_carry2;
-    B.Bi->grid_cells = s_cells;
+    B.Bi->grid_cells = (s_carry << kBlockBits) + s_carry2;
   }
 }
 
