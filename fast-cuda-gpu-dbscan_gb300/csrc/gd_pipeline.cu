@@ -1910,8 +1910,12 @@ __global__ void k_core_split(const gdl::Bufs B, int64_t n, int chunk, int clear)
 // classified first, as a whole and per point (wholly inside eps: count, wholly
 // outside: skip; from 1, 2, 5 points on the batch's core phase took 20.7, 20.1 and 18.7
 // ms, from 8 on 18.4, and no less beyond).
-// A chunk whose tests pass the budget sends its cell to the warp kernel, which
-// recomputes the whole cell.  Per-cell core counts are atomics (cleared before the
+// A chunk whose tests pass its budget sends its cell to the warp kernel, which
+// recomputes the whole cell.  The budget counts every candidate (most cells are not classified
+// first), so it is kCellBudget times the context's per point: a whole 3D stencil of 8 points per
+// cell.  (2M 3D points, uniform, 4 per cell, minPts 87, the mean neighbour count: core phase
+// 3.91 ms at one times the budget, 2.55 at two, four, eight and sixteen; 9 per cell: 6.03, 6.02,
+// 3.98, 3.97, 3.97.)  Per-cell core counts are atomics (cleared before the
 // launch).
 //
 // Passes [p0, p1).  3D runs pass 0 for every listed chunk first: a chunk with an
@@ -1923,6 +1927,7 @@ __global__ void k_core_split(const gdl::Bufs B, int64_t n, int chunk, int clear)
 #endif
 constexpr int kCoreChunk = GD_CORE_CHUNK;
 constexpr int kCoreBigCell = 8;
+constexpr int kCellBudget = 4;
 constexpr int kDecided = 0x3fffffff;
 template <int D, bool KEY64>
 __global__ void __launch_bounds__(kCoreThreads, kCoreCellMinBlocks)
@@ -1995,7 +2000,7 @@ k_core_cell(const gdl::Bufs B, int64_t n, int p0, int p1) {
           st.w5[k] = near << ((cc.c[k] - 2) & (St::SIDE - 1));
         }
       }
-      int budget = B.tn_core * present;
+      int budget = kCellBudget * B.tn_core * present;
       bool done = present == 0;
       // one occupied cell: place `bit` of block (row r, half h) of the stencil
       auto visit = [&](int q0, int qe, int bit, int r, int h) {
