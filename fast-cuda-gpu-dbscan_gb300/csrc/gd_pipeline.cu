@@ -2650,7 +2650,11 @@ k_union_scan(const gdl::Bufs B, int64_t n, int pass) {
 // expansion queries from the core point).  Cells whose id cannot improve on
 // the best so far are skipped; with classification, a cell wholly inside eps
 // gives its id without tests and one wholly outside is skipped.  A point whose
-// tests pass the budget sends its cell to the warp kernel.
+// tests pass the budget sends its cell to the warp kernel.  The own block comes first: in it
+// lie most of the near cells, whose first hit settles all cells of the same cluster (2M 3D
+// points, 4 per cell, half of them border points: label phase 646 us in block order, 389 so,
+// float64 mode 1841 and 874; cells within one of the own first in every block 344 and 514, but
+// 48.4 -> 50.8 ms on 4,096 instances, most of whose points are noise).
 template <int D, bool F32, bool KEY64>
 __global__ void __launch_bounds__(kBorderThreads, kBorderMinBlocks) k_border_point(const gdl::Bufs B, int64_t n) {
   using St = Stencil<D>;
@@ -2705,12 +2709,17 @@ __global__ void __launch_bounds__(kBorderThreads, kBorderMinBlocks) k_border_poi
         }
       }
       int best = INT_MAX, budget = B.tn_border;
-      // the blocks with core cells in the stencil, then their cells
+      // the blocks with core cells in the stencil, the own block's row and half first, then
+      // their cells
       StencilWords<D> W5;
       W5.init(st.w5);
       int ni = 0;
       uint32_t codes = 0;
-      for (int r = 0; r < St::ROWS; ++r) {
+      const int home = D == 3 ? ((cc.c[0] >> St::S) - st.b0[0]) * 2 + (cc.c[1] >> St::S) - st.b0[1]
+                              : (cc.c[0] >> St::S) - st.b0[0];
+      const int hz = (cc.c[D - 1] >> St::S) - st.b0[D - 1];
+      for (int tt = 0; tt < St::ROWS; ++tt) {
+        const int r = tt ^ home;
         const int64_t row = st.row(r, P);
         if (row < 0) continue;
         uint2 mk[2];
@@ -2722,13 +2731,16 @@ __global__ void __launch_bounds__(kBorderThreads, kBorderMinBlocks) k_border_poi
 #pragma unroll
         for (int h = 0; h < 2; ++h) w[h] = e[h] != kNoEnt ? B.ent[e[h]].core & u64_of(mk[h]) : 0ull;
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
-          if (w[h]) {
-            siw[ni][threadIdx.x] = w[h];
-            sie[ni][threadIdx.x] = e[h];
+        for (int g = 0; g < 2; ++g) {
+          const int h = g ^ hz;
+          const unsigned long long wh = h ? w[1] : w[0];
+          if (wh) {
+            siw[ni][threadIdx.x] = wh;
+            sie[ni][threadIdx.x] = h ? e[1] : e[0];
             codes |= (uint32_t)(2 * r + h) << (4 * ni);
             ++ni;
           }
+        }
       }
       unsigned long long w = 0, occ = 0;
       uint32_t base = 0;
