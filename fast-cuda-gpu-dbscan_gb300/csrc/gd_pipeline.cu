@@ -1915,7 +1915,10 @@ __global__ void k_core_split(const gdl::Bufs B, int64_t n, int chunk, int clear)
 // first), so it is kCellBudget times the context's per point: a whole 3D stencil of 8 points per
 // cell.  (2M 3D points, uniform, 4 per cell, minPts 87, the mean neighbour count: core phase
 // 3.91 ms at one times the budget, 2.55 at two, four, eight and sixteen; 9 per cell: 6.03, 6.02,
-// 3.98, 3.97, 3.97.)  Per-cell core counts are atomics (cleared before the
+// 3.98, 3.97, 3.97.)  A cell of more than a quarter of the budget that is not settled whole goes
+// to the warp kernel at once: its points are a long serial chain (200 clumps of 5,000 2D points,
+// spread 0.05 to 5 at eps 0.5, minPts 5 and 50: 376 and 1142 us without the rule, 136 and 255
+// from 64 points on, 144 and 284 from 128, 133 and 245 from 32, which costs even sets 1 to 8 %.)  Per-cell core counts are atomics (cleared before the
 // launch).
 //
 // Passes [p0, p1).  3D runs pass 0 for every listed chunk first: a chunk with an
@@ -2039,6 +2042,7 @@ k_core_cell(const gdl::Bufs B, int64_t n, int p0, int p1) {
             return;
           }
         }
+        if (qe - q0 > B.tn_core / 4) budget = 0;  // a crowded cell is a warp's work
         for (int q = q0; q < qe; ++q) {
           budget -= present;
           if (budget < 0) {
@@ -2170,8 +2174,11 @@ k_core_cell(const gdl::Bufs B, int64_t n, int p0, int p1) {
 // undecided cells cannot lift its count to minpts is no core point, untested.
 // Then the warp pools: each lane hands out its open candidates one at a time into
 // the warp's pair buffer until its count reaches minpts, and whenever the buffer
-// holds 32 pairs the warp tests them, a lane per pair.  A warp whose open
-// candidates pass 32 budgets sends its cells to the warp kernel.
+// holds 32 pairs the warp tests them, a lane per pair.  A point whose own open candidates pass
+// the budget sends its cell to the warp kernel, and so does a warp whose candidates pass 32 of
+// them.  (200 clumps of 5,000 2D points, spread 0.05 to 5 at eps 0.5, minPts 5 and 50: core phase
+// 851 and 1126 us with the warp's rule alone, a few lanes handing out thousands; 194 and 443 so,
+// 223 and 491 at twice the budget.)
 // Passes as in k_core_cell (2D: both in one walk).
 // a lane's open candidates are counted up to this many (32 lanes' sum fits an int)
 constexpr int kPoolCap = 0x03ffffff;
@@ -2326,13 +2333,15 @@ k_core_point(const gdl::Bufs B, int64_t n, int p0, int p1) {
       if (cnt >= minpts || (!split && ptot < kPoolCap && cnt + ptot < minpts)) ni = 0;
       if (ni == 0) ptot = 0;
     }
-    // ---- pooled tests
-    bool over = false;
+    // ---- pooled tests; a lane hands out one candidate per step, so that one of more than a
+    // budget of its own would keep the warp (its cell goes to the warp kernel)
+    bool over = ptot > B.tn_core;
+    if (over) ni = ptot = 0;
     int pool = ptot;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) pool += __shfl_xor_sync(kFull, pool, o);
     if (pool > 32 * B.tn_core) {  // too much for the warp: the warp kernel takes the cells
-      over = ni > 0;
+      over = over || ni > 0;
       ni = 0;
       pool = 0;
     }
