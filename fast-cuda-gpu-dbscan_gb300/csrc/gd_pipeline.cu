@@ -2456,6 +2456,17 @@ __device__ __forceinline__ int inline_link(const gdl::Bufs& B, int64_t n, int bA
   return 0;
 }
 
+// Pairs of cells that a thread does not search: it classifies the first cell's points one by
+// one, and skips the second one's that are not core points, without counting either.  (2M 3D
+// points at 40,000 Zipf-popular positions, the most popular one with 190,000 points, float32
+// mode: union phase 49.9 ms, 15.5 so; 400,000 2D points likewise 5.5 and 1.2; the line at 64 or
+// 1024 points within 5 %.)
+constexpr int kLinkPoints = 256;
+constexpr long long kLinkPairs = 1ll << 16;
+__device__ __forceinline__ bool crowded_pair(int na, int nb) {
+  return na > kLinkPoints || (long long)na * nb > kLinkPairs;
+}
+
 // Link between core cells m and c (at offset (ox, oy, oz) from m), m's
 // representative in ca: the representatives first -- on the workloads nine face
 // neighbours in ten are linked by that one test -- then the search.
@@ -2478,11 +2489,79 @@ __device__ __forceinline__ int cell_link(const gdl::Bufs& B, int64_t n, const De
     apart = !d2_le(d2, P.eps2);
   }
   if (apart && B.cellcore[m] == 1 && B.cellcore[c] == 1) return 0;  // the only pair
+  const int bA = B.reps[m], eA = B.reps[m + 1], bB = B.reps[c], eB = B.reps[c + 1];
+  if (crowded_pair(eA - bA, eB - bB)) return -1;
   const PredParams Q = pred_params(P);
   float oA[D];
   if (Q.prune) cell_origin32<D>(cc, P, oA);
-  return inline_link<D, F32>(B, n, B.reps[m], B.reps[m + 1], B.reps[c], B.reps[c + 1], oA, ox, oy,
-                             oz, P, Q, t);
+  return inline_link<D, F32>(B, n, bA, eA, bB, eB, oA, ox, oy, oz, P, Q, t);
+}
+
+// ---- link searches by a warp.
+// Core point a of one cell against the core points [b0, b1) of another: whether one is its
+// neighbour both ways.  A warp, a lane per candidate.
+template <int D, bool F32>
+__device__ __forceinline__ bool warp_link_row(const gdl::Bufs& B, int a, int b0, int b1,
+                                               const PredParams& Q, Tally& t) {
+  const int lane = threadIdx.x & 31;
+  double ax[D];
+  float af[D];
+  if (F32) ld_f<D>(B, a, af);
+  else ld_x<D>(B, a, ax);
+  for (int qb = b0; qb < b1; qb += 32) {
+    const int q = qb + lane;
+    bool hit = false;
+    if (q < b1 && B.core[q]) {
+      Cand<D, F32> c;
+      load_cand<D, F32>(c, B, q);
+      hit = link_test<D, F32>(ax, af, c, B, a, q, Q, t);
+    }
+    if (__any_sync(kFull, hit)) return true;
+  }
+  return false;
+}
+
+// The core points [a0, a0 + na), na <= 32, of the cell with origin oA against those of [b0, b1),
+// at offset o: whether a pair are neighbours both ways.  A lane per point of the first cell
+// finds out which of them have the other cell wholly inside or outside their reach; the others
+// are tested one by one with a lane per point of the other cell, or all at once with a lane each
+// and that cell's points one by one, whichever takes fewer steps.
+template <int D, bool F32>
+__device__ __forceinline__ bool warp_link_rows(const gdl::Bufs& B, int a0, int na, int b0, int b1,
+                                               const float* oA, const int* o, const PredParams& Q,
+                                               Tally& t) {
+  const int lane = threadIdx.x & 31;
+  int cls = -1;
+  double ax[D];
+  float af[D];
+  if (lane < na && B.core[a0 + lane]) {
+    cls = 0;
+    load_point<D, F32>(ax, af, B, a0 + lane, Q.prune != 0);
+    if (Q.prune) {
+      float u[D];
+      frac_pos<D>(af, oA, Q, u);
+      cls = classify<D>(u, o[0], o[1], o[2], Q);
+    }
+  }
+  if (__any_sync(kFull, cls > 0)) return true;  // (the other cell holds a core point)
+  unsigned open = __ballot_sync(kFull, cls == 0);
+  if (!open) return false;
+  if (__popc(open) * ((b1 - b0 + 31) / 32) > b1 - b0) {
+    for (int q = b0; q < b1; ++q) {
+      if (!B.core[q]) continue;
+      bool hit = false;
+      if (cls == 0) {
+        Cand<D, F32> c;
+        load_cand<D, F32>(c, B, q);
+        hit = link_test<D, F32>(ax, af, c, B, a0 + lane, q, Q, t);
+      }
+      if (__any_sync(kFull, hit)) return true;
+    }
+    return false;
+  }
+  for (; open; open &= open - 1)
+    if (warp_link_row<D, F32>(B, a0 + __ffs(open) - 1, b0, b1, Q, t)) return true;
+  return false;
 }
 
 // bit of offset (ox, oy, oz) in the kHalf[D][pass] table, or -1 if it is not there
@@ -3087,8 +3166,7 @@ __global__ void k_flood(const gdl::Bufs B) {
 // Heavy link searches, one warp per queued cell A: for each still-open
 // half-stencil neighbour B (pass 0: offsets within +-1, pass 1: the rest) whose
 // core points are in another component, look for one core-core pair that are
-// neighbours both ways (lanes over B's points, A's core points broadcast) and
-// unite the two cells.
+// neighbours both ways (warp_link_rows) and unite the two cells.
 template <int D, bool F32, bool KEY64>
 __global__ void __launch_bounds__(kCellThreads) k_union_heavy(const gdl::Bufs B, int64_t n, int pass) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -3109,6 +3187,8 @@ __global__ void __launch_bounds__(kCellThreads) k_union_heavy(const gdl::Bufs B,
     const DevParams& P = *cx.P;
     const PredParams Q = pred_params(P);
     const CellXYZ<D> cc = decompose<D>(cx.local, P);
+    float oA[D];
+    if (Q.prune) cell_origin32<D>(cc, P, oA);
     for (int t0 = 0; t0 < T.n; t0 += 32) {
       const int tt = t0 + lane;
       bool cand = false;
@@ -3132,22 +3212,11 @@ __global__ void __launch_bounds__(kCellThreads) k_union_heavy(const gdl::Bufs B,
         const int ceB = __shfl_sync(kFull, eB, src);
         const int ccB = __shfl_sync(kFull, cB, src);
         if (uf_find(B.parent, (int)m) == uf_find(B.parent, ccB)) continue;
+        const signed char* ob = T.o[t0 + src];
+        const int o[3] = {ob[0], ob[1], ob[2]};
         bool found = false;
-        for (int qb = cbB; qb < ceB && !found; qb += 32) {
-          const int q = qb + lane;
-          const bool valid = q < ceB && B.core[q];
-          Cand<D, F32> c;
-          if (valid) load_cand<D, F32>(c, B, q);
-          for (int a = b; a < e && !found; ++a) {
-            if (!B.core[a]) continue;
-            double ax[D];
-            float af[D];
-            if (F32) ld_f<D>(B, a, af);
-            else ld_x<D>(B, a, ax);
-            bool hit = valid && link_test<D, F32>(ax, af, c, B, a, q, Q, t);
-            found = __any_sync(kFull, hit);
-          }
-        }
+        for (int a = b; a < e && !found; a += 32)
+          found = warp_link_rows<D, F32>(B, a, min(32, e - a), cbB, ceB, oA, o, Q, t);
         if (found && lane == 0) uf_union(B.parent, (int)m, ccB);
         __syncwarp();
       }

@@ -322,8 +322,7 @@ struct SmallWalk {
 };
 
 // ---- link searches that a lane does not finish.  A lane of the union spends at most
-// kSmallLinkTests tests on a cell pair, and none on a pair of more than kSmallLanePairs point
-// pairs: a pair of crowded cells that are apart by a little more than eps would otherwise keep
+// kSmallLinkTests tests on a cell pair, and none on a crowded one (crowded_pair): a pair of crowded cells that are apart by a little more than eps would otherwise keep
 // one lane busy for |A| |B| tests while every other block waits at the barrier.  The cells with
 // open pairs are listed with those pairs as a mask (offsets of the step's half stencil) and
 // searched after the barrier, a warp per cell; pairs of more than kSmallWarpPairs point pairs
@@ -334,7 +333,7 @@ struct SmallWalk {
 // the listed cells in ptcell (each once per step), large pairs in ptpos: a pair of more than 2^17 point
 // pairs has a cell of more than 362 points, there are at most n / 363 of those, each in at
 // most 124 pairs (62 in each half of the 3D stencil), which is below n / 2.
-constexpr long long kSmallLanePairs = 1ll << 16, kSmallWarpPairs = 1ll << 17;
+constexpr long long kSmallWarpPairs = 1ll << 17;
 __host__ __device__ constexpr int small_big_cap(int n) { return n / 2; }
 
 constexpr int kShell3 = make_half(3, 1).n;
@@ -346,52 +345,6 @@ __device__ __forceinline__ int small_open_bit(int step, int ox, int oy, int oz) 
   const int ax = max(abs(ox), max(abs(oy), abs(oz)));
   if (step == 0) return half_bit<D>(0, ox, oy, oz);
   return D == 3 && ax > 1 ? kShell3 + half_bit<D>(2, ox, oy, oz) : half_bit<D>(1, ox, oy, oz);
-}
-
-// Core point a of one cell against the core points [b0, b1) of another: whether one is its
-// neighbour both ways.  A warp, a lane per candidate.
-template <int D, bool F32>
-__device__ __forceinline__ bool small_warp_row(const gdl::Bufs& B, int a, int b0, int b1,
-                                               const PredParams& Q, Tally& t) {
-  const int lane = threadIdx.x & 31;
-  double ax[D];
-  float af[D];
-  if (F32) ld_f<D>(B, a, af);
-  else ld_x<D>(B, a, ax);
-  for (int qb = b0; qb < b1; qb += 32) {
-    const int q = qb + lane;
-    bool hit = false;
-    if (q < b1 && B.core[q]) {
-      Cand<D, F32> c;
-      load_cand<D, F32>(c, B, q);
-      hit = link_test<D, F32>(ax, af, c, B, a, q, Q, t);
-    }
-    if (__any_sync(kFull, hit)) return true;
-  }
-  return false;
-}
-
-// The same for core points [a0, a0 + na), na <= 32, of the cell with origin oA: those that
-// have the other cell (at offset o) wholly inside or outside their reach need no tests.
-template <int D, bool F32>
-__device__ __forceinline__ bool small_warp_rows(const gdl::Bufs& B, int a0, int na, int b0, int b1,
-                                                const float* oA, const int* o, const PredParams& Q,
-                                                Tally& t) {
-  const int lane = threadIdx.x & 31;
-  int cls = -1;
-  if (lane < na && B.core[a0 + lane]) {
-    cls = 0;
-    if (Q.prune) {
-      float f[D], u[D];
-      ld_f<D>(B, a0 + lane, f);
-      frac_pos<D>(f, oA, Q, u);
-      cls = classify<D>(u, o[0], o[1], o[2], Q);
-    }
-  }
-  if (__any_sync(kFull, cls > 0)) return true;  // (the other cell holds a core point)
-  for (unsigned w = __ballot_sync(kFull, cls == 0); w; w &= w - 1)
-    if (small_warp_row<D, F32>(B, a0 + __ffs(w) - 1, b0, b1, Q, t)) return true;
-  return false;
 }
 
 // two cells' roots equal (one answer for the warp)
@@ -457,7 +410,7 @@ __device__ __noinline__ void small_link_cells(const gdl::Bufs& B, const SmallArg
         const int o[3] = {ob[0], ob[1], ob[2]};
         bool found = false;
         for (int a = (int)ra.x; a < (int)ra.y && !found; a += 32)
-          found = small_warp_rows<D, F32>(B, a, min(32, (int)ra.y - a), b0, b1, oA, o, Q, t);
+          found = warp_link_rows<D, F32>(B, a, min(32, (int)ra.y - a), b0, b1, oA, o, Q, t);
         if (found && lane == 0) uf_union(B.parent, m, cb);
         __syncwarp();
       }
@@ -482,7 +435,7 @@ __device__ __noinline__ void small_link_big(const gdl::Bufs& B, const SmallArgs&
     for (int a = (int)ra.x + w; a < (int)ra.y; a += W) {
       if (!B.core[a]) continue;
       if (small_same(B, m, c)) break;
-      if (small_warp_row<D, F32>(B, a, (int)rb.x, (int)rb.y, Q, t)) {
+      if (warp_link_row<D, F32>(B, a, (int)rb.x, (int)rb.y, Q, t)) {
         if ((threadIdx.x & 31) == 0) uf_union(B.parent, m, c);
         __syncwarp();
         break;
@@ -719,7 +672,7 @@ k_small_expand(const __grid_constant__ gdl::Bufs B, const __grid_constant__ Smal
         if (!linked && !(apart && single && B.cellcore[c] == 1)) {
           const uint2 q = A.crange[c];
           const int ox = wk.off(bit, 0), oy = wk.off(bit, 1), oz = D == 3 ? wk.off(bit, D - 1) : 0;
-          const int res = (long long)(r.y - r.x) * (q.y - q.x) > kSmallLanePairs
+          const int res = crowded_pair((int)(r.y - r.x), (int)(q.y - q.x))
                               ? -1
                               : inline_link<D, F32>(B, n, (int)r.x, (int)r.y, (int)q.x, (int)q.y,
                                                     oA, ox, oy, oz, P, Q, t);
