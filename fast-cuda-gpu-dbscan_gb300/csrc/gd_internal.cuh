@@ -247,7 +247,9 @@ enum Counter {
   kCtrWalkCursor3,
   kCtrWaitTimeouts,     // scan / sort launches whose look-back wait gave up (never expected)
   kCtrBlocks,           // blocks holding a core point (small runs: positions handed out)
-  kCtrCount = 18
+  kCtrSmallPairs,       // small runs: large cell pairs for blocks and for the grid, in each of
+                        // the union's two steps (4 words, cleared by the expand)
+  kCtrCount = 22
 };
 
 // Capacity of the list of one-directional core-core pairs (see k_asym_resolve).
@@ -282,7 +284,13 @@ struct SmallArgs {
 
 constexpr int kSmallThreads = 512;
 // pair tests one lane of a small run spends on a cell pair before the pair goes to a warp
-constexpr int kSmallLinkTests = 256;
+constexpr int kSmallLinkTests = 64;
+// open candidates from which a point goes to a warp (core count), and candidates that a lane
+// looks at for a point's border search before it does.  (Both lines at half and twice the value
+// on sets with crowded cells, 300 to 260,000 points, and on the blobs: 64 instead of 256 costs
+// 30,000 3D blob points 16 % and 128 2 %, 512 costs 260,000 points in clumps of different spread
+// 20 %; link tests at 256 cost 1,000 to 30,000 points at Zipf-popular positions 10 to 20 %.)
+constexpr int kSmallPointTests = 256;
 // Single runs of at most this many points take the small kernels when their grid has
 // a direct block table.  The lines lie where the general pipeline's launches stop
 // dominating: 2D 482 -> 341 us at 128k points, 510 -> 398 at 256k (blobs, float64); 3D

@@ -2546,7 +2546,7 @@ __device__ __forceinline__ bool warp_link_rows(const gdl::Bufs& B, int a0, int n
   if (__any_sync(kFull, cls > 0)) return true;  // (the other cell holds a core point)
   unsigned open = __ballot_sync(kFull, cls == 0);
   if (!open) return false;
-  if (__popc(open) * ((b1 - b0 + 31) / 32) > b1 - b0) {
+  if (5 * __popc(open) * ((b1 - b0 + 31) / 32) >= 4 * (b1 - b0)) {  // (its steps are the cheaper)
     for (int q = b0; q < b1; ++q) {
       if (!B.core[q]) continue;
       bool hit = false;

@@ -326,15 +326,18 @@ struct SmallWalk {
 // one lane busy for |A| |B| tests while every other block waits at the barrier.  The cells with
 // open pairs are listed with those pairs as a mask (offsets of the step's half stencil) and
 // searched after the barrier, a warp per cell; pairs of more than kSmallWarpPairs point pairs
-// then by the whole grid, one after the other.  (Two crowds of 5,000 points each, 1.1 eps
-// apart, float64, whole call: 0.70 ms in 2D and 0.79 in 3D; 20,000 each: 6.4 and 8.6.  The
-// general path's warp per pair: 234 and 304 ms; 4.5 and 5.5 s.)
+// then by a block each, and those of more than kSmallBlockPairs by the whole grid, one after the
+// other.  (Two crowds of 5,000 points each, 1.1 eps apart, float64, whole call: 0.70 ms in 2D
+// and 0.79 in 3D; 20,000 each: 6.4 and 8.6.  The general path's warp per pair: 234 and 304 ms;
+// 4.5 and 5.5 s.)
 // The lists lie in buffers of the index build that are free by now: each cell's mask in ptkey,
-// the listed cells in ptcell (each once per step), large pairs in ptpos: a pair of more than 2^17 point
-// pairs has a cell of more than 362 points, there are at most n / 363 of those, each in at
-// most 124 pairs (62 in each half of the 3D stencil), which is below n / 2.
-constexpr long long kSmallWarpPairs = 1ll << 17;
-__host__ __device__ constexpr int small_big_cap(int n) { return n / 2; }
+// the listed cells in ptcell (each once per step), large pairs in ptpos, n / 2 of them: the
+// blocks' from its start, which a warp searches itself where there is no room, the grid's from
+// its middle.  The latter's cells have more than 1,024 points on one side; there are at most
+// n / 1025 of those, each in at most 124 pairs (62 in each half of the 3D stencil): below n / 8.
+constexpr long long kSmallWarpPairs = 1ll << 14, kSmallBlockPairs = 1ll << 20;
+__host__ __device__ constexpr int small_block_cap(int n) { return n / 2 - n / 8; }
+__host__ __device__ constexpr int small_grid_cap(int n) { return n / 8; }
 
 constexpr int kShell3 = make_half(3, 1).n;
 static_assert(kShell3 + make_half(3, 2).n <= 64 && make_half(2, 1).n <= 64, "a mask per step");
@@ -398,13 +401,17 @@ __device__ __noinline__ void small_link_cells(const gdl::Bufs& B, const SmallArg
         const int cb = __shfl_sync(kFull, c, src);
         const int b0 = (int)__shfl_sync(kFull, rb.x, src), b1 = (int)__shfl_sync(kFull, rb.y, src);
         if (small_same(B, m, cb)) continue;
-        if ((long long)(ra.y - ra.x) * (b1 - b0) > kSmallWarpPairs) {
+        const long long tests = (long long)(ra.y - ra.x) * (b1 - b0);
+        if (tests > kSmallWarpPairs) {
+          const bool grid = tests > kSmallBlockPairs;
+          int room = 0;
           if (lane == 0) {
-            const unsigned long long at = atomicAdd(nbig, 1ull);
-            if (at < (unsigned long long)small_big_cap(A.n))
-              big[at] = make_uint2((uint32_t)m, (uint32_t)cb);
+            const unsigned long long at = atomicAdd(nbig + (grid ? 1 : 0), 1ull);
+            room = at < (unsigned long long)(grid ? small_grid_cap(A.n) : small_block_cap(A.n));
+            if (room)
+              big[(grid ? small_block_cap(A.n) : 0) + at] = make_uint2((uint32_t)m, (uint32_t)cb);
           }
-          continue;
+          if (__shfl_sync(kFull, room, 0)) continue;
         }
         const signed char* ob = k < n0 ? kHalf[D - 2][step].o[k] : kHalf[D - 2][2].o[k - n0];
         const int o[3] = {ob[0], ob[1], ob[2]};
@@ -419,34 +426,152 @@ __device__ __noinline__ void small_link_cells(const gdl::Bufs& B, const SmallArg
   flush_tally(t, B.ctr);
 }
 
-// The large pairs, each by the whole grid: a warp per point of the first cell.
+// A large pair: a warp (w of W) per point of the first cell.
+template <int D, bool F32>
+__device__ __forceinline__ void small_link_pair(const gdl::Bufs& B, const SmallArgs& A, uint2 pair,
+                                                int w, int W, const PredParams& Q, Tally& t) {
+  const int m = (int)pair.x, c = (int)pair.y;
+  const uint2 ra = A.crange[m], rb = A.crange[c];
+  for (int a = (int)ra.x + w; a < (int)ra.y; a += W) {
+    if (!B.core[a]) continue;
+    if (small_same(B, m, c)) break;
+    if (warp_link_row<D, F32>(B, a, (int)rb.x, (int)rb.y, Q, t)) {
+      if ((threadIdx.x & 31) == 0) uf_union(B.parent, m, c);
+      __syncwarp();
+      break;
+    }
+  }
+}
+
+// The large pairs: a block each, then the whole grid.
 template <int D, bool F32>
 __device__ __noinline__ void small_link_big(const gdl::Bufs& B, const SmallArgs& A,
-                                            const DevParams& P, int pairs) {
-  const int W = gridDim.x * (kSmallThreads / 32);
-  const int w = blockIdx.x * (kSmallThreads / 32) + (threadIdx.x >> 5);
+                                            const DevParams& P, const unsigned long long* nbig) {
+  constexpr int NW = kSmallThreads / 32;
+  const int w = threadIdx.x >> 5;
   const PredParams Q = pred_params(P);
   const uint2* big = reinterpret_cast<const uint2*>(A.ptpos);
-  pairs = min(pairs, small_big_cap(A.n));
+  const int nb = (int)min(nbig[0], (unsigned long long)small_block_cap(A.n));
+  const int ng = (int)min(nbig[1], (unsigned long long)small_grid_cap(A.n));
   Tally t;
-  for (int p = 0; p < pairs; ++p) {
-    const int m = (int)big[p].x, c = (int)big[p].y;
-    const uint2 ra = A.crange[m], rb = A.crange[c];
-    for (int a = (int)ra.x + w; a < (int)ra.y; a += W) {
-      if (!B.core[a]) continue;
-      if (small_same(B, m, c)) break;
-      if (warp_link_row<D, F32>(B, a, (int)rb.x, (int)rb.y, Q, t)) {
-        if ((threadIdx.x & 31) == 0) uf_union(B.parent, m, c);
-        __syncwarp();
-        break;
+  for (int p = blockIdx.x; p < nb; p += gridDim.x)
+    small_link_pair<D, F32>(B, A, big[p], w, NW, Q, t);
+  for (int p = 0; p < ng; ++p)
+    small_link_pair<D, F32>(B, A, big[small_block_cap(A.n) + p], blockIdx.x * NW + w,
+                            gridDim.x * NW, Q, t);
+  flush_tally(t, B.ctr);
+}
+
+// ---- points with many open candidates, a warp each.  A group of 4 or 8 lanes tests them a
+// lane per block, one per step: a point beside a crowded cell would keep one lane busy for
+// thousands of steps, and the warp with it.  (260,000 2D points in clumps with spreads from
+// 0.01 to 20 at eps 0.5, float64, minPts 4, whole call: 3.43 ms, so 0.75.)
+// Neighbours of point i (sorted position), counted up to minpts.
+template <int D, bool F32>
+__device__ __noinline__ int small_count_point(const gdl::Bufs& B, const SmallArgs& A,
+                                              const DevParams& P, int i, int minpts) {
+  using W = SmallWalk<D>;
+  const int lane = threadIdx.x & 31;
+  const PredParams Q = pred_params(P);
+  const bool prune = Q.prune != 0;
+  const int m = (int)A.pcell[i];
+  const uint2 own = A.crange[m];
+  int cnt = (int)(own.y - own.x);
+  double px[D];
+  float pf[D], u[D];
+  load_point<D, F32>(px, pf, B, i, prune);
+  Tally t;
+  for (int g = 0; g < W::G && cnt < minpts; ++g) {
+    W wk;
+    wk.init(B, P, A.cellkey[m], g);
+    if (prune) {
+      float o[D];
+      cell_origin32<D>(wk.cc, P, o);
+      frac_pos<D>(pf, o, Q, u);
+    }
+    const EntHead h = ent_head(B, wk.e);
+    for (unsigned long long v = h.occ & wk.mask(wk.st.w5); v && cnt < minpts; v &= v - 1) {
+      const int bit = __ffsll((long long)v) - 1;
+      const int c = ent_cell(h.occ, h.base, bit);
+      if (c == m) continue;
+      const int cls = prune ? classify<D>(u, wk.off(bit, 0), wk.off(bit, 1),
+                                          D == 3 ? wk.off(bit, D - 1) : 0, Q) : 0;
+      if (cls < 0) continue;
+      const uint2 r = A.crange[c];
+      if (cls > 0) {
+        cnt += (int)(r.y - r.x);
+        continue;
+      }
+      for (uint32_t q0 = r.x; q0 < r.y && cnt < minpts; q0 += 32) {
+        const uint32_t q = q0 + lane;
+        bool hit = false;
+        if (q < r.y) {
+          Cand<D, F32> cd;
+          load_cand<D, F32>(cd, B, q);
+          hit = pair_test<D, F32>(px, pf, cd, B, q, i, true, Q, t);
+        }
+        cnt += __popc(__ballot_sync(kFull, hit));
       }
     }
   }
   flush_tally(t, B.ctr);
+  return cnt;
 }
 
-// Two blocks' registers fit an SM, so that two runs on different streams do not wait for each
-// other's end (one block per SM: 118 registers, no spills, and within 1 % of the time).
+// Smallest cluster id below `best` among the cells whose core points have point i in their
+// neighbourhood, else `best`.
+template <int D, bool F32>
+__device__ __noinline__ int small_border_point(const gdl::Bufs& B, const SmallArgs& A,
+                                               const DevParams& P, int i, int best) {
+  using W = SmallWalk<D>;
+  const int lane = threadIdx.x & 31;
+  const PredParams Q = pred_params(P);
+  const bool prune = Q.prune != 0;
+  const int m = (int)A.pcell[i];
+  double px[D];
+  float pf[D], u[D];
+  load_point<D, F32>(px, pf, B, i, prune);
+  Tally t;
+  for (int g = 0; g < W::G; ++g) {
+    W wk;
+    wk.init(B, P, A.cellkey[m], g);
+    if (wk.e == kNoEnt) continue;
+    if (prune) {
+      float o[D];
+      cell_origin32<D>(wk.cc, P, o);
+      frac_pos<D>(pf, o, Q, u);
+    }
+    const EntHead h = ent_head(B, wk.e);
+    for (unsigned long long v = ent_tail(B, wk.e).core & wk.mask(wk.st.w5); v; v &= v - 1) {
+      const int bit = __ffsll((long long)v) - 1;
+      const int c = ent_cell(h.occ, h.base, bit);
+      const int cB = B.cellcid[c];
+      if (cB >= best) continue;
+      const int cls = prune ? classify<D>(u, wk.off(bit, 0), wk.off(bit, 1),
+                                          D == 3 ? wk.off(bit, D - 1) : 0, Q) : 0;
+      if (cls < 0) continue;
+      bool in = cls > 0;
+      const uint2 r = A.crange[c];
+      for (uint32_t q0 = r.x; q0 < r.y && !in; q0 += 32) {
+        const uint32_t q = q0 + lane;
+        bool hit = false;
+        if (q < r.y && B.core[q]) {
+          Cand<D, F32> cd;
+          load_cand<D, F32>(cd, B, q);
+          hit = pair_test<D, F32>(px, pf, cd, B, q, i, false, Q, t);
+        }
+        in = __any_sync(kFull, hit);
+      }
+      if (in) best = cB;
+    }
+  }
+  flush_tally(t, B.ctr);
+  return best;
+}
+
+// Two blocks' registers fit an SM, so that runs on different streams do not wait for each
+// other's end (100,000 2D points, 4 threads with a context each: 7,600 runs a second, with one
+// block per SM, which needs no spills, 5,300; one thread: 4,030 and 4,140).
 template <int D, bool F32>
 __global__ void __launch_bounds__(kSmallThreads, 2)
 k_small_expand(const __grid_constant__ gdl::Bufs B, const __grid_constant__ SmallArgs A, int minpts,
@@ -487,6 +612,7 @@ k_small_expand(const __grid_constant__ gdl::Bufs B, const __grid_constant__ Smal
     B.ent[A.cellkey[m] >> kBlockBits].core = 0;
   }
   for (int k = t0; k < nwf; k += T) B.fbits[k] = 0;
+  if (t0 < 4) B.ctr[kCtrSmallPairs + t0] = 0;
   for (int i0 = t0 - lane; i0 < n; i0 += T) {
     const int i = i0 + lane;
     bool walk = false;
@@ -559,7 +685,9 @@ k_small_expand(const __grid_constant__ gdl::Bufs B, const __grid_constant__ Smal
       open += __shfl_xor_sync(kFull, open, o);
     }
     int cnt = own + add;
-    bool more = valid && cnt < minpts && cnt + open >= minpts && w != 0;
+    const bool undecided = valid && cnt < minpts && cnt + open >= minpts;
+    const bool heavy = undecided && open > kSmallPointTests;  // (the whole group)
+    bool more = undecided && !heavy && w != 0;
     uint32_t q = 0, qe = 0;
     while (true) {
       bool hit = false;
@@ -578,6 +706,11 @@ k_small_expand(const __grid_constant__ gdl::Bufs B, const __grid_constant__ Smal
       cnt += __popc(__ballot_sync(kFull, hit) & grp);
       more = more && cnt < minpts && (q < qe || w != 0);
       if (!__any_sync(kFull, more)) break;
+    }
+    for (unsigned hv = __ballot_sync(kFull, heavy && g == 0); hv; hv &= hv - 1) {
+      const int src = __ffs(hv) - 1;
+      const int c = small_count_point<D, F32>(B, A, P, __shfl_sync(kFull, i, src), minpts);
+      if (src == (lane & ~(W::G - 1))) cnt = c;
     }
     if (valid && g == 0) {
       const bool isc = cnt >= minpts;
@@ -606,7 +739,7 @@ k_small_expand(const __grid_constant__ gdl::Bufs B, const __grid_constant__ Smal
   // from one parent load.  Pairs that pass a lane's budget follow after the barrier.
   for (int step = 0; step < 2; ++step) {
     unsigned long long* nopen = B.ctr + (step == 0 ? kCtrHeavyCore : kCtrHeavyUnion);
-    unsigned long long* nbig = B.ctr + (step == 0 ? kCtrHeavyBorder : kCtrWalkCursor3);
+    unsigned long long* nbig = B.ctr + kCtrSmallPairs + 2 * step;
     for (int m = g0; m < M; m += gT) {
       if (B.cellcore[m] == 0) continue;  // (the whole group)
       const uint64_t ck = A.cellkey[m];
@@ -688,9 +821,9 @@ k_small_expand(const __grid_constant__ gdl::Bufs B, const __grid_constant__ Smal
     if (listed) {
       small_link_cells<D, F32>(B, A, P, step, listed, nbig);
       if (!grid_barrier(A, timeouts)) return;
-      const int pairs = (int)*reinterpret_cast<volatile unsigned long long*>(nbig);
-      if (pairs) {
-        small_link_big<D, F32>(B, A, P, pairs);
+      const volatile unsigned long long* nb = nbig;
+      if (nb[0] + nb[1]) {
+        small_link_big<D, F32>(B, A, P, nbig);
         if (!grid_barrier(A, timeouts)) return;
       }
     }
@@ -753,12 +886,14 @@ k_small_expand(const __grid_constant__ gdl::Bufs B, const __grid_constant__ Smal
     if (out) out[B.ids[i]] = best;
     else B.lab[i] = best;
   }
-  for (int j = g0; j < L; j += gT) {
-    const int i = (int)A.list[j];
-    if (B.core[i]) continue;  // (the whole group)
-    const int m = (int)A.pcell[i];
-    int best = INT_MAX;
-    {
+  for (int j0 = (t0 - lane) / W::G; j0 < L; j0 += gT) {
+    const int j = j0 + lane / W::G;
+    const int i = j < L ? (int)A.list[j] : 0;
+    const bool search = j < L && !B.core[i];  // (the whole group)
+    int best = INT_MAX, budget = kSmallPointTests;
+    bool heavy = false;
+    if (search) {
+      const int m = (int)A.pcell[i];
       W wk;
       wk.init(B, P, A.cellkey[m], g);
       unsigned long long w = 0;
@@ -774,7 +909,7 @@ k_small_expand(const __grid_constant__ gdl::Bufs B, const __grid_constant__ Smal
           cell_origin32<D>(wk.cc, P, o);
           frac_pos<D>(pf, o, Q, u);
         }
-        while (w) {
+        while (w && !heavy) {
           const int bit = __ffsll((long long)w) - 1;
           w &= w - 1;
           const int c = ent_cell(h.occ, h.base, bit);
@@ -789,6 +924,10 @@ k_small_expand(const __grid_constant__ gdl::Bufs B, const __grid_constant__ Smal
           }
           const uint2 q = A.crange[c];
           for (uint32_t qq = q.x; qq < q.y; ++qq) {
+            if (budget-- == 0) {
+              heavy = true;
+              break;
+            }
             if (!B.core[qq]) continue;
             Cand<D, F32> cd;
             load_cand<D, F32>(cd, B, qq);
@@ -799,12 +938,20 @@ k_small_expand(const __grid_constant__ gdl::Bufs B, const __grid_constant__ Smal
           }
         }
       }
-#pragma unroll
-      for (int o = W::G / 2; o > 0; o >>= 1) best = min(best, __shfl_xor_sync(grp, best, o));
-      if (best == INT_MAX) best = kNoise;
-      noise += g == 0 && best == kNoise;
     }
-    if (g == 0) {
+#pragma unroll
+    for (int o = W::G / 2; o > 0; o >>= 1) best = min(best, __shfl_xor_sync(kFull, best, o));
+    // (a group's lowest lane stands for it)
+    const unsigned hb = __ballot_sync(kFull, heavy);
+    for (unsigned hv = __ballot_sync(kFull, g == 0 && (hb & grp)); hv; hv &= hv - 1) {
+      const int src = __ffs(hv) - 1;
+      const int b = small_border_point<D, F32>(B, A, P, __shfl_sync(kFull, i, src),
+                                               __shfl_sync(kFull, best, src));
+      if (src == (lane & ~(W::G - 1))) best = b;
+    }
+    if (search && g == 0) {
+      if (best == INT_MAX) best = kNoise;
+      noise += best == kNoise;
       if (out) out[B.ids[i]] = best;
       else B.lab[i] = best;
     }

@@ -33,8 +33,9 @@ def _expected(who):
 
 @pytest.mark.parametrize("prec", [0, 1])
 @pytest.mark.parametrize("d", [2, 3])
-@pytest.mark.parametrize("sizes", [(16, 16), (16, 17), (256, 256), (256, 257), (362, 362),
-                                   (363, 362), (5, 20_000), (30_000, 30_000), (5000, 7, 5000)])
+@pytest.mark.parametrize("sizes", [(16, 16), (16, 17), (128, 128), (129, 128), (256, 256),
+                                   (256, 257), (257, 5), (362, 362), (363, 362), (1024, 1024),
+                                   (1025, 1024), (5, 20_000), (30_000, 30_000), (5000, 7, 5000)])
 def test_unlinked_and_last_pair_linked(gpu_ctx, gd, prec, d, sizes):
     rng = np.random.default_rng(sum(sizes) + d)
     pts, who = _crowds(d, sizes, 1.1, rng)
