@@ -289,8 +289,11 @@ constexpr int kSmallLinkTests = 64;
 // looks at for a point's border search before it does.  (Both lines at half and twice the value
 // on sets with crowded cells, 300 to 260,000 points, and on the blobs: 64 instead of 256 costs
 // 30,000 3D blob points 16 % and 128 2 %, 512 costs 260,000 points in clumps of different spread
-// 20 %; link tests at 256 cost 1,000 to 30,000 points at Zipf-popular positions 10 to 20 %.)
-constexpr int kSmallPointTests = 256;
+// 20 %; link tests at 256 cost 1,000 to 30,000 points at Zipf-popular positions 10 to 20 %.
+// Float32 tests cost a lane less beside the classification that a warp does again: at 256 and
+// 512, 130,000 3D points of a few per position take 1.35 and 1.23 times as long as at 1024; at
+// 2048 260,000 points in clumps 1.25 times.)
+constexpr int kSmallPointTests = 256, kSmallPointTests32 = 1024;
 // Single runs of at most this many points take the small kernels when their grid has
 // a direct block table.  The lines lie where the general pipeline's launches stop
 // dominating: 2D 482 -> 341 us at 128k points, 510 -> 398 at 256k (blobs, float64); 3D

@@ -686,7 +686,7 @@ k_small_expand(const __grid_constant__ gdl::Bufs B, const __grid_constant__ Smal
     }
     int cnt = own + add;
     const bool undecided = valid && cnt < minpts && cnt + open >= minpts;
-    const bool heavy = undecided && open > kSmallPointTests;  // (the whole group)
+    const bool heavy = undecided && open > (F32 ? kSmallPointTests32 : kSmallPointTests);  // (the whole group)
     bool more = undecided && !heavy && w != 0;
     uint32_t q = 0, qe = 0;
     while (true) {
