@@ -245,7 +245,7 @@ enum Counter {
   kCtrCells2D,          // cells of 2D instances (they sort first)
   kCtrWalkCursor2,      // walk-list entries handed out (2D, 3D); cleared before each walk launch
   kCtrWalkCursor3,
-  kCtrWaitTimeouts,     // scan / sort launches whose look-back wait gave up (never expected)
+  kCtrWaitTimeouts,     // look-back waits (scans, sort) and small runs' barrier waits that gave up
   kCtrBlocks,           // blocks holding a core point (small runs: positions handed out)
   kCtrSmallPairs,       // small runs: large cell pairs for blocks and for the grid, in each of
                         // the union's two steps (4 words, cleared by the expand)

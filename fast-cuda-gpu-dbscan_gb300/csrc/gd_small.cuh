@@ -21,7 +21,7 @@
 // is reported (kCtrWaitTimeouts): the host then takes the general path.
 
 
-constexpr unsigned kBarrierPolls = 1u << 25;  // 2 s and more
+constexpr unsigned kBarrierPolls = 1u << 25;  // 2 s of sleep, about 15 s with the loads
 
 // All blocks of the launch; false when the wait gave up (the block must leave).
 __device__ __forceinline__ bool grid_barrier(const SmallArgs& A, unsigned long long* timeouts) {

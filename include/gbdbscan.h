@@ -117,7 +117,8 @@ gd_status gd_ctx_trim(gd_ctx* ctx);
 /* No counterpart in the reference.  With graphs enabled (the default), the
    second gd_expand on one index build captures the expand launches into a CUDA
    graph and later gd_expand calls on that index (other minpts) replay it with
-   one launch.  (Small runs expand in one kernel anyway and capture nothing.)  A new index build, a tuning change or gd_ctx_trim drops it. */
+   one launch.  (Small runs expand in one kernel anyway and capture nothing.)  A
+   new index build, a tuning change or gd_ctx_trim drops it. */
 gd_status gd_ctx_set_graphs(gd_ctx* ctx, int32_t enable);
 
 /* ---- the pipeline, stage by stage ---------------------------------------- */
@@ -178,7 +179,10 @@ gd_status gd_batch_dbscan(gd_ctx* ctx, int32_t count, const gd_instance* inst,
    compile-time constants, common.h:10-25).  Parameters that change speed but
    never labels: the cell side as a multiple of eps per dimension (see
    gd_ctx_set_cell_mults) and the pair tests one thread spends on a core
-   count, a link search and a border search before the work goes to a warp. */
+   count, a link search and a border search before the work goes to a warp (a
+   float32 core count: four times as many per point, on cells of up to a quarter
+   of them).  Small runs (one instance, at most 262144 points in 2D and 131072 in
+   3D) use the multipliers and have budgets of their own. */
 typedef struct gd_tuning {
   double mult2d;          /* (0.5, 1/sqrt(2)); 0 = default */
   double mult3d;          /* (0.5, 1/sqrt(3)); 0 = default */
