@@ -1915,11 +1915,12 @@ __global__ void k_core_split(const gdl::Bufs B, int64_t n, int chunk, int clear)
 // first), so it is kCellBudget times the context's per point: a whole 3D stencil of 8 points per
 // cell.  (2M 3D points, uniform, 4 per cell, minPts 87, the mean neighbour count: core phase
 // 3.91 ms at one times the budget, 2.55 at two, four, eight and sixteen; 9 per cell: 6.03, 6.02,
-// 3.98, 3.97, 3.97.)  A cell of more than a quarter of the budget that is not settled whole goes
-// to the warp kernel at once: its points are a long serial chain (200 clumps of 5,000 2D points,
-// spread 0.05 to 5 at eps 0.5, minPts 5 and 50: 376 and 1142 us without the rule, 136 and 255
-// from 64 points on, 144 and 284 from 128, 133 and 245 from 32, which costs even sets 1 to 8 %.)  Per-cell core counts are atomics (cleared before the
-// launch).
+// 3.98, 3.97, 3.97.)  A cell of more than half the budget that is not settled whole goes to the
+// warp kernel at once: its points are a long serial chain (200 clumps of 5,000 2D points, spread
+// 0.05 to 5 at eps 0.5, minPts 5 and 50: 381 and 1129 us without the rule, 147 and 282 from 128
+// points on, 134 and 270 from 64, 157 and 354 from 256; five minPts on 1M even 2D points take 0.6 %
+// longer with the line at 128 than without the rule, 2 % at 64).  Per-cell core counts are atomics
+// (cleared before the launch).
 //
 // Passes [p0, p1).  3D runs pass 0 for every listed chunk first: a chunk with an
 // undecided point keeps its points' counts in lab[] (kDecided for decided ones)
@@ -2042,7 +2043,7 @@ k_core_cell(const gdl::Bufs B, int64_t n, int p0, int p1) {
             return;
           }
         }
-        if (qe - q0 > B.tn_core / 4) budget = 0;  // a crowded cell is a warp's work
+        if (qe - q0 > B.tn_core / 2) budget = 0;  // a crowded cell is a warp's work
         for (int q = q0; q < qe; ++q) {
           budget -= present;
           if (budget < 0) {

@@ -180,8 +180,8 @@ gd_status gd_batch_dbscan(gd_ctx* ctx, int32_t count, const gd_instance* inst,
    never labels: the cell side as a multiple of eps per dimension (see
    gd_ctx_set_cell_mults) and the pair tests one thread spends on a core
    count, a link search and a border search before the work goes to a warp (a
-   float32 core count: four times as many per point, on cells of up to a quarter
-   of them).  Small runs (one instance, at most 262144 points in 2D and 131072 in
+   float32 core count: four times as many per point, on cells of up to half of
+   them).  Small runs (one instance, at most 262144 points in 2D and 131072 in
    3D) use the multipliers and have budgets of their own. */
 typedef struct gd_tuning {
   double mult2d;          /* (0.5, 1/sqrt(2)); 0 = default */
