@@ -2525,8 +2525,8 @@ __device__ __forceinline__ bool warp_link_row(const gdl::Bufs& B, int a, int b0,
 // The core points [a0, a0 + na), na <= 32, of the cell with origin oA against those of [b0, b1),
 // at offset o: whether a pair are neighbours both ways.  A lane per point of the first cell
 // finds out which of them have the other cell wholly inside or outside their reach; the others
-// are tested one by one with a lane per point of the other cell, or all at once with a lane each
-// and that cell's points one by one, whichever takes fewer steps.
+// are tested all at once with a lane each and the other cell's points one by one, or one by one
+// with a lane per point of that cell, whichever takes fewer steps.
 template <int D, bool F32>
 __device__ __forceinline__ bool warp_link_rows(const gdl::Bufs& B, int a0, int na, int b0, int b1,
                                                const float* oA, const int* o, const PredParams& Q,
@@ -2547,7 +2547,8 @@ __device__ __forceinline__ bool warp_link_rows(const gdl::Bufs& B, int a0, int n
   if (__any_sync(kFull, cls > 0)) return true;  // (the other cell holds a core point)
   unsigned open = __ballot_sync(kFull, cls == 0);
   if (!open) return false;
-  if (5 * __popc(open) * ((b1 - b0 + 31) / 32) >= 4 * (b1 - b0)) {  // (its steps are the cheaper)
+  // (the steps of the first way are the cheaper)
+  if (5ll * __popc(open) * ((b1 - b0 + 31) / 32) >= 4ll * (b1 - b0)) {
     for (int q = b0; q < b1; ++q) {
       if (!B.core[q]) continue;
       bool hit = false;
@@ -3167,9 +3168,11 @@ __global__ void k_flood(const gdl::Bufs B) {
 // Heavy link searches, one warp per queued cell A: for each still-open
 // half-stencil neighbour B (pass 0: offsets within +-1, pass 1: the rest) whose
 // core points are in another component, look for one core-core pair that are
-// neighbours both ways (warp_link_rows) and unite the two cells.
+// neighbours both ways (warp_link_rows) and unite the two cells.  (Two blocks per SM leave room
+// for the search without spills: two crowds of 8,000 points, float32 mode, 350 -> 327 ms.)
 template <int D, bool F32, bool KEY64>
-__global__ void __launch_bounds__(kCellThreads) k_union_heavy(const gdl::Bufs B, int64_t n, int pass) {
+__global__ void __launch_bounds__(kCellThreads, 2)
+k_union_heavy(const gdl::Bufs B, int64_t n, int pass) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int LB = B.Bi->LB;
   int64_t mlo, mhi;

@@ -322,18 +322,19 @@ struct SmallWalk {
 };
 
 // ---- link searches that a lane does not finish.  A lane of the union spends at most
-// kSmallLinkTests tests on a cell pair, and none on a crowded one (crowded_pair): a pair of crowded cells that are apart by a little more than eps would otherwise keep
-// one lane busy for |A| |B| tests while every other block waits at the barrier.  The cells with
-// open pairs are listed with those pairs as a mask (offsets of the step's half stencil) and
-// searched after the barrier, a warp per cell; pairs of more than kSmallWarpPairs point pairs
+// kSmallLinkTests tests on a cell pair, and none on a crowded one (crowded_pair): two crowded
+// cells that are apart by a little more than eps would otherwise keep one lane busy for |A| |B|
+// tests while every other block waits at the barrier.  The cells with open pairs are listed with
+// those pairs as a mask (offsets of the step's half stencil) and searched after the barrier, a
+// warp per cell; pairs of more than kSmallWarpPairs point pairs
 // then by a block each, and those of more than kSmallBlockPairs by the whole grid, one after the
 // other.  (Two crowds of 5,000 points each, 1.1 eps apart, float64, whole call: 0.70 ms in 2D
-// and 0.79 in 3D; 20,000 each: 6.4 and 8.6.  The general path's warp per pair: 234 and 304 ms;
-// 4.5 and 5.5 s.)
+// and 0.79 in 3D; 20,000 each: 6.4 and 8.6.  The general path's warp per pair: 0.25 and 0.32 s;
+// 4.8 and 6.1 s.)
 // The lists lie in buffers of the index build that are free by now: each cell's mask in ptkey,
 // the listed cells in ptcell (each once per step), large pairs in ptpos, n / 2 of them: the
-// blocks' from its start, which a warp searches itself where there is no room, the grid's from
-// its middle.  The latter's cells have more than 1,024 points on one side; there are at most
+// blocks' in its first 3 n / 8, the grid's behind them; a warp searches a pair itself where there
+// is no room.  The grid's cells have more than 1,024 points on one side; there are at most
 // n / 1025 of those, each in at most 124 pairs (62 in each half of the 3D stencil): below n / 8.
 constexpr long long kSmallWarpPairs = 1ll << 14, kSmallBlockPairs = 1ll << 20;
 __host__ __device__ constexpr int small_block_cap(int n) { return n / 2 - n / 8; }
@@ -686,7 +687,8 @@ k_small_expand(const __grid_constant__ gdl::Bufs B, const __grid_constant__ Smal
     }
     int cnt = own + add;
     const bool undecided = valid && cnt < minpts && cnt + open >= minpts;
-    const bool heavy = undecided && open > (F32 ? kSmallPointTests32 : kSmallPointTests);  // (the whole group)
+    // (the whole group)
+    const bool heavy = undecided && open > (F32 ? kSmallPointTests32 : kSmallPointTests);
     bool more = undecided && !heavy && w != 0;
     uint32_t q = 0, qe = 0;
     while (true) {
